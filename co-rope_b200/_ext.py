@@ -17,7 +17,7 @@ LIB_PATH = os.path.join(_HERE, "libcorope_b200.so")
 HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200.h")
 DEBUG_HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200_debug.h")
 
-SOURCES = ["abi.cu", "rope_general.cu", "rope_fwd_sm100.cu", "rope_bwd_sm100.cu", "corope_general.cu", "corope_fwd_mma.cu", "corope_bwd_mma.cu", "noalloc.cu",
+SOURCES = ["abi.cu", "rope_general.cu", "rope_prepass.cu", "rope_fwd_sm100.cu", "rope_bwd_sm100.cu", "corope_general.cu", "corope_fwd_mma.cu", "corope_bwd_mma.cu", "noalloc.cu",
            "debug.cu"]
 
 DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
@@ -85,6 +85,8 @@ def lib():
             L.corope_status_string.argtypes = [i32]
             L.corope_workspace_bytes.restype = sz
             L.corope_workspace_bytes.argtypes = [i32] * 7
+            L.corope_workspace_bytes_any_n.restype = sz
+            L.corope_workspace_bytes_any_n.argtypes = [i32] * 7
             L.corope_launch_count.restype = ctypes.c_uint64
             L.corope_launch_count.argtypes = []
             L.corope_set_kernel_policy.restype = i32
@@ -119,6 +121,10 @@ def lib():
             L.corope_rope_attn_fwd_freqs.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, sz, vp, vp]
             L.corope_rope_attn_bwd_freqs.restype = i32
             L.corope_rope_attn_bwd_freqs.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, sz, vp, vp]
+            L.corope_rope_attn_fwd_theta.restype = i32
+            L.corope_rope_attn_fwd_theta.argtypes = [vp, vp, vp, f32, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, sz, vp, vp, sp]
+            L.corope_rope_attn_bwd_theta.restype = i32
+            L.corope_rope_attn_bwd_theta.argtypes = [vp, vp, vp, vp, vp, vp, f32, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, vp, sz, vp, vp, sp]
             L.corope_flash_attn_fwd.restype = i32
             L.corope_flash_attn_fwd.argtypes = [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, vp, sz, vp, vp]
             L.corope_flash_attn_bwd.restype = i32
@@ -265,7 +271,7 @@ def check_status(device=None):
 
 
 def workspace(op, B, Hq, Hkv, N, D, dtype, device):
-    nbytes = lib().corope_workspace_bytes(op, B, Hq, Hkv, N, D, DTYPE_CODES[dtype])
+    nbytes = lib().corope_workspace_bytes_any_n(op, B, Hq, Hkv, N, D, DTYPE_CODES[dtype])
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device), int(nbytes)
 
 

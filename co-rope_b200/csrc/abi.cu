@@ -16,25 +16,24 @@ constexpr size_t kAlign = 256;
 bool head_dim_ok(int D) { return D == 32 || D == 64 || D == 128; }
 
 struct RopeWorkspace {
-    size_t packed_tab, synth_cos, synth_sin, rot, delta, dq_acc, pad[5], total;
+    size_t packed_tab, synth_cos, synth_sin, rot, delta, lse_pad, dq_acc, total;
+    bool tc;   // room for the tensor-core kernels
 };
 
-// 16-bit problems with D = 64 and N % 128 == 0 run zero-padded to D = 128 on the tensor-core kernels (half of the MMA work
-// is on zeros, which still is an order of magnitude faster than the CUDA-core kernels); the workspace then also holds the
-// padded copies.
-bool rope_d64_padded(int N, int D, int dtype) { return D == 64 && dtype != COROPE_DTYPE_F32 && N % 128 == 0; }
+// Rows per head of the backward's side inputs (LSE, delta): whole 128-row blocks, so that every tile's 64 values start on the
+// 16-byte boundary that bulk copies need.
+int side_pitch_for(int N) { return (N + 127) / 128 * 128; }
 
 // Hq query heads, Hkv K / V heads (equal for the fused-RoPE ops).  `synth`: room for fp32 cos / sin tables [N, D/2] that the
-// entry points taking frequencies instead of tables fill in.
-RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth) {
+// entry points taking frequencies instead of tables fill in.  `any_n`: room for the tensor-core kernels whatever N is, not only
+// for multiples of 128.
+RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth, bool any_n) {
     RopeWorkspace w{};
-    const bool padded = rope_d64_padded(N, D, dtype);
-    const int Dk = padded ? 128 : D;                 // head dimension the kernels see
-    const bool tc = dtype != COROPE_DTYPE_F32 && Dk == 128;
-    const size_t q_elems = (size_t)B * Hq * N * Dk, kv_elems = (size_t)B * Hkv * N * Dk;
+    w.tc = rope_tc_supported(D, dtype) && (any_n || N % 128 == 0);
+    const size_t q_elems = (size_t)B * Hq * N * D, kv_elems = (size_t)B * Hkv * N * D;
     size_t off = 0;
     w.packed_tab = off;
-    off += align_up((size_t)N * (Dk / 2) * sizeof(uint32_t) + 64, kAlign);   // + the work counter behind the table
+    off += align_up((size_t)N * (D / 2) * sizeof(uint32_t) + 64, kAlign);   // + the work counter behind the table
     if (synth) {
         w.synth_cos = off;
         off += align_up((size_t)N * (D / 2) * sizeof(float), kAlign);
@@ -42,25 +41,27 @@ RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int
         off += align_up((size_t)N * (D / 2) * sizeof(float), kAlign);
     }
     w.rot = off;   // tensor-core kernels: fp16 copy of the rotated K (forward) / rotated and scaled Q (backward)
-    if (tc) off += align_up((bwd ? q_elems : kv_elems) * 2, kAlign);
+    if (w.tc) off += align_up((bwd ? q_elems : kv_elems) * 2, kAlign);
     if (bwd) {
+        const size_t side = align_up((size_t)B * Hq * side_pitch_for(N) * sizeof(float), kAlign);
         w.delta = off;
-        off += align_up((size_t)B * Hq * N * sizeof(float), kAlign);
+        off += side;
+        w.lse_pad = off;
+        if (w.tc && N % 128 != 0) off += side;
         w.dq_acc = off;
-        if (tc) off += align_up(q_elems * sizeof(float), kAlign);
-    }
-    if (padded) {
-        // forward: q, v, o (k before its rotation shares o's buffer: needs the larger of the two); backward: k, v, dO / dq,
-        // dk (q before its rotation shares dk's buffer), dv
-        const size_t fwd_sizes[3] = {q_elems, kv_elems, q_elems};
-        const size_t bwd_sizes[5] = {kv_elems, kv_elems, q_elems, q_elems, kv_elems};
-        for (int i = 0; i < (bwd ? 5 : 3); ++i) {
-            w.pad[i] = off;
-            off += align_up((bwd ? bwd_sizes[i] : fwd_sizes[i]) * 2, kAlign);
-        }
+        if (w.tc) off += align_up(q_elems * sizeof(float), kAlign);
     }
     w.total = off < kAlign ? kAlign : off;
     return w;
+}
+
+// What corope_workspace_bytes answers for the fused-RoPE and plain ops.  16-bit D = 64 problems with N % 128 == 0 once ran
+// zero-padded to D = 128 and callers were told 16 (forward) / 32 (backward) bytes per element of q; that bound stays in force.
+size_t rope_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth) {
+    const size_t need = rope_workspace_layout(bwd, B, Hq, Hkv, N, D, dtype, synth, false).total;
+    if (D != 64 || dtype == COROPE_DTYPE_F32 || N % 128 != 0) return need;
+    const size_t told = align_up((size_t)B * Hq * N * D * (bwd ? 32 : 16), kAlign);
+    return need > told ? need : told;
 }
 
 struct GqaWorkspace {
@@ -187,15 +188,28 @@ const char* corope_status_string(int status) {
 size_t corope_workspace_bytes(int op, int B, int Hq, int Hkv, int N, int D, int dtype) {
     if (B <= 0 || Hq <= 0 || Hkv <= 0 || N <= 0 || D <= 0) return 0;
     switch (op) {
-        case COROPE_OP_ROPE_FWD: return rope_workspace_layout(false, B, Hq, Hq, N, D, dtype, false).total;
-        case COROPE_OP_ROPE_BWD: return rope_workspace_layout(true, B, Hq, Hq, N, D, dtype, false).total;
-        case COROPE_OP_ROPE_FWD_FREQS: return rope_workspace_layout(false, B, Hq, Hq, N, D, dtype, true).total;
-        case COROPE_OP_ROPE_BWD_FREQS: return rope_workspace_layout(true, B, Hq, Hq, N, D, dtype, true).total;
-        case COROPE_OP_FLASH_FWD: return Hq % Hkv ? 0 : rope_workspace_layout(false, B, Hq, Hkv, N, D, dtype, false).total;
-        case COROPE_OP_FLASH_BWD: return Hq % Hkv ? 0 : rope_workspace_layout(true, B, Hq, Hkv, N, D, dtype, false).total;
+        case COROPE_OP_ROPE_FWD: return rope_workspace_bytes(false, B, Hq, Hq, N, D, dtype, false);
+        case COROPE_OP_ROPE_BWD: return rope_workspace_bytes(true, B, Hq, Hq, N, D, dtype, false);
+        case COROPE_OP_ROPE_FWD_FREQS: return rope_workspace_bytes(false, B, Hq, Hq, N, D, dtype, true);
+        case COROPE_OP_ROPE_BWD_FREQS: return rope_workspace_bytes(true, B, Hq, Hq, N, D, dtype, true);
+        case COROPE_OP_FLASH_FWD: return Hq % Hkv ? 0 : rope_workspace_bytes(false, B, Hq, Hkv, N, D, dtype, false);
+        case COROPE_OP_FLASH_BWD: return Hq % Hkv ? 0 : rope_workspace_bytes(true, B, Hq, Hkv, N, D, dtype, false);
         case COROPE_OP_GQA_FWD: return gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype).total;
         case COROPE_OP_GQA_BWD: return gqa_workspace_layout(true, B, Hq, Hkv, N, D, dtype).total;
         default: return 0;
+    }
+}
+
+size_t corope_workspace_bytes_any_n(int op, int B, int Hq, int Hkv, int N, int D, int dtype) {
+    if (B <= 0 || Hq <= 0 || Hkv <= 0 || N <= 0 || D <= 0) return 0;
+    switch (op) {
+        case COROPE_OP_ROPE_FWD: return rope_workspace_layout(false, B, Hq, Hq, N, D, dtype, false, true).total;
+        case COROPE_OP_ROPE_BWD: return rope_workspace_layout(true, B, Hq, Hq, N, D, dtype, false, true).total;
+        case COROPE_OP_ROPE_FWD_FREQS: return rope_workspace_layout(false, B, Hq, Hq, N, D, dtype, true, true).total;
+        case COROPE_OP_ROPE_BWD_FREQS: return rope_workspace_layout(true, B, Hq, Hq, N, D, dtype, true, true).total;
+        case COROPE_OP_FLASH_FWD: return Hq % Hkv ? 0 : rope_workspace_layout(false, B, Hq, Hkv, N, D, dtype, false, true).total;
+        case COROPE_OP_FLASH_BWD: return Hq % Hkv ? 0 : rope_workspace_layout(true, B, Hq, Hkv, N, D, dtype, false, true).total;
+        default: return corope_workspace_bytes(op, B, Hq, Hkv, N, D, dtype);
     }
 }
 
@@ -209,13 +223,15 @@ int corope_last_kernel_family(int op) { return (op >= 0 && op < 4) ? g_last_fami
 
 namespace {
 
-// Where the rotation comes from: caller tables (cos / sin + row stride), per-pair frequencies (tables are synthesized into
-// the workspace first), or nothing at all (plain attention).
+// Where the rotation comes from: caller tables (cos / sin + row stride), per-pair frequencies (given, or those of a base theta),
+// or nothing at all (plain attention).
 struct Rotation {
     const float* cos = nullptr;
     const float* sin = nullptr;
     int64_t stride = 0;
     const float* inv_freq = nullptr;
+    float theta = 0.f;
+    bool freqs = false;   // tables are synthesized from inv_freq (or theta when it is null)
     bool none = false;
 };
 
@@ -261,25 +277,46 @@ bool strides_positive(const Strides& st, int D) { return st.n >= D && st.b >= 0 
 // ops whose kernel family is recorded: the fused-RoPE pair also stands for its variants
 constexpr int kFamFwd = COROPE_OP_ROPE_FWD, kFamBwd = COROPE_OP_ROPE_BWD;
 
+// The workspace layout a call runs with: the one with room for the tensor-core kernels at any N when the caller's workspace has
+// it (corope_workspace_bytes_any_n), else the one of corope_workspace_bytes.
+int pick_workspace(RopeWorkspace& w, bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth, const void* ws, size_t have) {
+    w = rope_workspace_layout(bwd, B, Hq, Hkv, N, D, dtype, synth, true);
+    if (have >= w.total) return check_workspace(ws, have, w.total);
+    w = rope_workspace_layout(bwd, B, Hq, Hkv, N, D, dtype, synth, false);
+    return check_workspace(ws, have, w.total);
+}
+
+// Tensor-core kernels: packed table in the workspace, or where the pre-pass gets it from.
+int table_source(TableSource& src, const Rotation& rot, uint32_t* tab, int N, int D, cudaStream_t s) {
+    if (rot.freqs) {
+        src.packed = true;
+        return launch_synth_packed(rot.inv_freq, rot.theta, tab, N, D / 2, s);
+    }
+    if (!rot.none) src.cos = rot.cos, src.sin = rot.sin, src.stride = rot.stride;
+    return COROPE_OK;
+}
+// General kernels: fp32 tables.
+int fp32_tables(RopeParams& p, const Rotation& rot, void* workspace, const RopeWorkspace& w, cudaStream_t s) {
+    p.cos = rot.none ? nullptr : rot.cos; p.sin = rot.none ? nullptr : rot.sin; p.table_stride = rot.stride;
+    if (!rot.freqs) return COROPE_OK;
+    float* c = reinterpret_cast<float*>((char*)workspace + w.synth_cos);
+    float* sn = reinterpret_cast<float*>((char*)workspace + w.synth_sin);
+    p.cos = c; p.sin = sn; p.table_stride = p.D / 2;
+    return launch_synth_tables(rot.inv_freq, rot.theta, c, sn, p.N, p.D / 2, s);
+}
+
 int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, void* o, float* lse2, int B, int Hq, int Hkv, int N, int D,
                   int dtype, int causal, float sm_scale, void* workspace, size_t workspace_bytes, int* status_word, void* stream,
                   const corope_strides_t* strides = nullptr) {
     if (!q || !k || !v || !o || !lse2) return COROPE_ERR_NULL_POINTER;
-    if (!rot.none && !rot.inv_freq && (!rot.cos || !rot.sin)) return COROPE_ERR_NULL_POINTER;
+    if (!rot.none && !rot.freqs && (!rot.cos || !rot.sin)) return COROPE_ERR_NULL_POINTER;
     if (int e = check_common(B, Hq, N, D, dtype)) return e;
     if (Hkv <= 0 || Hq % Hkv != 0) return COROPE_ERR_BAD_GROUP;
-    RopeWorkspace w = rope_workspace_layout(false, B, Hq, Hkv, N, D, dtype, rot.inv_freq != nullptr);
-    if (int e = check_workspace(workspace, workspace_bytes, w.total)) return e;
+    RopeWorkspace w;
+    if (int e = pick_workspace(w, false, B, Hq, Hkv, N, D, dtype, rot.freqs, workspace, workspace_bytes)) return e;
     cudaStream_t s = (cudaStream_t)stream;
-    if (rot.inv_freq) {
-        float* c = reinterpret_cast<float*>((char*)workspace + w.synth_cos);
-        float* sn = reinterpret_cast<float*>((char*)workspace + w.synth_sin);
-        if (int e = launch_synth_tables(rot.inv_freq, c, sn, N, D / 2, s)) return e;
-        rot.cos = c; rot.sin = sn; rot.stride = D / 2;
-    }
     RopeParams p{};
     p.q = q; p.k = k; p.v = v; p.out_o = o; p.lse2 = lse2;
-    p.cos = rot.none ? nullptr : rot.cos; p.sin = rot.none ? nullptr : rot.sin; p.table_stride = rot.stride;
     p.B = B; p.H = Hq; p.Hkv = Hkv; p.no_rope = rot.none ? 1 : 0;
     p.N = N; p.D = D; p.causal = causal ? 1 : 0; p.sm_scale = sm_scale; p.status = status_word;
     set_strides(p, strides, Hq, Hkv, N, D);
@@ -287,42 +324,25 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
     // rows are moved with TMA / 16-byte vectors on the tensor-core paths; otherwise the CUDA-core kernels take over
     const bool vec = vec_ok(q, p.sq) && vec_ok(k, p.sk) && vec_ok(v, p.sv) && vec_ok(o, p.so);
     const int policy = vec ? g_policy.load() : 1;
-    if (policy == 0 && rope_d64_padded(N, D, dtype)) {
-        // D = 64: zero-padded copies of q, k, v in the layout that keeps the rotation pairs together, the D = 128 kernels, o back
+    const bool whole = N % 128 == 0;
+    if (w.tc && policy != 1 && (policy == 0 || whole)) {
         uint32_t* tab = reinterpret_cast<uint32_t*>((char*)workspace + w.packed_tab);
-        void* k_rot = (char*)workspace + w.rot;
-        void* qp = (char*)workspace + w.pad[0];
-        void* vp = (char*)workspace + w.pad[1];
-        void* op = (char*)workspace + w.pad[2];   // first the padded k (until it is rotated), then the padded output
-        if (int e = launch_pack_tables(p.cos, p.sin, p.table_stride, tab, N, 64, s, 32)) return e;
-        const PadSpec in3[3] = {{q, qp, p.sq, Hq, 1}, {k, op, p.sk, Hkv, 1}, {v, vp, p.sv, Hkv, 0}};
-        if (int e = launch_pad_d64_many(3, in3, B, N, false, dtype, s)) return e;
-        if (int e = launch_rope_prerotate(op, contiguous_strides(Hkv, N, 128), k_rot, tab, B, Hkv, N, 1.0f, dtype, s)) return e;
-        const Strides so_caller = p.so;
-        p.q = qp; p.k = op; p.v = vp; p.out_o = op; p.D = 128;
-        set_strides(p, nullptr, Hq, Hkv, N, 128);   // the padded copies are contiguous
-        p.packed_tab = tab;
-        p.sched_counter = reinterpret_cast<int*>(tab + (size_t)N * 64);
-        p.k_rot = k_rot;
-        g_last_family[kFamFwd] = 1;
-        if (int e = launch_rope_fwd_tc(p, dtype, s)) return e;
-        return launch_unpad_d64(op, o, so_caller, B, Hq, N, 0, dtype, s);
-    }
-    if (policy != 1 && rope_fwd_tc_supported(B, Hq, N, D, dtype, causal)) {
-        uint32_t* tab = reinterpret_cast<uint32_t*>((char*)workspace + w.packed_tab);
-        if (int e = launch_pack_tables(p.cos, p.sin, p.table_stride, tab, N, D / 2, s)) return e;
+        TableSource src;
+        if (int e = table_source(src, rot, tab, N, D, s)) return e;
         p.packed_tab = tab;
         p.sched_counter = reinterpret_cast<int*>(tab + (size_t)N * (D / 2));
         // policy 2: every K tile is rotated in shared memory by the main kernel, nothing rotated is written to HBM (for plain
         // attention the "rotation" by the identity table is what brings K to fp16, the format Q is written in)
         if (policy == 0) {
-            void* k_rot = (char*)workspace + w.rot;
-            if (int e = launch_rope_prerotate(k, p.sk, k_rot, tab, B, Hkv, N, 1.0f, dtype, s)) return e;
-            p.k_rot = k_rot;
+            p.k_rot = (char*)workspace + w.rot;
+            if (int e = launch_rope_fwd_prepass(p, src, tab, dtype, s)) return e;
+        } else if (!src.packed) {
+            if (int e = launch_pack_tables(src, tab, N, D / 2, s)) return e;
         }
-        g_last_family[kFamFwd] = 1;
+        g_last_family[kFamFwd] = whole ? 1 : 0;
         return launch_rope_fwd_tc(p, dtype, s);
     }
+    if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
     g_last_family[kFamFwd] = 0;
     return launch_rope_fwd_general(p, dtype, s);
 }
@@ -331,23 +351,16 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
                   void* dk, void* dv, int B, int Hq, int Hkv, int N, int D, int dtype, int causal, float sm_scale, void* workspace,
                   size_t workspace_bytes, int* status_word, void* stream, const corope_strides_t* strides = nullptr) {
     if (!q || !k || !v || !o || !d_o || !lse2 || !dq || !dk || !dv) return COROPE_ERR_NULL_POINTER;
-    if (!rot.none && !rot.inv_freq && (!rot.cos || !rot.sin)) return COROPE_ERR_NULL_POINTER;
+    if (!rot.none && !rot.freqs && (!rot.cos || !rot.sin)) return COROPE_ERR_NULL_POINTER;
     if (int e = check_common(B, Hq, N, D, dtype)) return e;
     if (Hkv <= 0 || Hq % Hkv != 0) return COROPE_ERR_BAD_GROUP;
-    RopeWorkspace w = rope_workspace_layout(true, B, Hq, Hkv, N, D, dtype, rot.inv_freq != nullptr);
-    if (int e = check_workspace(workspace, workspace_bytes, w.total)) return e;
+    RopeWorkspace w;
+    if (int e = pick_workspace(w, true, B, Hq, Hkv, N, D, dtype, rot.freqs, workspace, workspace_bytes)) return e;
     cudaStream_t s = (cudaStream_t)stream;
-    if (rot.inv_freq) {
-        float* c = reinterpret_cast<float*>((char*)workspace + w.synth_cos);
-        float* sn = reinterpret_cast<float*>((char*)workspace + w.synth_sin);
-        if (int e = launch_synth_tables(rot.inv_freq, c, sn, N, D / 2, s)) return e;
-        rot.cos = c; rot.sin = sn; rot.stride = D / 2;
-    }
     RopeParams p{};
     p.q = q; p.k = k; p.v = v; p.o = o; p.d_o = d_o; p.dq = dq; p.dk = dk; p.dv = dv;
     p.lse2 = const_cast<float*>(lse2);
     p.delta = reinterpret_cast<float*>((char*)workspace + w.delta);
-    p.cos = rot.none ? nullptr : rot.cos; p.sin = rot.none ? nullptr : rot.sin; p.table_stride = rot.stride;
     p.B = B; p.H = Hq; p.Hkv = Hkv; p.no_rope = rot.none ? 1 : 0;
     p.N = N; p.D = D; p.causal = causal ? 1 : 0; p.sm_scale = sm_scale; p.status = status_word;
     set_strides(p, strides, Hq, Hkv, N, D);
@@ -356,47 +369,30 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
     const bool vec = vec_ok(q, p.sq) && vec_ok(k, p.sk) && vec_ok(v, p.sv) && vec_ok(o, p.so) && vec_ok(d_o, p.sdo) && vec_ok(dq, p.sdq) &&
                      vec_ok(dk, p.sdk) && vec_ok(dv, p.sdv);
     const int policy = vec ? g_policy.load() : 1;
-    const bool tc_direct = policy != 1 && !(policy == 0 && rope_d64_padded(N, D, dtype)) && rope_bwd_tc_supported(B, Hq, N, D, dtype, causal);
-    if (!(tc_direct && policy == 0))   // the tensor-core path at D = 128 computes delta in its fused pre-pass
-        if (int e = launch_rope_delta(p, dtype, s)) return e;
-    if (policy == 0 && rope_d64_padded(N, D, dtype)) {
+    const bool whole = N % 128 == 0;
+    if (w.tc && policy != 1 && (policy == 0 || whole)) {
         uint32_t* tab = reinterpret_cast<uint32_t*>((char*)workspace + w.packed_tab);
-        void* q_rot = (char*)workspace + w.rot;
-        void* kp = (char*)workspace + w.pad[0];
-        void* vp = (char*)workspace + w.pad[1];
-        void* dop = (char*)workspace + w.pad[2];   // padded dO; after the main kernel the padded dq (the finalize kernel writes it)
-        void* dkp = (char*)workspace + w.pad[3];   // first the padded q (until it is rotated), then the padded dk
-        void* dvp = (char*)workspace + w.pad[4];
-        if (int e = launch_pack_tables(p.cos, p.sin, p.table_stride, tab, N, 64, s, 32)) return e;
-        const PadSpec in4[4] = {{q, dkp, p.sq, Hq, 1}, {k, kp, p.sk, Hkv, 1}, {v, vp, p.sv, Hkv, 0}, {d_o, dop, p.sdo, Hq, 0}};
-        if (int e = launch_pad_d64_many(4, in4, B, N, false, dtype, s)) return e;
-        if (int e = launch_rope_prerotate(dkp, contiguous_strides(Hq, N, 128), q_rot, tab, B, Hq, N, sm_scale * kLog2e, dtype, s)) return e;
-        const Strides sdq_caller = p.sdq, sdk_caller = p.sdk, sdv_caller = p.sdv;
-        p.q = dkp; p.k = kp; p.v = vp; p.d_o = dop; p.dq = dop; p.dk = dkp; p.dv = dvp; p.D = 128;
-        set_strides(p, nullptr, Hq, Hkv, N, 128);   // the padded copies are contiguous
+        TableSource src;
+        if (int e = table_source(src, rot, tab, N, D, s)) return e;
         p.packed_tab = tab;
-        p.sched_counter = reinterpret_cast<int*>(tab + (size_t)N * 64);   // zeroed by the table pack
+        p.sched_counter = reinterpret_cast<int*>(tab + (size_t)N * (D / 2));   // zeroed with the table
         p.dq_acc = reinterpret_cast<float*>((char*)workspace + w.dq_acc);
-        p.q_rot = q_rot;
-        g_last_family[kFamBwd] = 1;
-        if (int e = launch_rope_bwd_tc(p, dtype, s)) return e;
-        const PadSpec out3[3] = {{dq, dop, sdq_caller, Hq, 1}, {dk, dkp, sdk_caller, Hkv, 1}, {dv, dvp, sdv_caller, Hkv, 0}};
-        return launch_pad_d64_many(3, out3, B, N, true, dtype, s);
-    }
-    if (tc_direct) {
-        uint32_t* tab = reinterpret_cast<uint32_t*>((char*)workspace + w.packed_tab);
-        if (int e = launch_pack_tables(p.cos, p.sin, p.table_stride, tab, N, D / 2, s)) return e;
-        p.packed_tab = tab;
-        p.sched_counter = reinterpret_cast<int*>(tab + (size_t)N * (D / 2));   // zeroed by the table pack
-        p.dq_acc = reinterpret_cast<float*>((char*)workspace + w.dq_acc);
-        if (policy == 0) {   // policy 2: every Q tile is rotated in shared memory by the main kernel, nothing rotated is written to HBM
+        p.side_pitch = side_pitch_for(N);
+        p.lse_pad = whole ? lse2 : reinterpret_cast<const float*>((char*)workspace + w.lse_pad);
+        if (policy == 0) {
             p.q_rot = (char*)workspace + w.rot;
-            if (int e = launch_rope_bwd_prepass(p, dtype, s)) return e;   // delta, rotated Q, cleared dQ accumulator
+            if (int e = launch_rope_bwd_prepass(p, src, tab, dtype, s)) return e;   // table, delta, rotated Q, cleared dQ accumulator
             p.dq_acc_zeroed = 1;
+        } else {   // policy 2: every Q tile is rotated in shared memory by the main kernel, nothing rotated is written to HBM
+            if (int e = launch_rope_delta(p, dtype, s)) return e;
+            if (!src.packed)
+                if (int e = launch_pack_tables(src, tab, N, D / 2, s)) return e;
         }
-        g_last_family[kFamBwd] = 1;
+        g_last_family[kFamBwd] = whole ? 1 : 0;
         return launch_rope_bwd_tc(p, dtype, s);
     }
+    if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
+    if (int e = launch_rope_delta(p, dtype, s)) return e;
     g_last_family[kFamBwd] = 0;
     return launch_rope_bwd_general(p, dtype, s);
 }
@@ -409,6 +405,13 @@ Rotation from_tables(const float* cos, const float* sin, int64_t stride) {
 Rotation from_freqs(const float* inv_freq) {
     Rotation r;
     r.inv_freq = inv_freq;
+    r.freqs = true;
+    return r;
+}
+Rotation from_theta(float theta) {
+    Rotation r;
+    r.theta = theta;
+    r.freqs = true;
     return r;
 }
 Rotation no_rotation() {
@@ -479,6 +482,20 @@ int corope_rope_attn_bwd_freqs(const void* q, const void* k, const void* v, cons
     if (!inv_freq) return COROPE_ERR_NULL_POINTER;
     return rope_bwd_impl(q, k, v, o, d_o, lse2, from_freqs(inv_freq), dq, dk, dv, B, H, H, N, D, dtype, causal, sm_scale, workspace,
                          workspace_bytes, status_word, stream);
+}
+
+int corope_rope_attn_fwd_theta(const void* q, const void* k, const void* v, float theta, void* o, float* lse2, int B, int H, int N, int D,
+                               int dtype, int causal, float sm_scale, void* workspace, size_t workspace_bytes, int* status_word, void* stream,
+                               const corope_strides_t* strides) {
+    return rope_fwd_impl(q, k, v, from_theta(theta), o, lse2, B, H, H, N, D, dtype, causal, sm_scale, workspace, workspace_bytes, status_word,
+                         stream, strides);
+}
+
+int corope_rope_attn_bwd_theta(const void* q, const void* k, const void* v, const void* o, const void* d_o, const float* lse2, float theta,
+                               void* dq, void* dk, void* dv, int B, int H, int N, int D, int dtype, int causal, float sm_scale,
+                               void* workspace, size_t workspace_bytes, int* status_word, void* stream, const corope_strides_t* strides) {
+    return rope_bwd_impl(q, k, v, o, d_o, lse2, from_theta(theta), dq, dk, dv, B, H, H, N, D, dtype, causal, sm_scale, workspace,
+                         workspace_bytes, status_word, stream, strides);
 }
 
 int corope_flash_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse2, int B, int Hq, int Hkv, int N, int D, int dtype,

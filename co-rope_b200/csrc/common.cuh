@@ -94,6 +94,8 @@ struct RopeParams {
     const float* cos;
     const float* sin;
     int64_t table_stride;
+    const float* lse_pad;   // tensor-core backward: LSE with row pitch `side_pitch` (the caller's lse2, or a padded copy for ragged N)
+    int side_pitch;         // rows per head of lse_pad and delta in the tensor-core backward: N, or N rounded up to 128
     const uint32_t* packed_tab;  // [N, D/2] (cos, sin) pairs in 16-bit fixed point, built per call in the workspace
     int B, H, N, D;     // H = number of query heads
     int Hkv;            // number of K / V heads (H % Hkv == 0; query head h reads KV head h / (H / Hkv)); equals H for the fused-RoPE ops
@@ -252,6 +254,11 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y, const void* smem_src) {
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
                  "r"(smem_u32(smem_src)), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, int x, int y, int z, const void* smem_src) {
+    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
+                 "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -484,24 +491,31 @@ template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b
 template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) { return pack_bf162(a, b); }
 template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) { return pack_half2(a, b); }
 
-// In-place half-layout rotation of a ROWS x 128 tile held as two 128-byte-swizzled ROWS x 64 boxes
-// (columns [0,64) and [64,128)).  Element (r, c) of a box sits at r*128 + ((c/8) ^ (r%8))*16 + (c%8)*2, so the
-// pair (d, d+64) has the same offset in the two boxes.  8 consecutive threads cover one 128-byte row; 128 threads.
+// In-place half-layout rotation of ROWS rows of a tile held as 128-byte-swizzled boxes of 64 columns; 128 threads, 8 pairs
+// (d, d + D/2) per thread and step.  Element (r, c) of a box sits at r*128 + ((c/8) ^ (r%8))*16 + (c%8)*2.
+//   D = 128: two boxes, columns [0,64) and [64,128); a pair has the same offset in both; 8 threads per row.
+//   D = 64 : one box; the partner of 16-byte chunk u < 4 is chunk u + 4 of the same row, i.e. its swizzled position ^ 4; 4
+//            threads per row (two-way bank conflicts, on tiles that are rotated once per work item).
 // The result is written as fp16 whatever the input type T.  The packed (cos, sin) rows of the tile (16-bit fixed
 // point, see unpack_unorm_pair) are fetched into registers by load_table_regs, which does not depend on the tile
 // having landed: callers issue it before waiting for the TMA so that the L2 latency is hidden.
-template <int ROWS>
+template <int ROWS, int D>
 struct TabRegs {
-    uint4 t[ROWS / 16 * 2];
+    static constexpr int kRowsPerStep = 128 / (D / 16);
+    static constexpr int kSteps = ROWS / kRowsPerStep;
+    uint4 t[kSteps * 2];
 };
 
-template <int ROWS>
-__device__ __forceinline__ void load_table_regs(TabRegs<ROWS>& tr, const uint32_t* __restrict__ tab, int tid) {
+// Table rows row0 .. row0 + ROWS - 1; rows beyond the table (a tile that reaches past the head) repeat its last one.
+template <int ROWS, int D>
+__device__ __forceinline__ void load_table_regs(TabRegs<ROWS, D>& tr, const uint32_t* __restrict__ tab, int row0, int n_rows, int tid) {
+    constexpr int kThreadsPerRow = D / 16;
 #pragma unroll
-    for (int it = 0; it < ROWS / 16; ++it) {
-        const int row = it * 16 + (tid >> 3);
-        const int c = (tid & 7) ^ (row & 7);
-        const uint4* tp = reinterpret_cast<const uint4*>(tab + row * 64 + c * 8);
+    for (int it = 0; it < TabRegs<ROWS, D>::kSteps; ++it) {
+        const int row = it * TabRegs<ROWS, D>::kRowsPerStep + tid / kThreadsPerRow;
+        const int u = tid % kThreadsPerRow;
+        const int c = D == 128 ? u ^ (row & 7) : u;
+        const uint4* tp = reinterpret_cast<const uint4*>(tab + (size_t)min(row0 + row, n_rows - 1) * (D / 2) + c * 8);
         tr.t[2 * it] = __ldg(tp);
         tr.t[2 * it + 1] = __ldg(tp + 1);
     }
@@ -529,54 +543,61 @@ __device__ __forceinline__ void rotate_vec8(uint4& x1, uint4& x2, const uint4& t
     x2 = make_uint4(b[0], b[1], b[2], b[3]);
 }
 
-template <typename T, int ROWS, int BOX_BYTES = ROWS * 128, int BATCH = 4>
-__device__ __forceinline__ void rotate_tile_regs(uint8_t* tile, const TabRegs<ROWS>& tr, int tid, float scale) {
-    constexpr int kBoxBytes = BOX_BYTES;   // distance between the [0,64) and [64,128) column boxes (ROWS may be part of a taller tile)
-    constexpr int kIters = ROWS / 16;
-    constexpr int kBatch = BATCH;                                    // rows in flight per thread: loads first, then math, then stores
+template <typename T, int ROWS, int D, int BOX_BYTES, int BATCH>
+__device__ __forceinline__ void rotate_tile_regs(uint8_t* tile, const TabRegs<ROWS, D>& tr, int tid, float scale) {
+    constexpr int kSteps = TabRegs<ROWS, D>::kSteps;
+    constexpr int kStepBytes = TabRegs<ROWS, D>::kRowsPerStep * 128;
+    constexpr int kBatch = BATCH < kSteps ? BATCH : kSteps;          // rows in flight per thread: loads first, then math, then stores
     const float k1 = scale * (1.f / 32768.f), k0 = -257.f * scale;   // decode constants with the scale folded in
-    uint8_t* base = tile + (tid >> 3) * 128 + (tid & 7) * 16;
+    const int row = tid / (D / 16), u = tid % (D / 16);              // (row & 7) is the same in every step
+    uint8_t* p1 = tile + row * 128 + (D == 128 ? u : u ^ (row & 7)) * 16;
+    uint8_t* p2 = D == 128 ? p1 + BOX_BYTES : tile + row * 128 + (u ^ (row & 7) ^ 4) * 16;
 #pragma unroll
-    for (int h = 0; h < kIters; h += kBatch) {
+    for (int h = 0; h < kSteps; h += kBatch) {
         uint4 x1[kBatch], x2[kBatch];
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            x1[u] = *reinterpret_cast<const uint4*>(base + (h + u) * 2048);
-            x2[u] = *reinterpret_cast<const uint4*>(base + kBoxBytes + (h + u) * 2048);
+        for (int v = 0; v < kBatch; ++v) {
+            x1[v] = *reinterpret_cast<const uint4*>(p1 + (h + v) * kStepBytes);
+            x2[v] = *reinterpret_cast<const uint4*>(p2 + (h + v) * kStepBytes);
         }
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            rotate_vec8<T>(x1[u], x2[u], tr.t[2 * (h + u)], tr.t[2 * (h + u) + 1], k1, k0);
+        for (int v = 0; v < kBatch; ++v) {
+            rotate_vec8<T>(x1[v], x2[v], tr.t[2 * (h + v)], tr.t[2 * (h + v) + 1], k1, k0);
         }
 #pragma unroll
-        for (int u = 0; u < kBatch; ++u) {
-            *reinterpret_cast<uint4*>(base + (h + u) * 2048) = x1[u];
-            *reinterpret_cast<uint4*>(base + kBoxBytes + (h + u) * 2048) = x2[u];
+        for (int v = 0; v < kBatch; ++v) {
+            *reinterpret_cast<uint4*>(p1 + (h + v) * kStepBytes) = x1[v];
+            *reinterpret_cast<uint4*>(p2 + (h + v) * kStepBytes) = x2[v];
         }
     }
 }
 
 #endif  // __CUDACC__
 
-// Same for a 2-D row-major fp32 tensor without swizzle (box_cols * 4 bytes a multiple of 16, box_cols <= 256): used for
-// bulk reduce-add stores of dense shared-memory tiles.
-inline int encode_tensor_map_2d_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                 CUtensorMapFloatOOBfill);
-    static EncodeFn fn = nullptr;
-    if (!fn) {
+// cuTensorMapEncodeTiled through the runtime's driver entry point (no link-time libcuda dependency); null when unavailable.
+typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                      const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                      CUtensorMapFloatOOBfill);
+inline TensorMapEncodeFn tensor_map_encoder() {
+    static const TensorMapEncodeFn fn = [] {
         void* sym = nullptr;
         cudaDriverEntryPointQueryResult qres;
-        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres);
-        if (e != cudaSuccess || qres != cudaDriverEntryPointSuccess || !sym) return COROPE_ERR_NO_DEVICE;
-        fn = (EncodeFn)sym;
-    }
-    cuuint64_t gdim[2] = {cols, rows};
-    cuuint64_t gstride[1] = {cols * 4};
-    cuuint32_t box[2] = {box_cols, box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        const cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres);
+        return e == cudaSuccess && qres == cudaDriverEntryPointSuccess ? (TensorMapEncodeFn)sym : nullptr;
+    }();
+    return fn;
+}
+
+// A row-major fp32 tensor [rows, cols] (slices == 0) or [slices, rows, cols] without swizzle (box_cols * 4 bytes a multiple of 16,
+// box_cols <= 256): bulk reduce-add of dense shared-memory tiles; rows of a box beyond `rows` are clipped.
+inline int encode_tensor_map_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t slices, uint32_t box_rows, uint32_t box_cols) {
+    const TensorMapEncodeFn fn = tensor_map_encoder();
+    if (!fn) return COROPE_ERR_NO_DEVICE;
+    cuuint64_t gdim[3] = {cols, rows, slices};
+    cuuint64_t gstride[2] = {cols * 4, rows * cols * 4};
+    cuuint32_t box[3] = {box_cols, box_rows, 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, slices ? 3 : 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : COROPE_ERR_TENSOR_MAP;
 }
@@ -593,29 +614,28 @@ int kernel_policy();
 int launch_rope_fwd_general(const RopeParams& p, int dtype, cudaStream_t s);
 int launch_rope_bwd_general(const RopeParams& p, int dtype, cudaStream_t s);
 int launch_rope_delta(const RopeParams& p, int dtype, cudaStream_t s);
-// tensor-core backward, D = 128, 16-bit: delta, the rotated fp16 copy of Q (scaled by sm_scale * log2e) into p.q_rot and a
-// zeroed p.dq_acc in one launch; sets nothing in p
-int launch_rope_bwd_prepass(const RopeParams& p, int dtype, cudaStream_t s);
-// cos == nullptr packs the identity rotation (plain attention)
-int launch_pack_tables(const float* cos, const float* sin, int64_t stride, uint32_t* packed, int N, int half_d, cudaStream_t s, int half_src = -1);
-// cos / sin tables [N, half_d] fp32 for positions 0 .. N-1 from per-pair frequencies: angle = float(n) * inv_freq[d]
-int launch_synth_tables(const float* inv_freq, float* cos_out, float* sin_out, int N, int half_d, cudaStream_t s);
-// x / out: [B, H, N, 64] with strides st (the padded side is contiguous [B*H*N, 128])
-int launch_unpad_d64(const void* xp, void* out, const Strides& st, int B, int H, int N, int rope_layout, int dtype, cudaStream_t s);
-// one tensor of a batched pad / un-pad launch: the caller's [B, H, N, 64] tensor with its strides and its padded copy
-struct PadSpec {
-    const void* tensor;   // written by an un-pad
-    void* padded;
-    Strides strides;
-    int H;
-    int rope_layout;
+// What the tensor-core kernels need before they run (rope_prepass.cu).
+// Where the (cos, sin) pairs of a position come from.
+struct TableSource {
+    const float* cos = nullptr;      // fp32 tables with row stride `stride`; null (and no packed table) = identity rotation
+    const float* sin = nullptr;
+    int64_t stride = 0;
+    bool packed = false;             // the packed table has already been written (launch_synth_packed)
 };
-int launch_pad_d64_many(int n, const PadSpec* specs, int B, int N, bool unpad, int dtype, cudaStream_t s);
-int launch_rope_prerotate(const void* x, const Strides& st, void* out_f16, const uint32_t* packed, int B, int H, int N, float scale,
-                          int dtype, cudaStream_t s);   // H = heads of x; out is contiguous [B*H*N, 128]
-bool rope_fwd_tc_supported(int B, int H, int N, int D, int dtype, int causal);
+// packed [N, half_d] table alone, + the zeroed work counter behind it
+int launch_pack_tables(const TableSource& src, uint32_t* packed, int N, int half_d, cudaStream_t s);
+// cos / sin tables [N, half_d] fp32 for positions 0 .. N-1: angle = float(n) * inv_freq[d], inv_freq from the array or, when it
+// is null, 1 / theta^(2 d / (2 half_d))
+int launch_synth_tables(const float* inv_freq, float theta, float* cos_out, float* sin_out, int N, int half_d, cudaStream_t s);
+// the same straight into the packed table, + the zeroed work counter
+int launch_synth_packed(const float* inv_freq, float theta, uint32_t* packed, int N, int half_d, cudaStream_t s);
+// forward: packed table (unless src.packed) and the rotated fp16 copy of K into p.k_rot
+int launch_rope_fwd_prepass(const RopeParams& p, const TableSource& src, uint32_t* packed, int dtype, cudaStream_t s);
+// backward: packed table (unless src.packed), delta, the rotated fp16 copy of Q (scaled by sm_scale * log2e) into p.q_rot, a zeroed
+// p.dq_acc and, for ragged N, the padded LSE copy into p.lse_pad
+int launch_rope_bwd_prepass(const RopeParams& p, const TableSource& src, uint32_t* packed, int dtype, cudaStream_t s);
+bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types, D = 64 or 128
 int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
-bool rope_bwd_tc_supported(int B, int H, int N, int D, int dtype, int causal);
 int launch_rope_bwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 bool gqa_fwd_mma_supported(int N, int D, int dtype);
 int launch_gqa_bwd_mma(const GqaParams& p, int dtype, cudaStream_t s);
@@ -623,22 +643,12 @@ int launch_gqa_fwd_mma(const GqaParams& p, int dtype, cudaStream_t s);
 int launch_gqa_fwd_general(const GqaParams& p, int dtype, cudaStream_t s);
 int launch_gqa_bwd_general(const GqaParams& p, int dtype, cudaStream_t s);
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link-time libcuda dependency).
 // Encodes a 2-D row-major [rows, cols] tensor of 16-bit elements with a [box_rows, box_cols] box and
 // 128-byte swizzle (box_cols * 2 bytes must be 128).  Returns 0 on success.
 inline int encode_tensor_map_2d_sw128(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows,
                                       uint32_t box_cols, int dtype, uint64_t row_stride_elems = 0) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                 CUtensorMapFloatOOBfill);
-    static EncodeFn fn = nullptr;
-    if (!fn) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres);
-        if (e != cudaSuccess || qres != cudaDriverEntryPointSuccess || !sym) return COROPE_ERR_NO_DEVICE;
-        fn = (EncodeFn)sym;
-    }
+    const TensorMapEncodeFn fn = tensor_map_encoder();
+    if (!fn) return COROPE_ERR_NO_DEVICE;
     cuuint64_t gdim[2] = {cols, rows};
     cuuint64_t gstride[1] = {(row_stride_elems ? row_stride_elems : cols) * 2};
     cuuint32_t box[2] = {box_cols, box_rows};
@@ -653,17 +663,8 @@ inline int encode_tensor_map_2d_sw128(CUtensorMap* out, const void* base, uint64
 // a 4-D map with dimensions (D, N, H, B) and a [box_rows, box_cols] box inside one head.  Rows beyond N read as zeros.
 inline int encode_tensor_map_4d_sw128(CUtensorMap* out, const void* base, uint64_t B, uint64_t H, uint64_t N, uint64_t D, const Strides& st,
                                       uint32_t box_rows, uint32_t box_cols, int dtype) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                 CUtensorMapFloatOOBfill);
-    static EncodeFn fn = nullptr;
-    if (!fn) {
-        void* sym = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &sym, cudaEnableDefault, &qres);
-        if (e != cudaSuccess || qres != cudaDriverEntryPointSuccess || !sym) return COROPE_ERR_NO_DEVICE;
-        fn = (EncodeFn)sym;
-    }
+    const TensorMapEncodeFn fn = tensor_map_encoder();
+    if (!fn) return COROPE_ERR_NO_DEVICE;
     cuuint64_t gdim[4] = {D, N, H, B};
     // a dimension of extent 1 is never stepped over, but its stride still has to be a valid one
     cuuint64_t gstride[3] = {(cuuint64_t)st.n * 2, (cuuint64_t)(H > 1 ? st.h : st.n * (int64_t)N) * 2, (cuuint64_t)(B > 1 ? st.b : st.n * (int64_t)N) * 2};
@@ -675,10 +676,11 @@ inline int encode_tensor_map_4d_sw128(CUtensorMap* out, const void* base, uint64
     return r == CUDA_SUCCESS ? 0 : COROPE_ERR_TENSOR_MAP;
 }
 
-// 2-D map when the rows collapse, else 4-D; `flat` tells the kernel which coordinates to use
+// 2-D map when the rows collapse, else 4-D; `flat` tells the kernel which coordinates to use.  A ragged N (last tile of a head
+// only partly filled) always takes the 4-D form, whose rows beyond N read as zeros instead of the next head's rows.
 inline int encode_rows_map(CUtensorMap* out, bool* flat, const void* base, int B, int H, int N, int D, const Strides& st, uint32_t box_rows,
                            uint32_t box_cols, int dtype) {
-    *flat = rows_collapse(st, H, N);
+    *flat = rows_collapse(st, H, N) && N % 128 == 0;
     if (*flat) return encode_tensor_map_2d_sw128(out, base, (uint64_t)B * H * N, D, box_rows, box_cols, dtype, (uint64_t)st.n);
     return encode_tensor_map_4d_sw128(out, base, B, H, N, D, st, box_rows, box_cols, dtype);
 }

@@ -32,5 +32,5 @@ extern "C" int corope_debug_expire_wait(int* status_word, unsigned max_polls, vo
 
 extern "C" int corope_debug_synth_tables(const float* inv_freq, float* cos_out, float* sin_out, int N, int half_d, void* stream) {
     if (!inv_freq || !cos_out || !sin_out || N <= 0 || half_d <= 0) return COROPE_ERR_NULL_POINTER;
-    return corope::launch_synth_tables(inv_freq, cos_out, sin_out, N, half_d, (cudaStream_t)stream);
+    return corope::launch_synth_tables(inv_freq, 0.f, cos_out, sin_out, N, half_d, (cudaStream_t)stream);
 }

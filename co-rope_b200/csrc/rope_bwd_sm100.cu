@@ -1,6 +1,6 @@
 // Fused-RoPE flash-attention backward (causal or full) for sm_100a: TMA -> shared memory -> in-place rotation of K
 // (once) and of every Q tile -> five tcgen05 MMAs per (K block, Q tile) pair with TMEM accumulators.
-// 16-bit inputs, D = 128, N % 128 == 0.
+// 16-bit inputs, D = 64 or 128, any N.
 //
 // Work unit = one K/V block of 128 keys of one (batch, head): the CTA sweeps the query tiles (64 rows each) at or
 // below the block's diagonal.  CTAs are persistent (one per SM) and take units from a global counter, the first unit
@@ -34,17 +34,13 @@
 namespace corope {
 namespace {
 
-constexpr int kD = 128;
 constexpr int kBK = 128;                 // keys per CTA
 constexpr int kBQ = 64;                  // query rows per step
 constexpr int kStages = 3;               // Q / dO ring.  With 2 stages the sweep is latency-bound on this ring (1.56 ms against 1.08 ms
                                          // with 3); a 4th stage gave nothing, so its 32 KiB stage the dQ~ tile for the bulk reduce instead
-constexpr int kKVBytes = kBK * kD * 2;   // 32 KiB
-constexpr int kKVBox = kKVBytes / 2;
-constexpr int kQBytes = kBQ * kD * 2;    // 16 KiB
-constexpr int kQBox = kQBytes / 2;
+constexpr int kKVBox = kBK * 64 * 2;     // 16 KiB: a K / V block is one (D = 64) or two (D = 128) boxes of 64 columns
+constexpr int kQBox = kBQ * 64 * 2;      // 8 KiB: the same for a Q / dO tile
 constexpr int kDsBytes = kBK * kBQ * 2;  // 16 KiB
-constexpr int kDqBytes = kBQ * kD * 4;   // 32 KiB: dQ~ tile [64 queries][128] fp32, dense, staged for the bulk reduce-add
 constexpr int kThreads = 768;             // six warpgroups: control (TMA, MMA, 2 spare) | rotation (2) | softmax A | softmax B | dQ drain
 constexpr int kMmaWarp = 1;
 constexpr int kRotWarp0 = 4, kSmxWarp0 = 12, kDrainWarp0 = 20;
@@ -103,20 +99,22 @@ __device__ __forceinline__ int fetch_unit(uint64_t* bars, volatile int* unit_rin
     return w;
 }
 
-constexpr size_t kSmemData = 2 * kKVBytes + kStages * 2 * kQBytes + 2 * kDsBytes + kDqBytes + kStages * 2 * kBQ * sizeof(float);
+// K, V | Q ring, dO ring | dS^T x 2 | dQ~ tile [64 queries][D] fp32, dense, staged for the bulk reduce-add | LSE, delta ring
+constexpr size_t smem_data(int D) { return 2 * kBK * D * 2 + kStages * 2 * kBQ * D * 2 + 2 * kDsBytes + kBQ * D * 4 + kStages * 2 * kBQ * sizeof(float); }
 constexpr size_t kSmemSlack = 512;       // room to round the dynamic shared memory base up to 1024 bytes (checked at run time)
-constexpr size_t kSmemBytes = kSmemData + NUM_BARS * 8 + 64 + kSmemSlack;
-static_assert(kSmemBytes <= 232448, "shared memory budget");
+constexpr size_t smem_bytes(int D) { return smem_data(D) + NUM_BARS * 8 + 64 + kSmemSlack; }
+static_assert(smem_bytes(128) <= 232448, "shared memory budget");
 
 constexpr uint32_t TS0 = 0, TD0 = 128, TDV = 256, TDK = 384;
 
 // kPlain: one query head per K / V head and every tensor's rows evenly spaced (all contiguous MHA calls): the group and
 // layout arithmetic folds away at compile time (it measured 1 - 2 % of the kernel when left to run-time flags).
-template <typename T, bool kPlain>
+template <typename T, bool kPlain, int kD>
 __global__ void __launch_bounds__(kThreads, 1)
 rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapDO,
                       const __grid_constant__ CUtensorMap mapDQ, RopeParams p) {
+    constexpr int kKVBytes = kBK * kD * 2, kQBytes = kBQ * kD * 2, kDqBytes = kBQ * kD * 4;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* sK = sm;
@@ -136,16 +134,19 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int G = kPlain ? 1 : p.H / p.Hkv;   // query heads per K / V head (1 for the fused-RoPE ops)
     const bool flat_q = kPlain || p.flat_q, flat_do = kPlain || p.flat_do, flat_k = kPlain || p.flat_k, flat_v = kPlain || p.flat_v;
     const int BH = p.B * p.Hkv;           // units are taken per K / V head; a unit sweeps the query tiles of all G heads of its group
-    const int n_kb = N / kBK;
+    const int n_kb = (N + kBK - 1) / kBK;
     const int n_units = BH * n_kb;
     const bool causal = p.causal != 0;
     // per unit (jb, bh): first query row visited q_first = causal ? jb * kBK : 0 (causal: the block's own diagonal),
-    // spg = (N - q_first) / kBQ steps per query head (even) and n_steps = G * spg, so the two-buffer indices of a unit's
-    // first step are always 0.  Step s works on query head bh * G + s / spg, rows q_first + (s % spg) * kBQ .. + kBQ - 1.
+    // spg = (n_pad - q_first) / kBQ steps per query head (even, so n_steps >= 2) and n_steps = G * spg.  For N not a multiple of
+    // 128 the last block of keys and the last steps reach past the head: Q, dO, K and V rows there read as zeros (4-D maps), the
+    // LSE copy holds +inf for them (P = 0, so such a query adds nothing), and a key at or beyond N has P = 0 by the causal mask
+    // for every query inside the head, by an explicit mask otherwise.  Step s works on query head bh * G + s / spg, rows q_first + (s % spg) * kBQ .. + kBQ - 1.
     // (no division when every K / V head has a single query head: then s < spg)
     auto step_head = [&](int spg, int s) { return G == 1 ? 0 : s / spg; };
     auto step_q0 = [&](int q_first, int spg, int s) { return q_first + (G == 1 ? s : s % spg) * kBQ; };
     auto step_row = [&](int bh, int q_first, int spg, int s) { return (bh * G + step_head(spg, s)) * N + step_q0(q_first, spg, s); };
+    const int n_pad = n_kb * kBK;         // N rounded up to whole blocks (= N for kPlain)
 
     if (reinterpret_cast<uintptr_t>(sm) - reinterpret_cast<uintptr_t>(smem_raw) > kSmemSlack) {   // base less aligned than assumed
         if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, COROPE_DEV_WAIT_EXPIRED | 0xfff);
@@ -211,34 +212,35 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 if (w < 0) break;
                 const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
                 const int q_first = causal ? un.jb * kBK : 0;
-                const int spg = (N - q_first) / kBQ, n_steps = G * spg;
+                const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
                 auto load_step = [&](int s) -> bool {
                     const int gs = g + s, st = gs % kStages;
                     if (gs >= kStages && !mbar_wait(&bars[QDO_EMPTY + st], ((gs / kStages) - 1) & 1, p.status, QDO_EMPTY, abort_flag)) return false;
-                    const int qr = step_row(un.bh, q_first, spg, s);   // flat row of the contiguous side inputs (LSE, delta)
+                    const int qr = step_row(un.bh, q_first, spg, s);   // flat row of Q, dO
+                    const int sr = kPlain ? qr : (un.bh * G + step_head(spg, s)) * p.side_pitch + step_q0(q_first, spg, s);   // of the side inputs (LSE, delta)
                     mbar_arrive_expect_tx(&bars[QDO_FULL + st], 2 * kQBytes + 2 * kBQ * (uint32_t)sizeof(float));
                     if (flat_q) {
                         tma_load_2d(sQ + st * kQBytes, &mapQ, 0, qr, &bars[QDO_FULL + st]);
-                        tma_load_2d(sQ + st * kQBytes + kQBox, &mapQ, 64, qr, &bars[QDO_FULL + st]);
+                        if (kD == 128) tma_load_2d(sQ + st * kQBytes + kQBox, &mapQ, 64, qr, &bars[QDO_FULL + st]);
                     }
                     if (flat_do) {
                         tma_load_2d(sDO + st * kQBytes, &mapDO, 0, qr, &bars[QDO_FULL + st]);
-                        tma_load_2d(sDO + st * kQBytes + kQBox, &mapDO, 64, qr, &bars[QDO_FULL + st]);
+                        if (kD == 128) tma_load_2d(sDO + st * kQBytes + kQBox, &mapDO, 64, qr, &bars[QDO_FULL + st]);
                     }
                     if (!flat_q || !flat_do) {   // 4-D maps: (row, head, batch) coordinates
                         const int qhead = un.bh * G + step_head(spg, s), q0 = step_q0(q_first, spg, s);
                         const int qb = qhead / p.H, qh = qhead % p.H;
                         if (!flat_q) {
                             tma_load_4d(sQ + st * kQBytes, &mapQ, 0, q0, qh, qb, &bars[QDO_FULL + st]);
-                            tma_load_4d(sQ + st * kQBytes + kQBox, &mapQ, 64, q0, qh, qb, &bars[QDO_FULL + st]);
+                            if (kD == 128) tma_load_4d(sQ + st * kQBytes + kQBox, &mapQ, 64, q0, qh, qb, &bars[QDO_FULL + st]);
                         }
                         if (!flat_do) {
                             tma_load_4d(sDO + st * kQBytes, &mapDO, 0, q0, qh, qb, &bars[QDO_FULL + st]);
-                            tma_load_4d(sDO + st * kQBytes + kQBox, &mapDO, 64, q0, qh, qb, &bars[QDO_FULL + st]);
+                            if (kD == 128) tma_load_4d(sDO + st * kQBytes + kQBox, &mapDO, 64, q0, qh, qb, &bars[QDO_FULL + st]);
                         }
                     }
-                    bulk_load_1d(sLD + st * 2 * kBQ, p.lse2 + qr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
-                    bulk_load_1d(sLD + st * 2 * kBQ + kBQ, p.delta + qr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
+                    bulk_load_1d(sLD + st * 2 * kBQ, p.lse_pad + sr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
+                    bulk_load_1d(sLD + st * 2 * kBQ + kBQ, p.delta + sr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
                     return true;
                 };
                 // the first two Q / dO tiles only need ring stages, which the last steps of the previous unit free: ask
@@ -249,10 +251,10 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 const int kr = un.jb * kBK, kb = un.bh / p.Hkv, kh = un.bh % p.Hkv;
                 mbar_arrive_expect_tx(&bars[K_FULL], kKVBytes);
                 tma_load_rows(sK, &mapK, flat_k, 0, kr, kh, kb, p.Hkv, N, &bars[K_FULL]);
-                tma_load_rows(sK + kKVBox, &mapK, flat_k, 64, kr, kh, kb, p.Hkv, N, &bars[K_FULL]);
+                if (kD == 128) tma_load_rows(sK + kKVBox, &mapK, flat_k, 64, kr, kh, kb, p.Hkv, N, &bars[K_FULL]);
                 mbar_arrive_expect_tx(&bars[V_FULL], kKVBytes);
                 tma_load_rows(sV, &mapV, flat_v, 0, kr, kh, kb, p.Hkv, N, &bars[V_FULL]);
-                tma_load_rows(sV + kKVBox, &mapV, flat_v, 64, kr, kh, kb, p.Hkv, N, &bars[V_FULL]);
+                if (kD == 128) tma_load_rows(sV + kKVBox, &mapV, flat_v, 64, kr, kh, kb, p.Hkv, N, &bars[V_FULL]);
                 for (int s = 2; ok && s < n_steps; ++s) ok = load_step(s);
                 g += n_steps;
             }
@@ -268,7 +270,9 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             const uint32_t id_dp = make_idesc(kTFmt, kTFmt, 0, 0, kBK, kBQ);     // dP^T: T x T, both K-major
             const uint32_t id_dv = make_idesc(kTFmt, kTFmt, 0, 1, kBK, kD);      // dV  : P^T (TMEM) x dO (MN-major)
             const uint32_t id_dk = make_idesc(0, 0, 0, 1, kBK, kD);              // dK~ : dS^T (K-major) x Q~ (MN-major)
-            const uint32_t id_dq = make_idesc(0, 0, 1, 1, kD, kBQ);              // dQ~^T: K~ (MN-major) x dS^T (MN-major)
+            // dQ~^T: K~ (MN-major) x dS^T (MN-major).  M = 128 = head dim; at D = 64 the upper 64 rows of A are whatever lies behind the
+            // K block (the V block) and the upper 64 lanes of the result are not read: an M = 64 MMA would take as long
+            const uint32_t id_dq = make_idesc(0, 0, 1, 1, 128, kBQ);
             constexpr uint32_t kHi = sdesc_hi(1024);
             // The buffers follow one another in shared memory (K | V | Q ring | dO ring | dS^T x 2) and the address field of
             // a descriptor (address >> 4, 14 bits) cannot wrap below 256 KiB, so every descriptor is the one of K plus a
@@ -317,7 +321,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 const int w = fetch_unit(bars, unit_ring, n, lane, p.status, abort_flag);
                 if (w < 0) break;
                 const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
-                const int n_steps = G * ((N - (causal ? un.jb * kBK : 0)) / kBQ);
+                const int n_steps = G * ((n_pad - (causal ? un.jb * kBK : 0)) / kBQ);
                 {
                     const int st0 = g % kStages, b0 = g & 1;
                     ok = mbar_wait_warp(&bars[K_ROT], n & 1, p.status, K_ROT, abort_flag) && mbar_wait_warp(&bars[V_FULL], n & 1, p.status, V_FULL, abort_flag) &&
@@ -377,25 +381,25 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (w < 0) break;
             const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
             const int q_first = causal ? un.jb * kBK : 0;
-            const int spg = (N - q_first) / kBQ, n_steps = G * spg;
+            const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
             {
-                TabRegs<kBQ> trk;
-                load_table_regs<kBQ>(trk, p.packed_tab + (size_t)(un.jb * kBK + rg * kBQ) * (kD / 2), tid);
+                TabRegs<kBQ, kD> trk;
+                load_table_regs(trk, p.packed_tab, un.jb * kBK + rg * kBQ, N, tid);
                 if (!(ok = mbar_wait_warp(&bars[K_FULL], n & 1, p.status, K_FULL, abort_flag))) break;
-                rotate_tile_regs<T, kBQ, kKVBox, 2>(sK + rg * kBQ * 128, trk, tid, 1.0f);
+                rotate_tile_regs<T, kBQ, kD, kKVBox, 2>(sK + rg * kBQ * 128, trk, tid, 1.0f);
                 fence_proxy_async();
                 mbar_arrive_warp(&bars[K_ROT], lane);
             }
             if (q_pre) continue;
-            TabRegs<kQHalf> tr;
-            load_table_regs<kQHalf>(tr, p.packed_tab + (size_t)(q_first + rg * kQHalf) * (kD / 2), tid);
+            TabRegs<kQHalf, kD> tr;
+            load_table_regs(tr, p.packed_tab, q_first + rg * kQHalf, N, tid);
             for (int s = 0; s < n_steps; ++s) {
                 const int gs = g + s, st = gs % kStages;
                 if (!(ok = mbar_wait_warp(&bars[QDO_FULL + st], (gs / kStages) & 1, p.status, QDO_FULL, abort_flag))) break;
-                rotate_tile_regs<T, kQHalf, kQBox, 2>(sQ + st * kQBytes + rg * kQHalf * 128, tr, tid, p.sm_scale * kLog2e);
+                rotate_tile_regs<T, kQHalf, kD, kQBox, 2>(sQ + st * kQBytes + rg * kQHalf * 128, tr, tid, p.sm_scale * kLog2e);
                 fence_proxy_async();
                 mbar_arrive_warp(&bars[Q_ROT + st], lane);
-                if (s + 1 < n_steps) load_table_regs<kQHalf>(tr, p.packed_tab + (size_t)(step_q0(q_first, spg, s + 1) + rg * kQHalf) * (kD / 2), tid);
+                if (s + 1 < n_steps) load_table_regs(tr, p.packed_tab, step_q0(q_first, spg, s + 1) + rg * kQHalf, N, tid);
             }
             g += n_steps;
         }
@@ -414,8 +418,9 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
         const int jb = un.jb;
         const int q_first = causal ? jb * kBK : 0;
-        const int spg = (N - q_first) / kBQ, n_steps = G * spg;
+        const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
         const int key = jb * kBK + row;
+        const bool key_out = !kPlain && key >= N;   // beyond the head: masked (full attention), not stored
         for (int s = 0; s < n_steps; ++s) {
             const int gs = g + s, u = gs >> 1, st = gs % kStages, b = gs & 1;
             const uint32_t tS = tmem + lane_base + TS0 + b * 64;
@@ -443,8 +448,8 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                     const float2 d2 = *reinterpret_cast<const float2*>(dlt + c0);
                     float p0 = fast_exp2(__uint_as_float(rs[2 * i]) - l2.x);
                     float p1 = fast_exp2(__uint_as_float(rs[2 * i + 1]) - l2.y);
-                    if (diag && key > q0 + c0) p0 = 0.f;
-                    if (diag && key > q0 + c0 + 1) p1 = 0.f;
+                    if ((diag && key > q0 + c0) || key_out) p0 = 0.f;
+                    if ((diag && key > q0 + c0 + 1) || key_out) p1 = 0.f;
                     const float s0 = p0 * (__uint_as_float(rd[2 * i]) - d2.x);
                     const float s1 = p1 * (__uint_as_float(rd[2 * i + 1]) - d2.y);
                     pp[i] = pack2<T>(p0, p1);
@@ -470,7 +475,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (wg == 0) {
                 T* dst = reinterpret_cast<T*>(p.dv) + (kPlain ? ((int64_t)un.bh * N + key) * p.sdv.n : row_offset(p.sdv, p.Hkv, un.bh, key));
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {
+                for (int c = 0; c < kD / 32; ++c) {
                     uint32_t r[32];
                     COROPE_TMEM_LD32(tmem + lane_base + TDV + c * 32, r);
                     tmem_wait_ld();
@@ -478,17 +483,19 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
 #pragma unroll
                     for (int i = 0; i < 16; ++i) pk[i] = pack2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
                     uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
+                    if (!key_out) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) d4[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+                        for (int i = 0; i < 4; ++i) d4[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+                    }
                 }
             } else {
                 T* dst = reinterpret_cast<T*>(p.dk) + (kPlain ? ((int64_t)un.bh * N + key) * p.sdk.n : row_offset(p.sdk, p.Hkv, un.bh, key));
-                const uint32_t* tab = p.packed_tab + (size_t)key * (kD / 2);
+                const uint32_t* tab = p.packed_tab + (size_t)(kPlain ? key : min(key, N - 1)) * (kD / 2);
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                for (int c = 0; c < kD / 64; ++c) {
                     uint32_t r1[32], r2[32];
                     COROPE_TMEM_LD32(tmem + lane_base + TDK + c * 32, r1);
-                    COROPE_TMEM_LD32(tmem + lane_base + TDK + 64 + c * 32, r2);
+                    COROPE_TMEM_LD32(tmem + lane_base + TDK + kD / 2 + c * 32, r2);
                     tmem_wait_ld();
                     uint32_t o1[16], o2[16];
 #pragma unroll
@@ -501,11 +508,13 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                         o2[i] = pack2<T>((b0 * cs0.x - a0 * cs0.y) * kLn2, (b1 * cs1.x - a1 * cs1.y) * kLn2);
                     }
                     uint4* d1 = reinterpret_cast<uint4*>(dst + c * 32);
-                    uint4* d2 = reinterpret_cast<uint4*>(dst + 64 + c * 32);
+                    uint4* d2 = reinterpret_cast<uint4*>(dst + kD / 2 + c * 32);
+                    if (!key_out) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        d1[i] = make_uint4(o1[4 * i], o1[4 * i + 1], o1[4 * i + 2], o1[4 * i + 3]);
-                        d2[i] = make_uint4(o2[4 * i], o2[4 * i + 1], o2[4 * i + 2], o2[4 * i + 3]);
+                        for (int i = 0; i < 4; ++i) {
+                            d1[i] = make_uint4(o1[4 * i], o1[4 * i + 1], o1[4 * i + 2], o1[4 * i + 3]);
+                            d2[i] = make_uint4(o2[4 * i], o2[4 * i + 1], o2[4 * i + 2], o2[4 * i + 3]);
+                        }
                     }
                 }
             }
@@ -529,7 +538,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (w < 0) break;
         const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
         const int q_first = causal ? un.jb * kBK : 0;
-        const int spg = (N - q_first) / kBQ, n_steps = G * spg;
+        const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
         for (int s = 0; s < n_steps; ++s) {
             const int gs = g + s, b = gs & 1;
             if (!(ok = mbar_wait_warp(&bars[DQ_DONE + b], (gs >> 1) & 1, p.status, DQ_DONE + b, abort_flag))) break;
@@ -546,14 +555,18 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (threadIdx.x == kDrainWarp0 * 32) bulk_wait_group_read0();   // the previous reduce has finished reading the tile
             named_bar_sync(1, 128);
             float* tile = sDQ + dcol;
+            if (kD == 128 || dcol < kD) {   // D = 64: the upper two warps hold the unused half of the MMA's rows
 #pragma unroll
-            for (int i = 0; i < 32; ++i) tile[i * kD] = __uint_as_float(r0[i]);
+                for (int i = 0; i < 32; ++i) tile[i * kD] = __uint_as_float(r0[i]);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) tile[(32 + i) * kD] = __uint_as_float(r1[i]);
+                for (int i = 0; i < 32; ++i) tile[(32 + i) * kD] = __uint_as_float(r1[i]);
+            }
             fence_proxy_async();
             named_bar_sync(1, 128);
             if (threadIdx.x == kDrainWarp0 * 32) {
-                tma_reduce_add_2d(&mapDQ, 0, step_row(un.bh, q_first, spg, s), sDQ);
+                const int q0 = step_q0(q_first, spg, s);
+                if (kPlain) tma_reduce_add_2d(&mapDQ, 0, step_row(un.bh, q_first, spg, s), sDQ);
+                else if (q0 < N) tma_reduce_add_3d(&mapDQ, 0, q0, un.bh * G + step_head(spg, s), sDQ);   // rows beyond the head are clipped
                 bulk_commit_group();
             }
         }
@@ -568,20 +581,20 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     }
 }
 
-// dQ = inverse_rotate(dQ~ accumulator) * sm_scale; one thread per (row, 4 consecutive d < 64): 16-byte loads of the
-// accumulator halves and of the packed (cos, sin) table the main kernel used (the caller's own tables may be narrower than
-// 64 columns when a D = 64 problem runs zero-padded; the packed table then holds the identity in columns 32..63), 8-byte stores
-template <typename T>
+// dQ = inverse_rotate(dQ~ accumulator) * sm_scale; one thread per (row, 4 consecutive d < D/2): 16-byte loads of the
+// accumulator halves and of the packed (cos, sin) table the main kernel used, 8-byte stores
+template <typename T, int kD>
 __global__ void rope_bwd_dq_finalize_kernel(const float* __restrict__ acc, T* __restrict__ dq, const uint32_t* __restrict__ packed,
                                             size_t rows, int N, float scale, Strides sdq, int H, int flat) {
+    constexpr int kHalf = kD / 2, kPerRow = kD / 8;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= rows * 16) return;
-    const size_t row = idx >> 4;
-    const int d = (int)(idx & 15) * 4;
+    if (idx >= rows * kPerRow) return;
+    const size_t row = idx / kPerRow;
+    const int d = (int)(idx % kPerRow) * 4;
     const int pos = (int)((unsigned)row % (unsigned)N);
     const float4 a1 = *reinterpret_cast<const float4*>(acc + row * kD + d);
-    const float4 a2 = *reinterpret_cast<const float4*>(acc + row * kD + d + 64);
-    const uint4 t4 = __ldg(reinterpret_cast<const uint4*>(packed + (size_t)pos * (kD / 2) + d));
+    const float4 a2 = *reinterpret_cast<const float4*>(acc + row * kD + d + kHalf);
+    const uint4 t4 = __ldg(reinterpret_cast<const uint4*>(packed + (size_t)pos * kHalf + d));
     const float2 cs[4] = {unpack_unorm_pair(t4.x), unpack_unorm_pair(t4.y), unpack_unorm_pair(t4.z), unpack_unorm_pair(t4.w)};
     const float x1[4] = {a1.x, a1.y, a1.z, a1.w}, x2[4] = {a2.x, a2.y, a2.z, a2.w};
     uint2 o1, o2;
@@ -591,10 +604,10 @@ __global__ void rope_bwd_dq_finalize_kernel(const float* __restrict__ acc, T* __
     o2.y = pack2<T>((x2[2] * cs[2].x - x1[2] * cs[2].y) * scale, (x2[3] * cs[3].x - x1[3] * cs[3].y) * scale);
     T* out = dq + (flat ? (int64_t)row * sdq.n : row_offset(sdq, H, (int)((unsigned)row / (unsigned)N), pos));
     *reinterpret_cast<uint2*>(out + d) = o1;
-    *reinterpret_cast<uint2*>(out + d + 64) = o2;
+    *reinterpret_cast<uint2*>(out + d + kHalf) = o2;
 }
 
-template <typename T>
+template <typename T, int kD>
 int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     CUtensorMap mq, mk, mv, mdo, mdq;
     const uint64_t rows = (uint64_t)p.B * p.H * p.N;
@@ -610,38 +623,34 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     if (int e = encode_rows_map(&mv, &fv, p.v, p.B, p.Hkv, p.N, kD, p.sv, kBK, 64, dtype)) return e;
     pp.flat_q = fq; pp.flat_do = fdo; pp.flat_k = fk; pp.flat_v = fv;
     pp.head_chunk = head_chunk_for(p.N);
-    if (int e = encode_tensor_map_2d_f32(&mdq, p.dq_acc, rows, kD, kBQ, kD)) return e;
     cudaError_t e = p.dq_acc_zeroed ? cudaSuccess : cudaMemsetAsync(p.dq_acc, 0, rows * kD * sizeof(float), s);
     if (e != cudaSuccess) return (int)e;
     const bool plain = p.H == p.Hkv && fq && fdo && fk && fv && rows_collapse(p.sdk, p.Hkv, p.N) && rows_collapse(p.sdv, p.Hkv, p.N);
-    auto kern = plain ? rope_bwd_sm100_kernel<T, true> : rope_bwd_sm100_kernel<T, false>;
+    // the dQ accumulator as rows of all heads, or (3-D) head by head so that a last, partly filled tile ends with its head
+    if (int er = encode_tensor_map_f32(&mdq, p.dq_acc, plain ? rows : (uint64_t)p.N, kD, plain ? 0 : (uint64_t)p.B * p.H, kBQ, kD)) return er;
+    auto kern = plain ? rope_bwd_sm100_kernel<T, true, kD> : rope_bwd_sm100_kernel<T, false, kD>;
+    constexpr size_t kSmemBytes = smem_bytes(kD);
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     int dev = 0, sms = 0;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-    const unsigned units = (unsigned)((p.N / kBK) * p.B * p.Hkv);
+    const unsigned units = (unsigned)(((p.N + kBK - 1) / kBK) * p.B * p.Hkv);
     const unsigned grid = units < (unsigned)sms ? units : (unsigned)sms;   // persistent: one CTA per SM
     kern<<<grid, kThreads, kSmemBytes, s>>>(mq, mk, mv, mdo, mdq, pp); count_launch();
     e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
-    const size_t n = rows * 16;
-    rope_bwd_dq_finalize_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p.dq_acc, reinterpret_cast<T*>(p.dq), p.packed_tab, rows, p.N,
-                                                                              p.sm_scale, p.sdq, p.H, rows_collapse(p.sdq, p.H, p.N) ? 1 : 0); count_launch();
+    const size_t n = rows * (kD / 8);
+    rope_bwd_dq_finalize_kernel<T, kD><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p.dq_acc, reinterpret_cast<T*>(p.dq), p.packed_tab, rows, p.N,
+                                                                                  p.sm_scale, p.sdq, p.H, rows_collapse(p.sdq, p.H, p.N) ? 1 : 0); count_launch();
     return (int)cudaGetLastError();
 }
 
 }  // namespace
 
-bool rope_bwd_tc_supported(int B, int H, int N, int D, int dtype, int causal) {
-    (void)B; (void)H;
-    (void)causal;
-    return D == kD && (dtype == COROPE_DTYPE_BF16 || dtype == COROPE_DTYPE_F16) && N % kBK == 0;
-}
-
 int launch_rope_bwd_tc(const RopeParams& p, int dtype, cudaStream_t s) {
-    if (dtype == COROPE_DTYPE_BF16) return launch_t<__nv_bfloat16>(p, dtype, s);
-    return launch_t<__half>(p, dtype, s);
+    if (dtype == COROPE_DTYPE_BF16) return p.D == 64 ? launch_t<__nv_bfloat16, 64>(p, dtype, s) : launch_t<__nv_bfloat16, 128>(p, dtype, s);
+    return p.D == 64 ? launch_t<__half, 64>(p, dtype, s) : launch_t<__half, 128>(p, dtype, s);
 }
 
 }  // namespace corope

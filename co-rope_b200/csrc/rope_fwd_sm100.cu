@@ -1,5 +1,5 @@
 // Fused-RoPE flash-attention forward (causal or full) for sm_100a: TMA -> shared memory -> in-place rotation ->
-// tcgen05 MMAs with TMEM accumulators -> online softmax in registers.  16-bit inputs, D = 128.
+// tcgen05 MMAs with TMEM accumulators -> online softmax in registers.  16-bit inputs, D = 64 or 128, any N.
 //
 // A work item is 256 consecutive query rows (two 128-row tiles, "Q0" and "Q1") of one (batch, head) with the K/V
 // tiles 0 .. 2t+1 they can see.  CTAs are persistent (one per SM) and take items from a global counter, heaviest
@@ -11,13 +11,13 @@
 //                 per item) and of every K tile as it lands, in place in shared memory, as fp16
 //   warps 12-19   two softmax groups of Q0, each taking 64 of the 128 key columns: thread = row; half an S row from
 //                 TMEM into registers, half-row max exchanged with the partner group, exp2, row sum, P written back
-//                 over S in TMEM, lazy rescale of its 64 O columns in TMEM, final normalise + store
+//                 over S in TMEM, lazy rescale of its half of the O columns in TMEM, final normalise + store
 //   warps 20-27   the same for Q1
 // TMEM columns: S0 [0,128) S1 [128,256) O0 [256,384) O1 [384,512); P_i (16-bit) is written over S_i: keys 0-63 in
 // columns 0-31, keys 64-127 in columns 64-95 (each softmax group writes only over columns it has already read).
 // MMA order per K tile j:  PV0(j) QK0(j+1) | PV1(j) QK1(j+1)  so that one group's softmax overlaps the
 // other group's MMAs.
-// K tiles come in one of two ways.  By default a pre-pass (rope_prerotate_d128_kernel) has written a rotated fp16 copy
+// K tiles come in one of two ways.  By default a pre-pass (rope_fwd_prepass_kernel) has written a rotated fp16 copy
 // of K to the workspace and the K ring loads that copy: every K tile is consumed by up to N/256 work items, and rotating
 // it in shared memory for each of them cost 14 % of the kernel (issue slots and shared-memory port time that the softmax
 // and the MMA operand fetch need), more than the copy's extra HBM traffic.  With p.k_rot == nullptr (kernel policy 2 of
@@ -31,13 +31,11 @@
 namespace corope {
 namespace {
 
-constexpr int kD = 128;
 constexpr int kBM = 128;
 constexpr int kBN = 128;
 constexpr int kKStages = 3;
 constexpr int kVStages = 2;
-constexpr int kTileBytes = kBM * kD * 2;   // 32 KiB: two 128 x 64 boxes
-constexpr int kBoxBytes = kTileBytes / 2;
+constexpr int kBoxBytes = kBM * 64 * 2;    // 16 KiB: a tile of 128 rows is one (D = 64) or two (D = 128) boxes of 64 columns
 constexpr int kThreads = 896;          // seven warpgroups: control (TMA K, TMA V, MMA, spare) | rotation (2) | softmax of Q0 (2) | of Q1 (2)
 constexpr int kMmaWarp = 2;
 constexpr int kRotWarp0 = 4;
@@ -71,11 +69,10 @@ enum Bar {
     NUM_BARS = ITEM_EMPTY + kItemSlots
 };
 
-constexpr size_t kSmemTiles = (size_t)(2 + kKStages + kVStages) * kTileBytes;
 constexpr size_t kXchBytes = 2 * 2 * kBM * sizeof(float);         // half-row maxima / sums exchanged between the two groups of a Q tile
 constexpr size_t kSmemSlack = 512;     // room to round the dynamic shared memory base up to 1024 bytes (checked at run time)
-constexpr size_t kSmemBytes = kSmemTiles + kXchBytes + NUM_BARS * 8 + 64 + kSmemSlack;
-static_assert(kSmemBytes <= 232448, "shared memory budget");  // + alignment slack (tmem slot, abort flag and the item ring live in the 64)
+constexpr size_t smem_bytes(int D) { return (size_t)(2 + kKStages + kVStages) * kBM * D * 2 + kXchBytes + NUM_BARS * 8 + 64 + kSmemSlack; }
+static_assert(smem_bytes(128) <= 232448, "shared memory budget");  // + alignment slack (tmem slot, abort flag and the item ring live in the 64)
 
 // Work items (one = 256 query rows of one head) in the order CTAs take them: heads in chunks of kHeadChunk so that
 // the items in flight at one time share few heads (their K/V stay in L2), heaviest query blocks first inside a chunk.
@@ -118,7 +115,7 @@ __device__ __forceinline__ int fetch_item(uint64_t* bars, volatile int* item_rin
 
 // kPlain: one query head per K / V head and every tensor's rows evenly spaced (all contiguous MHA calls): the group and
 // layout arithmetic folds away at compile time (it measured 1 - 2 % of the kernel when left to run-time flags).
-template <typename T, bool kPlain>
+template <typename T, bool kPlain, int kD>
 __global__ void __launch_bounds__(kThreads, 1)
 rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                       const __grid_constant__ CUtensorMap mapV, RopeParams p) {
@@ -126,6 +123,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // one format).  For bf16 the row sums are taken from the rounded P, which keeps the normalised weights consistent:
     // measured max-abs error of O at the Llama-7B-4K shape is unchanged (0.0080, rounding of the bf16 output itself 0.0077).
     constexpr bool kPBf16 = Elem<T>::kDtype == COROPE_DTYPE_BF16;
+    constexpr int kTileBytes = kBM * kD * 2;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* sQ = sm;
@@ -142,14 +140,15 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int BH = p.B * p.H;
     const int G = kPlain ? 1 : p.H / p.Hkv;   // query heads per K / V head (1 for the fused-RoPE ops); query head bh reads KV head bh / G
     const bool flat_q = kPlain || p.flat_q, flat_k = kPlain || p.flat_k, flat_v = kPlain || p.flat_v;
-    // N is a multiple of 128: when it is not a multiple of 256 the last item of a head has only Q0; its Q1 tile (and, causal,
-    // the K tile behind the diagonal) lies beyond the head -- TMA fetches the next head's rows there (2-D maps) or zeros (4-D
-    // maps and behind the tensor); the results are finite and are not stored
+    // When N is not a multiple of 256 the last item of a head reaches past it: its Q1 tile (and, causal, the K tile behind the
+    // diagonal) may lie beyond the head, and for N not a multiple of 128 its last tile is partly filled.  TMA fetches the next
+    // head's rows there (2-D maps, whole tiles only) or zeros (4-D maps and behind the tensor); rows at or beyond N are not
+    // stored, and keys at or beyond N are masked: by the causal mask for every row that is stored, explicitly otherwise.
     const int n_qt = (N + 2 * kBM - 1) / (2 * kBM);
     const int n_items = n_qt * BH;
     // K tiles an item sees: up to its diagonal (causal: Q0 one tile less than Q1), or all of them
     const bool causal = p.causal != 0;
-    const int nk_all = N / kBN;   // full attention: every tile that lies inside the head
+    const int nk_all = (N + kBN - 1) / kBN;   // full attention: every tile that starts inside the head
     // Persistent CTAs with a dynamic schedule: the first item of CTA c is c, further ones come from a global counter
     // (heavy items first, so the greedy order balances to a few percent; a static round-robin was 19 % off).  The K
     // producer fetches an item, publishes it in a small shared-memory ring and every other role reads it from there.
@@ -228,7 +227,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                         const int r = wi.t * 2 * kBM + i * kBM;   // rows at or beyond N (a head's last, half-empty item) read as zeros
                         mbar_arrive_expect_tx(&bars[Q_FULL + i], kTileBytes);
                         tma_load_rows(sQ + i * kTileBytes, &mapQ, flat_q, 0, r, qh, qb, p.H, N, &bars[Q_FULL + i]);
-                        tma_load_rows(sQ + i * kTileBytes + kBoxBytes, &mapQ, flat_q, 64, r, qh, qb, p.H, N, &bars[Q_FULL + i]);
+                        if (kD == 128) tma_load_rows(sQ + i * kTileBytes + kBoxBytes, &mapQ, flat_q, 64, r, qh, qb, p.H, N, &bars[Q_FULL + i]);
                     }
                     for (int j = 0; ok && j < nk; ++j, ++gk) {
                         const int r = j * kBN;
@@ -236,7 +235,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                         if (gk >= kKStages && !(ok = mbar_wait(&bars[K_EMPTY + ks], ((gk / kKStages) - 1) & 1, p.status, K_EMPTY, abort_flag))) break;
                         mbar_arrive_expect_tx(&bars[K_FULL + ks], kTileBytes);
                         tma_load_rows(sK + ks * kTileBytes, &mapK, flat_k, 0, r, kh, kb, p.Hkv, N, &bars[K_FULL + ks]);
-                        tma_load_rows(sK + ks * kTileBytes + kBoxBytes, &mapK, flat_k, 64, r, kh, kb, p.Hkv, N, &bars[K_FULL + ks]);
+                        if (kD == 128) tma_load_rows(sK + ks * kTileBytes + kBoxBytes, &mapK, flat_k, 64, r, kh, kb, p.Hkv, N, &bars[K_FULL + ks]);
                     }
                 }
             }
@@ -258,7 +257,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                         if (gv >= kVStages && !(ok = mbar_wait(&bars[V_EMPTY + vs], ((gv / kVStages) - 1) & 1, p.status, V_EMPTY, abort_flag))) break;
                         mbar_arrive_expect_tx(&bars[V_FULL + vs], kTileBytes);
                         tma_load_rows(sV + vs * kTileBytes, &mapV, flat_v, 0, r, kh, kb, p.Hkv, N, &bars[V_FULL + vs]);
-                        tma_load_rows(sV + vs * kTileBytes + kBoxBytes, &mapV, flat_v, 64, r, kh, kb, p.Hkv, N, &bars[V_FULL + vs]);
+                        if (kD == 128) tma_load_rows(sV + vs * kTileBytes + kBoxBytes, &mapV, flat_v, 64, r, kh, kb, p.Hkv, N, &bars[V_FULL + vs]);
                     }
                 }
             }
@@ -357,7 +356,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const int tid = (threadIdx.x - kRotWarp0 * 32) & 127;
         constexpr int kHalfRows = kBM / 2;
         bool ok = true;
-        TabRegs<kHalfRows> tr;
+        TabRegs<kHalfRows, kD> tr;
         int gk = 0;
         for (int n = 0; ok; ++n) {
             const int w = fetch_item(bars, item_ring, n, lane, true, p.status, abort_flag);
@@ -365,23 +364,23 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             const WorkItem wi = work_item(w, n_qt, BH, p.head_chunk);
             const int nk = causal ? 2 * wi.t + 2 : nk_all;
             for (int i = 0; i < 2 && ok; ++i) {
-                load_table_regs<kHalfRows>(tr, p.packed_tab + (size_t)(wi.t * 2 * kBM + i * kBM + rg * kHalfRows) * (kD / 2), tid);
+                load_table_regs(tr, p.packed_tab, wi.t * 2 * kBM + i * kBM + rg * kHalfRows, N, tid);
                 if (!(ok = mbar_wait_warp(&bars[Q_FULL + i], n & 1, p.status, Q_FULL, abort_flag))) break;
-                rotate_tile_regs<T, kHalfRows, kBoxBytes, 1>(sQ + i * kTileBytes + rg * kHalfRows * 128, tr, tid, p.sm_scale * kLog2e);
+                rotate_tile_regs<T, kHalfRows, kD, kBoxBytes, 1>(sQ + i * kTileBytes + rg * kHalfRows * 128, tr, tid, p.sm_scale * kLog2e);
                 fence_proxy_async();
                 mbar_arrive_warp(&bars[Q_ROT + i], lane);
             }
             if (!ok) break;
             // K tiles: only when no pre-pass has rotated them; otherwise the MMA warp takes them straight from the TMA barriers
             if (p.k_rot != nullptr) continue;
-            load_table_regs<kHalfRows>(tr, p.packed_tab + (size_t)(rg * kHalfRows) * (kD / 2), tid);
+            load_table_regs(tr, p.packed_tab, rg * kHalfRows, N, tid);
             for (int j = 0; j < nk; ++j, ++gk) {
                 const int ks = gk % kKStages;
                 if (!(ok = mbar_wait_warp(&bars[K_FULL + ks], (gk / kKStages) & 1, p.status, K_FULL, abort_flag))) break;
-                rotate_tile_regs<T, kHalfRows, kBoxBytes, 1>(sK + ks * kTileBytes + rg * kHalfRows * 128, tr, tid, 1.0f);
+                rotate_tile_regs<T, kHalfRows, kD, kBoxBytes, 1>(sK + ks * kTileBytes + rg * kHalfRows * 128, tr, tid, 1.0f);
                 fence_proxy_async();
                 mbar_arrive_warp(&bars[K_ROT + ks], lane);
-                if (j + 1 < nk) load_table_regs<kHalfRows>(tr, p.packed_tab + (size_t)((j + 1) * kBN + rg * kHalfRows) * (kD / 2), tid);
+                if (j + 1 < nk) load_table_regs(tr, p.packed_tab, (j + 1) * kBN + rg * kHalfRows, N, tid);
             }
         }
     } else {
@@ -400,7 +399,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const int pair_bar = 1 + wg * 4 + quad;   // named barrier of the two warps that hold the same 32 rows
         const uint32_t lane_base = (uint32_t)(quad * 32) << 16;
         const uint32_t tS = tmem + lane_base + wg * 128 + half * 64;          // this group's 64 S columns; its P goes over their start
-        const uint32_t tO = tmem + lane_base + 256 + wg * 128 + half * 64;    // this group's 64 O columns
+        const uint32_t tO = tmem + lane_base + 256 + wg * 128 + half * (kD / 2);   // this group's half of the O columns
         float* xmine = xch + (wg * 2 + half) * kBM + row;
         const float* xother = xch + (wg * 2 + (half ^ 1)) * kBM + row;
         int gs = 0;   // S tiles of this Q tile so far (across items): parity of S_FULL / O_FULL and of the exchange slots
@@ -419,11 +418,13 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 COROPE_TMEM_LD32(tS, s0);
                 COROPE_TMEM_LD32(tS + 32, s1);
                 tmem_wait_ld();
-                if (diag) {   // causal mask on the diagonal tile: key column > query row
+                if (diag || (!kPlain && !causal && (j + 1) * kBN > N)) {
+                    // causal mask on the diagonal tile (key column > query row); full attention: keys beyond the head
+                    const int last = (diag ? row : N - 1 - j * kBN) - half * 64;
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
-                        if (half * 64 + i > row) s0[i] = 0xff800000u;
-                        if (half * 64 + 32 + i > row) s1[i] = 0xff800000u;
+                        if (i > last) s0[i] = 0xff800000u;
+                        if (32 + i > last) s1[i] = 0xff800000u;
                     }
                 }
                 float mx0 = -INFINITY, mx1 = -INFINITY;
@@ -474,7 +475,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                     tc_fence_after();
                     const float alpha = fast_exp2(m_old - m);
 #pragma unroll
-                    for (int c = 0; c < 2; ++c) {
+                    for (int c = 0; c < kD / 64; ++c) {
                         uint32_t r[32];
                         COROPE_TMEM_LD32(tO + c * 32, r);
                         tmem_wait_ld();
@@ -491,7 +492,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             }
             if (!ok) break;
             // output of this item: total row sum from the two halves, wait for the last P V, normalise, store this
-            // group's 64 head-dim columns; then hand O back to the MMA issuer
+            // group's half of the head-dim columns; then hand O back to the MMA issuer
             *xmine = l;
             named_bar_sync(pair_bar, 64);
             const float l_tot = l + *xother;
@@ -499,12 +500,12 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (!(ok = mbar_wait_warp(&bars[O_FULL + wg], (gs - 1) & 1, p.status, O_FULL + wg, abort_flag))) break;
             tc_fence_after();
             const float inv = 1.f / l_tot;
-            const bool in_head = (2 * wi.t + wg) * kBM < N;   // false for the Q1 tile of a head's last, half-empty item
+            const bool in_head = (2 * wi.t + wg) * kBM + (kPlain ? 0 : row) < N;   // false for rows of a head's last item beyond the head
             const size_t grow = (size_t)wi.bh * N + (size_t)(2 * wi.t + wg) * kBM + row;   // row of the (contiguous) LSE
-            T* orow = reinterpret_cast<T*>(p.out_o) + half * 64 +
+            T* orow = reinterpret_cast<T*>(p.out_o) + half * (kD / 2) +
                       (kPlain ? (int64_t)grow * p.so.n : row_offset(p.so, p.H, wi.bh, (2 * wi.t + wg) * kBM + row));
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
+            for (int c = 0; c < kD / 64; ++c) {
                 uint32_t r[32];
                 COROPE_TMEM_LD32(tO + c * 32, r);
                 tmem_wait_ld();
@@ -530,7 +531,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     }
 }
 
-template <typename T>
+template <typename T, int kD>
 int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     CUtensorMap mq, mk, mv;
     // maps over the caller's q / k / v with their own strides (2-D when the rows collapse, else 4-D: head dim, row, head, batch);
@@ -545,7 +546,8 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     pp.flat_q = fq; pp.flat_k = fk; pp.flat_v = fv;
     pp.head_chunk = head_chunk_for(p.N);
     const bool plain = p.H == p.Hkv && fq && fk && fv && rows_collapse(p.so, p.H, p.N);
-    auto kern = plain ? rope_fwd_sm100_kernel<T, true> : rope_fwd_sm100_kernel<T, false>;
+    auto kern = plain ? rope_fwd_sm100_kernel<T, true, kD> : rope_fwd_sm100_kernel<T, false, kD>;
+    constexpr size_t kSmemBytes = smem_bytes(kD);
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
     if (e != cudaSuccess) return (int)e;
     const unsigned items = (unsigned)(((p.N + 2 * kBM - 1) / (2 * kBM)) * p.B * p.H);
@@ -559,15 +561,11 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
 
 }  // namespace
 
-bool rope_fwd_tc_supported(int B, int H, int N, int D, int dtype, int causal) {
-    (void)B; (void)H;
-    (void)causal;
-    return D == kD && (dtype == COROPE_DTYPE_BF16 || dtype == COROPE_DTYPE_F16) && N % kBM == 0;
-}
+bool rope_tc_supported(int D, int dtype) { return (D == 64 || D == 128) && (dtype == COROPE_DTYPE_BF16 || dtype == COROPE_DTYPE_F16); }
 
 int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s) {
-    if (dtype == COROPE_DTYPE_BF16) return launch_t<__nv_bfloat16>(p, dtype, s);
-    return launch_t<__half>(p, dtype, s);
+    if (dtype == COROPE_DTYPE_BF16) return p.D == 64 ? launch_t<__nv_bfloat16, 64>(p, dtype, s) : launch_t<__nv_bfloat16, 128>(p, dtype, s);
+    return p.D == 64 ? launch_t<__half, 64>(p, dtype, s) : launch_t<__half, 128>(p, dtype, s);
 }
 
 }  // namespace corope

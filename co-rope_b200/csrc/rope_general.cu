@@ -372,155 +372,6 @@ __global__ void __launch_bounds__(kThreads) rope_bwd_dkdv_general_kernel(RopePar
     }
 }
 
-// cos/sin fp32 tables -> compact [N][D/2] table of (cos, sin) pairs in 16-bit offset-binary fixed point
-// (see pack_unorm_pair): half the bytes of the fp32 tables with an absolute error of 1.5e-5.
-// half_src < half_d: the caller's tables have half_src columns; the pairs beyond them get the identity rotation (used when
-// a D = 64 problem is run zero-padded on the D = 128 kernels).
-__global__ void pack_tables_kernel(const float* __restrict__ cosT, const float* __restrict__ sinT, int64_t ts, uint32_t* __restrict__ out,
-                                   int N, int half_d, int half_src) {
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx == 0) out[(size_t)N * half_d] = 0u;   // the word after the table: work counter of the persistent forward kernel
-    if (idx >= (size_t)N * half_d) return;
-    int n = (int)(idx / half_d), d = (int)(idx % half_d);
-    out[idx] = (cosT != nullptr && d < half_src) ? pack_unorm_pair(cosT[n * ts + d], sinT[n * ts + d]) : pack_unorm_pair(1.f, 0.f);
-}
-
-// cos / sin tables for positions 0 .. N-1 from the per-pair frequencies, as precompute_freqs_cis forms them
-// (fused-rope/rope_attn_pytorch.py:33-47): angle = float(position) * inv_freq[d] in fp32, then cos / sin of it.
-__global__ void synth_tables_kernel(const float* __restrict__ inv_freq, float* __restrict__ cosT, float* __restrict__ sinT, int N, int half_d) {
-    size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (size_t)N * half_d) return;
-    const int n = (int)(idx / half_d), d = (int)(idx % half_d);
-    const float ang = __fmul_rn((float)n, inv_freq[d]);
-    float sn, cs;
-    sincosf(ang, &sn, &cs);
-    cosT[idx] = cs;
-    sinT[idx] = sn;
-}
-
-// D = 64 <-> D = 128 with zero padding, 16-byte chunks.  "rope" layout keeps the half-layout pairs together for the
-// D = 128 kernels: first half of the row (32 columns) to columns 0..31, second half to columns 64..95; "plain" layout
-// puts the 64 columns first.  Everything else is zero, so dot products and rotations are unchanged.
-template <typename T>
-__global__ void __launch_bounds__(256) unpad_d64_kernel(const T* __restrict__ xp, T* __restrict__ out, size_t rows, int rope_layout, RowAddr ax) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // rows * 8 output chunks
-    if (idx >= rows * 8) return;
-    const size_t r = idx >> 3;
-    const int c = (int)(idx & 7);
-    const int src = rope_layout ? (c < 4 ? c : c + 4) : c;
-    *reinterpret_cast<uint4*>(out + flat_row_offset(ax, r) + c * 8) = *reinterpret_cast<const uint4*>(xp + r * 128 + src * 8);
-}
-
-// Up to four tensors per launch (blockIdx.y picks the tensor): the D = 64 problems that take this path are small, and their
-// time is made of launches.
-struct PadJob {
-    const void* src;
-    void* dst;
-    size_t rows;
-    int rope_layout;
-    RowAddr addr;
-};
-struct PadJobs {
-    PadJob j[4];
-};
-template <typename T>
-__global__ void __launch_bounds__(256) pad_d64_many_kernel(PadJobs jobs) {
-    const PadJob& jb = jobs.j[blockIdx.y];
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // rows * 16 output chunks
-    if (idx >= jb.rows * 16) return;
-    const size_t r = idx >> 4;
-    const int c = (int)(idx & 15);
-    int src = -1;
-    if (jb.rope_layout) {
-        if (c < 4) src = c;
-        else if (c >= 8 && c < 12) src = c - 4;
-    } else if (c < 8) {
-        src = c;
-    }
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (src >= 0) v = *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(jb.src) + flat_row_offset(jb.addr, r) + src * 8);
-    *reinterpret_cast<uint4*>(reinterpret_cast<T*>(jb.dst) + r * 128 + c * 8) = v;
-}
-template <typename T>
-__global__ void __launch_bounds__(256) unpad_d64_many_kernel(PadJobs jobs) {
-    const PadJob& jb = jobs.j[blockIdx.y];   // src = padded copy, dst = the caller's tensor
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // rows * 8 output chunks
-    if (idx >= jb.rows * 8) return;
-    const size_t r = idx >> 3;
-    const int c = (int)(idx & 7);
-    const int src = jb.rope_layout ? (c < 4 ? c : c + 4) : c;
-    *reinterpret_cast<uint4*>(reinterpret_cast<T*>(jb.dst) + flat_row_offset(jb.addr, r) + c * 8) =
-        *reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(jb.src) + r * 128 + src * 8);
-}
-
-// Rotation as a pass of its own, for the tensor-core kernels at D = 128: out[r, :] = rot(x[r, :]) * scale as fp16, with the
-// same packed table and the same arithmetic as the in-kernel rotation (rotate_vec8), so both give identical bits.  The
-// forward uses it for K (every K tile is consumed by up to N/256 work items; rotating it once here instead of once per
-// consumer removes the rotation from the forward's inner loop), the backward for Q (consumed by every key block below
-// its diagonal).  One thread = 8 pairs of one row: two 16-byte loads, 32 bytes of table, two 16-byte stores.
-template <typename T>
-__global__ void __launch_bounds__(256) rope_prerotate_d128_kernel(const T* __restrict__ x, __half* __restrict__ out,
-                                                                   const uint32_t* __restrict__ tab, size_t rows, int N, float scale, RowAddr ax) {
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= rows * 8) return;
-    const size_t row = idx >> 3;
-    const int c = (int)(idx & 7) * 8;
-    const int n = (int)(row % (size_t)N);
-    const uint4* src = reinterpret_cast<const uint4*>(x + flat_row_offset(ax, row) + c);
-    uint4 x1 = __ldg(src), x2 = __ldg(src + 8);
-    const uint4* tp = reinterpret_cast<const uint4*>(tab + (size_t)n * 64 + c);
-    const uint4 t0 = __ldg(tp), t1 = __ldg(tp + 1);
-    rotate_vec8<T>(x1, x2, t0, t1, scale * (1.f / 32768.f), -257.f * scale);
-    uint4* dst = reinterpret_cast<uint4*>(out + row * 128 + c);
-    dst[0] = x1;
-    dst[8] = x2;
-}
-
-// Everything the tensor-core backward needs before its main kernel, in one pass over the rows (16 threads per row):
-// delta = rowsum(O * dO), the rotated and scaled fp16 copy of Q (threads 0-7 of a row: 8 pairs each, same arithmetic as
-// rope_prerotate_d128_kernel) and a zeroed row of the fp32 dQ accumulator (32 bytes per thread).  One launch instead of
-// a memset and two kernels; all three parts are bound by the same HBM traffic.
-template <typename T>
-__global__ void __launch_bounds__(256) rope_bwd_prepass_d128_kernel(const T* __restrict__ q, const T* __restrict__ o, const T* __restrict__ d_o,
-                                                                     const uint32_t* __restrict__ tab, __half* __restrict__ q_rot,
-                                                                     float* __restrict__ delta, float* __restrict__ dq_acc, size_t rows, int N,
-                                                                     float scale, RowAddr aq, RowAddr ao, RowAddr ado) {
-    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t row = t >> 4;
-    const int part = (int)(t & 15);
-    const bool live = row < rows;
-    float s = 0.f;
-    if (live) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(o + flat_row_offset(ao, row)) + part);
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(d_o + flat_row_offset(ado, row)) + part);
-        if (part < 8) {
-            const int c = part * 8;
-            const int n = (int)(row % (size_t)N);
-            const uint4* src = reinterpret_cast<const uint4*>(q + flat_row_offset(aq, row) + c);
-            uint4 x1 = __ldg(src), x2 = __ldg(src + 8);
-            const uint4* tp = reinterpret_cast<const uint4*>(tab + (size_t)n * 64 + c);
-            const uint4 t0 = __ldg(tp), t1 = __ldg(tp + 1);
-            rotate_vec8<T>(x1, x2, t0, t1, scale * (1.f / 32768.f), -257.f * scale);
-            uint4* dst = reinterpret_cast<uint4*>(q_rot + row * 128 + c);
-            dst[0] = x1;
-            dst[8] = x2;
-        }
-        uint4* z = reinterpret_cast<uint4*>(dq_acc + row * 128) + part * 2;
-        z[0] = make_uint4(0u, 0u, 0u, 0u);
-        z[1] = make_uint4(0u, 0u, 0u, 0u);
-        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float2 fa = unpack2<T>(aw[i]), fb = unpack2<T>(bw[i]);
-            s = fmaf(fa.x, fb.x, s);
-            s = fmaf(fa.y, fb.y, s);
-        }
-    }
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (part == 0 && live) delta[row] = s;
-}
-
 template <typename T, int D>
 int launch_fwd_t(const RopeParams& p, cudaStream_t s) {
     size_t smem = sizeof(float) * (kRows * D + kTile * (D + 1) + kTile * D);
@@ -615,82 +466,6 @@ int launch_rope_delta(const RopeParams& p, int dtype, cudaStream_t s) {
             break;
         default: return COROPE_ERR_BAD_DTYPE;
     }
-    return (int)cudaGetLastError();
-}
-
-int launch_rope_prerotate(const void* x, const Strides& st, void* out_f16, const uint32_t* packed, int B, int H, int N, float scale, int dtype,
-                          cudaStream_t s) {
-    const size_t rows = (size_t)B * H * N;
-    const unsigned grid = (unsigned)((rows * 8 + 255) / 256);
-    if (dtype == COROPE_DTYPE_BF16)
-        rope_prerotate_d128_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)x, (__half*)out_f16, packed, rows, N, scale, row_addr(st, H, N));
-    else
-        rope_prerotate_d128_kernel<__half><<<grid, 256, 0, s>>>((const __half*)x, (__half*)out_f16, packed, rows, N, scale, row_addr(st, H, N));
-    count_launch();
-    return (int)cudaGetLastError();
-}
-
-int launch_rope_bwd_prepass(const RopeParams& p, int dtype, cudaStream_t s) {
-    const size_t rows = (size_t)p.B * p.H * p.N;
-    const unsigned grid = (unsigned)((rows * 16 + 255) / 256);
-    const float scale = p.sm_scale * kLog2e;
-    if (dtype == COROPE_DTYPE_BF16)
-        rope_bwd_prepass_d128_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)p.q, (const __nv_bfloat16*)p.o, (const __nv_bfloat16*)p.d_o,
-                                                                        p.packed_tab, (__half*)const_cast<void*>(p.q_rot), p.delta, p.dq_acc, rows, p.N, scale, row_addr(p.sq, p.H, p.N), row_addr(p.so, p.H, p.N), row_addr(p.sdo, p.H, p.N));
-    else
-        rope_bwd_prepass_d128_kernel<__half><<<grid, 256, 0, s>>>((const __half*)p.q, (const __half*)p.o, (const __half*)p.d_o, p.packed_tab,
-                                                                 (__half*)const_cast<void*>(p.q_rot), p.delta, p.dq_acc, rows, p.N, scale, row_addr(p.sq, p.H, p.N), row_addr(p.so, p.H, p.N), row_addr(p.sdo, p.H, p.N));
-    count_launch();
-    return (int)cudaGetLastError();
-}
-
-int launch_pack_tables(const float* cos, const float* sin, int64_t stride, uint32_t* packed, int N, int half_d, cudaStream_t s, int half_src) {
-    size_t n = (size_t)N * half_d;
-    pack_tables_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(cos, sin, stride, packed, N, half_d, half_src < 0 ? half_d : half_src);
-    count_launch();
-    return (int)cudaGetLastError();
-}
-
-int launch_synth_tables(const float* inv_freq, float* cos_out, float* sin_out, int N, int half_d, cudaStream_t s) {
-    size_t n = (size_t)N * half_d;
-    synth_tables_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(inv_freq, cos_out, sin_out, N, half_d);
-    count_launch();
-    return (int)cudaGetLastError();
-}
-
-// n <= 4 tensors [B, H_i, N, 64] <-> their zero-padded [B, H_i, N, 128] copies in one launch (unpad: the other direction)
-int launch_pad_d64_many(int n, const PadSpec* specs, int B, int N, bool unpad, int dtype, cudaStream_t s) {
-    PadJobs jobs{};
-    size_t max_rows = 0;
-    for (int i = 0; i < n; ++i) {
-        const size_t rows = (size_t)B * specs[i].H * N;
-        jobs.j[i].src = unpad ? specs[i].padded : specs[i].tensor;
-        jobs.j[i].dst = unpad ? const_cast<void*>(specs[i].tensor) : specs[i].padded;
-        jobs.j[i].rows = rows;
-        jobs.j[i].rope_layout = specs[i].rope_layout;
-        jobs.j[i].addr = row_addr(specs[i].strides, specs[i].H, N);
-        max_rows = rows > max_rows ? rows : max_rows;
-    }
-    const dim3 grid((unsigned)((max_rows * (unpad ? 8 : 16) + 255) / 256), (unsigned)n);
-    if (dtype == COROPE_DTYPE_BF16) {
-        if (unpad) unpad_d64_many_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(jobs);
-        else pad_d64_many_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(jobs);
-    } else {
-        if (unpad) unpad_d64_many_kernel<__half><<<grid, 256, 0, s>>>(jobs);
-        else pad_d64_many_kernel<__half><<<grid, 256, 0, s>>>(jobs);
-    }
-    count_launch();
-    return (int)cudaGetLastError();
-}
-
-int launch_unpad_d64(const void* xp, void* out, const Strides& st, int B, int H, int N, int rope_layout, int dtype, cudaStream_t s) {
-    const size_t rows = (size_t)B * H * N;
-    const unsigned grid = (unsigned)((rows * 8 + 255) / 256);
-    if (dtype == COROPE_DTYPE_BF16)
-        unpad_d64_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>((const __nv_bfloat16*)xp, (__nv_bfloat16*)out, rows, rope_layout, row_addr(st, H, N));
-    else
-        unpad_d64_kernel<__half><<<grid, 256, 0, s>>>((const __half*)xp, (__half*)out, rows, rope_layout, row_addr(st, H, N));
-    count_launch();
     return (int)cudaGetLastError();
 }
 

@@ -81,12 +81,16 @@ int corope_status_mirror_clear(int* status_word, int* host_mirror, void* stream)
 const char* corope_status_string(int status);
 
 /* Bytes of caller-provided scratch (device memory, 256-byte aligned) an op needs.  Contents
- * need not be initialised by the caller.  For MHA pass Hkv == Hq.  For 16-bit inputs at D = 128 the
- * fused-RoPE ops keep a rotated fp16 copy of K (forward) or Q (backward) there, so the size grows
- * with B*H*N*D (forward: 2 bytes per element of k; backward: 6 bytes per element of q).  16-bit
- * inputs at D = 64 with N % 128 == 0 are run zero-padded to D = 128 and also keep their padded copies
- * there (forward: 16 bytes per element of q; backward: 32).  Always ask this function. */
+ * need not be initialised by the caller.  For MHA pass Hkv == Hq.  For 16-bit inputs at D = 64 or 128 with
+ * N % 128 == 0 the fused-RoPE and plain ops keep a rotated fp16 copy of K (forward) or Q (backward) there, so the
+ * size grows with B*H*N*D (forward: 2 bytes per element of k; backward: 6 bytes per element of q; for D = 64 this
+ * function answers 16 and 32 per element of q).  Always ask this function. */
 size_t corope_workspace_bytes(int op, int B, int Hq, int Hkv, int N, int D, int dtype);
+
+/* The size with which an op runs on the tensor-core kernels at every N, not only at whole tiles.  A call that is handed at
+ * least this much uses them; with corope_workspace_bytes() bytes a ragged N runs on the CUDA-core kernels.
+ * Never more than corope_workspace_bytes() where N is a whole number of tiles. */
+size_t corope_workspace_bytes_any_n(int op, int B, int Hq, int Hkv, int N, int D, int dtype);
 
 /*
  * Fused RoPE attention forward.  Replaces the launch in _attention.forward
@@ -182,6 +186,21 @@ int corope_rope_attn_bwd_freqs(const void* q, const void* k, const void* v, cons
                                int B, int H, int N, int D, int dtype, int causal, float sm_scale,
                                void* workspace, size_t workspace_bytes,
                                int* status_word, void* stream);
+
+/* The same from the base theta: inv_freq[d] = 1 / theta^(2d/D) is formed on the device too, in fp32 as precompute_freqs_cis forms
+ * it.  Workspace: COROPE_OP_ROPE_FWD_FREQS / COROPE_OP_ROPE_BWD_FREQS.  `strides` as in the *_strided entry points (NULL =
+ * contiguous). */
+int corope_rope_attn_fwd_theta(const void* q, const void* k, const void* v, float theta,
+                               void* o, float* lse2,
+                               int B, int H, int N, int D, int dtype, int causal, float sm_scale,
+                               void* workspace, size_t workspace_bytes,
+                               int* status_word, void* stream, const corope_strides_t* strides);
+int corope_rope_attn_bwd_theta(const void* q, const void* k, const void* v, const void* o, const void* d_o,
+                               const float* lse2, float theta,
+                               void* dq, void* dk, void* dv,
+                               int B, int H, int N, int D, int dtype, int causal, float sm_scale,
+                               void* workspace, size_t workspace_bytes,
+                               int* status_word, void* stream, const corope_strides_t* strides);
 
 /*
  * Plain flash attention (no RoPE) with grouped K / V heads.  Replaces _attention.forward / .backward of the reference's

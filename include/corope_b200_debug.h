@@ -23,7 +23,8 @@ extern "C" {
  */
 int corope_set_kernel_policy(int policy);
 
-/* Which kernel family the last call of each op (COROPE_OP_*) used in this process: 0 general, 1 tensor-core. */
+/* Which kernel family the last call of each op (COROPE_OP_*) used in this process: 1 = tensor-core kernels at whole tiles
+ * (N a multiple of 128, Co-RoPE: of 64), 0 = anything else: the CUDA-core kernels, or a ragged N whichever kernels ran it. */
 int corope_last_kernel_family(int op);
 
 /* Number of GPU kernel launches this library has issued in this process so far. */

@@ -1,0 +1,83 @@
+"""Lengths that are not whole tiles, on the tensor-core kernels: one key, one short of / one beyond the 64-row steps, the 128-row
+blocks and the 256-row work items; both head dimensions, causal and full, with and without rotation, grouped heads, transposed
+buffers.  Tolerances as in test_gpu_parity.py."""
+
+import os
+
+import pytest
+import torch
+
+import oracle
+from helpers import check16, draw, ext, pkg
+
+pytestmark = pytest.mark.gpu
+
+TOL_FWD_16, TOL_BWD_16 = 1e-2, 2e-2
+
+
+def _label():
+    return os.environ.get("PYTEST_CURRENT_TEST", "?").split("::")[-1].split(" ")[0]
+
+
+def _check(outs, refs, dtype):
+    check16(_label() + " O", outs[0], refs[0], TOL_FWD_16, dtype, strict=True)
+    for name, got, ref in zip(("dQ", "dK", "dV"), outs[1:], refs[1:]):
+        check16(_label() + " " + name, got, ref, TOL_BWD_16, dtype)
+
+
+def _run(fn, q, k, v, do, *args):
+    qd, kd, vd = (t.cuda().requires_grad_(True) for t in (q, k, v))
+    o = fn(qd, kd, vd, *args)
+    o.backward(do.cuda())
+    ext.check_status()
+    return tuple(t.detach().float().cpu() for t in (o, qd.grad, kd.grad, vd.grad))
+
+
+@pytest.mark.parametrize("N", [1, 63, 65, 127, 129, 193, 255, 257, 449])
+@pytest.mark.parametrize("D,causal,dtype", [(128, True, torch.bfloat16), (128, False, torch.float16), (64, True, torch.float16),
+                                            (64, False, torch.bfloat16)])
+def test_rope_at_tile_edges(N, D, causal, dtype):
+    B, H = 1, 3
+    q, k, v, do = (draw((B, H, N, D), 200 + i, dtype) for i in range(4))
+    cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
+    s = D ** -0.5
+    outs = _run(pkg.fused_rope_attention, q, k, v, do, causal, s, cos.cuda(), sin.cuda())
+    refs = (oracle.rope_attn_fwd(q, k, v, causal, s, cos, sin),) + tuple(oracle.rope_attn_bwd(q, k, v, do, causal, s, cos, sin))
+    _check(outs, refs, dtype)
+
+
+@pytest.mark.parametrize("N,D,causal", [(200, 128, True), (300, 64, False), (1000, 64, True), (129, 128, False)])
+def test_grouped_heads_in_transposed_buffers(N, D, causal):
+    B, Hq, Hkv, dtype = 2, 6, 2, torch.bfloat16
+    q, do = (draw((B, N, Hq, D), 210 + i, dtype).transpose(1, 2) for i in range(2))
+    k, v = (draw((B, N, Hkv, D), 212 + i, dtype).transpose(1, 2) for i in range(2))
+    s = D ** -0.5
+    outs = _run(pkg.flash_attention, q, k, v, do, causal, s)
+    refs = (oracle.attn_gqa_fwd(q, k, v, causal, s),) + tuple(oracle.attn_gqa_bwd(q, k, v, do, causal, s))
+    _check(outs, refs, dtype)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+def test_rows_of_the_next_head_are_not_seen(causal):
+    # head 1 holds values 100 times as large (its V and dO even infinite in one element): head 0 must not change by a bit
+    B, H, N, D, dtype = 1, 2, 200, 128, torch.bfloat16
+    q, k, v, do = (draw((B, H, N, D), 220 + i, dtype) for i in range(4))
+    base = _run(pkg.flash_attention, q, k, v, do, causal, D ** -0.5)
+    for t in (q, k, v, do):
+        t[:, 1] *= 100
+    v[0, 1, 0, 0] = do[0, 1, 0, 0] = float("inf")
+    outs = _run(pkg.flash_attention, q, k, v, do, causal, D ** -0.5)
+    for i, (a, b) in enumerate(zip(base, outs)):
+        if i == 1:   # dQ is summed with floating-point reductions in an order that varies
+            assert (a[:, 0] - b[:, 0]).abs().max().item() < 1e-2
+        else:
+            assert torch.equal(a[:, 0], b[:, 0])
+
+
+def test_theta_with_a_ragged_length():
+    B, H, N, D, dtype = 2, 2, 333, 64, torch.bfloat16
+    q, k, v, do = (draw((B, H, N, D), 230 + i, dtype) for i in range(4))
+    cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
+    outs = _run(pkg.fused_rope_attention_theta, q, k, v, do, False, D ** -0.5, 10000.0)
+    refs = (oracle.rope_attn_fwd(q, k, v, False, D ** -0.5, cos, sin),) + tuple(oracle.rope_attn_bwd(q, k, v, do, False, D ** -0.5, cos, sin))
+    _check(outs, refs, dtype)
