@@ -1,12 +1,17 @@
-"""Loader for the C-ABI library (libcorope_b200.so) and thin ctypes call helpers.
+"""Loader for the C-ABI library (libcorope_b200.so) and for the extension module in front of it (_corope_torch), which
+carries the entry points' checks, allocations and autograd nodes in C++; ctypes access to the library for everything else.
 
-The library is built in-tree by `build()` (nvcc, sm_100a only).  There is no fallback:
-if the library is missing or a CUDA device is absent, the attention entry points raise.
+Both are built in-tree by `build()` (nvcc, sm_100a only; g++ for the module).  There is no fallback:
+if they are missing or a CUDA device is absent, the attention entry points raise.
 """
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import subprocess
+import sys
+import sysconfig
 import threading
 
 import torch
@@ -14,6 +19,7 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, "csrc")
 LIB_PATH = os.path.join(_HERE, "libcorope_b200.so")
+NATIVE_PATH = os.path.join(_HERE, "_corope_torch.so")
 HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200.h")
 DEBUG_HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200_debug.h")
 
@@ -36,11 +42,38 @@ def _nvcc():
     return "nvcc"
 
 
+def _newer(target, deps):
+    return os.path.exists(target) and all(os.path.getmtime(target) >= os.path.getmtime(d) for d in deps)
+
+
+def _run(cmd, what):
+    r = subprocess.run(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("%s failed: %s\n%s" % (what, " ".join(cmd), r.stdout))
+
+
+def _build_native(force):
+    """The extension module: host code only, against torch's headers and the C ABI."""
+    src = os.path.join(_CSRC, "torch_binding.cpp")
+    if not force and _newer(NATIVE_PATH, [src, HEADER_PATH, LIB_PATH]):
+        return
+    from torch.utils import cpp_extension
+
+    cuda_home = os.path.dirname(os.path.dirname(_nvcc())) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    includes = cpp_extension.include_paths() + [os.path.join(cuda_home, "include"), sysconfig.get_paths()["include"]]
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    _run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_EXTENSION_NAME=_corope_torch", "-DTORCH_API_INCLUDE_EXTENSION_H",
+          "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + ["-isystem" + p for p in includes] +
+         [src, "-o", NATIVE_PATH, LIB_PATH, "-Wl,-rpath,$ORIGIN", "-L" + torch_lib, "-L" + os.path.join(cuda_home, "lib64"),
+          "-ltorch_python", "-ltorch", "-ltorch_cuda", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-lcudart"], "g++")
+
+
 def build(force=False, verbose=False):
-    """Compile csrc/*.cu into libcorope_b200.so for sm_100a (cross-compiles without a GPU)."""
+    """Compile csrc/*.cu into libcorope_b200.so for sm_100a (cross-compiles without a GPU) and the extension module beside it."""
     srcs = [os.path.join(_CSRC, s) for s in SOURCES]
     deps = srcs + [os.path.join(_CSRC, "common.cuh"), os.path.join(_CSRC, "corope_mma.cuh"), HEADER_PATH, DEBUG_HEADER_PATH]
-    if not force and os.path.exists(LIB_PATH) and all(os.path.getmtime(LIB_PATH) >= os.path.getmtime(d) for d in deps):
+    if not force and _newer(LIB_PATH, deps):
+        _build_native(force)
         return LIB_PATH
     objs = []
     procs = []
@@ -58,11 +91,30 @@ def build(force=False, verbose=False):
             raise RuntimeError("nvcc failed: %s\n%s" % (" ".join(cmd), out))
         if verbose and out:
             print(out)
-    link = [_nvcc(), "-shared", "-o", LIB_PATH] + objs + ["-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"]
-    r = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
-    if r.returncode != 0:
-        raise RuntimeError("link failed: %s\n%s" % (" ".join(link), r.stdout))
+    _run([_nvcc(), "-shared", "-Xlinker", "-soname=libcorope_b200.so", "-o", LIB_PATH] + objs + ["-gencode", "arch=compute_100a,code=sm_100a", "-lcudart"], "link")
+    _build_native(force)
     return LIB_PATH
+
+
+_native = None
+
+
+def native():
+    """The loaded extension module.  Raises if it has not been built -- there is no other code path."""
+    global _native
+    if _native is None:
+        lib()
+        with _lock:
+            mod = sys.modules.get("_corope_torch")   # one copy per process, whatever name this package was imported under
+            if mod is None:
+                if not os.path.exists(NATIVE_PATH):
+                    raise RuntimeError("corope_b200: %s is missing; build it with `python -c \"import __graft_entry__ as g; g.build()\"`." % NATIVE_PATH)
+                loader = importlib.machinery.ExtensionFileLoader("_corope_torch", NATIVE_PATH)
+                mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_corope_torch", loader))
+                loader.exec_module(mod)
+                sys.modules["_corope_torch"] = mod
+            _native = mod
+    return _native
 
 
 def lib():
@@ -154,27 +206,12 @@ def strides_of(**tensors):
     return st
 
 
-def kernel_layout(t):
-    """`t` itself when the kernels can take its layout directly (unit stride along the head dimension, no overlapping
-    or broadcast strides), else a contiguous copy."""
-    if t.stride(-1) == 1 and all(s > 0 for s in t.stride()) and t.stride(2) >= t.shape[3]:
-        return t
-    return t.contiguous()
-
-
-def require_cuda(t):
-    if not t.is_cuda:
-        raise RuntimeError("corope_b200 runs on CUDA tensors only (got a %s tensor); there is no CPU path." % t.device.type)
-
-
 class _DeviceStatus:
-    """The device status word of one GPU with a pinned host mirror that the library's side stream refreshes after every call."""
+    """The device status word of one GPU and its pinned host mirror (both owned by the extension module)."""
 
     def __init__(self, index):
-        dev = torch.device("cuda", index)
         self.index = index
-        self.word = torch.zeros(1, dtype=torch.int32, device=dev)
-        self.mirror = torch.zeros(1, dtype=torch.int32).pin_memory()
+        self.word, self.mirror = native().device_status(index)
         self.word_ptr = self.word.data_ptr()
         self.mirror_ptr = self.mirror.data_ptr()
         self.mirror_view = (ctypes.c_int * 1).from_address(self.mirror_ptr)   # a plain int read, no tensor indexing per call
@@ -186,11 +223,7 @@ def _status(device):
         key = torch.cuda.current_device()
     st = _status_words.get(key)
     if st is None:
-        with _lock:
-            st = _status_words.get(key)
-            if st is None:
-                st = _DeviceStatus(key)
-                _status_words[key] = st
+        st = _status_words.setdefault(key, _DeviceStatus(key))
     return st
 
 
@@ -206,11 +239,9 @@ def _status_message(v):
 
 
 def pre_call(device):
-    """Called by the attention entry points before they launch: raises if an EARLIER call on this device left the status
-    word set.  Reads only the pinned host mirror (no synchronisation); the mirror is refreshed by post_call(), so the error
-    surfaces at the first call after the failing one has finished on the GPU.  The word is cleared before raising."""
-    if getattr(_batched, "depth", 0) > 0:
-        return
+    """What the attention entry points do before they launch: raises if an EARLIER call on this device left the status word
+    set, clearing it.  Reads only the pinned host mirror (no synchronisation), which a failing kernel writes itself, so the
+    error surfaces at the first call after the failing one has run on the GPU."""
     st = _status(device)
     v = st.mirror_view[0]
     if v != 0:
@@ -219,43 +250,30 @@ def pre_call(device):
         raise RuntimeError("corope_b200: an earlier kernel reported device status 0x%x: %s" % (v, _status_message(v)))
 
 
-_batched = threading.local()
-
-
 class batched_status:
-    """Context manager for callers that make many library calls in a row (the host pipeline): the per-call look at the
-    mirror and its refresh are done once, on entry and on exit, instead of around every call."""
+    """Context manager around many library calls in a row (the host pipeline, a graph capture): looks at the mirror on entry."""
 
     def __init__(self, device):
         self.device = device
 
     def __enter__(self):
         pre_call(self.device)
-        _batched.depth = getattr(_batched, "depth", 0) + 1
         return self
 
     def __exit__(self, *exc):
-        _batched.depth -= 1
-        if exc[0] is None:
-            post_call(self.device)
         return False
 
 
 def post_call(device, stream=None):
-    """Called after a launch: the library's side stream copies the status word to its pinned mirror once the caller's stream
-    gets there (the caller's stream itself only records an event).  The caller has the device current."""
-    if getattr(_batched, "depth", 0) > 0:
-        return
+    """Refreshes the mirror of a word that something other than this library's kernels may have set: the library's side stream
+    copies it once the caller's stream gets there (the caller's stream itself only records an event)."""
     if torch.cuda.is_current_stream_capturing():
         return
     st = _status(device)
     if stream is None:
         stream = torch.cuda.current_stream(st.index).cuda_stream
-    if torch.cuda.current_device() == st.index:
+    with torch.cuda.device(st.index):   # the library's side stream belongs to the current device
         lib().corope_status_mirror_refresh(st.word_ptr, st.mirror_ptr, stream)
-    else:   # the library's side stream belongs to the current device
-        with torch.cuda.device(st.index):
-            lib().corope_status_mirror_refresh(st.word_ptr, st.mirror_ptr, stream)
 
 
 def check_status(device=None):
@@ -273,17 +291,6 @@ def check_status(device=None):
 def workspace(op, B, Hq, Hkv, N, D, dtype, device):
     nbytes = lib().corope_workspace_bytes_any_n(op, B, Hq, Hkv, N, D, DTYPE_CODES[dtype])
     return torch.empty(max(int(nbytes), 256), dtype=torch.uint8, device=device), int(nbytes)
-
-
-def raise_for_status(code, what):
-    if code == 0:
-        return
-    msg = lib().corope_status_string(code).decode()
-    if code == -3:
-        raise AssertionError("%s: %s" % (what, msg))
-    if code in (-6,):
-        raise ValueError("%s: %s" % (what, msg))
-    raise RuntimeError("%s failed with status %d: %s" % (what, code, msg))
 
 
 def stream_ptr(device):

@@ -105,11 +105,22 @@ int check_workspace(const void* ws, size_t have, size_t need) {
 
 }  // namespace
 
+int sm_count() {
+    static std::atomic<int> known[64];
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 148;
+    if (dev >= 0 && dev < 64 && (sms = known[dev].load(std::memory_order_relaxed)) > 0) return sms;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return 148;
+    if (dev >= 0 && dev < 64) known[dev].store(sms, std::memory_order_relaxed);
+    return sms;
+}
 void count_launch(int n) { g_launches.fetch_add((unsigned long long)n); }
 void note_kernel_family(int op, int family) {
     if (op >= 0 && op < 4) g_last_family[op] = family;
 }
 int kernel_policy() { return g_policy.load(); }
+
+int* status_mirror_of(const int* status_word);   // below, beside the registration
 
 }  // namespace corope
 
@@ -163,6 +174,29 @@ int corope_status_mirror_clear(int* status_word, int* host_mirror, void* stream)
     if (e == cudaSuccess) e = cudaMemsetAsync(status_word, 0, sizeof(int), (cudaStream_t)stream);
     *host_mirror = 0;
     return (int)e;
+}
+
+// Registered (word, mirror) pairs: a handful per process, looked up by every launch.
+namespace {
+struct MirrorPair {
+    std::atomic<const int*> word{nullptr};
+    std::atomic<int*> mirror{nullptr};
+};
+MirrorPair g_pairs[128];
+}  // namespace
+
+int corope_status_mirror_register(const int* status_word, int* host_mirror) {
+    if (!status_word || !host_mirror) return COROPE_ERR_NULL_POINTER;
+    void* dev = nullptr;
+    if (cudaError_t e = cudaHostGetDevicePointer(&dev, host_mirror, 0)) return (int)e;
+    std::lock_guard<std::mutex> lock(g_mirror_mutex);
+    for (MirrorPair& p : g_pairs)
+        if (p.word.load() == nullptr || p.word.load() == status_word) {
+            p.mirror.store(static_cast<int*>(dev));
+            p.word.store(status_word);
+            return COROPE_OK;
+        }
+    return COROPE_ERR_TOO_LARGE;
 }
 
 const char* corope_status_string(int status) {
@@ -318,7 +352,7 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
     RopeParams p{};
     p.q = q; p.k = k; p.v = v; p.out_o = o; p.lse2 = lse2;
     p.B = B; p.H = Hq; p.Hkv = Hkv; p.no_rope = rot.none ? 1 : 0;
-    p.N = N; p.D = D; p.causal = causal ? 1 : 0; p.sm_scale = sm_scale; p.status = status_word;
+    p.N = N; p.D = D; p.causal = causal ? 1 : 0; p.sm_scale = sm_scale; p.status = status_word; p.status_mirror = status_mirror_of(status_word);
     set_strides(p, strides, Hq, Hkv, N, D);
     if (!strides_positive(p.sq, D) || !strides_positive(p.sk, D) || !strides_positive(p.sv, D) || !strides_positive(p.so, D)) return COROPE_ERR_BAD_STRIDE;
     // rows are moved with TMA / 16-byte vectors on the tensor-core paths; otherwise the CUDA-core kernels take over
@@ -362,7 +396,7 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
     p.lse2 = const_cast<float*>(lse2);
     p.delta = reinterpret_cast<float*>((char*)workspace + w.delta);
     p.B = B; p.H = Hq; p.Hkv = Hkv; p.no_rope = rot.none ? 1 : 0;
-    p.N = N; p.D = D; p.causal = causal ? 1 : 0; p.sm_scale = sm_scale; p.status = status_word;
+    p.N = N; p.D = D; p.causal = causal ? 1 : 0; p.sm_scale = sm_scale; p.status = status_word; p.status_mirror = status_mirror_of(status_word);
     set_strides(p, strides, Hq, Hkv, N, D);
     for (const Strides* st : {&p.sq, &p.sk, &p.sv, &p.so, &p.sdo, &p.sdq, &p.sdk, &p.sdv})
         if (!strides_positive(*st, D)) return COROPE_ERR_BAD_STRIDE;
@@ -421,6 +455,16 @@ Rotation no_rotation() {
 }
 
 }  // namespace
+
+int* corope::status_mirror_of(const int* status_word) {
+    if (status_word)
+        for (const MirrorPair& p : g_pairs) {
+            const int* w = p.word.load();
+            if (w == status_word) return p.mirror.load();
+            if (w == nullptr) break;
+        }
+    return nullptr;
+}
 
 extern "C" {
 
@@ -532,7 +576,7 @@ int corope_gqa_fwd_strided(const void* q, const void* k, const void* v, void* o,
     if (int e = check_workspace(workspace, workspace_bytes, w.total)) return e;
     GqaParams p{};
     p.q = q; p.k = k; p.v = v; p.out_o = o; p.lse2 = lse2; p.a_diag = a_diag;
-    p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.N = N; p.D = D; p.sm_scale = sm_scale; p.theta = theta; p.status = status_word;
+    p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.N = N; p.D = D; p.sm_scale = sm_scale; p.theta = theta; p.status = status_word; p.status_mirror = status_mirror_of(status_word);
     set_gqa_strides(p, strides);
     if (!strides_positive(p.sq, D) || !strides_positive(p.sk, D) || !strides_positive(p.sv, D) || !strides_positive(p.so, D)) return COROPE_ERR_BAD_STRIDE;
     // the tensor-core kernels read K and V in 16-byte vectors and store O in element pairs
@@ -567,7 +611,7 @@ int corope_gqa_bwd_strided(const void* q, const void* k, const void* v, const vo
     p.delta = reinterpret_cast<float*>((char*)workspace + w.delta);
     p.dk_acc = reinterpret_cast<float*>((char*)workspace + w.dk_acc);
     p.dv_acc = reinterpret_cast<float*>((char*)workspace + w.dv_acc);
-    p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.N = N; p.D = D; p.sm_scale = sm_scale; p.theta = theta; p.status = status_word;
+    p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.G = Hq / Hkv; p.N = N; p.D = D; p.sm_scale = sm_scale; p.theta = theta; p.status = status_word; p.status_mirror = status_mirror_of(status_word);
     set_gqa_strides(p, strides);
     for (const Strides* st : {&p.sq, &p.sk, &p.sv, &p.so, &p.sdo, &p.sdq, &p.sdk, &p.sdv})
         if (!strides_positive(*st, D)) return COROPE_ERR_BAD_STRIDE;

@@ -7,6 +7,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/corope_b200.h"
 
 namespace corope {
@@ -103,6 +105,7 @@ struct RopeParams {
     int causal;
     float sm_scale;
     int* status;
+    int* status_mirror; // host memory that a failing kernel copies the status word to, or null
     int* sched_counter; // zeroed word in the workspace: next work item / unit of the persistent tensor-core kernels
     int head_chunk;     // heads per chunk of the persistent kernels' work order (set by their launchers)
     const void* k_rot;  // forward: [B,H,N,D] fp16, K already rotated by the pre-pass; null = the kernel rotates K tiles itself
@@ -134,6 +137,7 @@ struct GqaParams {
     float sm_scale;
     float theta;
     int* status;
+    int* status_mirror;   // see RopeParams
     Strides sq, sk, sv, so, sdo, sdq, sdk, sdv;   // strides of q, k, v, o (forward output or backward input), dO, dq, dk, dv
 };
 
@@ -187,6 +191,12 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
     *abort_flag = 1;
     if (status) atomicCAS(status, 0, COROPE_DEV_WAIT_EXPIRED | id);
     return false;
+}
+// A kernel that gave up leaves its code in the host mirror too, so that the host learns of it without a copy or a synchronisation.
+__device__ __forceinline__ void report_to_mirror(const int* status, int* mirror) {
+    if (status == nullptr || mirror == nullptr) return;
+    *reinterpret_cast<volatile int*>(mirror) = *reinterpret_cast<const volatile int*>(status);
+    __threadfence_system();
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int id, volatile int* abort_flag) {
     return mbar_wait_limited(bar, parity, status, id, abort_flag, kWaitLimit);
@@ -602,6 +612,20 @@ inline int encode_tensor_map_f32(CUtensorMap* out, const void* base, uint64_t ro
     return r == CUDA_SUCCESS ? 0 : COROPE_ERR_TENSOR_MAP;
 }
 
+int* status_mirror_of(const int* status_word);   // device address of the registered host mirror, or null
+// Host costs paid once instead of per launch: the SM count of the current device, and the opt-in to large dynamic shared memory of
+// a kernel on it (`done` is a static of the call site, one bit per device).
+int sm_count();
+template <typename K>
+inline int allow_smem(K kernel, size_t bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    if (cudaError_t e = cudaGetDevice(&dev)) return (int)e;
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done.load(std::memory_order_relaxed) & bit) return 0;
+    if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) return (int)e;
+    done.fetch_or(bit);
+    return 0;
+}
 // Every kernel launch of the library bumps this counter (read through corope_launch_count()).
 void count_launch(int n = 1);
 // Diagnostics kept by abi.cu (see include/corope_b200_debug.h): which kernel family an op took last, and the policy in force.

@@ -525,7 +525,10 @@ __global__ void __launch_bounds__(kThreads, 1) corope_bwd_mma_kernel(GqaParams p
                 }
         }
     }
-    if (__any_sync(0xffffffffu, range_clamped) && lane == 0 && p.status) atomicCAS(p.status, 0, COROPE_DEV_RANGE);
+    if (__any_sync(0xffffffffu, range_clamped) && lane == 0 && p.status) {
+        atomicCAS(p.status, 0, COROPE_DEV_RANGE);
+        report_to_mirror(p.status, p.status_mirror);
+    }
 #pragma unroll
     for (int x2 = 0; x2 < 2; ++x2) {
         if (2 * c + x2 >= G) continue;
@@ -551,11 +554,13 @@ int launch_g(const GqaParams& p, cudaStream_t s) {
     if (e != cudaSuccess) return (int)e;
     if (p.N <= 8192) {
         auto kern = corope_bwd_mma_kernel<T, G, true>;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)) != cudaSuccess) return (int)e;
+        static std::atomic<uint64_t> smem_ok;
+        if (int er = allow_smem(kern, kSmemBytes, smem_ok)) return er;
         kern<<<grid, kThreads, kSmemBytes, s>>>(p);
     } else {
         auto kern = corope_bwd_mma_kernel<T, G, false>;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)) != cudaSuccess) return (int)e;
+        static std::atomic<uint64_t> smem_ok;
+        if (int er = allow_smem(kern, kSmemBytes, smem_ok)) return er;
         kern<<<grid, kThreads, kSmemBytes, s>>>(p);
     }
     count_launch();

@@ -260,11 +260,13 @@ int launch_g(const GqaParams& p, cudaStream_t s) {
     // phases up to a few thousand radians (N <= 8192) go to the hardware sin / cos directly
     if (p.N <= 8192) {
         auto kern = corope_fwd_mma_kernel<T, G, true>;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)) != cudaSuccess) return (int)e;
+        static std::atomic<uint64_t> smem_ok;
+        if (int er = allow_smem(kern, kSmemBytes, smem_ok)) return er;
         kern<<<grid, kThreads, kSmemBytes, s>>>(p);
     } else {
         auto kern = corope_fwd_mma_kernel<T, G, false>;
-        if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes)) != cudaSuccess) return (int)e;
+        static std::atomic<uint64_t> smem_ok;
+        if (int er = allow_smem(kern, kSmemBytes, smem_ok)) return er;
         kern<<<grid, kThreads, kSmemBytes, s>>>(p);
     }
     count_launch();

@@ -456,8 +456,8 @@ int launch_fwd_g(const GqaParams& p, cudaStream_t s) {
     constexpr bool kAcc = (Elem<T>::kDtype == COROPE_DTYPE_F32);
     size_t smem = sizeof(float) * ((size_t)G * kWarps * D + kTile * (D + kPad) + kTile * D + D / 2);
     auto kern = corope_fwd_general_kernel<T, D, G, kAcc>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
+    static std::atomic<uint64_t> smem_ok;
+    if (int er = allow_smem(kern, smem, smem_ok)) return er;
     dim3 grid((p.N + kWarps - 1) / kWarps, p.B * p.Hkv);
     kern<<<grid, kThreads, smem, s>>>(p); count_launch();
     return (int)cudaGetLastError();
@@ -468,8 +468,8 @@ int launch_bwd_g(const GqaParams& p, cudaStream_t s) {
     constexpr bool kAcc = (Elem<T>::kDtype == COROPE_DTYPE_F32);
     size_t smem = sizeof(float) * ((size_t)2 * G * kWarps * D + 2 * kTile * (D + kPad) + 2 * kTile * D + D / 2 + (size_t)kWarps * (2 * G + 2) * kTile);
     auto kern = corope_bwd_general_kernel<T, D, G, kAcc>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
+    static std::atomic<uint64_t> smem_ok;
+    if (int er = allow_smem(kern, smem, smem_ok)) return er;
     dim3 grid((p.N + kWarps - 1) / kWarps, p.B * p.Hkv);
     kern<<<grid, kThreads, smem, s>>>(p); count_launch();
     return (int)cudaGetLastError();

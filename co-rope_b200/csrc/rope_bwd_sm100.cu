@@ -575,6 +575,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (threadIdx.x == kDrainWarp0 * 32) bulk_wait_group0();   // all reduces have landed before the CTA exits
     }
     __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) report_to_mirror(p.status, p.status_mirror);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -630,11 +631,9 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     if (int er = encode_tensor_map_f32(&mdq, p.dq_acc, plain ? rows : (uint64_t)p.N, kD, plain ? 0 : (uint64_t)p.B * p.H, kBQ, kD)) return er;
     auto kern = plain ? rope_bwd_sm100_kernel<T, true, kD> : rope_bwd_sm100_kernel<T, false, kD>;
     constexpr size_t kSmemBytes = smem_bytes(kD);
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return (int)e;
-    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+    static std::atomic<uint64_t> smem_ok[2];
+    if (int er = allow_smem(kern, kSmemBytes, smem_ok[plain])) return er;
+    const int sms = sm_count();
     const unsigned units = (unsigned)(((p.N + kBK - 1) / kBK) * p.B * p.Hkv);
     const unsigned grid = units < (unsigned)sms ? units : (unsigned)sms;   // persistent: one CTA per SM
     kern<<<grid, kThreads, kSmemBytes, s>>>(mq, mk, mv, mdo, mdq, pp); count_launch();

@@ -525,6 +525,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         tc_fence_before();
     }
     __syncthreads();
+    if (threadIdx.x == 0 && *abort_flag) report_to_mirror(p.status, p.status_mirror);
     if (warp == kMmaWarp) {
         tc_fence_after();
         tmem_dealloc(tmem, 512);
@@ -548,12 +549,10 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     const bool plain = p.H == p.Hkv && fq && fk && fv && rows_collapse(p.so, p.H, p.N);
     auto kern = plain ? rope_fwd_sm100_kernel<T, true, kD> : rope_fwd_sm100_kernel<T, false, kD>;
     constexpr size_t kSmemBytes = smem_bytes(kD);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
-    if (e != cudaSuccess) return (int)e;
+    static std::atomic<uint64_t> smem_ok[2];
+    if (int e = allow_smem(kern, kSmemBytes, smem_ok[plain])) return e;
     const unsigned items = (unsigned)(((p.N + 2 * kBM - 1) / (2 * kBM)) * p.B * p.H);
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    const int sms = sm_count();
     const unsigned grid = items < (unsigned)sms ? items : (unsigned)sms;   // persistent: one CTA per SM
     kern<<<grid, kThreads, kSmemBytes, s>>>(mq, mk, mv, pp); count_launch();
     return (int)cudaGetLastError();

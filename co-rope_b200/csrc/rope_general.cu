@@ -376,8 +376,8 @@ template <typename T, int D>
 int launch_fwd_t(const RopeParams& p, cudaStream_t s) {
     size_t smem = sizeof(float) * (kRows * D + kTile * (D + 1) + kTile * D);
     auto kern = rope_fwd_general_kernel<T, D>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
+    static std::atomic<uint64_t> smem_ok;
+    if (int er = allow_smem(kern, smem, smem_ok)) return er;
     dim3 grid((p.N + kRows - 1) / kRows, p.B * p.H);
     kern<<<grid, kThreads, smem, s>>>(p); count_launch();
     return (int)cudaGetLastError();
@@ -389,17 +389,16 @@ int launch_bwd_t(const RopeParams& p, cudaStream_t s) {
     {
         size_t smem = sizeof(float) * (2 * kRows * D + 2 * kTile * (D + 1));
         auto kern = rope_bwd_dq_general_kernel<T, D>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
+        static std::atomic<uint64_t> smem_ok;
+        if (int er = allow_smem(kern, smem, smem_ok)) return er;
         kern<<<grid, kThreads, smem, s>>>(p); count_launch();
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return (int)e;
+        if (cudaError_t e = cudaGetLastError()) return (int)e;
     }
     {
         size_t smem = sizeof(float) * (2 * kRows * D + 2 * kTile * (D + 1) + 2 * kTile);
         auto kern = rope_bwd_dkdv_general_kernel<T, D>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
+        static std::atomic<uint64_t> smem_ok;
+        if (int er = allow_smem(kern, smem, smem_ok)) return er;
         dim3 grid_kv((p.N + kRows - 1) / kRows, p.B * p.Hkv);   // one CTA per 32 keys of a KV head; it sums over the group's query heads
         kern<<<grid_kv, kThreads, smem, s>>>(p); count_launch();
         return (int)cudaGetLastError();

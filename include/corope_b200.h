@@ -12,7 +12,7 @@
  * kernel exits cleanly.  While the word is non-zero, later tensor-core launches that are given the
  * same word return without computing (their outputs are then undefined): read and clear it on the
  * host after synchronising.  The Python modules of this package do that for the caller: every call
- * first looks at a pinned host mirror of the word that the previous call's stream refreshed, and
+ * first looks at a pinned host mirror of the word, which a failing kernel writes too, and
  * raises (and clears the word) if it was set.
  *
  * Supported value range of 16-bit inputs: the tensor-core kernels feed fp16 operands to the MMAs
@@ -73,9 +73,12 @@ int corope_abi_version(void);
  * Host mirror of a status word, for callers that want to learn of a device-side error without ever synchronising:
  * `_refresh` makes a side stream of the library copy *status_word to *host_mirror (pinned host memory) once `stream` has
  * executed everything enqueued so far -- `stream` itself only records an event -- so that reading *host_mirror on the host
- * before a later call shows whether an earlier call failed.  `_clear` resets both (it waits for the side stream first).
+ * before a later call shows whether an earlier call failed.  `_register` lets the kernels themselves write a failure to the
+ * mirror of the word they are handed (nothing has to be enqueued behind a call then).  `_clear` resets both (it waits for
+ * the side stream first).
  * No counterpart in the reference, whose kernels report nothing.
  */
+int corope_status_mirror_register(const int* status_word, int* host_mirror);
 int corope_status_mirror_refresh(const int* status_word, int* host_mirror, void* stream);
 int corope_status_mirror_clear(int* status_word, int* host_mirror, void* stream);
 const char* corope_status_string(int status);

@@ -1,0 +1,49 @@
+"""The C++ host path of the entry points: a device-side failure reaches the host without any call in between, and output
+gradients and masks in forms a caller may hand over."""
+
+import pytest
+import torch
+
+import oracle
+from helpers import check16, draw, ext, fused_attention, pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def test_a_failing_kernel_writes_the_host_mirror_itself():
+    dev = torch.device("cuda", 0)
+    ext.check_status(dev)
+    word = ext.status_word(dev)
+    assert ext.lib().corope_debug_expire_wait(word.data_ptr(), 100, torch.cuda.current_stream(dev).cuda_stream) == 0
+    torch.cuda.synchronize()
+    q, k, v = (draw((1, 1, 128, 64), i, torch.bfloat16).cuda() for i in range(3))
+    with pytest.raises(RuntimeError, match="0x107e"):
+        pkg.flash_attention(q, k, v, True, 0.125)
+    pkg.flash_attention(q, k, v, True, 0.125)   # cleared
+    ext.check_status(dev)
+
+
+def test_broadcast_output_gradient_and_partial_requires_grad():
+    # o.sum().backward() hands over a dO with zero strides; only v asks for a gradient
+    B, H, N, D = 1, 2, 160, 64
+    q, k, v = (draw((B, H, N, D), 300 + i, torch.bfloat16) for i in range(3))
+    cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
+    vd = v.cuda().requires_grad_(True)
+    qd = q.cuda()
+    fused_attention(qd, k.cuda(), vd, True, D ** -0.5, cos.cuda(), sin.cuda(), False).sum().backward()
+    ext.check_status()
+    ref = oracle.rope_attn_bwd(q, k, v, torch.ones_like(q), True, D ** -0.5, cos, sin)[2]
+    assert qd.grad is None
+    # dV of an all-ones gradient is the same for every column: sums of P over the queries, up to ~7 here, each of N terms rounded to bf16
+    check16("broadcast dO dV", vd.grad.float().cpu(), ref, 2e-2, torch.bfloat16)
+
+
+def test_wrong_tables_and_dtypes_raise_the_python_errors():
+    q = torch.zeros(1, 1, 128, 64, device="cuda", dtype=torch.bfloat16)
+    t = torch.zeros(100, 64, device="cuda")
+    with pytest.raises(ValueError, match="cover"):
+        fused_attention(q, q, q, True, 1.0, t, t)
+    with pytest.raises(AssertionError):
+        fused_attention(q, q, q.float(), True, 1.0, t, t)
+    with pytest.raises(AssertionError):
+        pkg.flash_attention(q, q, q[..., :32], True, 1.0)
