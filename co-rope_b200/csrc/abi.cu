@@ -426,8 +426,9 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
         return launch_rope_bwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
-    if (int e = launch_rope_delta(p, dtype, s)) return e;
     g_last_family[kFamBwd] = 0;
+    if (dtype == COROPE_DTYPE_F32) return launch_rope_bwd_fp32(p, s);
+    if (int e = launch_rope_delta(p, dtype, s)) return e;
     return launch_rope_bwd_general(p, dtype, s);
 }
 

@@ -636,7 +636,8 @@ int kernel_policy();
 // host launchers implemented by the kernel translation units (return cudaError_t as int)
 // ---------------------------------------------------------------------------------------------
 int launch_rope_fwd_general(const RopeParams& p, int dtype, cudaStream_t s);
-int launch_rope_bwd_general(const RopeParams& p, int dtype, cudaStream_t s);
+int launch_rope_bwd_general(const RopeParams& p, int dtype, cudaStream_t s);   // 16-bit types, delta computed before
+int launch_rope_bwd_fp32(const RopeParams& p, cudaStream_t s);                 // delta included
 int launch_rope_delta(const RopeParams& p, int dtype, cudaStream_t s);
 // What the tensor-core kernels need before they run (rope_prepass.cu).
 // Where the (cos, sin) pairs of a position come from.

@@ -1,16 +1,15 @@
-// General fused-RoPE attention kernels: fp32 arithmetic on the CUDA cores, any N, causal or not,
-// D in {32, 64, 128}, inputs fp32 / bf16 / fp16.  This is the accuracy path (fp32 inputs must match
-// the fp32 reference to 1e-4, which rules out 16-bit tensor-core operands) and the path for shapes the
-// tensor-core kernels do not take.  Q and every K tile are rotated while being staged into shared
-// memory; rotated values never go back to HBM.
+// General fused-RoPE attention backward for 16-bit inputs: fp32 arithmetic on the CUDA cores, any N, causal or not, D in
+// {32, 64, 128}.  The path for the shapes and layouts the tensor-core kernels do not take (D = 32, strides that are no multiples
+// of 16 bytes); the forward of those and everything in fp32 is in rope_fp32.cu.  Q and every K tile are rotated while being staged
+// into shared memory; rotated values never go back to HBM.
 //
-// Tiling: one CTA = 32 rows (queries for fwd / dQ, keys for dK / dV), 4 warps x 8 rows; the other
+// Tiling: one CTA = 32 rows (queries for dQ, keys for dK / dV), 4 warps x 8 rows; the other
 // operand streams through shared memory in tiles of 32.  Within a warp, lane = column of the
 // 32 x 32 score tile for the dot products, and lane = head-dim column (lane + 32 c) for the
 // accumulators.
 //
-// Math follows fused-rope/rope_attn_pytorch.py:108-155 (forward) and :187-222 (backward); the exp2-domain
-// softmax and the log2-domain LSE follow fused-rope/fused_rope_attn.py:103-114, 316.
+// Math follows fused-rope/rope_attn_pytorch.py:187-222; the exp2-domain softmax and the log2-domain LSE follow
+// fused-rope/fused_rope_attn.py:103-114, 316.
 #include "common.cuh"
 
 namespace corope {
@@ -21,11 +20,6 @@ constexpr int kTile = 32;     // streamed rows per step
 constexpr int kThreads = 128;
 constexpr int kRowsPerWarp = 8;
 
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -120,74 +114,6 @@ __device__ __forceinline__ void store_inverse_rotated(T* dst_row, const float (&
             dst_row[d] = Elem<T>::from_f32((a1 * c + a2 * s) * scale);
             dst_row[d + H2] = Elem<T>::from_f32((a2 * c - a1 * s) * scale);
         }
-    }
-}
-
-// ------------------------------------------------------------------------------------------------
-// forward
-// ------------------------------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void __launch_bounds__(kThreads) rope_fwd_general_kernel(RopeParams p) {
-    constexpr int NC = D / 32;
-    extern __shared__ __align__(16) float smem[];
-    float* q_s = smem;                       // [32][D]     rotated * sm_scale * log2e
-    float* k_s = q_s + kRows * D;            // [32][D+1]   rotated
-    float* v_s = k_s + kTile * (D + 1);      // [32][D]
-
-    const int N = p.N;
-    const int bh = blockIdx.y;
-    const int m0 = (gridDim.x - 1 - blockIdx.x) * kRows;  // longest causal rows first
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kvh = bh / (p.H / p.Hkv);   // [B, H] flattened -> [B, Hkv] flattened: the heads of a group are adjacent
-    const T* Q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, 0);
-    const T* K = reinterpret_cast<const T*>(p.k) + row_offset(p.sk, p.Hkv, kvh, 0);
-    const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0);
-    T* O = reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.H, bh, 0);
-
-    stage_rows<T, D, D, true>(q_s, Q, p.sq.n, m0, N, p.cos, p.sin, p.table_stride, p.sm_scale * kLog2e);
-
-    float m[kRowsPerWarp], l[kRowsPerWarp], acc[kRowsPerWarp][NC];
-#pragma unroll
-    for (int r = 0; r < kRowsPerWarp; ++r) {
-        m[r] = -INFINITY;
-        l[r] = 0.f;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) acc[r][c] = 0.f;
-    }
-    const int row0 = warp * kRowsPerWarp;
-    const int n_end = p.causal ? min(N, m0 + kRows) : N;
-    for (int j0 = 0; j0 < n_end; j0 += kTile) {
-        __syncthreads();
-        stage_rows<T, D, D + 1, true>(k_s, K, p.sk.n, j0, N, p.cos, p.sin, p.table_stride, 1.f);
-        stage_rows<T, D, D, false>(v_s, V, p.sv.n, j0, N, nullptr, nullptr, 0, 1.f);
-        __syncthreads();
-        float s[kRowsPerWarp];
-        dot_rows<D>(s, q_s, row0, k_s, lane);
-        const int j = j0 + lane;
-#pragma unroll
-        for (int r = 0; r < kRowsPerWarp; ++r) {
-            const int i = m0 + row0 + r;
-            bool ok = (j < N) && (!p.causal || j <= i);
-            float sv = ok ? s[r] : -INFINITY;
-            float mx = fmaxf(m[r], warp_max(sv));
-            float alpha = (mx == -INFINITY) ? 1.f : exp2f(m[r] - mx);
-            float pv = (mx == -INFINITY || !ok) ? 0.f : exp2f(sv - mx);
-            l[r] = l[r] * alpha + warp_sum(pv);
-            m[r] = mx;
-#pragma unroll
-            for (int c = 0; c < NC; ++c) acc[r][c] *= alpha;
-            s[r] = pv;
-        }
-        accumulate_cols<D, D>(acc, s, v_s, lane);
-    }
-#pragma unroll
-    for (int r = 0; r < kRowsPerWarp; ++r) {
-        const int i = m0 + row0 + r;
-        if (i >= N) continue;
-        float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
-#pragma unroll
-        for (int c = 0; c < NC; ++c) O[(int64_t)i * p.so.n + lane + 32 * c] = Elem<T>::from_f32(acc[r][c] * inv);
-        if (lane == 0) p.lse2[(size_t)bh * N + i] = m[r] + log2f(l[r]);
     }
 }
 
@@ -373,17 +299,6 @@ __global__ void __launch_bounds__(kThreads) rope_bwd_dkdv_general_kernel(RopePar
 }
 
 template <typename T, int D>
-int launch_fwd_t(const RopeParams& p, cudaStream_t s) {
-    size_t smem = sizeof(float) * (kRows * D + kTile * (D + 1) + kTile * D);
-    auto kern = rope_fwd_general_kernel<T, D>;
-    static std::atomic<uint64_t> smem_ok;
-    if (int er = allow_smem(kern, smem, smem_ok)) return er;
-    dim3 grid((p.N + kRows - 1) / kRows, p.B * p.H);
-    kern<<<grid, kThreads, smem, s>>>(p); count_launch();
-    return (int)cudaGetLastError();
-}
-
-template <typename T, int D>
 int launch_bwd_t(const RopeParams& p, cudaStream_t s) {
     dim3 grid((p.N + kRows - 1) / kRows, p.B * p.H);
     {
@@ -406,31 +321,22 @@ int launch_bwd_t(const RopeParams& p, cudaStream_t s) {
 }
 
 template <typename T>
-int dispatch_d(const RopeParams& p, cudaStream_t s, bool bwd) {
+int dispatch_d(const RopeParams& p, cudaStream_t s) {
     switch (p.D) {
-        case 32: return bwd ? launch_bwd_t<T, 32>(p, s) : launch_fwd_t<T, 32>(p, s);
-        case 64: return bwd ? launch_bwd_t<T, 64>(p, s) : launch_fwd_t<T, 64>(p, s);
-        case 128: return bwd ? launch_bwd_t<T, 128>(p, s) : launch_fwd_t<T, 128>(p, s);
+        case 32: return launch_bwd_t<T, 32>(p, s);
+        case 64: return launch_bwd_t<T, 64>(p, s);
+        case 128: return launch_bwd_t<T, 128>(p, s);
         default: return COROPE_ERR_BAD_HEAD_DIM;
     }
 }
 
 }  // namespace
 
-int launch_rope_fwd_general(const RopeParams& p, int dtype, cudaStream_t s) {
-    switch (dtype) {
-        case COROPE_DTYPE_F32: return dispatch_d<float>(p, s, false);
-        case COROPE_DTYPE_BF16: return dispatch_d<__nv_bfloat16>(p, s, false);
-        case COROPE_DTYPE_F16: return dispatch_d<__half>(p, s, false);
-        default: return COROPE_ERR_BAD_DTYPE;
-    }
-}
-
+// gradients of 16-bit tensors; delta has been computed
 int launch_rope_bwd_general(const RopeParams& p, int dtype, cudaStream_t s) {
     switch (dtype) {
-        case COROPE_DTYPE_F32: return dispatch_d<float>(p, s, true);
-        case COROPE_DTYPE_BF16: return dispatch_d<__nv_bfloat16>(p, s, true);
-        case COROPE_DTYPE_F16: return dispatch_d<__half>(p, s, true);
+        case COROPE_DTYPE_BF16: return dispatch_d<__nv_bfloat16>(p, s);
+        case COROPE_DTYPE_F16: return dispatch_d<__half>(p, s);
         default: return COROPE_ERR_BAD_DTYPE;
     }
 }
@@ -453,9 +359,6 @@ int launch_rope_delta(const RopeParams& p, int dtype, cudaStream_t s) {
     const int warps = 8;
     unsigned blocks = (unsigned)((rows + warps - 1) / warps);
     switch (dtype) {
-        case COROPE_DTYPE_F32:
-            rope_delta_kernel<float><<<blocks, warps * 32, 0, s>>>((const float*)p.o, (const float*)p.d_o, p.delta, rows, p.D, row_addr(p.so, p.H, p.N), row_addr(p.sdo, p.H, p.N)); count_launch();
-            break;
         case COROPE_DTYPE_BF16:
             rope_delta_kernel<__nv_bfloat16>
                 <<<blocks, warps * 32, 0, s>>>((const __nv_bfloat16*)p.o, (const __nv_bfloat16*)p.d_o, p.delta, rows, p.D, row_addr(p.so, p.H, p.N), row_addr(p.sdo, p.H, p.N)); count_launch();

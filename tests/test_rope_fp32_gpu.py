@@ -1,0 +1,50 @@
+"""The fp32 CUDA-core kernels at the edges of their 32- and 64-row tiles, for each head dimension, grouped heads and rows that
+cannot be moved in vectors; tolerance: the 1e-4 of the other fp32 tests."""
+
+import pytest
+import torch
+
+import oracle
+from helpers import draw, ext, maxdiff, pkg
+
+pytestmark = pytest.mark.gpu
+
+TOL_32 = 1e-4
+
+
+def _run(fn, q, k, v, do, *args):
+    qd, kd, vd = (t.requires_grad_(True) for t in (q, k, v))
+    o = fn(qd, kd, vd, *args)
+    o.backward(do)
+    ext.check_status()
+    return tuple(t.detach().float().cpu() for t in (o, qd.grad, kd.grad, vd.grad))
+
+
+@pytest.mark.parametrize("N", [1, 31, 33, 64, 65, 130])
+@pytest.mark.parametrize("D,causal", [(32, True), (64, False), (64, True), (128, True), (128, False)])
+def test_rope_fp32_at_tile_edges(N, D, causal):
+    q, k, v, do = (draw((1, 2, N, D), 400 + i, torch.float32) for i in range(4))
+    cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
+    s = D ** -0.5
+    outs = _run(pkg.fused_rope_attention, *(t.cuda() for t in (q, k, v, do)), causal, s, cos.cuda(), sin.cuda())
+    refs = (oracle.rope_attn_fwd(q, k, v, causal, s, cos, sin),) + tuple(oracle.rope_attn_bwd(q, k, v, do, causal, s, cos, sin))
+    for a, b in zip(outs, refs):
+        assert maxdiff(a, b) < TOL_32
+
+
+@pytest.mark.parametrize("pad", [0, 1])
+def test_grouped_heads_many_ctas_and_unaligned_rows(pad):
+    # enough 64-row tiles to fill the chip (the 64-row forward CTA), 4 query heads per K / V head, rows of 64 + pad floats
+    B, Hq, Hkv, N, D = 2, 16, 4, 330, 64
+
+    def make(heads, seed):
+        t = draw((B, heads, N, D), seed, torch.float32)
+        buf = torch.zeros((B, heads, N, D + pad), device="cuda")
+        buf[..., :D] = t.cuda()
+        return t, buf[..., :D]
+
+    (q, qv), (do, dov), (k, kv), (v, vv) = make(Hq, 410), make(Hq, 411), make(Hkv, 412), make(Hkv, 413)
+    outs = _run(pkg.flash_attention, qv.detach(), kv.detach(), vv.detach(), dov, True, D ** -0.5)
+    refs = (oracle.attn_gqa_fwd(q, k, v, True, D ** -0.5),) + tuple(oracle.attn_gqa_bwd(q, k, v, do, True, D ** -0.5))
+    for a, b in zip(outs, refs):
+        assert maxdiff(a, b) < TOL_32
