@@ -16,20 +16,18 @@ constexpr size_t kAlign = 256;
 bool head_dim_ok(int D) { return D == 32 || D == 64 || D == 128; }
 
 struct RopeWorkspace {
-    size_t packed_tab, synth_cos, synth_sin, rot, delta, lse_pad, dq_acc, total;
-    bool tc;   // room for the tensor-core kernels
+    size_t packed_tab, synth_cos, synth_sin, rot, delta, dq_acc, total;
+    bool tc;      // room for the tcgen05 kernels
+    bool split;   // room for the split-operand kernels
 };
 
-// Rows per head of the backward's side inputs (LSE, delta): whole 128-row blocks, so that every tile's 64 values start on the
-// 16-byte boundary that bulk copies need.
-int side_pitch_for(int N) { return (N + 127) / 128 * 128; }
-
 // Hq query heads, Hkv K / V heads (equal for the fused-RoPE ops).  `synth`: room for fp32 cos / sin tables [N, D/2] that the
-// entry points taking frequencies instead of tables fill in.  `any_n`: room for the tensor-core kernels whatever N is, not only
+// entry points taking frequencies instead of tables fill in.  `any_n`: room for tensor-core kernels whatever N is, not only
 // for multiples of 128.
 RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth, bool any_n) {
     RopeWorkspace w{};
-    w.tc = rope_tc_supported(D, dtype) && (any_n || N % 128 == 0);
+    w.tc = rope_tc_supported(D, dtype) && N % 128 == 0;
+    w.split = rope_tc_supported(D, dtype) && N % 128 != 0 && any_n;
     const size_t q_elems = (size_t)B * Hq * N * D, kv_elems = (size_t)B * Hkv * N * D;
     size_t off = 0;
     w.packed_tab = off;
@@ -40,14 +38,12 @@ RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int
         w.synth_sin = off;
         off += align_up((size_t)N * (D / 2) * sizeof(float), kAlign);
     }
-    w.rot = off;   // tensor-core kernels: fp16 copy of the rotated K (forward) / rotated and scaled Q (backward)
+    w.rot = off;   // tcgen05 kernels: fp16 copy of the rotated K (forward) / rotated and scaled Q (backward); the other ones: bf16 hi and lo
     if (w.tc) off += align_up((bwd ? q_elems : kv_elems) * 2, kAlign);
+    if (w.split) off += align_up(rope_split_workspace_bytes(bwd, B, Hq, Hkv, N, D), kAlign);
     if (bwd) {
-        const size_t side = align_up((size_t)B * Hq * side_pitch_for(N) * sizeof(float), kAlign);
         w.delta = off;
-        off += side;
-        w.lse_pad = off;
-        if (w.tc && N % 128 != 0) off += side;
+        off += align_up((size_t)B * Hq * N * sizeof(float), kAlign);
         w.dq_acc = off;
         if (w.tc) off += align_up(q_elems * sizeof(float), kAlign);
     }
@@ -311,7 +307,7 @@ bool strides_positive(const Strides& st, int D) { return st.n >= D && st.b >= 0 
 // ops whose kernel family is recorded: the fused-RoPE pair also stands for its variants
 constexpr int kFamFwd = COROPE_OP_ROPE_FWD, kFamBwd = COROPE_OP_ROPE_BWD;
 
-// The workspace layout a call runs with: the one with room for the tensor-core kernels at any N when the caller's workspace has
+// The workspace layout a call runs with: the one with room for the split-operand kernels when the caller's workspace has
 // it (corope_workspace_bytes_any_n), else the one of corope_workspace_bytes.
 int pick_workspace(RopeWorkspace& w, bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth, const void* ws, size_t have) {
     w = rope_workspace_layout(bwd, B, Hq, Hkv, N, D, dtype, synth, true);
@@ -358,8 +354,7 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
     // rows are moved with TMA / 16-byte vectors on the tensor-core paths; otherwise the CUDA-core kernels take over
     const bool vec = vec_ok(q, p.sq) && vec_ok(k, p.sk) && vec_ok(v, p.sv) && vec_ok(o, p.so);
     const int policy = vec ? g_policy.load() : 1;
-    const bool whole = N % 128 == 0;
-    if (w.tc && policy != 1 && (policy == 0 || whole)) {
+    if (w.tc && policy != 1) {
         uint32_t* tab = reinterpret_cast<uint32_t*>((char*)workspace + w.packed_tab);
         TableSource src;
         if (int e = table_source(src, rot, tab, N, D, s)) return e;
@@ -373,11 +368,13 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
         } else if (!src.packed) {
             if (int e = launch_pack_tables(src, tab, N, D / 2, s)) return e;
         }
-        g_last_family[kFamFwd] = whole ? 1 : 0;
+        g_last_family[kFamFwd] = 1;
         return launch_rope_fwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
     g_last_family[kFamFwd] = 0;
+    // ragged N, rows that can be moved in 16-byte vectors: split operands at fp32 accuracy (rope_split.cu has both sides' figures)
+    if (w.split && policy == 0) return launch_rope_fwd_split(p, (char*)workspace + w.rot, dtype, s);
     return launch_rope_fwd_general(p, dtype, s);
 }
 
@@ -403,16 +400,13 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
     const bool vec = vec_ok(q, p.sq) && vec_ok(k, p.sk) && vec_ok(v, p.sv) && vec_ok(o, p.so) && vec_ok(d_o, p.sdo) && vec_ok(dq, p.sdq) &&
                      vec_ok(dk, p.sdk) && vec_ok(dv, p.sdv);
     const int policy = vec ? g_policy.load() : 1;
-    const bool whole = N % 128 == 0;
-    if (w.tc && policy != 1 && (policy == 0 || whole)) {
+    if (w.tc && policy != 1) {
         uint32_t* tab = reinterpret_cast<uint32_t*>((char*)workspace + w.packed_tab);
         TableSource src;
         if (int e = table_source(src, rot, tab, N, D, s)) return e;
         p.packed_tab = tab;
         p.sched_counter = reinterpret_cast<int*>(tab + (size_t)N * (D / 2));   // zeroed with the table
         p.dq_acc = reinterpret_cast<float*>((char*)workspace + w.dq_acc);
-        p.side_pitch = side_pitch_for(N);
-        p.lse_pad = whole ? lse2 : reinterpret_cast<const float*>((char*)workspace + w.lse_pad);
         if (policy == 0) {
             p.q_rot = (char*)workspace + w.rot;
             if (int e = launch_rope_bwd_prepass(p, src, tab, dtype, s)) return e;   // table, delta, rotated Q, cleared dQ accumulator
@@ -422,13 +416,14 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
             if (!src.packed)
                 if (int e = launch_pack_tables(src, tab, N, D / 2, s)) return e;
         }
-        g_last_family[kFamBwd] = whole ? 1 : 0;
+        g_last_family[kFamBwd] = 1;
         return launch_rope_bwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
     g_last_family[kFamBwd] = 0;
     if (dtype == COROPE_DTYPE_F32) return launch_rope_bwd_fp32(p, s);
     if (int e = launch_rope_delta(p, dtype, s)) return e;
+    if (w.split && policy == 0) return launch_rope_bwd_split(p, (char*)workspace + w.rot, dtype, s);
     return launch_rope_bwd_general(p, dtype, s);
 }
 

@@ -96,8 +96,6 @@ struct RopeParams {
     const float* cos;
     const float* sin;
     int64_t table_stride;
-    const float* lse_pad;   // tensor-core backward: LSE with row pitch `side_pitch` (the caller's lse2, or a padded copy for ragged N)
-    int side_pitch;         // rows per head of lse_pad and delta in the tensor-core backward: N, or N rounded up to 128
     const uint32_t* packed_tab;  // [N, D/2] (cos, sin) pairs in 16-bit fixed point, built per call in the workspace
     int B, H, N, D;     // H = number of query heads
     int Hkv;            // number of K / V heads (H % Hkv == 0; query head h reads KV head h / (H / Hkv)); equals H for the fused-RoPE ops
@@ -264,11 +262,6 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y, const void* smem_src) {
     asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map),
                  "r"(smem_u32(smem_src)), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, int x, int y, int z, const void* smem_src) {
-    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
-                 "r"(smem_u32(smem_src)), "r"(x), "r"(y), "r"(z)
                  : "memory");
 }
 __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
@@ -598,16 +591,16 @@ inline TensorMapEncodeFn tensor_map_encoder() {
     return fn;
 }
 
-// A row-major fp32 tensor [rows, cols] (slices == 0) or [slices, rows, cols] without swizzle (box_cols * 4 bytes a multiple of 16,
-// box_cols <= 256): bulk reduce-add of dense shared-memory tiles; rows of a box beyond `rows` are clipped.
-inline int encode_tensor_map_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t slices, uint32_t box_rows, uint32_t box_cols) {
+// A row-major fp32 tensor [rows, cols] without swizzle (box_cols * 4 bytes a multiple of 16, box_cols <= 256): bulk reduce-add of
+// dense shared-memory tiles.
+inline int encode_tensor_map_f32(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint32_t box_rows, uint32_t box_cols) {
     const TensorMapEncodeFn fn = tensor_map_encoder();
     if (!fn) return COROPE_ERR_NO_DEVICE;
-    cuuint64_t gdim[3] = {cols, rows, slices};
-    cuuint64_t gstride[2] = {cols * 4, rows * cols * 4};
-    cuuint32_t box[3] = {box_cols, box_rows, 1};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, slices ? 3 : 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint64_t gdim[2] = {cols, rows};
+    cuuint64_t gstride[1] = {cols * 4};
+    cuuint32_t box[2] = {box_cols, box_rows};
+    cuuint32_t estr[2] = {1, 1};
+    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                     CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : COROPE_ERR_TENSOR_MAP;
 }
@@ -656,10 +649,15 @@ int launch_synth_tables(const float* inv_freq, float theta, float* cos_out, floa
 int launch_synth_packed(const float* inv_freq, float theta, uint32_t* packed, int N, int half_d, cudaStream_t s);
 // forward: packed table (unless src.packed) and the rotated fp16 copy of K into p.k_rot
 int launch_rope_fwd_prepass(const RopeParams& p, const TableSource& src, uint32_t* packed, int dtype, cudaStream_t s);
-// backward: packed table (unless src.packed), delta, the rotated fp16 copy of Q (scaled by sm_scale * log2e) into p.q_rot, a zeroed
-// p.dq_acc and, for ragged N, the padded LSE copy into p.lse_pad
+// backward: packed table (unless src.packed), delta, the rotated fp16 copy of Q (scaled by sm_scale * log2e) into p.q_rot and a zeroed
+// p.dq_acc
 int launch_rope_bwd_prepass(const RopeParams& p, const TableSource& src, uint32_t* packed, int dtype, cudaStream_t s);
 bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types, D = 64 or 128
+// 16-bit tensors at any N, D = 64 or 128, 16-byte aligned rows: split operands, `ws` of rope_split_workspace_bytes; backward with
+// delta computed before
+size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D);
+int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
+int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
 int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 int launch_rope_bwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 bool gqa_fwd_mma_supported(int N, int D, int dtype);
@@ -701,11 +699,10 @@ inline int encode_tensor_map_4d_sw128(CUtensorMap* out, const void* base, uint64
     return r == CUDA_SUCCESS ? 0 : COROPE_ERR_TENSOR_MAP;
 }
 
-// 2-D map when the rows collapse, else 4-D; `flat` tells the kernel which coordinates to use.  A ragged N (last tile of a head
-// only partly filled) always takes the 4-D form, whose rows beyond N read as zeros instead of the next head's rows.
+// 2-D map when the rows collapse, else 4-D; `flat` tells the kernel which coordinates to use.
 inline int encode_rows_map(CUtensorMap* out, bool* flat, const void* base, int B, int H, int N, int D, const Strides& st, uint32_t box_rows,
                            uint32_t box_cols, int dtype) {
-    *flat = rows_collapse(st, H, N) && N % 128 == 0;
+    *flat = rows_collapse(st, H, N);
     if (*flat) return encode_tensor_map_2d_sw128(out, base, (uint64_t)B * H * N, D, box_rows, box_cols, dtype, (uint64_t)st.n);
     return encode_tensor_map_4d_sw128(out, base, B, H, N, D, st, box_rows, box_cols, dtype);
 }

@@ -59,7 +59,7 @@ extern "C" int corope_rope_attn_fwd_noalloc(const void* q, const void* k, const 
     p.sq = p.sk = p.sv = p.so = contiguous_strides(H, N, D);
     // the kernel-selection policy of the diagnostics header applies here too: 1 = general kernels; 0 and 2 both mean the
     // tensor-core kernel with its in-kernel K rotation (this entry point has no room for a rotated copy)
-    if (kernel_policy() != 1 && rope_tc_supported(D, dtype) && ((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0 &&
+    if (kernel_policy() != 1 && rope_tc_supported(D, dtype) && D == 128 && N % 128 == 0 && ((uintptr_t)q % 16) == 0 && ((uintptr_t)k % 16) == 0 && ((uintptr_t)v % 16) == 0 &&
         ((uintptr_t)o % 16) == 0) {
         uint32_t* table = nullptr;
         if (int e = scratch_on_current_device(&table)) return e;
@@ -69,7 +69,7 @@ extern "C" int corope_rope_attn_fwd_noalloc(const void* q, const void* k, const 
         if (int e = launch_pack_tables(src, table, N, D / 2, s)) return e;
         p.packed_tab = table;
         p.sched_counter = reinterpret_cast<int*>(table + (size_t)N * (D / 2));
-        note_kernel_family(COROPE_OP_ROPE_FWD, N % 128 == 0 ? 1 : 0);
+        note_kernel_family(COROPE_OP_ROPE_FWD, 1);
         return launch_rope_fwd_tc(p, dtype, s);
     }
     note_kernel_family(COROPE_OP_ROPE_FWD, 0);

@@ -1,6 +1,6 @@
 // Fused-RoPE flash-attention backward (causal or full) for sm_100a: TMA -> shared memory -> in-place rotation of K
 // (once) and of every Q tile -> five tcgen05 MMAs per (K block, Q tile) pair with TMEM accumulators.
-// 16-bit inputs, D = 64 or 128, any N.
+// 16-bit inputs, D = 64 or 128, N % 128 == 0.
 //
 // Work unit = one K/V block of 128 keys of one (batch, head): the CTA sweeps the query tiles (64 rows each) at or
 // below the block's diagonal.  CTAs are persistent (one per SM) and take units from a global counter, the first unit
@@ -134,19 +134,15 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int G = kPlain ? 1 : p.H / p.Hkv;   // query heads per K / V head (1 for the fused-RoPE ops)
     const bool flat_q = kPlain || p.flat_q, flat_do = kPlain || p.flat_do, flat_k = kPlain || p.flat_k, flat_v = kPlain || p.flat_v;
     const int BH = p.B * p.Hkv;           // units are taken per K / V head; a unit sweeps the query tiles of all G heads of its group
-    const int n_kb = (N + kBK - 1) / kBK;
+    const int n_kb = N / kBK;
     const int n_units = BH * n_kb;
     const bool causal = p.causal != 0;
     // per unit (jb, bh): first query row visited q_first = causal ? jb * kBK : 0 (causal: the block's own diagonal),
-    // spg = (n_pad - q_first) / kBQ steps per query head (even, so n_steps >= 2) and n_steps = G * spg.  For N not a multiple of
-    // 128 the last block of keys and the last steps reach past the head: Q, dO, K and V rows there read as zeros (4-D maps), the
-    // LSE copy holds +inf for them (P = 0, so such a query adds nothing), and a key at or beyond N has P = 0 by the causal mask
-    // for every query inside the head, by an explicit mask otherwise.  Step s works on query head bh * G + s / spg, rows q_first + (s % spg) * kBQ .. + kBQ - 1.
+    // spg = (N - q_first) / kBQ steps per query head (even, so n_steps >= 2) and n_steps = G * spg.  Step s works on query head bh * G + s / spg, rows q_first + (s % spg) * kBQ .. + kBQ - 1.
     // (no division when every K / V head has a single query head: then s < spg)
     auto step_head = [&](int spg, int s) { return G == 1 ? 0 : s / spg; };
     auto step_q0 = [&](int q_first, int spg, int s) { return q_first + (G == 1 ? s : s % spg) * kBQ; };
     auto step_row = [&](int bh, int q_first, int spg, int s) { return (bh * G + step_head(spg, s)) * N + step_q0(q_first, spg, s); };
-    const int n_pad = n_kb * kBK;         // N rounded up to whole blocks (= N for kPlain)
 
     if (reinterpret_cast<uintptr_t>(sm) - reinterpret_cast<uintptr_t>(smem_raw) > kSmemSlack) {   // base less aligned than assumed
         if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, COROPE_DEV_WAIT_EXPIRED | 0xfff);
@@ -212,12 +208,11 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 if (w < 0) break;
                 const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
                 const int q_first = causal ? un.jb * kBK : 0;
-                const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
+                const int spg = (N - q_first) / kBQ, n_steps = G * spg;
                 auto load_step = [&](int s) -> bool {
                     const int gs = g + s, st = gs % kStages;
                     if (gs >= kStages && !mbar_wait(&bars[QDO_EMPTY + st], ((gs / kStages) - 1) & 1, p.status, QDO_EMPTY, abort_flag)) return false;
-                    const int qr = step_row(un.bh, q_first, spg, s);   // flat row of Q, dO
-                    const int sr = kPlain ? qr : (un.bh * G + step_head(spg, s)) * p.side_pitch + step_q0(q_first, spg, s);   // of the side inputs (LSE, delta)
+                    const int qr = step_row(un.bh, q_first, spg, s);   // flat row of Q, dO, LSE, delta
                     mbar_arrive_expect_tx(&bars[QDO_FULL + st], 2 * kQBytes + 2 * kBQ * (uint32_t)sizeof(float));
                     if (flat_q) {
                         tma_load_2d(sQ + st * kQBytes, &mapQ, 0, qr, &bars[QDO_FULL + st]);
@@ -239,8 +234,8 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                             if (kD == 128) tma_load_4d(sDO + st * kQBytes + kQBox, &mapDO, 64, q0, qh, qb, &bars[QDO_FULL + st]);
                         }
                     }
-                    bulk_load_1d(sLD + st * 2 * kBQ, p.lse_pad + sr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
-                    bulk_load_1d(sLD + st * 2 * kBQ + kBQ, p.delta + sr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
+                    bulk_load_1d(sLD + st * 2 * kBQ, p.lse2 + qr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
+                    bulk_load_1d(sLD + st * 2 * kBQ + kBQ, p.delta + qr, kBQ * sizeof(float), &bars[QDO_FULL + st]);
                     return true;
                 };
                 // the first two Q / dO tiles only need ring stages, which the last steps of the previous unit free: ask
@@ -321,7 +316,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 const int w = fetch_unit(bars, unit_ring, n, lane, p.status, abort_flag);
                 if (w < 0) break;
                 const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
-                const int n_steps = G * ((n_pad - (causal ? un.jb * kBK : 0)) / kBQ);
+                const int n_steps = G * ((N - (causal ? un.jb * kBK : 0)) / kBQ);
                 {
                     const int st0 = g % kStages, b0 = g & 1;
                     ok = mbar_wait_warp(&bars[K_ROT], n & 1, p.status, K_ROT, abort_flag) && mbar_wait_warp(&bars[V_FULL], n & 1, p.status, V_FULL, abort_flag) &&
@@ -381,7 +376,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (w < 0) break;
             const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
             const int q_first = causal ? un.jb * kBK : 0;
-            const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
+            const int spg = (N - q_first) / kBQ, n_steps = G * spg;
             {
                 TabRegs<kBQ, kD> trk;
                 load_table_regs(trk, p.packed_tab, un.jb * kBK + rg * kBQ, N, tid);
@@ -418,9 +413,8 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
         const int jb = un.jb;
         const int q_first = causal ? jb * kBK : 0;
-        const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
+        const int spg = (N - q_first) / kBQ, n_steps = G * spg;
         const int key = jb * kBK + row;
-        const bool key_out = !kPlain && key >= N;   // beyond the head: masked (full attention), not stored
         for (int s = 0; s < n_steps; ++s) {
             const int gs = g + s, u = gs >> 1, st = gs % kStages, b = gs & 1;
             const uint32_t tS = tmem + lane_base + TS0 + b * 64;
@@ -448,8 +442,8 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                     const float2 d2 = *reinterpret_cast<const float2*>(dlt + c0);
                     float p0 = fast_exp2(__uint_as_float(rs[2 * i]) - l2.x);
                     float p1 = fast_exp2(__uint_as_float(rs[2 * i + 1]) - l2.y);
-                    if ((diag && key > q0 + c0) || key_out) p0 = 0.f;
-                    if ((diag && key > q0 + c0 + 1) || key_out) p1 = 0.f;
+                    if (diag && key > q0 + c0) p0 = 0.f;
+                    if (diag && key > q0 + c0 + 1) p1 = 0.f;
                     const float s0 = p0 * (__uint_as_float(rd[2 * i]) - d2.x);
                     const float s1 = p1 * (__uint_as_float(rd[2 * i + 1]) - d2.y);
                     pp[i] = pack2<T>(p0, p1);
@@ -483,14 +477,12 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
 #pragma unroll
                     for (int i = 0; i < 16; ++i) pk[i] = pack2<T>(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
                     uint4* d4 = reinterpret_cast<uint4*>(dst + c * 32);
-                    if (!key_out) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) d4[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
-                    }
+                    for (int i = 0; i < 4; ++i) d4[i] = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
                 }
             } else {
                 T* dst = reinterpret_cast<T*>(p.dk) + (kPlain ? ((int64_t)un.bh * N + key) * p.sdk.n : row_offset(p.sdk, p.Hkv, un.bh, key));
-                const uint32_t* tab = p.packed_tab + (size_t)(kPlain ? key : min(key, N - 1)) * (kD / 2);
+                const uint32_t* tab = p.packed_tab + (size_t)key * (kD / 2);
 #pragma unroll
                 for (int c = 0; c < kD / 64; ++c) {
                     uint32_t r1[32], r2[32];
@@ -509,12 +501,10 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                     }
                     uint4* d1 = reinterpret_cast<uint4*>(dst + c * 32);
                     uint4* d2 = reinterpret_cast<uint4*>(dst + kD / 2 + c * 32);
-                    if (!key_out) {
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            d1[i] = make_uint4(o1[4 * i], o1[4 * i + 1], o1[4 * i + 2], o1[4 * i + 3]);
-                            d2[i] = make_uint4(o2[4 * i], o2[4 * i + 1], o2[4 * i + 2], o2[4 * i + 3]);
-                        }
+                    for (int i = 0; i < 4; ++i) {
+                        d1[i] = make_uint4(o1[4 * i], o1[4 * i + 1], o1[4 * i + 2], o1[4 * i + 3]);
+                        d2[i] = make_uint4(o2[4 * i], o2[4 * i + 1], o2[4 * i + 2], o2[4 * i + 3]);
                     }
                 }
             }
@@ -538,7 +528,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (w < 0) break;
         const Unit un = unit_of(w, n_kb, BH, p.head_chunk);
         const int q_first = causal ? un.jb * kBK : 0;
-        const int spg = (n_pad - q_first) / kBQ, n_steps = G * spg;
+        const int spg = (N - q_first) / kBQ, n_steps = G * spg;
         for (int s = 0; s < n_steps; ++s) {
             const int gs = g + s, b = gs & 1;
             if (!(ok = mbar_wait_warp(&bars[DQ_DONE + b], (gs >> 1) & 1, p.status, DQ_DONE + b, abort_flag))) break;
@@ -564,9 +554,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             fence_proxy_async();
             named_bar_sync(1, 128);
             if (threadIdx.x == kDrainWarp0 * 32) {
-                const int q0 = step_q0(q_first, spg, s);
-                if (kPlain) tma_reduce_add_2d(&mapDQ, 0, step_row(un.bh, q_first, spg, s), sDQ);
-                else if (q0 < N) tma_reduce_add_3d(&mapDQ, 0, q0, un.bh * G + step_head(spg, s), sDQ);   // rows beyond the head are clipped
+                tma_reduce_add_2d(&mapDQ, 0, step_row(un.bh, q_first, spg, s), sDQ);
                 bulk_commit_group();
             }
         }
@@ -627,14 +615,13 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     cudaError_t e = p.dq_acc_zeroed ? cudaSuccess : cudaMemsetAsync(p.dq_acc, 0, rows * kD * sizeof(float), s);
     if (e != cudaSuccess) return (int)e;
     const bool plain = p.H == p.Hkv && fq && fdo && fk && fv && rows_collapse(p.sdk, p.Hkv, p.N) && rows_collapse(p.sdv, p.Hkv, p.N);
-    // the dQ accumulator as rows of all heads, or (3-D) head by head so that a last, partly filled tile ends with its head
-    if (int er = encode_tensor_map_f32(&mdq, p.dq_acc, plain ? rows : (uint64_t)p.N, kD, plain ? 0 : (uint64_t)p.B * p.H, kBQ, kD)) return er;
+    if (int er = encode_tensor_map_f32(&mdq, p.dq_acc, rows, kD, kBQ, kD)) return er;
     auto kern = plain ? rope_bwd_sm100_kernel<T, true, kD> : rope_bwd_sm100_kernel<T, false, kD>;
     constexpr size_t kSmemBytes = smem_bytes(kD);
     static std::atomic<uint64_t> smem_ok[2];
     if (int er = allow_smem(kern, kSmemBytes, smem_ok[plain])) return er;
     const int sms = sm_count();
-    const unsigned units = (unsigned)(((p.N + kBK - 1) / kBK) * p.B * p.Hkv);
+    const unsigned units = (unsigned)((p.N / kBK) * p.B * p.Hkv);
     const unsigned grid = units < (unsigned)sms ? units : (unsigned)sms;   // persistent: one CTA per SM
     kern<<<grid, kThreads, kSmemBytes, s>>>(mq, mk, mv, mdo, mdq, pp); count_launch();
     e = cudaGetLastError();

@@ -1,5 +1,5 @@
 // Fused-RoPE flash-attention forward (causal or full) for sm_100a: TMA -> shared memory -> in-place rotation ->
-// tcgen05 MMAs with TMEM accumulators -> online softmax in registers.  16-bit inputs, D = 64 or 128, any N.
+// tcgen05 MMAs with TMEM accumulators -> online softmax in registers.  16-bit inputs, D = 64 or 128, N % 128 == 0.
 //
 // A work item is 256 consecutive query rows (two 128-row tiles, "Q0" and "Q1") of one (batch, head) with the K/V
 // tiles 0 .. 2t+1 they can see.  CTAs are persistent (one per SM) and take items from a global counter, heaviest
@@ -140,15 +140,14 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int BH = p.B * p.H;
     const int G = kPlain ? 1 : p.H / p.Hkv;   // query heads per K / V head (1 for the fused-RoPE ops); query head bh reads KV head bh / G
     const bool flat_q = kPlain || p.flat_q, flat_k = kPlain || p.flat_k, flat_v = kPlain || p.flat_v;
-    // When N is not a multiple of 256 the last item of a head reaches past it: its Q1 tile (and, causal, the K tile behind the
-    // diagonal) may lie beyond the head, and for N not a multiple of 128 its last tile is partly filled.  TMA fetches the next
-    // head's rows there (2-D maps, whole tiles only) or zeros (4-D maps and behind the tensor); rows at or beyond N are not
-    // stored, and keys at or beyond N are masked: by the causal mask for every row that is stored, explicitly otherwise.
+    // N is a multiple of 128: when it is not a multiple of 256 the last item of a head has only Q0; its Q1 tile (and, causal,
+    // the K tile behind the diagonal) lies beyond the head -- TMA fetches the next head's rows there (2-D maps) or zeros (4-D
+    // maps and behind the tensor); the results are finite and are not stored
     const int n_qt = (N + 2 * kBM - 1) / (2 * kBM);
     const int n_items = n_qt * BH;
     // K tiles an item sees: up to its diagonal (causal: Q0 one tile less than Q1), or all of them
     const bool causal = p.causal != 0;
-    const int nk_all = (N + kBN - 1) / kBN;   // full attention: every tile that starts inside the head
+    const int nk_all = N / kBN;   // full attention: every tile of the head
     // Persistent CTAs with a dynamic schedule: the first item of CTA c is c, further ones come from a global counter
     // (heavy items first, so the greedy order balances to a few percent; a static round-robin was 19 % off).  The K
     // producer fetches an item, publishes it in a small shared-memory ring and every other role reads it from there.
@@ -418,9 +417,8 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                 COROPE_TMEM_LD32(tS, s0);
                 COROPE_TMEM_LD32(tS + 32, s1);
                 tmem_wait_ld();
-                if (diag || (!kPlain && !causal && (j + 1) * kBN > N)) {
-                    // causal mask on the diagonal tile (key column > query row); full attention: keys beyond the head
-                    const int last = (diag ? row : N - 1 - j * kBN) - half * 64;
+                if (diag) {   // causal mask on the diagonal tile: key column > query row
+                    const int last = row - half * 64;
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
                         if (i > last) s0[i] = 0xff800000u;
@@ -500,7 +498,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             if (!(ok = mbar_wait_warp(&bars[O_FULL + wg], (gs - 1) & 1, p.status, O_FULL + wg, abort_flag))) break;
             tc_fence_after();
             const float inv = 1.f / l_tot;
-            const bool in_head = (2 * wi.t + wg) * kBM + (kPlain ? 0 : row) < N;   // false for rows of a head's last item beyond the head
+            const bool in_head = (2 * wi.t + wg) * kBM < N;   // false for the Q1 tile of a head's last, half-empty item
             const size_t grow = (size_t)wi.bh * N + (size_t)(2 * wi.t + wg) * kBM + row;   // row of the (contiguous) LSE
             T* orow = reinterpret_cast<T*>(p.out_o) + half * (kD / 2) +
                       (kPlain ? (int64_t)grow * p.so.n : row_offset(p.so, p.H, wi.bh, (2 * wi.t + wg) * kBM + row));

@@ -1,6 +1,5 @@
 // Passes over the inputs that the tensor-core fused-RoPE kernels need before they run: the packed (cos, sin) table, the rotated
-// fp16 copy of K (forward) or of Q (backward), and for the backward delta = rowsum(O * dO), a cleared fp32 dQ accumulator and,
-// for ragged N, an LSE copy whose heads start on 128-row boundaries.
+// fp16 copy of K (forward) or of Q (backward), and for the backward delta = rowsum(O * dO) and a cleared fp32 dQ accumulator.
 //
 // Rotating once here instead of once per consumer (a K tile is consumed by up to N/256 forward items, a Q tile by every key
 // block at or below its diagonal) takes the rotation out of the main kernels' inner loops.  All of it is bound by HBM.
@@ -99,12 +98,12 @@ __global__ void __launch_bounds__(kThreads) rope_fwd_prepass_kernel(const T* __r
 }
 
 // Backward: D / 8 threads per row; each takes 8 elements of O . dO and 32 bytes of the accumulator row, the lower half of them
-// also 8 pairs of Q.  Positions run over n_pad rows per head; the ones beyond N only exist in the side inputs.
+// also 8 pairs of Q.  
 template <typename T, int D, int MODE>
 __global__ void __launch_bounds__(kThreads) rope_bwd_prepass_kernel(const T* __restrict__ q, const T* __restrict__ o, const T* __restrict__ d_o,
-                                                                    PrepassTable tab, const float* __restrict__ lse2, float* __restrict__ lse_pad,
+                                                                    PrepassTable tab,
                                                                     __half* __restrict__ q_rot, float* __restrict__ delta, float* __restrict__ dq_acc,
-                                                                    int N, int n_pad, int BH, int heads_per_block, float scale, RowAddr aq,
+                                                                    int N, int BH, int heads_per_block, float scale, RowAddr aq,
                                                                     RowAddr ao, RowAddr ado) {
     constexpr int kPerRow = D / 8, kRows = kThreads / kPerRow, kUnroll = 2;
     const int n = blockIdx.x * kRows + threadIdx.x / kPerRow;
@@ -163,11 +162,7 @@ __global__ void __launch_bounds__(kThreads) rope_bwd_prepass_kernel(const T* __r
                 z[0] = make_uint4(0u, 0u, 0u, 0u);
                 z[1] = make_uint4(0u, 0u, 0u, 0u);
             }
-            if (part == 0 && n < n_pad) {
-                const size_t side = (size_t)(h + u) * n_pad + n;
-                delta[side] = s;                                                // 0 beyond the head
-                if (lse_pad != nullptr) lse_pad[side] = live ? lse2[row] : INFINITY;   // P = exp2(S - inf) = 0 there
-            }
+            if (live && part == 0) delta[row] = s;
         }
     }
 }
@@ -241,11 +236,10 @@ int fwd_prepass_t(const RopeParams& p, const PrepassTable& tab, cudaStream_t s) 
 template <typename T, int D, int MODE>
 int bwd_prepass_t(const RopeParams& p, const PrepassTable& tab, cudaStream_t s) {
     constexpr int kRows = kThreads / (D / 8);
-    const int BH = p.B * p.H, pb = (p.side_pitch + kRows - 1) / kRows, hpb = heads_per_block_for(pb, BH);
+    const int BH = p.B * p.H, pb = (p.N + kRows - 1) / kRows, hpb = heads_per_block_for(pb, BH);
     const dim3 grid(pb, (BH + hpb - 1) / hpb);
-    float* lse_pad = p.lse_pad != p.lse2 ? const_cast<float*>(p.lse_pad) : nullptr;
-    rope_bwd_prepass_kernel<T, D, MODE><<<grid, kThreads, 0, s>>>((const T*)p.q, (const T*)p.o, (const T*)p.d_o, tab, p.lse2, lse_pad,
-                                                                  (__half*)const_cast<void*>(p.q_rot), p.delta, p.dq_acc, p.N, p.side_pitch, BH, hpb,
+    rope_bwd_prepass_kernel<T, D, MODE><<<grid, kThreads, 0, s>>>((const T*)p.q, (const T*)p.o, (const T*)p.d_o, tab,
+                                                                  (__half*)const_cast<void*>(p.q_rot), p.delta, p.dq_acc, p.N, BH, hpb,
                                                                   p.sm_scale * kLog2e, row_addr(p.sq, p.H, p.N), row_addr(p.so, p.H, p.N),
                                                                   row_addr(p.sdo, p.H, p.N));
     count_launch();

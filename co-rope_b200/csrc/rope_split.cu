@@ -1,0 +1,529 @@
+// Fused-RoPE / plain attention for 16-bit tensors at lengths that are not whole 128-row tiles, D = 64 or 128: tensor-core products
+// (mma.sync m16n8k16) with fp32 precision kept by splitting.  Every fp32 operand x enters the MMAs as hi + lo, hi = x rounded to 16
+// bits and lo = (x - hi) rounded:
+//     S  = Q~ K~^T        Q~, K~ rotated in fp32, both split into bf16 pairs    3 MMAs (hi hi, hi lo, lo hi; lo lo is below 2^-17)
+//     dP = dO V^T         inputs as they are                                    1 MMA
+//     O += P V, dV += P^T dO     P split into the inputs' own type              2 MMAs
+//     dQ += dS K~, dK += dS^T Q~  dS split into bf16                            3 MMAs
+// bf16 for everything that is not bounded, so that no magnitude of the inputs leaves the range.  These lengths have always run with
+// fp32 operands and keep that accuracy (2-norm error against 64-bit arithmetic, N(0, 1) inputs, B1 H4 N1777 D128 causal, f16:
+// O 2.008e-4 and dV 2.04e-4, dQ and dK 2.25e-4, all of it the rounding of the results, to the third digit what the CUDA-core kernels
+// show; the tcgen05 kernels with their 16-bit P and Q~, K~: 3.6e-4, 3.9e-4, 4.7e-4).  The pairs carry 16 bits: scores of some
+// hundred would begin to show in f16 results.
+//
+// B1 H32 N1777 D128 bf16 causal forward 222 us (116 TFLOP/s; the CUDA-core kernel 909 us), B4 H16 N1000 D64 bf16 full forward +
+// backward 613 us (94 TFLOP/s; 3473 us).
+// What bounds it: the tensor pipe (mma.sync) and, next to it, the shared-memory port: a warp's 16 rows read every streamed tile,
+// hi and lo, once per product.  tcgen05 would need the split tiles of all operands resident (Q~ hi / lo, K~ hi / lo, V of 128 x 128:
+// 160 KB before any ring), so one stage of everything and no overlap.
+//
+// Math: fused-rope/rope_attn_pytorch.py:108-155 (forward), :187-222 (backward); exp2-domain softmax and log2-domain LSE as
+// fused-rope/fused_rope_attn.py:103-114, 316.
+#include "common.cuh"
+
+namespace corope {
+namespace {
+
+constexpr int kThreads = 128;   // 4 warps of 16 rows
+constexpr int kRows = 64;       // rows a CTA owns
+
+// ------------------------------------------------------------------------------------------------ operands
+// row-major 16-bit tile in shared memory: rows of D elements + 16 bytes, so that 8 consecutive rows of an ldmatrix fall into
+// distinct bank groups
+template <int D> struct Pitch { static constexpr int kBytes = 2 * D + 16; };
+
+__device__ __forceinline__ void ldm_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldm_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+// byte offsets of a lane's ldmatrix row inside a tile.  A operand (16 rows x 16 k): registers a0..a3.  B operand from a tile with
+// k contiguous: (b0, b1) of columns 0-7, then of columns 8-15.  B operand from a tile with the columns contiguous (.trans): the same.
+template <int D> __device__ __forceinline__ uint32_t lane_a(int lane) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * Pitch<D>::kBytes + (lane >> 4) * 16; }
+template <int D> __device__ __forceinline__ uint32_t lane_b(int lane) { return ((lane & 7) + (lane >> 4) * 8) * Pitch<D>::kBytes + ((lane >> 3) & 1) * 16; }
+template <int D> __device__ __forceinline__ uint32_t lane_bt(int lane) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * Pitch<D>::kBytes + (lane >> 4) * 16; }
+
+template <typename T> __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
+template <> __device__ __forceinline__ void mma<__nv_bfloat16>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <> __device__ __forceinline__ void mma<__half>(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// d += (ah + al) (bh + bl) without the product of the two small halves
+__device__ __forceinline__ void mma_split(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], uint32_t bh0, uint32_t bh1, uint32_t bl0,
+                                          uint32_t bl1) {
+    mma<__nv_bfloat16>(d, ah, bh0, bh1);
+    mma<__nv_bfloat16>(d, ah, bl0, bl1);
+    mma<__nv_bfloat16>(d, al, bh0, bh1);
+}
+template <typename T>
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    hi = pack2<T>(a, b);
+    const float2 f = unpack2<T>(hi);
+    lo = pack2<T>(a - f.x, b - f.y);
+}
+// two neighbouring 8-column accumulator tiles as the A operand of one k-step, split
+template <typename T>
+__device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[4], float scale, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
+    split2<T>(c0[0] * scale, c0[1] * scale, hi[0], lo[0]);
+    split2<T>(c0[2] * scale, c0[3] * scale, hi[1], lo[1]);
+    split2<T>(c1[0] * scale, c1[1] * scale, hi[2], lo[2]);
+    split2<T>(c1[2] * scale, c1[3] * scale, hi[3], lo[3]);
+}
+
+// 16 bytes global -> shared, zeros when `have` is false (the address is then not read)
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool have) {
+    const int bytes = have ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
+
+// ROWS rows [r0, r0 + ROWS) of X (row stride xs elements) into a padded tile, rows at or beyond N as zeros
+template <int D, int ROWS, typename E>
+__device__ __forceinline__ void load_rows(uint32_t dst, const E* X, int64_t xs, int r0, int N) {
+    constexpr int kPerRow = D / 8;
+#pragma unroll
+    for (int it = 0; it < ROWS * kPerRow / kThreads; ++it) {
+        const int idx = threadIdx.x + it * kThreads, r = idx / kPerRow, ch = idx % kPerRow, pos = r0 + r;
+        const bool have = pos < N;
+        cp16(dst + r * Pitch<D>::kBytes + ch * 16, X + (int64_t)(have ? pos : 0) * xs + ch * 8, have);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// pre-pass: rows of X rotated in fp32, times `scale`, as bf16 hi and lo copies [B, H, N, D].  One thread per 8 pairs.
+// ------------------------------------------------------------------------------------------------
+template <typename T, int D>
+__global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__ X, RowAddr ax, const float* __restrict__ cosT, const float* __restrict__ sinT,
+                                                           int64_t ts, float scale, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, size_t rows) {
+    constexpr int kPerRow = D / 16;
+    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t row = idx / kPerRow;
+    if (row >= rows) return;
+    const int d = (int)(idx % kPerRow) * 8, n = (int)(row % (size_t)ax.N);
+    const T* src = X + flat_row_offset(ax, row) + d;
+    const uint4 xa = *reinterpret_cast<const uint4*>(src), xb = *reinterpret_cast<const uint4*>(src + D / 2);
+    const uint32_t a[4] = {xa.x, xa.y, xa.z, xa.w}, b[4] = {xb.x, xb.y, xb.z, xb.w};
+    uint32_t ha[4], la[4], hb[4], lb[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
+        float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
+        if (cosT != nullptr) {   // null tables: plain attention
+            const float *c = cosT + (int64_t)n * ts + d + 2 * e, *s = sinT + (int64_t)n * ts + d + 2 * e;
+            c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
+        }
+        split2<__nv_bfloat16>((fa.x * c0 - fb.x * s0) * scale, (fa.y * c1 - fb.y * s1) * scale, ha[e], la[e]);
+        split2<__nv_bfloat16>((fb.x * c0 + fa.x * s0) * scale, (fb.y * c1 + fa.y * s1) * scale, hb[e], lb[e]);
+    }
+    __nv_bfloat16 *h = hi + row * D + d, *l = lo + row * D + d;
+    *reinterpret_cast<uint4*>(h) = make_uint4(ha[0], ha[1], ha[2], ha[3]);
+    *reinterpret_cast<uint4*>(h + D / 2) = make_uint4(hb[0], hb[1], hb[2], hb[3]);
+    *reinterpret_cast<uint4*>(l) = make_uint4(la[0], la[1], la[2], la[3]);
+    *reinterpret_cast<uint4*>(l + D / 2) = make_uint4(lb[0], lb[1], lb[2], lb[3]);
+}
+
+// ------------------------------------------------------------------------------------------------
+// forward: 64 query rows per CTA, key tiles of 64, double-buffered
+// ------------------------------------------------------------------------------------------------
+template <int D> struct Fwd {
+    static constexpr int kBN = 64;
+    static constexpr uint32_t kTile = kBN * Pitch<D>::kBytes;
+    static constexpr uint32_t kStage = 3 * kTile;   // K~ hi, K~ lo, V
+    static constexpr size_t kSmem = 2 * kStage;
+};
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kThreads, 2) rope_fwd_split_kernel(RopeParams p, const __nv_bfloat16* __restrict__ k_hi, const __nv_bfloat16* __restrict__ k_lo) {
+    using F = Fwd<D>;
+    constexpr int BN = F::kBN, KS = D / 16, NT = BN / 8, DT = D / 8;
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t sm = smem_u32(smem);
+    // heads run fastest and the longest causal rows come first
+    const int N = p.N, bh = blockIdx.x, kvh = bh / (p.H / p.Hkv);
+    const int m0 = (gridDim.y - 1 - blockIdx.y) * kRows;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+    const int row0 = m0 + warp * 16 + g;   // the lane's rows: row0 and row0 + 8
+    const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0);
+    const __nv_bfloat16 *KH = k_hi + (size_t)kvh * N * D, *KL = k_lo + (size_t)kvh * N * D;
+    auto load = [&](int j0, int buf) {
+        const uint32_t st = sm + buf * F::kStage;
+        load_rows<D, BN>(st, KH, D, j0, N);
+        load_rows<D, BN>(st + F::kTile, KL, D, j0, N);
+        load_rows<D, BN>(st + 2 * F::kTile, V, p.sv.n, j0, N);
+        cp_commit();
+    };
+    load(0, 0);
+
+    // Q~ = rotated q * sm_scale * log2e as A operands, split; both columns of a rotation pair belong to the same lane
+    uint32_t qh[KS][4], ql[KS][4];
+    {
+        const T* Q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, 0);
+        const float scale = p.sm_scale * kLog2e;
+#pragma unroll
+        for (int ks = 0; ks < KS / 2; ++ks)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const int pos = row0 + (x & 1) * 8, d = ks * 16 + (x >> 1) * 8 + c2;
+                float2 a = make_float2(0.f, 0.f), b = a;
+                float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
+                if (pos < N) {
+                    const T* q = Q + (int64_t)pos * p.sq.n + d;
+                    a = unpack2<T>(*reinterpret_cast<const uint32_t*>(q));
+                    b = unpack2<T>(*reinterpret_cast<const uint32_t*>(q + D / 2));
+                    if (p.cos != nullptr) {
+                        const float *c = p.cos + (int64_t)pos * p.table_stride + d, *s = p.sin + (int64_t)pos * p.table_stride + d;
+                        c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
+                    }
+                }
+                split2<__nv_bfloat16>((a.x * c0 - b.x * s0) * scale, (a.y * c1 - b.y * s1) * scale, qh[ks][x], ql[ks][x]);
+                split2<__nv_bfloat16>((b.x * c0 + a.x * s0) * scale, (b.y * c1 + a.y * s1) * scale, qh[ks + KS / 2][x], ql[ks + KS / 2][x]);
+            }
+    }
+    float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[DT][4];
+#pragma unroll
+    for (int n = 0; n < DT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+
+    const int n_end = p.causal ? min(N, m0 + kRows) : N;
+    int buf = 0;
+    for (int j0 = 0; j0 < n_end; j0 += BN, buf ^= 1) {
+        cp_wait_all();
+        __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
+        if (j0 + BN < n_end) load(j0 + BN, buf ^ 1);
+        const uint32_t kh = sm + buf * F::kStage + lane_b<D>(lane), kl = kh + F::kTile, vv = sm + buf * F::kStage + 2 * F::kTile + lane_bt<D>(lane);
+        float s[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+            for (int np = 0; np < NT / 2; ++np) {
+                uint32_t bh4[4], bl4[4];
+                ldm_x4(bh4, kh + np * 16 * Pitch<D>::kBytes + ks * 32);
+                ldm_x4(bl4, kl + np * 16 * Pitch<D>::kBytes + ks * 32);
+                mma_split(s[2 * np], qh[ks], ql[ks], bh4[0], bh4[1], bl4[0], bl4[1]);
+                mma_split(s[2 * np + 1], qh[ks], ql[ks], bh4[2], bh4[3], bl4[2], bl4[3]);
+            }
+        // keys the lane's rows do not see
+        if (j0 + BN > N || (p.causal && j0 + BN - 1 > m0 + warp * 16)) {
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {
+                    const int key = j0 + n * 8 + c2 + (x & 1);
+                    if (key >= N || (p.causal && key > row0 + (x >> 1) * 8)) s[n][x] = -INFINITY;
+                }
+        }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            float mx = m[r];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) mx = fmax3(mx, s[n][2 * r], s[n][2 * r + 1]);
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            const float ref = mx == -INFINITY ? 0.f : mx;   // a row that has seen no key yet
+            const float alpha = fast_exp2(m[r] - ref);
+            float sum = 0.f;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    s[n][2 * r + x] = fast_exp2(s[n][2 * r + x] - ref);
+                    sum += s[n][2 * r + x];
+                }
+            l[r] = l[r] * alpha + sum;   // this lane's columns only; the four lanes of a row are added at the end
+            m[r] = mx;
+#pragma unroll
+            for (int n = 0; n < DT; ++n) o[n][2 * r] *= alpha, o[n][2 * r + 1] *= alpha;
+        }
+#pragma unroll
+        for (int t = 0; t < BN / 16; ++t) {
+            uint32_t ph[4], pl[4];
+            split_a<T>(s[2 * t], s[2 * t + 1], 1.f, ph, pl);
+#pragma unroll
+            for (int dp = 0; dp < DT / 2; ++dp) {
+                uint32_t b[4];
+                ldm_x4_trans(b, vv + t * 16 * Pitch<D>::kBytes + dp * 32);
+                mma<T>(o[2 * dp], ph, b[0], b[1]);
+                mma<T>(o[2 * dp + 1], ph, b[2], b[3]);
+                mma<T>(o[2 * dp], pl, b[0], b[1]);
+                mma<T>(o[2 * dp + 1], pl, b[2], b[3]);
+            }
+        }
+    }
+    T* O = reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.H, bh, 0);
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        float sum = l[r];
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+        const int pos = row0 + 8 * r;
+        if (pos >= N) continue;
+        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        uint32_t* out = reinterpret_cast<uint32_t*>(O + (int64_t)pos * p.so.n + c2);
+#pragma unroll
+        for (int n = 0; n < DT; ++n) out[n * 4] = pack2<T>(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
+        if (c2 == 0) p.lse2[(size_t)bh * N + pos] = m[r] + log2f(sum);
+    }
+}
+
+// ------------------------------------------------------------------------------------------------
+// backward: two kernels of one form.  KV = false: dQ of 64 query rows, sweeping the keys.  KV = true: dK, dV of 64 keys, sweeping
+// the query rows of the group's heads (everything transposed).  The owned rows are the A operands, the streamed rows (32 per step)
+// the B operands of both score products, and the streamed rotated rows again those of the gradient product.  The scores are formed
+// twice (16 MMAs against 12), but every sum has one owner and one order: the same bits every time, and no fp32 accumulator of dQ.
+// ------------------------------------------------------------------------------------------------
+template <int D> struct Bwd {
+    static constexpr int kBS = 32;
+    static constexpr uint32_t kOwn = kRows * Pitch<D>::kBytes, kTile = kBS * Pitch<D>::kBytes, kStage = 3 * kTile;
+    static constexpr size_t kSmem = 3 * kOwn + 2 * kStage;
+};
+
+struct SplitRows {   // bf16 hi and lo copies [B, H, N, D]
+    const __nv_bfloat16 *hi, *lo;
+};
+
+template <typename T, int D, bool KV>
+__global__ void __launch_bounds__(kThreads, 2) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
+    using W = Bwd<D>;
+    constexpr int BS = W::kBS, KS = D / 16, NT = BS / 8, DT = D / 8;
+    // P^T of f16 tensors enters its product times 1024: a probability of a long row is far below 1, where f16 hi + lo runs out of
+    // exponent before it runs out of mantissa
+    constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 1024.f : 1.f;
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t sm = smem_u32(smem), stages = sm + 3 * W::kOwn;
+    const int N = p.N, G = p.H / p.Hkv;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+    const int own_head = blockIdx.x;                         // KV: a K / V head, otherwise a query head
+    const int kvh = KV ? own_head : own_head / G;
+    const int own0 = (KV ? blockIdx.y : gridDim.y - 1 - blockIdx.y) * kRows;   // long causal sweeps first
+    const int row0 = own0 + warp * 16 + g;                   // the lane's owned rows: row0 and row0 + 8
+    const int first = KV && p.causal ? own0 / BS * BS : 0, end = !KV && p.causal ? min(N, own0 + kRows) : N;
+    const int steps = (end - first + BS - 1) / BS, total = KV ? steps * G : steps;
+
+    auto load = [&](int step, int buf) {
+        const uint32_t st = stages + buf * W::kStage;
+        const int r0 = first + (KV ? step % steps : step) * BS;
+        if (KV) {
+            const int qh = kvh * G + step / steps;
+            load_rows<D, BS>(st, qs.hi + (size_t)qh * N * D, D, r0, N);
+            load_rows<D, BS>(st + W::kTile, qs.lo + (size_t)qh * N * D, D, r0, N);
+            load_rows<D, BS>(st + 2 * W::kTile, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, qh, 0), p.sdo.n, r0, N);
+        } else {
+            load_rows<D, BS>(st, ks.hi + (size_t)kvh * N * D, D, r0, N);
+            load_rows<D, BS>(st + W::kTile, ks.lo + (size_t)kvh * N * D, D, r0, N);
+            load_rows<D, BS>(st + 2 * W::kTile, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0), p.sv.n, r0, N);
+        }
+        cp_commit();
+    };
+    {
+        const SplitRows& own = KV ? ks : qs;
+        load_rows<D, kRows>(sm, own.hi + (size_t)own_head * N * D, D, own0, N);
+        load_rows<D, kRows>(sm + W::kOwn, own.lo + (size_t)own_head * N * D, D, own0, N);
+        if (KV)
+            load_rows<D, kRows>(sm + 2 * W::kOwn, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, own_head, 0), p.sv.n, own0, N);
+        else
+            load_rows<D, kRows>(sm + 2 * W::kOwn, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, own_head, 0), p.sdo.n, own0, N);
+        load(0, 0);
+    }
+    float lse_r[2], dl_r[2];
+    if (!KV) {
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+            const int pos = row0 + 8 * r;
+            lse_r[r] = pos < N ? p.lse2[(size_t)own_head * N + pos] : INFINITY;   // P = 0 beyond the head
+            dl_r[r] = pos < N ? p.delta[(size_t)own_head * N + pos] : 0.f;
+        }
+    }
+    float acc[DT][4], dv[KV ? DT : 1][4];   // dQ~ / dK~ and dV
+#pragma unroll
+    for (int n = 0; n < DT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+#pragma unroll
+    for (int n = 0; n < (KV ? DT : 1); ++n) dv[n][0] = dv[n][1] = dv[n][2] = dv[n][3] = 0.f;
+    const uint32_t ah_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane), al_addr = ah_addr + W::kOwn, ax_addr = ah_addr + 2 * W::kOwn;
+
+    for (int step = 0, buf = 0; step < total; ++step, buf ^= 1) {
+        cp_wait_all();
+        __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
+        if (step + 1 < total) load(step + 1, buf ^ 1);
+        const uint32_t st = stages + buf * W::kStage;
+        const int r0 = first + (KV ? step % steps : step) * BS;
+        float lse_c[NT][2], dl_c[NT][2];
+        if (KV) {
+            const size_t head = (size_t)(kvh * G + step / steps) * N;
+#pragma unroll
+            for (int n = 0; n < NT; ++n)
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int pos = r0 + n * 8 + c2 + x;
+                    lse_c[n][x] = pos < N ? p.lse2[head + pos] : INFINITY;
+                    dl_c[n][x] = pos < N ? p.delta[head + pos] : 0.f;
+                }
+        }
+        float s[NT][4], dp[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) s[n][x] = dp[n][x] = 0.f;
+        const uint32_t b_addr = st + lane_b<D>(lane);
+#pragma unroll
+        for (int k = 0; k < KS; ++k) {
+            uint32_t ah[4], al[4], ax[4];
+            ldm_x4(ah, ah_addr + k * 32);
+            ldm_x4(al, al_addr + k * 32);
+            ldm_x4(ax, ax_addr + k * 32);
+#pragma unroll
+            for (int np = 0; np < NT / 2; ++np) {
+                uint32_t bh4[4], bl4[4], bx[4];
+                ldm_x4(bh4, b_addr + np * 16 * Pitch<D>::kBytes + k * 32);
+                ldm_x4(bl4, b_addr + W::kTile + np * 16 * Pitch<D>::kBytes + k * 32);
+                ldm_x4(bx, b_addr + 2 * W::kTile + np * 16 * Pitch<D>::kBytes + k * 32);
+                mma_split(s[2 * np], ah, al, bh4[0], bh4[1], bl4[0], bl4[1]);
+                mma_split(s[2 * np + 1], ah, al, bh4[2], bh4[3], bl4[2], bl4[3]);
+                mma<T>(dp[2 * np], ax, bx[0], bx[1]);
+                mma<T>(dp[2 * np + 1], ax, bx[2], bx[3]);
+            }
+        }
+        // P and dS = P (dP - delta), in place of S and dP
+        const bool edge = KV ? (p.causal && r0 < own0 + warp * 16 + 15) : (r0 + BS > N || (p.causal && r0 + BS - 1 > own0 + warp * 16));
+#pragma unroll
+        for (int n = 0; n < NT; ++n)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                float pv = fast_exp2(s[n][x] - (KV ? lse_c[n][x & 1] : lse_r[x >> 1]));
+                if (edge) {
+                    const int own = row0 + (x >> 1) * 8, str = r0 + n * 8 + c2 + (x & 1);
+                    const bool seen = KV ? (!p.causal || own <= str) : (str < N && (!p.causal || str <= own));
+                    if (!seen) pv = 0.f;
+                }
+                dp[n][x] = pv * (dp[n][x] - (KV ? dl_c[n][x & 1] : dl_r[x >> 1]));
+                s[n][x] = pv;
+            }
+        const uint32_t t_addr = st + lane_bt<D>(lane);
+#pragma unroll
+        for (int t = 0; t < BS / 16; ++t) {
+            uint32_t dh[4], dl[4], ph[4], pl[4];
+            split_a<__nv_bfloat16>(dp[2 * t], dp[2 * t + 1], 1.f, dh, dl);
+            if (KV) split_a<T>(s[2 * t], s[2 * t + 1], kPScale, ph, pl);
+#pragma unroll
+            for (int d = 0; d < DT / 2; ++d) {
+                const uint32_t off = t * 16 * Pitch<D>::kBytes + d * 32;
+                uint32_t bh4[4], bl4[4];
+                ldm_x4_trans(bh4, t_addr + off);
+                ldm_x4_trans(bl4, t_addr + W::kTile + off);
+                mma_split(acc[2 * d], dh, dl, bh4[0], bh4[1], bl4[0], bl4[1]);
+                mma_split(acc[2 * d + 1], dh, dl, bh4[2], bh4[3], bl4[2], bl4[3]);
+                if (KV) {
+                    uint32_t bx[4];
+                    ldm_x4_trans(bx, t_addr + 2 * W::kTile + off);
+                    mma<T>(dv[KV ? 2 * d : 0], ph, bx[0], bx[1]);
+                    mma<T>(dv[KV ? 2 * d + 1 : 0], ph, bx[2], bx[3]);
+                    mma<T>(dv[KV ? 2 * d : 0], pl, bx[0], bx[1]);
+                    mma<T>(dv[KV ? 2 * d + 1 : 0], pl, bx[2], bx[3]);
+                }
+            }
+        }
+    }
+
+    // gradients of the rotated rows turned back (both columns of a pair belong to the same lane); Q~ carries sm_scale * log2e, so
+    // dK only takes the log2e off again
+    const float scale = KV ? kLn2 : p.sm_scale;
+    T* OUT = reinterpret_cast<T*>(KV ? p.dk : p.dq) + (KV ? row_offset(p.sdk, p.Hkv, own_head, 0) : row_offset(p.sdq, p.H, own_head, 0));
+    const int64_t out_stride = KV ? p.sdk.n : p.sdq.n;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int pos = row0 + 8 * r;
+        if (pos >= N) continue;
+        uint32_t* out = reinterpret_cast<uint32_t*>(OUT + (int64_t)pos * out_stride + c2);
+#pragma unroll
+        for (int n = 0; n < DT / 2; ++n) {
+            float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
+            if (p.cos != nullptr) {
+                const float *c = p.cos + (int64_t)pos * p.table_stride + n * 8 + c2, *s = p.sin + (int64_t)pos * p.table_stride + n * 8 + c2;
+                c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
+            }
+            const float a0 = acc[n][2 * r], a1 = acc[n][2 * r + 1], b0 = acc[n + DT / 2][2 * r], b1 = acc[n + DT / 2][2 * r + 1];
+            out[n * 4] = pack2<T>((a0 * c0 + b0 * s0) * scale, (a1 * c1 + b1 * s1) * scale);
+            out[n * 4 + D / 4] = pack2<T>((b0 * c0 - a0 * s0) * scale, (b1 * c1 - a1 * s1) * scale);
+        }
+        if (KV) {
+            uint32_t* o2 = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.dv) + row_offset(p.sdv, p.Hkv, own_head, pos) + c2);
+#pragma unroll
+            for (int n = 0; n < DT; ++n) o2[n * 4] = pack2<T>(dv[KV ? n : 0][2 * r] * (1.f / kPScale), dv[KV ? n : 0][2 * r + 1] * (1.f / kPScale));
+        }
+    }
+}
+
+// ------------------------------------------------------------------------------------------------ launchers
+template <typename T, int D>
+int split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, SplitRows out, cudaStream_t s) {
+    const size_t rows = (size_t)p.B * H * p.N;
+    split_rotate_kernel<T, D><<<(unsigned)((rows * (D / 16) + 255) / 256), 256, 0, s>>>((const T*)x, row_addr(st, H, p.N), p.cos, p.sin, p.table_stride, scale,
+                                                                                       const_cast<__nv_bfloat16*>(out.hi), const_cast<__nv_bfloat16*>(out.lo), rows);
+    count_launch();
+    return (int)cudaGetLastError();
+}
+SplitRows take_rows(__nv_bfloat16*& ws, int B, int H, int N, int D) {
+    const size_t n = (size_t)B * H * N * D;
+    SplitRows r{ws, ws + n};
+    ws += 2 * n;
+    return r;
+}
+
+template <typename T, int D>
+int fwd(const RopeParams& p, void* ws, cudaStream_t s) {
+    __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
+    const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D);
+    if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
+    auto kern = rope_fwd_split_kernel<T, D>;
+    static std::atomic<uint64_t> smem_ok;
+    if (int e = allow_smem(kern, Fwd<D>::kSmem, smem_ok)) return e;
+    kern<<<dim3(p.B * p.H, (p.N + kRows - 1) / kRows), kThreads, Fwd<D>::kSmem, s>>>(p, k.hi, k.lo);
+    count_launch();
+    return (int)cudaGetLastError();
+}
+template <typename T, int D>
+int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
+    __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
+    const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D), q = take_rows(at, p.B, p.H, p.N, D);
+    if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
+    if (int e = split_rows<T, D>(p.q, p.sq, p.H, p, p.sm_scale * kLog2e, q, s)) return e;
+    const unsigned blocks = (p.N + kRows - 1) / kRows;
+    auto kv = rope_bwd_split_kernel<T, D, true>;
+    auto dq = rope_bwd_split_kernel<T, D, false>;
+    static std::atomic<uint64_t> kv_ok, dq_ok;
+    if (int e = allow_smem(kv, Bwd<D>::kSmem, kv_ok)) return e;
+    if (int e = allow_smem(dq, Bwd<D>::kSmem, dq_ok)) return e;
+    kv<<<dim3(p.B * p.Hkv, blocks), kThreads, Bwd<D>::kSmem, s>>>(p, q, k);
+    count_launch();
+    if (cudaError_t e = cudaGetLastError()) return (int)e;
+    dq<<<dim3(p.B * p.H, blocks), kThreads, Bwd<D>::kSmem, s>>>(p, q, k);
+    count_launch();
+    return (int)cudaGetLastError();
+}
+
+}  // namespace
+
+size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D) {
+    return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 2 * sizeof(__nv_bfloat16);
+}
+
+int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
+    if (dtype == COROPE_DTYPE_BF16) return p.D == 64 ? fwd<__nv_bfloat16, 64>(p, ws, s) : fwd<__nv_bfloat16, 128>(p, ws, s);
+    return p.D == 64 ? fwd<__half, 64>(p, ws, s) : fwd<__half, 128>(p, ws, s);
+}
+
+// delta computed before
+int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
+    if (dtype == COROPE_DTYPE_BF16) return p.D == 64 ? bwd<__nv_bfloat16, 64>(p, ws, s) : bwd<__nv_bfloat16, 128>(p, ws, s);
+    return p.D == 64 ? bwd<__half, 64>(p, ws, s) : bwd<__half, 128>(p, ws, s);
+}
+
+}  // namespace corope

@@ -90,7 +90,8 @@ const char* corope_status_string(int status);
  * function answers 16 and 32 per element of q).  Always ask this function. */
 size_t corope_workspace_bytes(int op, int B, int Hq, int Hkv, int N, int D, int dtype);
 
-/* The size with which an op runs on the tensor-core kernels at every N, not only at whole tiles.  A call that is handed at
+/* The size with which an op runs on tensor cores at every N, not only at whole tiles: 16-bit D = 64 or 128 inputs of a ragged N
+ * then go to kernels that split every fp32 operand into two 16-bit ones and keep fp32 accuracy.  A call that is handed at
  * least this much uses them; with corope_workspace_bytes() bytes a ragged N runs on the CUDA-core kernels.
  * Never more than corope_workspace_bytes() where N is a whole number of tiles. */
 size_t corope_workspace_bytes_any_n(int op, int B, int Hq, int Hkv, int N, int D, int dtype);

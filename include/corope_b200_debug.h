@@ -24,7 +24,7 @@ extern "C" {
 int corope_set_kernel_policy(int policy);
 
 /* Which kernel family the last call of each op (COROPE_OP_*) used in this process: 1 = tensor-core kernels at whole tiles
- * (N a multiple of 128, Co-RoPE: of 64), 0 = anything else: the CUDA-core kernels, or a ragged N whichever kernels ran it. */
+ * (N a multiple of 128, Co-RoPE: of 64), 0 = the kernels with fp32 accuracy: on CUDA cores, or with split operands. */
 int corope_last_kernel_family(int op);
 
 /* Number of GPU kernel launches this library has issued in this process so far. */

@@ -1,4 +1,4 @@
-"""Lengths that are not whole tiles, on the tensor-core kernels: one key, one short of / one beyond the 64-row steps, the 128-row
+"""Lengths that are not whole tiles, on the split-operand kernels: one key, one short of / one beyond the 64-row steps, the 128-row
 blocks and the 256-row work items; both head dimensions, causal and full, with and without rotation, grouped heads, transposed
 buffers.  Tolerances as in test_gpu_parity.py."""
 
@@ -81,3 +81,36 @@ def test_theta_with_a_ragged_length():
     outs = _run(pkg.fused_rope_attention_theta, q, k, v, do, False, D ** -0.5, 10000.0)
     refs = (oracle.rope_attn_fwd(q, k, v, False, D ** -0.5, cos, sin),) + tuple(oracle.rope_attn_bwd(q, k, v, do, False, D ** -0.5, cos, sin))
     _check(outs, refs, dtype)
+
+
+def _exact(q, k, v, do, causal, s, cos, sin):
+    """The same in 64 bits: rotated attention and its gradients."""
+    q, k, v = (t.cuda().double().requires_grad_(True) for t in (q, k, v))
+    half = q.shape[-1] // 2
+    c, sn = cos[:, :half].cuda().double(), sin[:, :half].cuda().double()
+    qr, kr = (torch.cat((x[..., :half] * c - x[..., half:] * sn, x[..., half:] * c + x[..., :half] * sn), -1) for x in (q, k))
+    w = qr @ kr.transpose(-1, -2) * s
+    if causal:
+        w = w.masked_fill(torch.ones_like(w, dtype=torch.bool).triu(1), float("-inf"))
+    o = w.softmax(-1) @ v
+    return (o.detach(),) + torch.autograd.grad(o, (q, k, v), do.cuda().double())
+
+
+@pytest.mark.parametrize("scale", [1.0, 2.0])   # 2: scores with a standard deviation of 4
+@pytest.mark.parametrize("N,D,causal", [(1777, 128, True), (1000, 64, False), (65, 128, False), (129, 64, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_ragged_lengths_keep_fp32_accuracy(N, D, causal, dtype, scale):
+    """Rounding the result to p bits costs at most 2^-p of a value and about 0.8 * 2^-p of it in the 2-norm; nothing else may show.
+    dQ and dK also see delta = rowsum(O dO) of the rounded O, which every kernel of this package forms that way: its rounding error,
+    0.8 * 2^-p of sqrt(D) |O| |dO|, stands next to a dP - delta of about the same size, and grows against it as rows become one-hot,
+    so they are only looked at for scale 1."""
+    q, k, v, do = (draw((1, 2, N, D), 230 + i, dtype) * (scale if i < 2 else 1.0) for i in range(4))
+    cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
+    s = D ** -0.5
+    outs = _run(pkg.fused_rope_attention, q, k, v, do, causal, s, cos.cuda(), sin.cuda())
+    ulp = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    for name, got, ref in zip(("O", "dQ", "dK", "dV"), outs, _exact(q, k, v, do, causal, s, cos, sin)):
+        if scale != 1.0 and name in ("dQ", "dK"):
+            continue
+        err = ((got.double() - ref.cpu()).norm() / ref.cpu().norm()).item()
+        assert err < ulp * (1.0 if name in ("O", "dV") else 1.5), (name, err / ulp)
