@@ -18,7 +18,7 @@
 //     dq1_h += g K'1, dq2_h += g K'2;   dk1_j += (sum_h g q1) cos - (sum_h g q2) sin,  dk2_j += (sum_h g q2) cos + (sum_h g q1) sin
 //     gD_ij = - sum_h g_hij * sum_d w_d ( q1 (k1 sin - k2 cos) + q2 (k2 sin + k1 cos) )
 //     gz_ik = sum_{j<k} gD_ij (k <= i),  graw = gz z (1 - z) s,  dqL_i += graw k,  dk_k += graw qL_i
-// dK / dV partial sums of a CTA's 8 rows are combined in shared memory and added to fp32 global accumulators.
+// dK / dV partial sums of a CTA's 8 rows are combined in registers and added to fp32 global accumulators.
 #include "common.cuh"
 
 namespace corope {
@@ -238,27 +238,68 @@ __global__ void gqa_delta_kernel(const T* __restrict__ o, const T* __restrict__ 
     if (lane == 0) delta[row] = s;
 }
 
+// fp32 accumulators [rows, D] of dK (y = 0) and dV (y = 1) to the outputs' type and layout
 template <typename T>
-__global__ void gqa_finalize_kernel(const float* __restrict__ acc, T* __restrict__ out, size_t n, int D, RowAddr aout) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;   // over the contiguous fp32 accumulator [rows, D]
-    if (i < n) out[flat_row_offset(aout, i / (size_t)D) + (int)(i % (size_t)D)] = Elem<T>::from_f32(acc[i]);
+__global__ void gqa_finalize_kernel(const float* __restrict__ dk_acc, const float* __restrict__ dv_acc, T* __restrict__ dk, T* __restrict__ dv, size_t n,
+                                    int D, RowAddr adk, RowAddr adv) {
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const size_t row = i / (size_t)D;
+    const int d = (int)(i % (size_t)D);
+    if (blockIdx.y == 0)
+        dk[flat_row_offset(adk, row) + d] = Elem<T>::from_f32(dk_acc[i]);
+    else
+        dv[flat_row_offset(adv, row) + d] = Elem<T>::from_f32(dv_acc[i]);
 }
 
+// Shared memory of the backward (floats).  The (cos, sin) of every (row, key, pair) of a tile are kept from the score phase for the
+// two gradient phases where they fit and are worth it: sincosf costs some 40 instructions, the hardware approximations two.
+template <int D, int G, bool ACCURATE> struct BwdSmem {
+    static constexpr int kPitch = D + 2;                          // floats per (row, key) of the (cos, sin) table: lane = key writes 8 bytes without conflicts
+    static constexpr size_t kBase = (size_t)2 * G * kWarps * D + 2 * kTile * (D + kPad) + D / 2 + (size_t)kWarps * kTile * (2 * G + 2);
+    static constexpr size_t kTable = (size_t)kWarps * kTile * kPitch;
+    static constexpr bool kStore = (ACCURATE || D <= 64) && (kBase + kTable) * sizeof(float) <= 225 * 1024;
+    static constexpr size_t kBytes = (kBase + (kStore ? kTable : 0)) * sizeof(float);
+};
+
+// G floats that every lane of the warp reads at one address
+template <int G>
+__device__ __forceinline__ void load_heads(float (&x)[G], const float* src) {
+    if constexpr (G % 4 == 0) {
+#pragma unroll
+        for (int h = 0; h < G; h += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(src + h);
+            x[h] = v.x; x[h + 1] = v.y; x[h + 2] = v.z; x[h + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < G; ++h) x[h] = src[h];
+    }
+}
+
+// Three phases per tile of 32 keys.  A: warp = row, lane = key: scores, P, dS, mileage gradient.  B1: warp = row, lane = pair: dq.
+// B2: warp = 4 keys, lane = pair / column: dk and dv summed over the CTA's 8 rows in registers, one global reduction per tile.
+// (With one phase for dq, dk and dv the rows met in shared-memory atomics, fp32 compare-and-swap loops that all 8 warps aimed at the
+// same key: backward of B1 Hq8 Hkv2 N512 D64 fp32 341 against 181 us now, B1 Hq32 Hkv8 N1500 D128 bf16 5.64 against 3.30 ms.)  Bound by
+// issue slots and, at small grids, the latency of one CTA's chain of tiles.
 template <typename T, int D, int G, bool ACCURATE>
 __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams p) {
+    using M = BwdSmem<D, G, ACCURATE>;
     constexpr int H2 = D / 2;
     constexpr int NC = D / 32;                    // head-dim columns per lane
     constexpr int NPI = (H2 + 31) / 32;           // (d, d + D/2) pairs per lane
-    constexpr int kXch = (2 * G + 2) * kTile;     // floats exchanged per warp between the two phases
+    constexpr int kKeys = kTile / kWarps;         // keys per warp in phase B2
     extern __shared__ __align__(16) float smem[];
     float* q_s = smem;                            // [G][8][D]
     float* do_s = q_s + G * kWarps * D;           // [G][8][D]
-    float* k_s = do_s + G * kWarps * D;           // [32][D+1]
-    float* v_s = k_s + kTile * (D + kPad);           // [32][D+1]
-    float* dk_t = v_s + kTile * (D + kPad);          // [32][D] tile accumulators shared by the CTA's 8 rows
-    float* dv_t = dk_t + kTile * D;               // [32][D]
-    float* w_s = dv_t + kTile * D;                // [H2]
-    float* xch = w_s + H2;                        // [8][kXch]
+    float* k_s = do_s + G * kWarps * D;           // [32][D+4]
+    float* v_s = k_s + kTile * (D + kPad);        // [32][D+4]
+    float* xg = v_s + kTile * (D + kPad);         // [8][32][G] dS * sm_scale
+    float* xp = xg + kWarps * kTile * G;          // [8][32][G] P
+    float* xd = xp + kWarps * kTile * G;          // [8][32] Delta
+    float* xr = xd + kWarps * kTile;              // [8][32] graw
+    float* w_s = xr + kWarps * kTile;             // [H2]
+    float* cs_s = w_s + H2;                       // [8][32][D+2] (cos, sin) pairs
 
     const int N = p.N;
     const int bg = blockIdx.y;
@@ -271,17 +312,12 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
     const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, bg, 0);
     float* dk_acc = p.dk_acc + (size_t)bg * N * D;
     float* dv_acc = p.dv_acc + (size_t)bg * N * D;
-    float* xg = xch + warp * kXch;                // g[G][32]
-    float* xp = xg + G * kTile;                   // P[G][32]
-    float* xd = xp + G * kTile;                   // Delta[32]
-    float* xr = xd + kTile;                       // graw[32]
 
     for (int h = 0; h < G; ++h) {
         stage_plain<T, D>(q_s + h * kWarps * D, D, reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.Hq, (int)q_head0 + h, 0), p.sq.n, i0, kWarps, N);
         stage_plain<T, D>(do_s + h * kWarps * D, D, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.Hq, (int)q_head0 + h, 0), p.sdo.n, i0, kWarps, N);
     }
     for (int d = threadIdx.x; d < H2; d += kThreads) w_s[d] = 1.0f / powf(p.theta, (float)(2 * d) / (float)D);
-    for (int idx = threadIdx.x; idx < kTile * D; idx += kThreads) dk_t[idx] = dv_t[idx] = 0.f;
 
     float lse[G], dl[G], dq1[G][NPI], dq2[G][NPI];
 #pragma unroll
@@ -296,8 +332,18 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
     const float sc2 = p.sm_scale * kLog2e;
     const bool direct = p.N <= 8192;
     const int i_last = min(N - 1, i0 + kWarps - 1);
+    // (cos, sin) of row r, key jj, pair pd of the tile
+    auto phase = [&](int r, int jj, int pd, float* sn, float* cs) {
+        if (M::kStore) {
+            const float2 x = *reinterpret_cast<const float2*>(cs_s + (r * kTile + jj) * M::kPitch + 2 * pd);
+            *cs = x.x;
+            *sn = x.y;
+        } else {
+            sincos_phase<ACCURATE>(xd[r * kTile + jj] * w_s[pd], sn, cs, direct);
+        }
+    };
     for (int j0 = 0; j0 <= i_last; j0 += kTile) {
-        __syncthreads();   // previous tile's flush done, accumulators are zero
+        __syncthreads();   // the previous tile has been used
         stage_plain<T, D>(k_s, D + kPad, K, p.sk.n, j0, kTile, N);
         stage_plain<T, D>(v_s, D + kPad, V, p.sv.n, j0, kTile, N);
         __syncthreads();
@@ -308,6 +354,7 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
             const float* kr = k_s + lane * (D + kPad);
             const float* vr = v_s + lane * (D + kPad);
             const float* qL = q_s + warp * D;
+            float* cs_out = cs_s + (warp * kTile + lane) * M::kPitch;
             float dot = 0.f;
 #pragma unroll 4
             for (int d = 0; d < D; d += 4) {
@@ -337,6 +384,7 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
                 for (int e = 0; e < 4; ++e) {
                     float sn, cs;
                     sincos_phase<ACCURATE>(delta * wv[e], &sn, &cs, direct);
+                    if (M::kStore) *reinterpret_cast<float2*>(cs_out + 2 * (d + e)) = make_float2(cs, sn);
                     r1[e] = fmaf(k1a[e], cs, k2a[e] * sn);
                     r2[e] = fmaf(k2a[e], cs, -k1a[e] * sn);
                     wr1[e] = wv[e] * r1[e];
@@ -370,69 +418,114 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
                 }
             }
             float gD = 0.f;
+            const int at = warp * kTile + lane;
 #pragma unroll
             for (int h = 0; h < G; ++h) {
                 float pv = vis ? exp2f(s[h] * sc2 - lse[h]) : 0.f;
                 float gT = pv * (dp[h] - dl[h]) * p.sm_scale;
                 gD = fmaf(-gT, tq[h], gD);
-                xg[h * kTile + lane] = gT;
-                xp[h * kTile + lane] = pv;
+                xg[at * G + h] = gT;
+                xp[at * G + h] = pv;
             }
             const float gpre = warp_prefix_incl(gD, lane);
             const float gz = carry_g + gpre - gD;
             carry_g += __shfl_sync(0xffffffffu, gpre, 31);
-            xd[lane] = delta;
-            xr[lane] = vis ? gz * z * (1.f - z) * p.sm_scale : 0.f;
+            xd[at] = delta;
+            xr[at] = vis ? gz * z * (1.f - z) * p.sm_scale : 0.f;
             __syncwarp();
-            // ---------------- phase B: lane = head-dim pair / column
+            // ---------------- phase B1: lane = head-dim pair, the warp's own row
             const int jj_end = min(kTile, i - j0 + 1);
+#pragma unroll 2
             for (int jj = 0; jj < jj_end; ++jj) {
-                const float dlt = xd[jj], graw = xr[jj];
+                float gT[G];
+                load_heads<G>(gT, xg + (warp * kTile + jj) * G);
+                const float graw = xr[warp * kTile + jj];
 #pragma unroll
                 for (int pi = 0; pi < NPI; ++pi) {
                     const int pd = lane + 32 * pi;
                     if (pd < H2) {
                         float sn, cs;
-                        sincos_phase<ACCURATE>(dlt * w_s[pd], &sn, &cs, direct);
-                        float k1 = k_s[jj * (D + kPad) + pd], k2 = k_s[jj * (D + kPad) + pd + H2];
-                        float r1 = fmaf(k1, cs, k2 * sn);
-                        float r2 = fmaf(k2, cs, -k1 * sn);
-                        float a1 = 0.f, a2 = 0.f;
+                        phase(warp, jj, pd, &sn, &cs);
+                        const float k1 = k_s[jj * (D + kPad) + pd], k2 = k_s[jj * (D + kPad) + pd + H2];
+                        const float r1 = fmaf(k1, cs, k2 * sn);
+                        const float r2 = fmaf(k2, cs, -k1 * sn);
 #pragma unroll
                         for (int h = 0; h < G; ++h) {
-                            float gT = xg[h * kTile + jj];
-                            dq1[h][pi] = fmaf(gT, r1, dq1[h][pi]);
-                            dq2[h][pi] = fmaf(gT, r2, dq2[h][pi]);
-                            a1 = fmaf(gT, q_s[(h * kWarps + warp) * D + pd], a1);
-                            a2 = fmaf(gT, q_s[(h * kWarps + warp) * D + pd + H2], a2);
+                            dq1[h][pi] = fmaf(gT[h], r1, dq1[h][pi]);
+                            dq2[h][pi] = fmaf(gT[h], r2, dq2[h][pi]);
                         }
                         dq1[0][pi] = fmaf(graw, k1, dq1[0][pi]);
                         dq2[0][pi] = fmaf(graw, k2, dq2[0][pi]);
-                        float dk1 = a1 * cs - a2 * sn + graw * qL[pd];
-                        float dk2 = a2 * cs + a1 * sn + graw * qL[pd + H2];
-                        atomicAdd(&dk_t[jj * D + pd], dk1);
-                        atomicAdd(&dk_t[jj * D + pd + H2], dk2);
                     }
-                }
-#pragma unroll
-                for (int c = 0; c < NC; ++c) {
-                    const int col = lane + 32 * c;
-                    float a = 0.f;
-#pragma unroll
-                    for (int h = 0; h < G; ++h) a = fmaf(xp[h * kTile + jj], do_s[(h * kWarps + warp) * D + col], a);
-                    atomicAdd(&dv_t[jj * D + col], a);
                 }
             }
         }
         __syncthreads();
-        for (int idx = threadIdx.x; idx < kTile * D; idx += kThreads) {
-            int r = idx / D;
-            if (j0 + r < N && j0 + r <= i_last) {
-                atomicAdd(&dk_acc[(size_t)(j0 + r) * D + (idx % D)], dk_t[idx]);
-                atomicAdd(&dv_acc[(size_t)(j0 + r) * D + (idx % D)], dv_t[idx]);
+        // ---------------- phase B2: keys kKeys * warp .. of the tile, all rows that reach it
+        float dk1[kKeys][NPI], dk2[kKeys][NPI], dv[kKeys][NC];
+#pragma unroll
+        for (int kk = 0; kk < kKeys; ++kk) {
+#pragma unroll
+            for (int pi = 0; pi < NPI; ++pi) dk1[kk][pi] = dk2[kk][pi] = 0.f;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) dv[kk][c] = 0.f;
+        }
+        const int key0 = j0 + kKeys * warp;
+#pragma unroll 1
+        for (int r = max(0, key0 - i0); r <= i_last - i0; ++r) {   // rows before the warp's first key do not see any of its keys
+            float x[kKeys][G];
+#pragma unroll
+            for (int kk = 0; kk < kKeys; ++kk) load_heads<G>(x[kk], xg + (r * kTile + kKeys * warp + kk) * G);
+#pragma unroll
+            for (int pi = 0; pi < NPI; ++pi) {
+                const int pd = lane + 32 * pi;
+                if (pd < H2) {
+                    float a1[kKeys], a2[kKeys];
+#pragma unroll
+                    for (int kk = 0; kk < kKeys; ++kk) a1[kk] = a2[kk] = 0.f;
+#pragma unroll
+                    for (int h = 0; h < G; ++h) {
+                        const float q1 = q_s[(h * kWarps + r) * D + pd], q2 = q_s[(h * kWarps + r) * D + pd + H2];
+#pragma unroll
+                        for (int kk = 0; kk < kKeys; ++kk) {
+                            a1[kk] = fmaf(x[kk][h], q1, a1[kk]);
+                            a2[kk] = fmaf(x[kk][h], q2, a2[kk]);
+                        }
+                    }
+                    const float qL1 = q_s[r * D + pd], qL2 = q_s[r * D + pd + H2];
+#pragma unroll
+                    for (int kk = 0; kk < kKeys; ++kk) {
+                        float sn, cs;
+                        phase(r, kKeys * warp + kk, pd, &sn, &cs);
+                        const float graw = xr[r * kTile + kKeys * warp + kk];
+                        dk1[kk][pi] += a1[kk] * cs - a2[kk] * sn + graw * qL1;
+                        dk2[kk][pi] += a2[kk] * cs + a1[kk] * sn + graw * qL2;
+                    }
+                }
             }
-            dk_t[idx] = 0.f;
-            dv_t[idx] = 0.f;
+#pragma unroll
+            for (int kk = 0; kk < kKeys; ++kk) load_heads<G>(x[kk], xp + (r * kTile + kKeys * warp + kk) * G);
+#pragma unroll
+            for (int h = 0; h < G; ++h)
+#pragma unroll
+                for (int c = 0; c < NC; ++c) {
+                    const float gv = do_s[(h * kWarps + r) * D + lane + 32 * c];
+#pragma unroll
+                    for (int kk = 0; kk < kKeys; ++kk) dv[kk][c] = fmaf(x[kk][h], gv, dv[kk][c]);
+                }
+        }
+#pragma unroll
+        for (int kk = 0; kk < kKeys; ++kk) {
+            if (key0 + kk > i_last) continue;
+            float *dk_out = dk_acc + (size_t)(key0 + kk) * D + lane, *dv_out = dv_acc + (size_t)(key0 + kk) * D + lane;
+#pragma unroll
+            for (int pi = 0; pi < NPI; ++pi)
+                if (lane + 32 * pi < H2) {
+                    atomicAdd(dk_out + 32 * pi, dk1[kk][pi]);
+                    atomicAdd(dk_out + 32 * pi + H2, dk2[kk][pi]);
+                }
+#pragma unroll
+            for (int c = 0; c < NC; ++c) atomicAdd(dv_out + 32 * c, dv[kk][c]);
         }
     }
     if (i < N) {
@@ -466,7 +559,7 @@ int launch_fwd_g(const GqaParams& p, cudaStream_t s) {
 template <typename T, int D, int G>
 int launch_bwd_g(const GqaParams& p, cudaStream_t s) {
     constexpr bool kAcc = (Elem<T>::kDtype == COROPE_DTYPE_F32);
-    size_t smem = sizeof(float) * ((size_t)2 * G * kWarps * D + 2 * kTile * (D + kPad) + 2 * kTile * D + D / 2 + (size_t)kWarps * (2 * G + 2) * kTile);
+    constexpr size_t smem = BwdSmem<D, G, kAcc>::kBytes;
     auto kern = corope_bwd_general_kernel<T, D, G, kAcc>;
     static std::atomic<uint64_t> smem_ok;
     if (int er = allow_smem(kern, smem, smem_ok)) return er;
@@ -508,11 +601,11 @@ int bwd_all(const GqaParams& p, cudaStream_t s) {
                                                                            row_addr(p.sdo, p.Hq, p.N)); count_launch();
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
-    if ((e = cudaMemsetAsync(p.dk_acc, 0, kv_elems * sizeof(float), s)) != cudaSuccess) return (int)e;
-    if ((e = cudaMemsetAsync(p.dv_acc, 0, kv_elems * sizeof(float), s)) != cudaSuccess) return (int)e;
+    // dv_acc follows dk_acc in the workspace
+    if ((e = cudaMemsetAsync(p.dk_acc, 0, (size_t)(p.dv_acc + kv_elems - p.dk_acc) * sizeof(float), s)) != cudaSuccess) return (int)e;
     if (int r = p.use_mma ? launch_gqa_bwd_mma(p, Elem<T>::kDtype, s) : dispatch_gd<T>(p, s, true)) return r;
-    gqa_finalize_kernel<T><<<(unsigned)((kv_elems + 255) / 256), 256, 0, s>>>(p.dk_acc, (T*)p.dk, kv_elems, p.D, row_addr(p.sdk, p.Hkv, p.N)); count_launch();
-    gqa_finalize_kernel<T><<<(unsigned)((kv_elems + 255) / 256), 256, 0, s>>>(p.dv_acc, (T*)p.dv, kv_elems, p.D, row_addr(p.sdv, p.Hkv, p.N)); count_launch();
+    gqa_finalize_kernel<T><<<dim3((unsigned)((kv_elems + 255) / 256), 2), 256, 0, s>>>(p.dk_acc, p.dv_acc, (T*)p.dk, (T*)p.dv, kv_elems, p.D,
+                                                                                      row_addr(p.sdk, p.Hkv, p.N), row_addr(p.sdv, p.Hkv, p.N)); count_launch();
     return (int)cudaGetLastError();
 }
 
