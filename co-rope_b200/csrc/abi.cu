@@ -64,10 +64,16 @@ struct GqaWorkspace {
     size_t delta, dk_acc, dv_acc, k_pairs, v_half, total;
 };
 
-GqaWorkspace gqa_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype) {
+// `any_n`: room for the split-operand forward where the mma kernels do not apply.
+GqaWorkspace gqa_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool any_n) {
     GqaWorkspace w{};
     size_t off = 0;
     if (gqa_fwd_mma_supported(N, D, dtype)) {   // fp16 operand copies of K (pair order) and V for the tensor-core kernels
+        w.k_pairs = off;
+        off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
+        w.v_half = off;
+        off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
+    } else if (any_n && !bwd && gqa_split_supported(D, dtype)) {   // K in pair order, its own type; a copy of V if its rows are not aligned
         w.k_pairs = off;
         off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
         w.v_half = off;
@@ -224,8 +230,8 @@ size_t corope_workspace_bytes(int op, int B, int Hq, int Hkv, int N, int D, int 
         case COROPE_OP_ROPE_BWD_FREQS: return rope_workspace_bytes(true, B, Hq, Hq, N, D, dtype, true);
         case COROPE_OP_FLASH_FWD: return Hq % Hkv ? 0 : rope_workspace_bytes(false, B, Hq, Hkv, N, D, dtype, false);
         case COROPE_OP_FLASH_BWD: return Hq % Hkv ? 0 : rope_workspace_bytes(true, B, Hq, Hkv, N, D, dtype, false);
-        case COROPE_OP_GQA_FWD: return gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype).total;
-        case COROPE_OP_GQA_BWD: return gqa_workspace_layout(true, B, Hq, Hkv, N, D, dtype).total;
+        case COROPE_OP_GQA_FWD: return gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype, false).total;
+        case COROPE_OP_GQA_BWD: return gqa_workspace_layout(true, B, Hq, Hkv, N, D, dtype, false).total;
         default: return 0;
     }
 }
@@ -239,6 +245,7 @@ size_t corope_workspace_bytes_any_n(int op, int B, int Hq, int Hkv, int N, int D
         case COROPE_OP_ROPE_BWD_FREQS: return rope_workspace_layout(true, B, Hq, Hq, N, D, dtype, true, true).total;
         case COROPE_OP_FLASH_FWD: return Hq % Hkv ? 0 : rope_workspace_layout(false, B, Hq, Hkv, N, D, dtype, false, true).total;
         case COROPE_OP_FLASH_BWD: return Hq % Hkv ? 0 : rope_workspace_layout(true, B, Hq, Hkv, N, D, dtype, false, true).total;
+        case COROPE_OP_GQA_FWD: return gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype, true).total;
         default: return corope_workspace_bytes(op, B, Hq, Hkv, N, D, dtype);
     }
 }
@@ -568,7 +575,7 @@ int corope_gqa_fwd_strided(const void* q, const void* k, const void* v, void* o,
                            void* stream, const corope_strides_t* strides) {
     if (!q || !k || !v || !o || !lse2 || !a_diag) return COROPE_ERR_NULL_POINTER;
     if (int e = check_gqa(B, Hq, Hkv, N, D, dtype)) return e;
-    GqaWorkspace w = gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype);
+    GqaWorkspace w = gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype, false);
     if (int e = check_workspace(workspace, workspace_bytes, w.total)) return e;
     GqaParams p{};
     p.q = q; p.k = k; p.v = v; p.out_o = o; p.lse2 = lse2; p.a_diag = a_diag;
@@ -583,6 +590,13 @@ int corope_gqa_fwd_strided(const void* q, const void* k, const void* v, void* o,
         return launch_gqa_fwd_mma(p, dtype, (cudaStream_t)stream);
     }
     g_last_family[COROPE_OP_GQA_FWD] = 0;
+    // D = 64, a ragged N, or rows that the mma kernels cannot read: fp32 accuracy on tensor cores where the workspace has room
+    const GqaWorkspace any = gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype, true);
+    if (g_policy.load() == 0 && gqa_split_supported(D, dtype) && workspace_bytes >= any.total) {
+        p.k_pairs = reinterpret_cast<uint32_t*>((char*)workspace + any.k_pairs);
+        p.v_half = reinterpret_cast<__half*>((char*)workspace + any.v_half);
+        return launch_gqa_fwd_split(p, vec_ok(k, p.sk), vec_ok(v, p.sv), dtype, (cudaStream_t)stream);
+    }
     return launch_gqa_fwd_general(p, dtype, (cudaStream_t)stream);
 }
 
@@ -599,7 +613,7 @@ int corope_gqa_bwd_strided(const void* q, const void* k, const void* v, const vo
                            const corope_strides_t* strides) {
     if (!q || !k || !v || !o || !d_o || !lse2 || !a_diag || !dq || !dk || !dv) return COROPE_ERR_NULL_POINTER;
     if (int e = check_gqa(B, Hq, Hkv, N, D, dtype)) return e;
-    GqaWorkspace w = gqa_workspace_layout(true, B, Hq, Hkv, N, D, dtype);
+    GqaWorkspace w = gqa_workspace_layout(true, B, Hq, Hkv, N, D, dtype, false);
     if (int e = check_workspace(workspace, workspace_bytes, w.total)) return e;
     GqaParams p{};
     p.q = q; p.k = k; p.v = v; p.o = o; p.d_o = d_o; p.dq = dq; p.dk = dk; p.dv = dv;

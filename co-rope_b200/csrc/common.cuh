@@ -661,6 +661,10 @@ int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t
 int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 int launch_rope_bwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 bool gqa_fwd_mma_supported(int N, int D, int dtype);
+// 16-bit tensors, D = 64 or 128, any N and strides; k_vec / v_vec: rows of k / v are aligned to 16 bytes; p.k_pairs and (without v_vec)
+// p.v_half: workspace of 2 B Hkv N D bytes each
+bool gqa_split_supported(int D, int dtype);
+int launch_gqa_fwd_split(const GqaParams& p, bool k_vec, bool v_vec, int dtype, cudaStream_t s);
 int launch_gqa_bwd_mma(const GqaParams& p, int dtype, cudaStream_t s);
 int launch_gqa_fwd_mma(const GqaParams& p, int dtype, cudaStream_t s);
 int launch_gqa_fwd_general(const GqaParams& p, int dtype, cudaStream_t s);

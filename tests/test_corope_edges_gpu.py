@@ -1,0 +1,76 @@
+"""Co-RoPE outside the whole tiles of its mma kernels -- D = 64, ragged lengths, fp32 tensors -- at the edges of the 8-row CTAs and
+of the 32- and 64-key tiles, for every kind of group size; and the accuracy of the 16-bit results: rounding, nothing else."""
+
+import os
+
+import pytest
+import torch
+
+import oracle
+from helpers import check16, draw, maxdiff, run_corope
+
+pytestmark = pytest.mark.gpu
+
+TOL_32, TOL_FWD_16, TOL_BWD_16 = 1e-4, 1e-2, 2e-2
+
+
+def _label():
+    return os.environ.get("PYTEST_CURRENT_TEST", "?").split("::")[-1].split(" ")[0]
+
+
+def _case(B, Hq, Hkv, N, D, dtype, seed):
+    return tuple(draw((B, h, N, D), seed + x, dtype) for x, h in enumerate((Hq, Hkv, Hkv, Hq)))
+
+
+@pytest.mark.parametrize("N", [1, 9, 31, 33, 63, 65, 130])
+@pytest.mark.parametrize("D,Hq,Hkv", [(64, 4, 1), (128, 6, 2), (64, 8, 1), (128, 2, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_16_bit_edges(N, D, Hq, Hkv, dtype):
+    q, k, v, do = _case(1, Hq, Hkv, N, D, dtype, 500)
+    outs = run_corope(q, k, v, do, D ** -0.5, 10000.0)
+    check16(_label() + " O", outs[0], oracle.corope_gqa_fwd(q, k, v, True, D ** -0.5, 10000.0), TOL_FWD_16, dtype, strict=True)
+    for name, got, ref in zip("qkv", outs[1:], oracle.corope_gqa_bwd(q, k, v, do, True, D ** -0.5, 10000.0)):
+        check16(_label() + " d" + name, got, ref, TOL_BWD_16, dtype)
+
+
+@pytest.mark.parametrize("N", [1, 9, 33, 65])
+@pytest.mark.parametrize("D,Hq,Hkv", [(32, 4, 1), (64, 3, 1), (64, 8, 1), (128, 4, 2), (128, 8, 1), (128, 5, 1)])
+def test_fp32_edges(N, D, Hq, Hkv):
+    q, k, v, do = _case(2, Hq, Hkv, N, D, torch.float32, 520)
+    outs = run_corope(q, k, v, do, D ** -0.5, 10000.0)
+    refs = (oracle.corope_gqa_fwd(q, k, v, True, D ** -0.5, 10000.0),) + tuple(oracle.corope_gqa_bwd(q, k, v, do, True, D ** -0.5, 10000.0))
+    for x, (a, b) in enumerate(zip(outs, refs)):   # tolerances of the other fp32 Co-RoPE tests
+        assert maxdiff(a, b) < (TOL_32 if x == 0 else 2 * TOL_32)
+
+
+def _exact_o(q, k, v, s, theta):
+    """O in 64 bits."""
+    q, k, v = (t.double() for t in (q, k, v))
+    (B, Hq, N, D), Hkv = q.shape, k.shape[1]
+    G, half = Hq // Hkv, D // 2
+    w = theta ** (-torch.arange(0, D, 2, dtype=torch.float64, device=q.device) / D)
+    hidden = torch.ones(N, N, dtype=torch.bool, device=q.device).triu(1)
+    o = torch.empty_like(q)
+    for b in range(B):
+        for g in range(Hkv):
+            z = torch.sigmoid(q[b, g * G] @ k[b, g].T * s).masked_fill(hidden, 0.0)
+            a = z.cumsum(1)
+            delta = a.diagonal()[:, None] - a
+            score = 0
+            for p in range(half):
+                c, sn = torch.cos(delta * w[p]), torch.sin(delta * w[p])
+                k1, k2 = k[b, g, :, p], k[b, g, :, p + half]
+                score = score + q[b, g * G:(g + 1) * G, :, p, None] * (k1 * c + k2 * sn) + q[b, g * G:(g + 1) * G, :, p + half, None] * (k2 * c - k1 * sn)
+            o[b, g * G:(g + 1) * G] = (score * s).masked_fill(hidden, float("-inf")).softmax(-1) @ v[b, g]
+    return o
+
+
+@pytest.mark.parametrize("N,D", [(500, 128), (333, 64), (512, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_16_bit_results_are_rounded_only(N, D, dtype):
+    """Rounding to p bits costs about 0.8 * 2^-p of a value in the 2-norm; nothing else may show."""
+    q, k, v, do = _case(1, 8, 2, N, D, dtype, 540)
+    o = run_corope(q, k, v, do, D ** -0.5, 10000.0)[0]
+    ref = _exact_o(q.cuda(), k.cuda(), v.cuda(), D ** -0.5, 10000.0).cpu()
+    ulp = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    assert ((o.double() - ref).norm() / ref.norm()).item() < ulp
