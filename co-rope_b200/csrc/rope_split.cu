@@ -12,9 +12,11 @@
 // hundred would begin to show in f16 results.
 //
 // B1 H32 N1777 D128 bf16 causal forward 222 us (116 TFLOP/s; the CUDA-core kernel 909 us), B4 H16 N1000 D64 bf16 full forward +
-// backward 613 us (94 TFLOP/s; 3473 us).
-// What bounds it: the tensor pipe (mma.sync) and, next to it, the shared-memory port: a warp's 16 rows read every streamed tile,
-// hi and lo, once per product.  tcgen05 would need the split tiles of all operands resident (Q~ hi / lo, K~ hi / lo, V of 128 x 128:
+// backward 584 us (98 TFLOP/s; 3473 us).
+// What bounds it: mma.sync, measured at 553 TFLOP/s with all operands in registers (B200, 8 warps per SM), of which the split
+// products use about 300: with 8 warps per SM (D = 128: 255 registers; D = 64: 12 warps) the latency between a tile's ldmatrix, MMAs
+// and softmax is not fully hidden, and the shared-memory port is close behind, a warp's 16 rows reading every streamed tile, hi
+// and lo, once per product.  tcgen05 would need the split tiles of all operands resident (Q~ hi / lo, K~ hi / lo, V of 128 x 128:
 // 160 KB before any ring), so one stage of everything and no overlap.
 //
 // Math: fused-rope/rope_attn_pytorch.py:108-155 (forward), :187-222 (backward); exp2-domain softmax and log2-domain LSE as
@@ -55,12 +57,20 @@ template <> __device__ __forceinline__ void mma<__half>(float (&d)[4], const uin
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// four neighbouring accumulator tiles d += a b, b the two ldmatrix_x4 results of their columns: independent MMAs back to back
+template <typename T>
+__device__ __forceinline__ void mma4(float (*d)[4], const uint32_t (&a)[4], const uint32_t (&b0)[4], const uint32_t (&b1)[4]) {
+    mma<T>(d[0], a, b0[0], b0[1]);
+    mma<T>(d[1], a, b0[2], b0[3]);
+    mma<T>(d[2], a, b1[0], b1[1]);
+    mma<T>(d[3], a, b1[2], b1[3]);
+}
 // d += (ah + al) (bh + bl) without the product of the two small halves
-__device__ __forceinline__ void mma_split(float (&d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], uint32_t bh0, uint32_t bh1, uint32_t bl0,
-                                          uint32_t bl1) {
-    mma<__nv_bfloat16>(d, ah, bh0, bh1);
-    mma<__nv_bfloat16>(d, ah, bl0, bl1);
-    mma<__nv_bfloat16>(d, al, bh0, bh1);
+__device__ __forceinline__ void mma4_split(float (*d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh0)[4], const uint32_t (&bh1)[4],
+                                           const uint32_t (&bl0)[4], const uint32_t (&bl1)[4]) {
+    mma4<__nv_bfloat16>(d, ah, bh0, bh1);
+    mma4<__nv_bfloat16>(d, ah, bl0, bl1);
+    mma4<__nv_bfloat16>(d, al, bh0, bh1);
 }
 template <typename T>
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
@@ -141,7 +151,7 @@ template <int D> struct Fwd {
 };
 
 template <typename T, int D>
-__global__ void __launch_bounds__(kThreads, 2) rope_fwd_split_kernel(RopeParams p, const __nv_bfloat16* __restrict__ k_hi, const __nv_bfloat16* __restrict__ k_lo) {
+__global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kernel(RopeParams p, const __nv_bfloat16* __restrict__ k_hi, const __nv_bfloat16* __restrict__ k_lo) {
     using F = Fwd<D>;
     constexpr int BN = F::kBN, KS = D / 16, NT = BN / 8, DT = D / 8;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -204,12 +214,14 @@ __global__ void __launch_bounds__(kThreads, 2) rope_fwd_split_kernel(RopeParams 
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
-            for (int np = 0; np < NT / 2; ++np) {
-                uint32_t bh4[4], bl4[4];
-                ldm_x4(bh4, kh + np * 16 * Pitch<D>::kBytes + ks * 32);
-                ldm_x4(bl4, kl + np * 16 * Pitch<D>::kBytes + ks * 32);
-                mma_split(s[2 * np], qh[ks], ql[ks], bh4[0], bh4[1], bl4[0], bl4[1]);
-                mma_split(s[2 * np + 1], qh[ks], ql[ks], bh4[2], bh4[3], bl4[2], bl4[3]);
+            for (int np = 0; np < NT / 2; np += 2) {
+                constexpr uint32_t kNext = 16 * Pitch<D>::kBytes;
+                uint32_t bh0[4], bh1[4], bl0[4], bl1[4];
+                ldm_x4(bh0, kh + np * kNext + ks * 32);
+                ldm_x4(bh1, kh + (np + 1) * kNext + ks * 32);
+                ldm_x4(bl0, kl + np * kNext + ks * 32);
+                ldm_x4(bl1, kl + (np + 1) * kNext + ks * 32);
+                mma4_split(s + 2 * np, qh[ks], ql[ks], bh0, bh1, bl0, bl1);
             }
         // keys the lane's rows do not see
         if (j0 + BN > N || (p.causal && j0 + BN - 1 > m0 + warp * 16)) {
@@ -248,13 +260,12 @@ __global__ void __launch_bounds__(kThreads, 2) rope_fwd_split_kernel(RopeParams 
             uint32_t ph[4], pl[4];
             split_a<T>(s[2 * t], s[2 * t + 1], 1.f, ph, pl);
 #pragma unroll
-            for (int dp = 0; dp < DT / 2; ++dp) {
-                uint32_t b[4];
-                ldm_x4_trans(b, vv + t * 16 * Pitch<D>::kBytes + dp * 32);
-                mma<T>(o[2 * dp], ph, b[0], b[1]);
-                mma<T>(o[2 * dp + 1], ph, b[2], b[3]);
-                mma<T>(o[2 * dp], pl, b[0], b[1]);
-                mma<T>(o[2 * dp + 1], pl, b[2], b[3]);
+            for (int dp = 0; dp < DT / 2; dp += 2) {
+                uint32_t b0[4], b1[4];
+                ldm_x4_trans(b0, vv + t * 16 * Pitch<D>::kBytes + dp * 32);
+                ldm_x4_trans(b1, vv + t * 16 * Pitch<D>::kBytes + dp * 32 + 32);
+                mma4<T>(o + 2 * dp, ph, b0, b1);
+                mma4<T>(o + 2 * dp, pl, b0, b1);
             }
         }
     }
@@ -291,11 +302,17 @@ struct SplitRows {   // bf16 hi and lo copies [B, H, N, D]
 };
 
 template <typename T, int D, bool KV>
-__global__ void __launch_bounds__(kThreads, 2) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
+__global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
     using W = Bwd<D>;
     constexpr int BS = W::kBS, KS = D / 16, NT = BS / 8, DT = D / 8;
+    static_assert(NT == 4, "the score products of a step are four accumulator tiles");
     // P^T of f16 tensors enters its product times 1024: a probability of a long row is far below 1, where f16 hi + lo runs out of
     // exponent before it runs out of mantissa
+    // Owned A operands kept in registers (of hi, lo and the plain rows): an ldmatrix_x4 takes 4 cycles of the shared-memory port, an
+    // MMA 2 of the tensor pipe, and with all of them re-read a step's score products need 36 against 32.  D = 128 dQ has the
+    // registers (B1 H32 N1777 backward 686 -> 652 us, with the MMAs of four tiles back to back); at D = 64 a third CTA per SM is worth
+    // more (B4 H16 N1000 forward + backward 652 us with all three in registers and two CTAs, 584 us like this).
+    constexpr int kRegA = D == 64 || KV ? 0 : 2;
     constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 1024.f : 1.f;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sm = smem_u32(smem), stages = sm + 3 * W::kOwn;
@@ -347,11 +364,18 @@ __global__ void __launch_bounds__(kThreads, 2) rope_bwd_split_kernel(RopeParams 
     for (int n = 0; n < DT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
 #pragma unroll
     for (int n = 0; n < (KV ? DT : 1); ++n) dv[n][0] = dv[n][1] = dv[n][2] = dv[n][3] = 0.f;
-    const uint32_t ah_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane), al_addr = ah_addr + W::kOwn, ax_addr = ah_addr + 2 * W::kOwn;
+    const uint32_t ah_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane);   // of the hi rows; lo and plain rows follow
 
+    uint32_t own_a[kRegA > 0 ? kRegA : 1][KS][4];
     for (int step = 0, buf = 0; step < total; ++step, buf ^= 1) {
         cp_wait_all();
         __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
+        if (kRegA > 0 && step == 0) {
+#pragma unroll
+            for (int x = 0; x < kRegA; ++x)
+#pragma unroll
+                for (int k = 0; k < KS; ++k) ldm_x4(own_a[x][k], ah_addr + x * W::kOwn + k * 32);
+        }
         if (step + 1 < total) load(step + 1, buf ^ 1);
         const uint32_t st = stages + buf * W::kStage;
         const int r0 = first + (KV ? step % steps : step) * BS;
@@ -375,21 +399,20 @@ __global__ void __launch_bounds__(kThreads, 2) rope_bwd_split_kernel(RopeParams 
         const uint32_t b_addr = st + lane_b<D>(lane);
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
-            uint32_t ah[4], al[4], ax[4];
-            ldm_x4(ah, ah_addr + k * 32);
-            ldm_x4(al, al_addr + k * 32);
-            ldm_x4(ax, ax_addr + k * 32);
+            uint32_t a[3][4], b[3][2][4];   // of the hi, lo and plain rows
 #pragma unroll
-            for (int np = 0; np < NT / 2; ++np) {
-                uint32_t bh4[4], bl4[4], bx[4];
-                ldm_x4(bh4, b_addr + np * 16 * Pitch<D>::kBytes + k * 32);
-                ldm_x4(bl4, b_addr + W::kTile + np * 16 * Pitch<D>::kBytes + k * 32);
-                ldm_x4(bx, b_addr + 2 * W::kTile + np * 16 * Pitch<D>::kBytes + k * 32);
-                mma_split(s[2 * np], ah, al, bh4[0], bh4[1], bl4[0], bl4[1]);
-                mma_split(s[2 * np + 1], ah, al, bh4[2], bh4[3], bl4[2], bl4[3]);
-                mma<T>(dp[2 * np], ax, bx[0], bx[1]);
-                mma<T>(dp[2 * np + 1], ax, bx[2], bx[3]);
+            for (int x = 0; x < 3; ++x) {
+                if (x < kRegA) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) a[x][e] = own_a[x < kRegA ? x : 0][k][e];
+                } else {
+                    ldm_x4(a[x], ah_addr + x * W::kOwn + k * 32);
+                }
+#pragma unroll
+                for (int y = 0; y < 2; ++y) ldm_x4(b[x][y], b_addr + x * W::kTile + y * 16 * Pitch<D>::kBytes + k * 32);
             }
+            mma4<T>(dp, a[2], b[2][0], b[2][1]);
+            mma4_split(s, a[0], a[1], b[0][0], b[0][1], b[1][0], b[1][1]);
         }
         // P and dS = P (dP - delta), in place of S and dP
         const bool edge = KV ? (p.causal && r0 < own0 + warp * 16 + 15) : (r0 + BS > N || (p.causal && r0 + BS - 1 > own0 + warp * 16));
@@ -413,20 +436,20 @@ __global__ void __launch_bounds__(kThreads, 2) rope_bwd_split_kernel(RopeParams 
             split_a<__nv_bfloat16>(dp[2 * t], dp[2 * t + 1], 1.f, dh, dl);
             if (KV) split_a<T>(s[2 * t], s[2 * t + 1], kPScale, ph, pl);
 #pragma unroll
-            for (int d = 0; d < DT / 2; ++d) {
+            for (int d = 0; d < DT / 2; d += 2) {
                 const uint32_t off = t * 16 * Pitch<D>::kBytes + d * 32;
-                uint32_t bh4[4], bl4[4];
-                ldm_x4_trans(bh4, t_addr + off);
-                ldm_x4_trans(bl4, t_addr + W::kTile + off);
-                mma_split(acc[2 * d], dh, dl, bh4[0], bh4[1], bl4[0], bl4[1]);
-                mma_split(acc[2 * d + 1], dh, dl, bh4[2], bh4[3], bl4[2], bl4[3]);
+                uint32_t bh0[4], bh1[4], bl0[4], bl1[4];
+                ldm_x4_trans(bh0, t_addr + off);
+                ldm_x4_trans(bh1, t_addr + off + 32);
+                ldm_x4_trans(bl0, t_addr + W::kTile + off);
+                ldm_x4_trans(bl1, t_addr + W::kTile + off + 32);
+                mma4_split(acc + 2 * d, dh, dl, bh0, bh1, bl0, bl1);
                 if (KV) {
-                    uint32_t bx[4];
-                    ldm_x4_trans(bx, t_addr + 2 * W::kTile + off);
-                    mma<T>(dv[KV ? 2 * d : 0], ph, bx[0], bx[1]);
-                    mma<T>(dv[KV ? 2 * d + 1 : 0], ph, bx[2], bx[3]);
-                    mma<T>(dv[KV ? 2 * d : 0], pl, bx[0], bx[1]);
-                    mma<T>(dv[KV ? 2 * d + 1 : 0], pl, bx[2], bx[3]);
+                    uint32_t bx0[4], bx1[4];
+                    ldm_x4_trans(bx0, t_addr + 2 * W::kTile + off);
+                    ldm_x4_trans(bx1, t_addr + 2 * W::kTile + off + 32);
+                    mma4<T>(dv + (KV ? 2 * d : 0), ph, bx0, bx1);
+                    mma4<T>(dv + (KV ? 2 * d : 0), pl, bx0, bx1);
                 }
             }
         }
