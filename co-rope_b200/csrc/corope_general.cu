@@ -85,18 +85,87 @@ __device__ __forceinline__ void stage_plain(float* dst, int ld, const T* X, int6
     }
 }
 
+// fp32 tensors: K and V tiles by asynchronous copies into two buffers, the next tile in flight behind the current one.  (Small grids
+// put one CTA on an SM, which then waited for every tile's loads: B1 Hq8 Hkv2 N512 D64 forward + backward 287 -> 228 us, with P and
+// the leader dot products off the shuffle and multiply-add chains.)  16-bit tensors need a conversion and are staged through
+// registers; their grids are large.
+template <typename T, int D>
+struct Tiles {
+    static constexpr bool kAsync = sizeof(T) == 4;
+    static constexpr int kBufs = kAsync ? 2 : 1;
+};
+// kTile rows [r0, r0 + kTile) of X, rows at or beyond N as zeros (one commit group per call of the caller)
+template <int D>
+__device__ __forceinline__ void copy_tile(float* dst, int ld, const float* X, int64_t xs, int r0, int N, bool vec) {
+    if (vec) {
+#pragma unroll
+        for (int it = 0; it < kTile * D / 4 / kThreads; ++it) {
+            const int idx = threadIdx.x + it * kThreads, r = idx / (D / 4), d = idx % (D / 4) * 4;
+            const bool have = r0 + r < N;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst + r * ld + d)), "l"(X + (int64_t)(have ? r0 + r : 0) * xs + d),
+                         "r"(have ? 16 : 0)
+                         : "memory");
+        }
+    } else {
+        for (int idx = threadIdx.x; idx < kTile * D; idx += kThreads) {
+            const int r = idx / D, d = idx % D;
+            const bool have = r0 + r < N;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(dst + r * ld + d)), "l"(X + (int64_t)(have ? r0 + r : 0) * xs + d),
+                         "r"(have ? 4 : 0)
+                         : "memory");
+        }
+    }
+}
+__device__ __forceinline__ bool vec_rows(const float* X, int64_t xs) { return ((uintptr_t)X % 16) == 0 && xs % 4 == 0; }
+
+// dot product of two rows of D floats in shared memory: four independent chains
+template <int D>
+__device__ __forceinline__ float row_dot(const float* x, const float* y) {
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int d = 0; d < D; d += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + d);
+        const float4 b = *reinterpret_cast<const float4*>(y + d);
+        s[0] = fmaf(a.x, b.x, s[0]);
+        s[1] = fmaf(a.y, b.y, s[1]);
+        s[2] = fmaf(a.z, b.z, s[2]);
+        s[3] = fmaf(a.w, b.w, s[3]);
+    }
+    return (s[0] + s[1]) + (s[2] + s[3]);
+}
+
+// G floats that every lane of the warp reads at one address
+template <int G>
+__device__ __forceinline__ void load_heads(float (&x)[G], const float* src) {
+    if constexpr (G % 4 == 0) {
+#pragma unroll
+        for (int h = 0; h < G; h += 4) {
+            const float4 v = *reinterpret_cast<const float4*>(src + h);
+            x[h] = v.x; x[h + 1] = v.y; x[h + 2] = v.z; x[h + 3] = v.w;
+        }
+    } else {
+#pragma unroll
+        for (int h = 0; h < G; ++h) x[h] = src[h];
+    }
+}
+
 // ------------------------------------------------------------------------------------------------
 // forward
 // ------------------------------------------------------------------------------------------------
+template <typename T, int D, int G> constexpr size_t fwd_smem_bytes() {
+    return sizeof(float) * ((size_t)G * kWarps * D + Tiles<T, D>::kBufs * (kTile * (D + kPad) + kTile * D) + D / 2 + kWarps * kTile * G);
+}
 template <typename T, int D, int G, bool ACCURATE>
 __global__ void __launch_bounds__(kThreads) corope_fwd_general_kernel(GqaParams p) {
     constexpr int H2 = D / 2;
     constexpr int NC = D / 32;
     extern __shared__ __align__(16) float smem[];
-    float* q_s = smem;                         // [G][8][D]
-    float* k_s = q_s + G * kWarps * D;         // [32][D+1]
-    float* v_s = k_s + kTile * (D + kPad);        // [32][D]
-    float* w_s = v_s + kTile * D;              // [H2] inverse frequencies
+    using L = Tiles<T, D>;
+    float* q_s = smem;                                      // [G][8][D]
+    float* k_b = q_s + G * kWarps * D;                      // kBufs x [32][D+4]
+    float* v_b = k_b + L::kBufs * kTile * (D + kPad);       // kBufs x [32][D]
+    float* xp = v_b + L::kBufs * kTile * D;                 // [8][32][G] P
+    float* w_s = xp + kWarps * kTile * G;                   // [H2] inverse frequencies
 
     const int N = p.N;
     const int bg = blockIdx.y;                 // b * Hkv + g
@@ -124,27 +193,36 @@ __global__ void __launch_bounds__(kThreads) corope_fwd_general_kernel(GqaParams 
     const float sc2 = p.sm_scale * kLog2e;
     const bool direct = p.N <= 8192;
     const int i_last = min(N - 1, i0 + kWarps - 1);
-    for (int j0 = (i_last / kTile) * kTile; j0 >= 0; j0 -= kTile) {
-        __syncthreads();
-        stage_plain<T, D>(k_s, D + kPad, K, p.sk.n, j0, kTile, N);
-        stage_plain<T, D>(v_s, D, V, p.sv.n, j0, kTile, N);
-        __syncthreads();
+    const int j_first = (i_last / kTile) * kTile;
+    bool k_vec = false, v_vec = false;
+    if constexpr (L::kAsync) {
+        k_vec = vec_rows(K, p.sk.n), v_vec = vec_rows(V, p.sv.n);
+        copy_tile<D>(k_b, D + kPad, K, p.sk.n, j_first, N, k_vec);
+        copy_tile<D>(v_b, D, V, p.sv.n, j_first, N, v_vec);
+    }
+    int buf = 0;
+    for (int j0 = j_first; j0 >= 0; j0 -= kTile, buf ^= L::kBufs - 1) {
+        float *k_s = k_b + buf * kTile * (D + kPad), *v_s = v_b + buf * kTile * D;
+        if constexpr (L::kAsync) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
+            if (j0 >= kTile) {
+                copy_tile<D>(k_b + (buf ^ 1) * kTile * (D + kPad), D + kPad, K, p.sk.n, j0 - kTile, N, k_vec);
+                copy_tile<D>(v_b + (buf ^ 1) * kTile * D, D, V, p.sv.n, j0 - kTile, N, v_vec);
+            }
+        } else {
+            __syncthreads();
+            stage_plain<T, D>(k_s, D + kPad, K, p.sk.n, j0, kTile, N);
+            stage_plain<T, D>(v_s, D, V, p.sv.n, j0, kTile, N);
+            __syncthreads();
+        }
         if (i >= N) continue;
         const int j = j0 + lane;
         const bool vis = (j <= i);  // implies j < N
         const float* kr = k_s + lane * (D + kPad);
         const float* qL = q_s + warp * D;
         // leader score -> z   (16-byte shared-memory loads throughout: the loop is load-issue bound otherwise)
-        float dot = 0.f;
-#pragma unroll 4
-        for (int d = 0; d < D; d += 4) {
-            const float4 a = *reinterpret_cast<const float4*>(qL + d);
-            const float4 b = *reinterpret_cast<const float4*>(kr + d);
-            dot = fmaf(a.x, b.x, dot);
-            dot = fmaf(a.y, b.y, dot);
-            dot = fmaf(a.z, b.z, dot);
-            dot = fmaf(a.w, b.w, dot);
-        }
+        const float dot = row_dot<D>(qL, kr);
         float z = vis ? 1.f / (1.f + __expf(-dot * p.sm_scale)) : 0.f;
         // Delta_ij = sum_{k=j+1..i} z_ik = carry + (suffix over lanes above this one)
         float suf = warp_suffix_incl(z, lane);
@@ -189,29 +267,32 @@ __global__ void __launch_bounds__(kThreads) corope_fwd_general_kernel(GqaParams 
             float mx = fmaxf(m[h], warp_max(sv));
             float alpha = exp2f(m[h] - mx);   // first tile holds the diagonal, so mx is finite
             float pv = vis ? exp2f(sv - mx) : 0.f;
-            l[h] = l[h] * alpha + warp_sum(pv);
+            l[h] = l[h] * alpha + pv;         // this lane's keys only, added up at the end
             m[h] = mx;
 #pragma unroll
             for (int c = 0; c < NC; ++c) acc[h][c] *= alpha;
-            s[h] = pv;
+            xp[(warp * kTile + lane) * G + h] = pv;
         }
+        __syncwarp();
 #pragma unroll 4
         for (int jj = 0; jj < kTile; ++jj) {
             float vv[NC];
 #pragma unroll
             for (int c = 0; c < NC; ++c) vv[c] = v_s[jj * D + lane + 32 * c];
+            float pj[G];
+            load_heads<G>(pj, xp + (warp * kTile + jj) * G);
 #pragma unroll
-            for (int h = 0; h < G; ++h) {
-                float pj = __shfl_sync(0xffffffffu, s[h], jj);
+            for (int h = 0; h < G; ++h)
 #pragma unroll
-                for (int c = 0; c < NC; ++c) acc[h][c] = fmaf(pj, vv[c], acc[h][c]);
-            }
+                for (int c = 0; c < NC; ++c) acc[h][c] = fmaf(pj[h], vv[c], acc[h][c]);
         }
+        __syncwarp();   // every lane has read P before the next tile's overwrites it
     }
     if (i < N) {
 #pragma unroll
         for (int h = 0; h < G; ++h) {
             T* O = reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.Hq, (int)q_head0 + h, i);
+            l[h] = warp_sum(l[h]);
             float inv = 1.f / l[h];
 #pragma unroll
             for (int c = 0; c < NC; ++c) O[lane + 32 * c] = Elem<T>::from_f32(acc[h][c] * inv);
@@ -254,28 +335,17 @@ __global__ void gqa_finalize_kernel(const float* __restrict__ dk_acc, const floa
 
 // Shared memory of the backward (floats).  The (cos, sin) of every (row, key, pair) of a tile are kept from the score phase for the
 // two gradient phases where they fit and are worth it: sincosf costs some 40 instructions, the hardware approximations two.
-template <int D, int G, bool ACCURATE> struct BwdSmem {
+template <typename T, int D, int G, bool ACCURATE> struct BwdSmem {
     static constexpr int kPitch = D + 2;                          // floats per (row, key) of the (cos, sin) table: lane = key writes 8 bytes without conflicts
-    static constexpr size_t kBase = (size_t)2 * G * kWarps * D + 2 * kTile * (D + kPad) + D / 2 + (size_t)kWarps * kTile * (2 * G + 2);
-    static constexpr size_t kTable = (size_t)kWarps * kTile * kPitch;
-    static constexpr bool kStore = (ACCURATE || D <= 64) && (kBase + kTable) * sizeof(float) <= 225 * 1024;
-    static constexpr size_t kBytes = (kBase + (kStore ? kTable : 0)) * sizeof(float);
+    static constexpr size_t kTile2 = 2 * kTile * (D + kPad);      // one tile of K and of V
+    static constexpr size_t kBase = (size_t)2 * G * kWarps * D + kTile2 + D / 2 + (size_t)kWarps * kTile * (2 * G + 2);
+    static constexpr size_t kTable = (size_t)kWarps * kTile * kPitch, kMost = 225 * 1024 / sizeof(float);
+    static constexpr bool kStore = (ACCURATE || D <= 64) && kBase + kTable <= kMost;
+    // the second buffer of fp32 tiles where the table leaves room for it
+    static constexpr bool kAsync = Tiles<T, D>::kAsync && kBase + kTile2 + (kStore ? kTable : 0) <= kMost;
+    static constexpr int kBufs = kAsync ? 2 : 1;
+    static constexpr size_t kBytes = (kBase + (kAsync ? kTile2 : 0) + (kStore ? kTable : 0)) * sizeof(float);
 };
-
-// G floats that every lane of the warp reads at one address
-template <int G>
-__device__ __forceinline__ void load_heads(float (&x)[G], const float* src) {
-    if constexpr (G % 4 == 0) {
-#pragma unroll
-        for (int h = 0; h < G; h += 4) {
-            const float4 v = *reinterpret_cast<const float4*>(src + h);
-            x[h] = v.x; x[h + 1] = v.y; x[h + 2] = v.z; x[h + 3] = v.w;
-        }
-    } else {
-#pragma unroll
-        for (int h = 0; h < G; ++h) x[h] = src[h];
-    }
-}
 
 // Three phases per tile of 32 keys.  A: warp = row, lane = key: scores, P, dS, mileage gradient.  B1: warp = row, lane = pair: dq.
 // B2: warp = 4 keys, lane = pair / column: dk and dv summed over the CTA's 8 rows in registers, one global reduction per tile.
@@ -284,7 +354,7 @@ __device__ __forceinline__ void load_heads(float (&x)[G], const float* src) {
 // issue slots and, at small grids, the latency of one CTA's chain of tiles.
 template <typename T, int D, int G, bool ACCURATE>
 __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams p) {
-    using M = BwdSmem<D, G, ACCURATE>;
+    using M = BwdSmem<T, D, G, ACCURATE>;
     constexpr int H2 = D / 2;
     constexpr int NC = D / 32;                    // head-dim columns per lane
     constexpr int NPI = (H2 + 31) / 32;           // (d, d + D/2) pairs per lane
@@ -292,9 +362,9 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
     extern __shared__ __align__(16) float smem[];
     float* q_s = smem;                            // [G][8][D]
     float* do_s = q_s + G * kWarps * D;           // [G][8][D]
-    float* k_s = do_s + G * kWarps * D;           // [32][D+4]
-    float* v_s = k_s + kTile * (D + kPad);        // [32][D+4]
-    float* xg = v_s + kTile * (D + kPad);         // [8][32][G] dS * sm_scale
+    float* k_b = do_s + G * kWarps * D;           // kBufs x [32][D+4]
+    float* v_b = k_b + M::kBufs * kTile * (D + kPad);   // kBufs x [32][D+4]
+    float* xg = v_b + M::kBufs * kTile * (D + kPad);    // [8][32][G] dS * sm_scale
     float* xp = xg + kWarps * kTile * G;          // [8][32][G] P
     float* xd = xp + kWarps * kTile * G;          // [8][32] Delta
     float* xr = xd + kWarps * kTile;              // [8][32] graw
@@ -342,11 +412,28 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
             sincos_phase<ACCURATE>(xd[r * kTile + jj] * w_s[pd], sn, cs, direct);
         }
     };
-    for (int j0 = 0; j0 <= i_last; j0 += kTile) {
-        __syncthreads();   // the previous tile has been used
-        stage_plain<T, D>(k_s, D + kPad, K, p.sk.n, j0, kTile, N);
-        stage_plain<T, D>(v_s, D + kPad, V, p.sv.n, j0, kTile, N);
-        __syncthreads();
+    bool k_vec = false, v_vec = false;
+    if constexpr (M::kAsync) {
+        k_vec = vec_rows(K, p.sk.n), v_vec = vec_rows(V, p.sv.n);
+        copy_tile<D>(k_b, D + kPad, K, p.sk.n, 0, N, k_vec);
+        copy_tile<D>(v_b, D + kPad, V, p.sv.n, 0, N, v_vec);
+    }
+    int buf = 0;
+    for (int j0 = 0; j0 <= i_last; j0 += kTile, buf ^= M::kBufs - 1) {
+        float *k_s = k_b + buf * kTile * (D + kPad), *v_s = v_b + buf * kTile * (D + kPad);
+        if constexpr (M::kAsync) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();   // the tile has landed for every thread, and the previous one has been used
+            if (j0 + kTile <= i_last) {
+                copy_tile<D>(k_b + (buf ^ 1) * kTile * (D + kPad), D + kPad, K, p.sk.n, j0 + kTile, N, k_vec);
+                copy_tile<D>(v_b + (buf ^ 1) * kTile * (D + kPad), D + kPad, V, p.sv.n, j0 + kTile, N, v_vec);
+            }
+        } else {
+            __syncthreads();   // the previous tile has been used
+            stage_plain<T, D>(k_s, D + kPad, K, p.sk.n, j0, kTile, N);
+            stage_plain<T, D>(v_s, D + kPad, V, p.sv.n, j0, kTile, N);
+            __syncthreads();
+        }
         if (i < N && j0 <= i) {
             // ---------------- phase A: lane = key
             const int j = j0 + lane;
@@ -355,16 +442,7 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
             const float* vr = v_s + lane * (D + kPad);
             const float* qL = q_s + warp * D;
             float* cs_out = cs_s + (warp * kTile + lane) * M::kPitch;
-            float dot = 0.f;
-#pragma unroll 4
-            for (int d = 0; d < D; d += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(qL + d);
-                const float4 b = *reinterpret_cast<const float4*>(kr + d);
-                dot = fmaf(a.x, b.x, dot);
-                dot = fmaf(a.y, b.y, dot);
-                dot = fmaf(a.z, b.z, dot);
-                dot = fmaf(a.w, b.w, dot);
-            }
+            const float dot = row_dot<D>(qL, kr);
             const float z = vis ? 1.f / (1.f + __expf(-dot * p.sm_scale)) : 0.f;
             const float pre = warp_prefix_incl(z, lane);
             const float delta = a_ii - (carry_a + pre);
@@ -547,7 +625,7 @@ __global__ void __launch_bounds__(kThreads) corope_bwd_general_kernel(GqaParams 
 template <typename T, int D, int G>
 int launch_fwd_g(const GqaParams& p, cudaStream_t s) {
     constexpr bool kAcc = (Elem<T>::kDtype == COROPE_DTYPE_F32);
-    size_t smem = sizeof(float) * ((size_t)G * kWarps * D + kTile * (D + kPad) + kTile * D + D / 2);
+    constexpr size_t smem = fwd_smem_bytes<T, D, G>();
     auto kern = corope_fwd_general_kernel<T, D, G, kAcc>;
     static std::atomic<uint64_t> smem_ok;
     if (int er = allow_smem(kern, smem, smem_ok)) return er;
@@ -559,7 +637,7 @@ int launch_fwd_g(const GqaParams& p, cudaStream_t s) {
 template <typename T, int D, int G>
 int launch_bwd_g(const GqaParams& p, cudaStream_t s) {
     constexpr bool kAcc = (Elem<T>::kDtype == COROPE_DTYPE_F32);
-    constexpr size_t smem = BwdSmem<D, G, kAcc>::kBytes;
+    constexpr size_t smem = BwdSmem<T, D, G, kAcc>::kBytes;
     auto kern = corope_bwd_general_kernel<T, D, G, kAcc>;
     static std::atomic<uint64_t> smem_ok;
     if (int er = allow_smem(kern, smem, smem_ok)) return er;

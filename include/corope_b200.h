@@ -94,7 +94,7 @@ size_t corope_workspace_bytes(int op, int B, int Hq, int Hkv, int N, int D, int 
  * then go to kernels that split every fp32 operand into two 16-bit ones and keep fp32 accuracy; so does the Co-RoPE forward at D = 64,
  * a ragged N or rows that are not aligned to 16 bytes.  A call that is handed at
  * least this much uses them; with corope_workspace_bytes() bytes a ragged N runs on the CUDA-core kernels.
- * Never more than corope_workspace_bytes() where N is a whole number of tiles. */
+ * Never more than corope_workspace_bytes() where N is a whole number of tiles (Co-RoPE at D = 64 excepted). */
 size_t corope_workspace_bytes_any_n(int op, int B, int Hq, int Hkv, int N, int D, int dtype);
 
 /*
