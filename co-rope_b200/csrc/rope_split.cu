@@ -1,23 +1,28 @@
 // Fused-RoPE / plain attention for 16-bit tensors at lengths that are not whole 128-row tiles, D = 64 or 128: tensor-core products
-// (mma.sync m16n8k16) with fp32 precision kept by splitting.  Every fp32 operand x enters the MMAs as hi + lo, hi = x rounded to 16
-// bits and lo = (x - hi) rounded:
-//     S  = Q~ K~^T        Q~, K~ rotated in fp32, both split into bf16 pairs    3 MMAs (hi hi, hi lo, lo hi; lo lo is below 2^-17)
-//     dP = dO V^T         inputs as they are                                    1 MMA
-//     O += P V, dV += P^T dO     P split into the inputs' own type              2 MMAs
-//     dQ += dS K~, dK += dS^T Q~  dS split into bf16                            3 MMAs
-// bf16 for everything that is not bounded, so that no magnitude of the inputs leaves the range.  These lengths have always run with
-// fp32 operands and keep that accuracy (2-norm error against 64-bit arithmetic, N(0, 1) inputs, B1 H4 N1777 D128 causal, f16:
-// O 2.008e-4 and dV 2.04e-4, dQ and dK 2.25e-4, all of it the rounding of the results, to the third digit what the CUDA-core kernels
-// show; the tcgen05 kernels with their 16-bit P and Q~, K~: 3.6e-4, 3.9e-4, 4.7e-4).  The pairs carry 16 bits: scores of some
-// hundred would begin to show in f16 results.
+// (mma.sync m16n8k16) of fp32 operands.  Every fp32 operand x enters the MMAs as hi + mid + lo, hi = x rounded to 16 bits, mid = (x - hi)
+// rounded, lo = the rest.  Three bf16 numbers hold the 24 bits of an fp32 number exactly, so nothing is lost in the operands:
+//     S  = Q~ K~^T        Q~, K~ rotated in fp32, both split into bf16      6 MMAs (without mid lo, lo mid, lo lo: below 2^-24)
+//     dP = dO V^T         inputs as they are                                1 MMA
+//     O += P V, dV += P^T dO     P split into the inputs' own type          3 MMAs
+//     dQ += dS K~, dK += dS^T Q~  dS split into bf16                        6 MMAs
+// bf16 for everything that is not bounded, so that no magnitude of the inputs leaves the range.  P <= 1 of f16 tensors enters its
+// products times 2^14: the three numbers then reach down to 2^-38 of the row's largest probability.  The adder of the MMAs does not round to
+// nearest; the large products therefore go through short chains (their own accumulators for a row's scores, one 16-row step for the
+// sums over keys or queries), which fp32 additions join.
 //
-// B1 H32 N1777 D128 bf16 causal forward 222 us (116 TFLOP/s; the CUDA-core kernel 909 us), B4 H16 N1000 D64 bf16 full forward +
-// backward 584 us (98 TFLOP/s; 3473 us).
-// What bounds it: mma.sync, measured at 553 TFLOP/s with all operands in registers (B200, 8 warps per SM), of which the split
-// products use about 300: with 8 warps per SM (D = 128: 255 registers; D = 64: 12 warps) the latency between a tile's ldmatrix, MMAs
-// and softmax is not fully hidden, and the shared-memory port is close behind, a warp's 16 rows reading every streamed tile, hi
-// and lo, once per product.  tcgen05 would need the split tiles of all operands resident (Q~ hi / lo, K~ hi / lo, V of 128 x 128:
-// 160 KB before any ring), so one stage of everything and no overlap.
+// Error against 64-bit arithmetic next to the CUDA-core kernels with fp32 operands (N(0, 1) inputs, B1 H4 N1777 D128 causal f16): LSE
+// 3.75e-7 (3.87e-7), results that are not the exact one rounded: O 0.11 % (0.33 %), dV 0.21 % (0.36 %); with q and k times 4 (scores
+// with a standard deviation of 16) LSE 4.5e-6 (1.2e-5), O 0.29 % (0.71 %).  Two parts per operand (16 bits; half the MMAs, half the time)
+// had 2 to 10 times the error of the fp32 kernels.
+//
+// B1 H32 N1777 D128 bf16 causal forward 405 us (64 TFLOP/s; the CUDA-core kernel 909 us), backward 1262 us (5081 us); B4 H16 N1000 D64
+// bf16 full forward 244 us (572 us), backward 763 us (2890 us).  Below some 100 rows the CUDA-core forward is as fast or faster (B1 H1
+// N50 D128 12.6 against 16.8 us with the host's part), its backward never.
+// What bounds it: mma.sync, measured at 553 TFLOP/s with all operands in registers (B200, 8 warps per SM); with 8 warps per SM
+// (D = 128: 255 registers; D = 64: 12 warps) the latency between a tile's ldmatrix, MMAs and softmax is not fully hidden, and the
+// shared-memory port is close behind, a warp's 16 rows reading every streamed tile, all three parts of it, once per product.
+// Infinities in Q or K keep the scores they have in fp32; beyond that non-finite operands give NaN, also where fp32 sums would
+// have been infinite.
 //
 // Math: fused-rope/rope_attn_pytorch.py:108-155 (forward), :187-222 (backward); exp2-domain softmax and log2-domain LSE as
 // fused-rope/fused_rope_attn.py:103-114, 316.
@@ -25,9 +30,6 @@
 
 namespace corope {
 namespace {
-
-constexpr int kThreads = 128;   // 4 warps of 16 rows
-constexpr int kRows = 64;       // rows a CTA owns
 
 // ------------------------------------------------------------------------------------------------ operands
 // row-major 16-bit tile in shared memory: rows of D elements + 16 bytes, so that 8 consecutive rows of an ldmatrix fall into
@@ -65,26 +67,86 @@ __device__ __forceinline__ void mma4(float (*d)[4], const uint32_t (&a)[4], cons
     mma<T>(d[2], a, b1[0], b1[1]);
     mma<T>(d[3], a, b1[2], b1[3]);
 }
-// d += (ah + al) (bh + bl) without the product of the two small halves
-__device__ __forceinline__ void mma4_split(float (*d)[4], const uint32_t (&ah)[4], const uint32_t (&al)[4], const uint32_t (&bh0)[4], const uint32_t (&bh1)[4],
-                                           const uint32_t (&bl0)[4], const uint32_t (&bl1)[4]) {
-    mma4<__nv_bfloat16>(d, ah, bh0, bh1);
-    mma4<__nv_bfloat16>(d, ah, bl0, bl1);
-    mma4<__nv_bfloat16>(d, al, bh0, bh1);
+// d += t for four neighbouring accumulator tiles, rounded to nearest
+__device__ __forceinline__ void add4(float (*d)[4], const float (&t)[4][4]) {
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int x = 0; x < 4; ++x) d[n][x] += t[n][x];
+}
+// product of two split operands for four neighbouring accumulator tiles, b[part][two ldmatrix_x4 results]: hi hi into `d`, the five
+// smaller ones into `e`, smallest first
+__device__ __forceinline__ void mma4_split(float (*d)[4], float (*e)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2][4]) {
+    using B = __nv_bfloat16;
+    float t[4][4] = {};
+    mma4<B>(e, a[1], b[1][0], b[1][1]);
+    mma4<B>(e, a[0], b[2][0], b[2][1]);
+    mma4<B>(e, a[2], b[0][0], b[0][1]);
+    mma4<B>(t, a[0], b[0][0], b[0][1]);
+    mma4<B>(e, a[0], b[1][0], b[1][1]);
+    mma4<B>(e, a[1], b[0][0], b[0][1]);
+    add4(d, t);
+}
+// hi hi + the smaller products.  An infinity shows in hi hi with the sign it has in fp32; the other parts of such a product are
+// meaningless (0 or either infinity).
+__device__ __forceinline__ float join(float main, float small) { return fabsf(main) < INFINITY ? main + small : main; }
+// parts[] = hi, mid, lo of (a, b); a non-finite number is its own hi
+template <typename T>
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&parts)[3]) {
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        parts[x] = pack2<T>(a, b);
+        const float2 f = unpack2<T>(parts[x]);
+        a -= f.x;
+        b -= f.y;
+    }
 }
 template <typename T>
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
-    hi = pack2<T>(a, b);
-    const float2 f = unpack2<T>(hi);
-    lo = pack2<T>(a - f.x, b - f.y);
+__device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3]) {
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        parts[x] = pack2<T>(a, b);
+        const float2 f = unpack2<T>(parts[x]);
+        a = fabsf(a - f.x) < INFINITY ? a - f.x : 0.f;
+        b = fabsf(b - f.y) < INFINITY ? b - f.y : 0.f;
+    }
 }
-// two neighbouring 8-column accumulator tiles as the A operand of one k-step, split
+// two neighbouring 8-column accumulator tiles as the A operand of one k-step, split: a[part]
 template <typename T>
-__device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[4], float scale, uint32_t (&hi)[4], uint32_t (&lo)[4]) {
-    split2<T>(c0[0] * scale, c0[1] * scale, hi[0], lo[0]);
-    split2<T>(c0[2] * scale, c0[3] * scale, hi[1], lo[1]);
-    split2<T>(c1[0] * scale, c1[1] * scale, hi[2], lo[2]);
-    split2<T>(c1[2] * scale, c1[3] * scale, hi[3], lo[3]);
+__device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[4], float scale, uint32_t (&a)[3][4]) {
+    uint32_t w[4][3];
+    split3<T>(c0[0] * scale, c0[1] * scale, w[0]);
+    split3<T>(c0[2] * scale, c0[3] * scale, w[1]);
+    split3<T>(c1[0] * scale, c1[1] * scale, w[2]);
+    split3<T>(c1[2] * scale, c1[3] * scale, w[3]);
+#pragma unroll
+    for (int x = 0; x < 3; ++x)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) a[x][e] = w[e][x];
+}
+// P of f16 tensors enters its products times this
+template <typename T> constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 16384.f : 1.f;
+
+// d += P b for four neighbouring tiles of columns, one 16-row step: its own sum, then one fp32 addition
+template <typename T>
+__device__ __forceinline__ void add_products(float (*d)[4], const uint32_t (&a)[3][4], const uint32_t (&b0)[4], const uint32_t (&b1)[4]) {
+    float t[4][4] = {};
+    mma4<T>(t, a[2], b0, b1);
+    mma4<T>(t, a[1], b0, b1);
+    mma4<T>(t, a[0], b0, b1);
+    add4(d, t);
+}
+// the same with both operands split
+__device__ __forceinline__ void add_products_split(float (*d)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2][4]) {
+    float t[4][4] = {};
+    using B = __nv_bfloat16;
+    mma4<B>(t, a[1], b[1][0], b[1][1]);
+    mma4<B>(t, a[0], b[2][0], b[2][1]);
+    mma4<B>(t, a[2], b[0][0], b[0][1]);
+    mma4<B>(t, a[0], b[1][0], b[1][1]);
+    mma4<B>(t, a[1], b[0][0], b[0][1]);
+    mma4<B>(t, a[0], b[0][0], b[0][1]);
+    add4(d, t);
 }
 
 // 16 bytes global -> shared, zeros when `have` is false (the address is then not read)
@@ -96,23 +158,34 @@ __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_grou
 __device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // ROWS rows [r0, r0 + ROWS) of X (row stride xs elements) into a padded tile, rows at or beyond N as zeros
-template <int D, int ROWS, typename E>
+template <int D, int ROWS, int THREADS, typename E>
 __device__ __forceinline__ void load_rows(uint32_t dst, const E* X, int64_t xs, int r0, int N) {
     constexpr int kPerRow = D / 8;
 #pragma unroll
-    for (int it = 0; it < ROWS * kPerRow / kThreads; ++it) {
-        const int idx = threadIdx.x + it * kThreads, r = idx / kPerRow, ch = idx % kPerRow, pos = r0 + r;
+    for (int it = 0; it < ROWS * kPerRow / THREADS; ++it) {
+        const int idx = threadIdx.x + it * THREADS, r = idx / kPerRow, ch = idx % kPerRow, pos = r0 + r;
         const bool have = pos < N;
         cp16(dst + r * Pitch<D>::kBytes + ch * 16, X + (int64_t)(have ? pos : 0) * xs + ch * 8, have);
     }
 }
 
+struct SplitRows {   // three bf16 copies [B, H, N, D], `plane` elements apart: hi, mid, lo
+    __nv_bfloat16* rows;
+    size_t plane;
+};
+// the three parts of ROWS rows of head `head` into three tiles `step` bytes apart
+template <int D, int ROWS, int THREADS>
+__device__ __forceinline__ void load_split(uint32_t dst, uint32_t step, const SplitRows& x, int head, int r0, int N) {
+#pragma unroll
+    for (int part = 0; part < 3; ++part) load_rows<D, ROWS, THREADS>(dst + part * step, x.rows + part * x.plane + (size_t)head * N * D, D, r0, N);
+}
+
 // ------------------------------------------------------------------------------------------------
-// pre-pass: rows of X rotated in fp32, times `scale`, as bf16 hi and lo copies [B, H, N, D].  One thread per 8 pairs.
+// pre-pass: rows of X rotated in fp32, times `scale`, split.  One thread per 8 pairs.
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
 __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__ X, RowAddr ax, const float* __restrict__ cosT, const float* __restrict__ sinT,
-                                                           int64_t ts, float scale, __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo, size_t rows) {
+                                                           int64_t ts, float scale, SplitRows out, size_t rows) {
     constexpr int kPerRow = D / 16;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     const size_t row = idx / kPerRow;
@@ -121,7 +194,7 @@ __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__
     const T* src = X + flat_row_offset(ax, row) + d;
     const uint4 xa = *reinterpret_cast<const uint4*>(src), xb = *reinterpret_cast<const uint4*>(src + D / 2);
     const uint32_t a[4] = {xa.x, xa.y, xa.z, xa.w}, b[4] = {xb.x, xb.y, xb.z, xb.w};
-    uint32_t ha[4], la[4], hb[4], lb[4];
+    uint32_t pa[4][3], pb[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
@@ -130,58 +203,58 @@ __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__
             const float *c = cosT + (int64_t)n * ts + d + 2 * e, *s = sinT + (int64_t)n * ts + d + 2 * e;
             c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
         }
-        split2<__nv_bfloat16>((fa.x * c0 - fb.x * s0) * scale, (fa.y * c1 - fb.y * s1) * scale, ha[e], la[e]);
-        split2<__nv_bfloat16>((fb.x * c0 + fa.x * s0) * scale, (fb.y * c1 + fa.y * s1) * scale, hb[e], lb[e]);
+        split3_any<__nv_bfloat16>((fa.x * c0 - fb.x * s0) * scale, (fa.y * c1 - fb.y * s1) * scale, pa[e]);
+        split3_any<__nv_bfloat16>((fb.x * c0 + fa.x * s0) * scale, (fb.y * c1 + fa.y * s1) * scale, pb[e]);
     }
-    __nv_bfloat16 *h = hi + row * D + d, *l = lo + row * D + d;
-    *reinterpret_cast<uint4*>(h) = make_uint4(ha[0], ha[1], ha[2], ha[3]);
-    *reinterpret_cast<uint4*>(h + D / 2) = make_uint4(hb[0], hb[1], hb[2], hb[3]);
-    *reinterpret_cast<uint4*>(l) = make_uint4(la[0], la[1], la[2], la[3]);
-    *reinterpret_cast<uint4*>(l + D / 2) = make_uint4(lb[0], lb[1], lb[2], lb[3]);
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+        __nv_bfloat16* o = out.rows + part * out.plane + row * D + d;
+        *reinterpret_cast<uint4*>(o) = make_uint4(pa[0][part], pa[1][part], pa[2][part], pa[3][part]);
+        *reinterpret_cast<uint4*>(o + D / 2) = make_uint4(pb[0][part], pb[1][part], pb[2][part], pb[3][part]);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------
-// forward: 64 query rows per CTA, key tiles of 64, double-buffered
+// forward: 64 query rows per CTA (4 warps of 16), double-buffered key tiles of 64 (D = 64) or 32 keys
 // ------------------------------------------------------------------------------------------------
 template <int D> struct Fwd {
-    static constexpr int kBN = 64;
+    static constexpr int kThreads = 128, kRows = 64, kCtas = D == 64 ? 3 : 2;
+    static constexpr int kBN = D == 64 ? 64 : 32;
     static constexpr uint32_t kTile = kBN * Pitch<D>::kBytes;
-    static constexpr uint32_t kStage = 3 * kTile;   // K~ hi, K~ lo, V
+    static constexpr uint32_t kStage = 4 * kTile;   // K~ hi, mid, lo, V
     static constexpr size_t kSmem = 2 * kStage;
 };
 
 template <typename T, int D>
-__global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kernel(RopeParams p, const __nv_bfloat16* __restrict__ k_hi, const __nv_bfloat16* __restrict__ k_lo) {
+__global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_split_kernel(RopeParams p, SplitRows ks) {
     using F = Fwd<D>;
     constexpr int BN = F::kBN, KS = D / 16, NT = BN / 8, DT = D / 8;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sm = smem_u32(smem);
     // heads run fastest and the longest causal rows come first
     const int N = p.N, bh = blockIdx.x, kvh = bh / (p.H / p.Hkv);
-    const int m0 = (gridDim.y - 1 - blockIdx.y) * kRows;
+    const int m0 = (gridDim.y - 1 - blockIdx.y) * F::kRows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int row0 = m0 + warp * 16 + g;   // the lane's rows: row0 and row0 + 8
     const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0);
-    const __nv_bfloat16 *KH = k_hi + (size_t)kvh * N * D, *KL = k_lo + (size_t)kvh * N * D;
     auto load = [&](int j0, int buf) {
         const uint32_t st = sm + buf * F::kStage;
-        load_rows<D, BN>(st, KH, D, j0, N);
-        load_rows<D, BN>(st + F::kTile, KL, D, j0, N);
-        load_rows<D, BN>(st + 2 * F::kTile, V, p.sv.n, j0, N);
+        load_split<D, BN, F::kThreads>(st, F::kTile, ks, kvh, j0, N);
+        load_rows<D, BN, F::kThreads>(st + 3 * F::kTile, V, p.sv.n, j0, N);
         cp_commit();
     };
     load(0, 0);
 
     // Q~ = rotated q * sm_scale * log2e as A operands, split; both columns of a rotation pair belong to the same lane
-    uint32_t qh[KS][4], ql[KS][4];
+    uint32_t qa[KS][3][4];
     {
         const T* Q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, 0);
         const float scale = p.sm_scale * kLog2e;
 #pragma unroll
-        for (int ks = 0; ks < KS / 2; ++ks)
+        for (int ks2 = 0; ks2 < KS / 2; ++ks2)
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                const int pos = row0 + (x & 1) * 8, d = ks * 16 + (x >> 1) * 8 + c2;
+                const int pos = row0 + (x & 1) * 8, d = ks2 * 16 + (x >> 1) * 8 + c2;
                 float2 a = make_float2(0.f, 0.f), b = a;
                 float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
                 if (pos < N) {
@@ -193,36 +266,49 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kern
                         c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
                     }
                 }
-                split2<__nv_bfloat16>((a.x * c0 - b.x * s0) * scale, (a.y * c1 - b.y * s1) * scale, qh[ks][x], ql[ks][x]);
-                split2<__nv_bfloat16>((b.x * c0 + a.x * s0) * scale, (b.y * c1 + a.y * s1) * scale, qh[ks + KS / 2][x], ql[ks + KS / 2][x]);
+                uint32_t w[3];
+                split3_any<__nv_bfloat16>((a.x * c0 - b.x * s0) * scale, (a.y * c1 - b.y * s1) * scale, w);
+#pragma unroll
+                for (int part = 0; part < 3; ++part) qa[ks2][part][x] = w[part];
+                split3_any<__nv_bfloat16>((b.x * c0 + a.x * s0) * scale, (b.y * c1 + a.y * s1) * scale, w);
+#pragma unroll
+                for (int part = 0; part < 3; ++part) qa[ks2 + KS / 2][part][x] = w[part];
             }
     }
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[DT][4];
 #pragma unroll
     for (int n = 0; n < DT; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
 
-    const int n_end = p.causal ? min(N, m0 + kRows) : N;
+    const int n_end = p.causal ? min(N, m0 + F::kRows) : N;
     int buf = 0;
     for (int j0 = 0; j0 < n_end; j0 += BN, buf ^= 1) {
         cp_wait_all();
         __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
         if (j0 + BN < n_end) load(j0 + BN, buf ^ 1);
-        const uint32_t kh = sm + buf * F::kStage + lane_b<D>(lane), kl = kh + F::kTile, vv = sm + buf * F::kStage + 2 * F::kTile + lane_bt<D>(lane);
+        if (p.causal && j0 > m0 + warp * 16 + 15) continue;   // no key of the tile is seen by the warp's rows
+        const uint32_t st = sm + buf * F::kStage, kk = st + lane_b<D>(lane), vv = st + 3 * F::kTile + lane_bt<D>(lane);
         float s[NT][4];
 #pragma unroll
-        for (int n = 0; n < NT; ++n) s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+        for (int np = 0; np < NT / 4; ++np) {   // 32 keys
+            float (*main)[4] = s + 4 * np, small[4][4];
 #pragma unroll
-        for (int ks = 0; ks < KS; ++ks)
+            for (int n = 0; n < 4; ++n)
 #pragma unroll
-            for (int np = 0; np < NT / 2; np += 2) {
-                constexpr uint32_t kNext = 16 * Pitch<D>::kBytes;
-                uint32_t bh0[4], bh1[4], bl0[4], bl1[4];
-                ldm_x4(bh0, kh + np * kNext + ks * 32);
-                ldm_x4(bh1, kh + (np + 1) * kNext + ks * 32);
-                ldm_x4(bl0, kl + np * kNext + ks * 32);
-                ldm_x4(bl1, kl + (np + 1) * kNext + ks * 32);
-                mma4_split(s + 2 * np, qh[ks], ql[ks], bh0, bh1, bl0, bl1);
+                for (int x = 0; x < 4; ++x) main[n][x] = small[n][x] = 0.f;
+#pragma unroll
+            for (int k = 0; k < KS; ++k) {
+                uint32_t b[3][2][4];
+#pragma unroll
+                for (int part = 0; part < 3; ++part)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) ldm_x4(b[part][y], kk + part * F::kTile + (2 * np + y) * 16 * Pitch<D>::kBytes + k * 32);
+                mma4_split(main, small, qa[k], b);
             }
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) main[n][x] = join(main[n][x], small[n][x]);
+        }
         // keys the lane's rows do not see
         if (j0 + BN > N || (p.causal && j0 + BN - 1 > m0 + warp * 16)) {
 #pragma unroll
@@ -241,13 +327,13 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kern
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
             mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
             const float ref = mx == -INFINITY ? 0.f : mx;   // a row that has seen no key yet
-            const float alpha = fast_exp2(m[r] - ref);
+            const float alpha = exp2f(m[r] - ref);
             float sum = 0.f;
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    s[n][2 * r + x] = fast_exp2(s[n][2 * r + x] - ref);
+                    s[n][2 * r + x] = exp2f(s[n][2 * r + x] - ref);
                     sum += s[n][2 * r + x];
                 }
             l[r] = l[r] * alpha + sum;   // this lane's columns only; the four lanes of a row are added at the end
@@ -257,15 +343,14 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kern
         }
 #pragma unroll
         for (int t = 0; t < BN / 16; ++t) {
-            uint32_t ph[4], pl[4];
-            split_a<T>(s[2 * t], s[2 * t + 1], 1.f, ph, pl);
+            uint32_t pa[3][4];
+            split_a<T>(s[2 * t], s[2 * t + 1], kPScale<T>, pa);
 #pragma unroll
             for (int dp = 0; dp < DT / 2; dp += 2) {
                 uint32_t b0[4], b1[4];
                 ldm_x4_trans(b0, vv + t * 16 * Pitch<D>::kBytes + dp * 32);
                 ldm_x4_trans(b1, vv + t * 16 * Pitch<D>::kBytes + dp * 32 + 32);
-                mma4<T>(o + 2 * dp, ph, b0, b1);
-                mma4<T>(o + 2 * dp, pl, b0, b1);
+                add_products<T>(o + 2 * dp, pa, b0, b1);
             }
         }
     }
@@ -277,7 +362,7 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kern
         sum += __shfl_xor_sync(0xffffffffu, sum, 2);
         const int pos = row0 + 8 * r;
         if (pos >= N) continue;
-        const float inv = sum > 0.f ? 1.f / sum : 0.f;
+        const float inv = sum > 0.f ? (1.f / kPScale<T>) / sum : 0.f;
         uint32_t* out = reinterpret_cast<uint32_t*>(O + (int64_t)pos * p.so.n + c2);
 #pragma unroll
         for (int n = 0; n < DT; ++n) out[n * 4] = pack2<T>(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
@@ -286,36 +371,26 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_fwd_split_kern
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward: two kernels of one form.  KV = false: dQ of 64 query rows, sweeping the keys.  KV = true: dK, dV of 64 keys, sweeping
-// the query rows of the group's heads (everything transposed).  The owned rows are the A operands, the streamed rows (32 per step)
-// the B operands of both score products, and the streamed rotated rows again those of the gradient product.  The scores are formed
-// twice (16 MMAs against 12), but every sum has one owner and one order: the same bits every time, and no fp32 accumulator of dQ.
+// backward: two kernels of one form.  KV = false: dQ of the owned query rows, sweeping the keys.  KV = true: dK, dV of the owned keys,
+// sweeping the query rows of the group's heads (everything transposed).  The owned rows are the A operands, the streamed rows (32 per
+// step) the B operands of both score products, and the streamed rotated rows again those of the gradient product.  The scores are
+// formed twice (29 MMAs against 22), but every sum has one owner and one order: the same bits every time, and no fp32 accumulator
+// of dQ.
 // ------------------------------------------------------------------------------------------------
 template <int D> struct Bwd {
-    static constexpr int kBS = 32;
-    static constexpr uint32_t kOwn = kRows * Pitch<D>::kBytes, kTile = kBS * Pitch<D>::kBytes, kStage = 3 * kTile;
-    static constexpr size_t kSmem = 3 * kOwn + 2 * kStage;
-};
-
-struct SplitRows {   // bf16 hi and lo copies [B, H, N, D]
-    const __nv_bfloat16 *hi, *lo;
+    static constexpr int kThreads = D == 64 ? 128 : 256, kCtas = D == 64 ? 3 : 1;
+    static constexpr int kRows = kThreads / 2, kBS = 32;   // rows a CTA owns, 16 per warp; rows streamed per step
+    static constexpr uint32_t kOwn = kRows * Pitch<D>::kBytes, kTile = kBS * Pitch<D>::kBytes, kStage = 4 * kTile;
+    static constexpr size_t kSmem = 4 * kOwn + 2 * kStage;
 };
 
 template <typename T, int D, bool KV>
-__global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
+__global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
     using W = Bwd<D>;
-    constexpr int BS = W::kBS, KS = D / 16, NT = BS / 8, DT = D / 8;
+    constexpr int BS = W::kBS, KS = D / 16, NT = BS / 8, DT = D / 8, kThreads = W::kThreads, kRows = W::kRows;
     static_assert(NT == 4, "the score products of a step are four accumulator tiles");
-    // P^T of f16 tensors enters its product times 1024: a probability of a long row is far below 1, where f16 hi + lo runs out of
-    // exponent before it runs out of mantissa
-    // Owned A operands kept in registers (of hi, lo and the plain rows): an ldmatrix_x4 takes 4 cycles of the shared-memory port, an
-    // MMA 2 of the tensor pipe, and with all of them re-read a step's score products need 36 against 32.  D = 128 dQ has the
-    // registers (B1 H32 N1777 backward 686 -> 652 us, with the MMAs of four tiles back to back); at D = 64 a third CTA per SM is worth
-    // more (B4 H16 N1000 forward + backward 652 us with all three in registers and two CTAs, 584 us like this).
-    constexpr int kRegA = D == 64 || KV ? 0 : 2;
-    constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 1024.f : 1.f;
     extern __shared__ __align__(16) uint8_t smem[];
-    const uint32_t sm = smem_u32(smem), stages = sm + 3 * W::kOwn;
+    const uint32_t sm = smem_u32(smem), stages = sm + 4 * W::kOwn;
     const int N = p.N, G = p.H / p.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int own_head = blockIdx.x;                         // KV: a K / V head, otherwise a query head
@@ -330,26 +405,20 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_bwd_split_kern
         const int r0 = first + (KV ? step % steps : step) * BS;
         if (KV) {
             const int qh = kvh * G + step / steps;
-            load_rows<D, BS>(st, qs.hi + (size_t)qh * N * D, D, r0, N);
-            load_rows<D, BS>(st + W::kTile, qs.lo + (size_t)qh * N * D, D, r0, N);
-            load_rows<D, BS>(st + 2 * W::kTile, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, qh, 0), p.sdo.n, r0, N);
+            load_split<D, BS, kThreads>(st, W::kTile, qs, qh, r0, N);
+            load_rows<D, BS, kThreads>(st + 3 * W::kTile, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, qh, 0), p.sdo.n, r0, N);
         } else {
-            load_rows<D, BS>(st, ks.hi + (size_t)kvh * N * D, D, r0, N);
-            load_rows<D, BS>(st + W::kTile, ks.lo + (size_t)kvh * N * D, D, r0, N);
-            load_rows<D, BS>(st + 2 * W::kTile, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0), p.sv.n, r0, N);
+            load_split<D, BS, kThreads>(st, W::kTile, ks, kvh, r0, N);
+            load_rows<D, BS, kThreads>(st + 3 * W::kTile, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0), p.sv.n, r0, N);
         }
         cp_commit();
     };
-    {
-        const SplitRows& own = KV ? ks : qs;
-        load_rows<D, kRows>(sm, own.hi + (size_t)own_head * N * D, D, own0, N);
-        load_rows<D, kRows>(sm + W::kOwn, own.lo + (size_t)own_head * N * D, D, own0, N);
-        if (KV)
-            load_rows<D, kRows>(sm + 2 * W::kOwn, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, own_head, 0), p.sv.n, own0, N);
-        else
-            load_rows<D, kRows>(sm + 2 * W::kOwn, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, own_head, 0), p.sdo.n, own0, N);
-        load(0, 0);
-    }
+    load_split<D, kRows, kThreads>(sm, W::kOwn, KV ? ks : qs, own_head, own0, N);
+    if (KV)
+        load_rows<D, kRows, kThreads>(sm + 3 * W::kOwn, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, own_head, 0), p.sv.n, own0, N);
+    else
+        load_rows<D, kRows, kThreads>(sm + 3 * W::kOwn, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, own_head, 0), p.sdo.n, own0, N);
+    load(0, 0);
     float lse_r[2], dl_r[2];
     if (!KV) {
 #pragma unroll
@@ -364,92 +433,87 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_bwd_split_kern
     for (int n = 0; n < DT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
 #pragma unroll
     for (int n = 0; n < (KV ? DT : 1); ++n) dv[n][0] = dv[n][1] = dv[n][2] = dv[n][3] = 0.f;
-    const uint32_t ah_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane);   // of the hi rows; lo and plain rows follow
+    const uint32_t a_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane);   // of the hi rows; mid, lo and plain rows follow
 
-    uint32_t own_a[kRegA > 0 ? kRegA : 1][KS][4];
     for (int step = 0, buf = 0; step < total; ++step, buf ^= 1) {
         cp_wait_all();
         __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
-        if (kRegA > 0 && step == 0) {
-#pragma unroll
-            for (int x = 0; x < kRegA; ++x)
-#pragma unroll
-                for (int k = 0; k < KS; ++k) ldm_x4(own_a[x][k], ah_addr + x * W::kOwn + k * 32);
-        }
         if (step + 1 < total) load(step + 1, buf ^ 1);
         const uint32_t st = stages + buf * W::kStage;
         const int r0 = first + (KV ? step % steps : step) * BS;
-        float lse_c[NT][2], dl_c[NT][2];
-        if (KV) {
-            const size_t head = (size_t)(kvh * G + step / steps) * N;
-#pragma unroll
-            for (int n = 0; n < NT; ++n)
-#pragma unroll
-                for (int x = 0; x < 2; ++x) {
-                    const int pos = r0 + n * 8 + c2 + x;
-                    lse_c[n][x] = pos < N ? p.lse2[head + pos] : INFINITY;
-                    dl_c[n][x] = pos < N ? p.delta[head + pos] : 0.f;
-                }
-        }
-        float s[NT][4], dp[NT][4];
+        // no pair of the step's and the warp's rows is visible
+        if (p.causal && (KV ? r0 + BS - 1 < own0 + warp * 16 : r0 > own0 + warp * 16 + 15)) continue;
+        float s[NT][4], dp[NT][4], small[NT][4];
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) s[n][x] = dp[n][x] = 0.f;
+            for (int x = 0; x < 4; ++x) s[n][x] = dp[n][x] = small[n][x] = 0.f;
         const uint32_t b_addr = st + lane_b<D>(lane);
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
-            uint32_t a[3][4], b[3][2][4];   // of the hi, lo and plain rows
+            uint32_t a[3][4], ax[4], b[3][2][4], bx[2][4];   // split and plain rows
+#pragma unroll
+            for (int y = 0; y < 2; ++y) ldm_x4(bx[y], b_addr + 3 * W::kTile + y * 16 * Pitch<D>::kBytes + k * 32);
+            ldm_x4(ax, a_addr + 3 * W::kOwn + k * 32);
+            {
+                float t[4][4] = {};
+                mma4<T>(t, ax, bx[0], bx[1]);
+                add4(dp, t);
+            }
 #pragma unroll
             for (int x = 0; x < 3; ++x) {
-                if (x < kRegA) {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) a[x][e] = own_a[x < kRegA ? x : 0][k][e];
-                } else {
-                    ldm_x4(a[x], ah_addr + x * W::kOwn + k * 32);
-                }
+                ldm_x4(a[x], a_addr + x * W::kOwn + k * 32);
 #pragma unroll
                 for (int y = 0; y < 2; ++y) ldm_x4(b[x][y], b_addr + x * W::kTile + y * 16 * Pitch<D>::kBytes + k * 32);
             }
-            mma4<T>(dp, a[2], b[2][0], b[2][1]);
-            mma4_split(s, a[0], a[1], b[0][0], b[0][1], b[1][0], b[1][1]);
+            mma4_split(s, small, a, b);
         }
         // P and dS = P (dP - delta), in place of S and dP
+        const size_t head = KV ? (size_t)(kvh * G + step / steps) * N : 0;
         const bool edge = KV ? (p.causal && r0 < own0 + warp * 16 + 15) : (r0 + BS > N || (p.causal && r0 + BS - 1 > own0 + warp * 16));
 #pragma unroll
-        for (int n = 0; n < NT; ++n)
+        for (int n = 0; n < NT; ++n) {
+            float lse_c[2], dl_c[2];
+            if (KV) {
+#pragma unroll
+                for (int x = 0; x < 2; ++x) {
+                    const int pos = r0 + n * 8 + c2 + x;
+                    lse_c[x] = pos < N ? p.lse2[head + pos] : INFINITY;
+                    dl_c[x] = pos < N ? p.delta[head + pos] : 0.f;
+                }
+            }
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                float pv = fast_exp2(s[n][x] - (KV ? lse_c[n][x & 1] : lse_r[x >> 1]));
+                float pv = exp2f(join(s[n][x], small[n][x]) - (KV ? lse_c[x & 1] : lse_r[x >> 1]));
                 if (edge) {
                     const int own = row0 + (x >> 1) * 8, str = r0 + n * 8 + c2 + (x & 1);
                     const bool seen = KV ? (!p.causal || own <= str) : (str < N && (!p.causal || str <= own));
                     if (!seen) pv = 0.f;
                 }
-                dp[n][x] = pv * (dp[n][x] - (KV ? dl_c[n][x & 1] : dl_r[x >> 1]));
+                dp[n][x] = pv * (dp[n][x] - (KV ? dl_c[x & 1] : dl_r[x >> 1]));
                 s[n][x] = pv;
             }
+        }
         const uint32_t t_addr = st + lane_bt<D>(lane);
 #pragma unroll
         for (int t = 0; t < BS / 16; ++t) {
-            uint32_t dh[4], dl[4], ph[4], pl[4];
-            split_a<__nv_bfloat16>(dp[2 * t], dp[2 * t + 1], 1.f, dh, dl);
-            if (KV) split_a<T>(s[2 * t], s[2 * t + 1], kPScale, ph, pl);
+            uint32_t da[3][4], pa[3][4];
+            split_a<__nv_bfloat16>(dp[2 * t], dp[2 * t + 1], 1.f, da);
+            if (KV) split_a<T>(s[2 * t], s[2 * t + 1], kPScale<T>, pa);
 #pragma unroll
             for (int d = 0; d < DT / 2; d += 2) {
                 const uint32_t off = t * 16 * Pitch<D>::kBytes + d * 32;
-                uint32_t bh0[4], bh1[4], bl0[4], bl1[4];
-                ldm_x4_trans(bh0, t_addr + off);
-                ldm_x4_trans(bh1, t_addr + off + 32);
-                ldm_x4_trans(bl0, t_addr + W::kTile + off);
-                ldm_x4_trans(bl1, t_addr + W::kTile + off + 32);
-                mma4_split(acc + 2 * d, dh, dl, bh0, bh1, bl0, bl1);
+                uint32_t b[3][2][4];
+#pragma unroll
+                for (int x = 0; x < 3; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) ldm_x4_trans(b[x][y], t_addr + x * W::kTile + off + 32 * y);
+                add_products_split(acc + 2 * d, da, b);
                 if (KV) {
                     uint32_t bx0[4], bx1[4];
-                    ldm_x4_trans(bx0, t_addr + 2 * W::kTile + off);
-                    ldm_x4_trans(bx1, t_addr + 2 * W::kTile + off + 32);
-                    mma4<T>(dv + (KV ? 2 * d : 0), ph, bx0, bx1);
-                    mma4<T>(dv + (KV ? 2 * d : 0), pl, bx0, bx1);
+                    ldm_x4_trans(bx0, t_addr + 3 * W::kTile + off);
+                    ldm_x4_trans(bx1, t_addr + 3 * W::kTile + off + 32);
+                    add_products<T>(dv + (KV ? 2 * d : 0), pa, bx0, bx1);
                 }
             }
         }
@@ -477,9 +541,10 @@ __global__ void __launch_bounds__(kThreads, D == 64 ? 3 : 2) rope_bwd_split_kern
             out[n * 4 + D / 4] = pack2<T>((b0 * c0 - a0 * s0) * scale, (b1 * c1 - a1 * s1) * scale);
         }
         if (KV) {
+            constexpr float kUnscale = 1.f / kPScale<T>;
             uint32_t* o2 = reinterpret_cast<uint32_t*>(reinterpret_cast<T*>(p.dv) + row_offset(p.sdv, p.Hkv, own_head, pos) + c2);
 #pragma unroll
-            for (int n = 0; n < DT; ++n) o2[n * 4] = pack2<T>(dv[KV ? n : 0][2 * r] * (1.f / kPScale), dv[KV ? n : 0][2 * r + 1] * (1.f / kPScale));
+            for (int n = 0; n < DT; ++n) o2[n * 4] = pack2<T>(dv[KV ? n : 0][2 * r] * kUnscale, dv[KV ? n : 0][2 * r + 1] * kUnscale);
         }
     }
 }
@@ -489,45 +554,47 @@ template <typename T, int D>
 int split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, SplitRows out, cudaStream_t s) {
     const size_t rows = (size_t)p.B * H * p.N;
     split_rotate_kernel<T, D><<<(unsigned)((rows * (D / 16) + 255) / 256), 256, 0, s>>>((const T*)x, row_addr(st, H, p.N), p.cos, p.sin, p.table_stride, scale,
-                                                                                       const_cast<__nv_bfloat16*>(out.hi), const_cast<__nv_bfloat16*>(out.lo), rows);
+                                                                                       out, rows);
     count_launch();
     return (int)cudaGetLastError();
 }
 SplitRows take_rows(__nv_bfloat16*& ws, int B, int H, int N, int D) {
     const size_t n = (size_t)B * H * N * D;
-    SplitRows r{ws, ws + n};
-    ws += 2 * n;
+    SplitRows r{ws, n};
+    ws += 3 * n;
     return r;
 }
 
 template <typename T, int D>
 int fwd(const RopeParams& p, void* ws, cudaStream_t s) {
+    using F = Fwd<D>;
     __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
     const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D);
     if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
     auto kern = rope_fwd_split_kernel<T, D>;
     static std::atomic<uint64_t> smem_ok;
-    if (int e = allow_smem(kern, Fwd<D>::kSmem, smem_ok)) return e;
-    kern<<<dim3(p.B * p.H, (p.N + kRows - 1) / kRows), kThreads, Fwd<D>::kSmem, s>>>(p, k.hi, k.lo);
+    if (int e = allow_smem(kern, F::kSmem, smem_ok)) return e;
+    kern<<<dim3(p.B * p.H, (p.N + F::kRows - 1) / F::kRows), F::kThreads, F::kSmem, s>>>(p, k);
     count_launch();
     return (int)cudaGetLastError();
 }
 template <typename T, int D>
 int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
+    using W = Bwd<D>;
     __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
     const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D), q = take_rows(at, p.B, p.H, p.N, D);
     if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
     if (int e = split_rows<T, D>(p.q, p.sq, p.H, p, p.sm_scale * kLog2e, q, s)) return e;
-    const unsigned blocks = (p.N + kRows - 1) / kRows;
+    const unsigned blocks = (p.N + W::kRows - 1) / W::kRows;
     auto kv = rope_bwd_split_kernel<T, D, true>;
     auto dq = rope_bwd_split_kernel<T, D, false>;
     static std::atomic<uint64_t> kv_ok, dq_ok;
-    if (int e = allow_smem(kv, Bwd<D>::kSmem, kv_ok)) return e;
-    if (int e = allow_smem(dq, Bwd<D>::kSmem, dq_ok)) return e;
-    kv<<<dim3(p.B * p.Hkv, blocks), kThreads, Bwd<D>::kSmem, s>>>(p, q, k);
+    if (int e = allow_smem(kv, W::kSmem, kv_ok)) return e;
+    if (int e = allow_smem(dq, W::kSmem, dq_ok)) return e;
+    kv<<<dim3(p.B * p.Hkv, blocks), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     if (cudaError_t e = cudaGetLastError()) return (int)e;
-    dq<<<dim3(p.B * p.H, blocks), kThreads, Bwd<D>::kSmem, s>>>(p, q, k);
+    dq<<<dim3(p.B * p.H, blocks), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -535,7 +602,7 @@ int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
 }  // namespace
 
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D) {
-    return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 2 * sizeof(__nv_bfloat16);
+    return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 3 * sizeof(__nv_bfloat16);
 }
 
 int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {

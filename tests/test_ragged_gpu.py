@@ -2,6 +2,7 @@
 blocks and the 256-row work items; both head dimensions, causal and full, with and without rotation, grouped heads, transposed
 buffers.  Tolerances as in test_gpu_parity.py."""
 
+import math
 import os
 
 import pytest
@@ -114,3 +115,56 @@ def test_ragged_lengths_keep_fp32_accuracy(N, D, causal, dtype, scale):
             continue
         err = ((got.double() - ref.cpu()).norm() / ref.cpu().norm()).item()
         assert err < ulp * (1.0 if name in ("O", "dV") else 1.5), (name, err / ulp)
+
+
+def _exact_grads(q, k, v, do, o, causal, s, cos, sin):
+    """dQ, dK, dV in 64 bits with delta = rowsum(O dO) of the given rounded O, as the kernels form it."""
+    qd, kd, v, do, o = (t.cuda().double() for t in (q, k, v, do, o))
+    half = qd.shape[-1] // 2
+    c, sn = cos[:, :half].cuda().double(), sin[:, :half].cuda().double()
+    turn = lambda x, w: torch.cat((x[..., :half] * c - w * x[..., half:] * sn, x[..., half:] * c + w * x[..., :half] * sn), -1)   # w = -1: back
+    qr, kr = turn(qd, 1.0), turn(kd, 1.0)
+    w = qr @ kr.transpose(-1, -2) * s
+    if causal:
+        w = w.masked_fill(torch.ones_like(w, dtype=torch.bool).triu(1), float("-inf"))
+    p = w.softmax(-1)
+    ds = p * (do @ v.transpose(-1, -2) - (o * do).sum(-1, keepdim=True)) * s
+    return turn(ds @ kr, -1.0), turn(ds.transpose(-1, -2) @ qr, -1.0), p.transpose(-1, -2) @ do
+
+
+@pytest.mark.parametrize("scale", [1.0, 4.0, 6.0])   # scores with a standard deviation of 1, 16, 36
+@pytest.mark.parametrize("N,D,causal", [(1777, 128, True), (1000, 64, False), (1001, 64, True), (65, 128, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_ragged_lengths_are_as_accurate_as_fp32_kernels(N, D, causal, dtype, scale):
+    """Held against the CUDA-core kernels with fp32 operands (policy 1): the LSE, which is not rounded, by its error, the 16-bit results by
+    the share of them that are not the exact result rounded.  Both are proportional to the error before the rounding, and differ
+    by what the order of the sums gives (measured: 0.55 to 1.05 of the CUDA-core kernels' share); two 16-bit parts per operand instead of three
+    show 5 to 10 times the error."""
+    rope = pkg.fused_rope_attn
+    q, k, v, do = (draw((1, 4, N, D), 260 + i, dtype) * (scale if i < 2 else 1.0) for i in range(4))
+    cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
+    s = D ** -0.5
+    qd, kd, vd, dod, cd, sd = (t.cuda() for t in (q, k, v, do, cos, sin))
+    exact_o = _exact(q, k, v, do, causal, s, cos, sin)[0]
+    errors = {}
+    saved0 = rope._forward(qd, kd, vd, causal, s, cd, sd)
+    exact = _exact_grads(q, k, v, do, saved0[3], causal, s, cos, sin)
+    half = D // 2
+    c, sn = cos[:, :half].cuda().double(), sin[:, :half].cuda().double()
+    qr, kr = (torch.cat((x[..., :half] * c - x[..., half:] * sn, x[..., half:] * c + x[..., :half] * sn), -1) for x in (qd.double(), kd.double()))
+    w = qr @ kr.transpose(-1, -2) * s
+    if causal:
+        w = w.masked_fill(torch.ones_like(w, dtype=torch.bool).triu(1), float("-inf"))
+    lse = torch.logsumexp(w, -1) / math.log(2.0)
+    for policy in (0, 1):
+        prev = ext.lib().corope_set_kernel_policy(policy)
+        try:
+            saved = rope._forward(qd, kd, vd, causal, s, cd, sd)
+            grads = rope._backward(*saved0, dod, causal, s)   # both from one O and one LSE
+        finally:
+            ext.lib().corope_set_kernel_policy(prev)
+        ext.check_status()
+        errors[policy] = [(saved[4].double() - lse).pow(2).mean().sqrt().item()]
+        errors[policy] += [(a != b.to(dtype)).double().mean().item() for a, b in zip((saved[3],) + tuple(grads), (exact_o,) + exact)]
+    for name, new, old in zip(("LSE", "O", "dQ", "dK", "dV"), errors[0], errors[1]):
+        assert new <= 1.25 * old + (0.0 if name == "LSE" else 1e-4), (name, new, old)
