@@ -61,23 +61,25 @@ size_t rope_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D, int 
 }
 
 struct GqaWorkspace {
-    size_t delta, dk_acc, dv_acc, k_pairs, v_half, total;
+    size_t delta, dk_acc, dv_acc, k_pairs, v_half, k_scale, total;
 };
 
 // `any_n`: room for the split-operand forward where the mma kernels do not apply.
 GqaWorkspace gqa_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool any_n) {
     GqaWorkspace w{};
     size_t off = 0;
-    if (gqa_fwd_mma_supported(N, D, dtype)) {   // fp16 operand copies of K (pair order) and V for the tensor-core kernels
+    const bool split = any_n && !bwd && gqa_split_supported(D, dtype);
+    // fp16 operand copies of K (pair order) and V for the mma kernels; K in pair order, its own type, and a copy of V if its rows are
+    // not aligned for the split-operand forward
+    if (gqa_fwd_mma_supported(N, D, dtype) || split) {
         w.k_pairs = off;
         off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
         w.v_half = off;
         off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
-    } else if (any_n && !bwd && gqa_split_supported(D, dtype)) {   // K in pair order, its own type; a copy of V if its rows are not aligned
-        w.k_pairs = off;
-        off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
-        w.v_half = off;
-        off += align_up((size_t)B * Hkv * N * D * 2, kAlign);
+    }
+    if (split && dtype == COROPE_DTYPE_F16) {
+        w.k_scale = off;
+        off += align_up((size_t)B * Hkv * N * sizeof(float), kAlign);
     }
     if (bwd) {
         w.delta = off;
@@ -595,6 +597,7 @@ int corope_gqa_fwd_strided(const void* q, const void* k, const void* v, void* o,
     if (g_policy.load() == 0 && gqa_split_supported(D, dtype) && workspace_bytes >= any.total) {
         p.k_pairs = reinterpret_cast<uint32_t*>((char*)workspace + any.k_pairs);
         p.v_half = reinterpret_cast<__half*>((char*)workspace + any.v_half);
+        p.k_scale = reinterpret_cast<float*>((char*)workspace + any.k_scale);
         return launch_gqa_fwd_split(p, vec_ok(k, p.sk), vec_ok(v, p.sv), dtype, (cudaStream_t)stream);
     }
     return launch_gqa_fwd_general(p, dtype, (cudaStream_t)stream);

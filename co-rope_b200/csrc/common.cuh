@@ -130,6 +130,7 @@ struct GqaParams {
     float* dv_acc;   // [B,Hkv,N,D] fp32
     uint32_t* k_pairs;  // tensor-core forward: [B,Hkv,N,D/2] fp16 (k1, k2) pairs in MMA operand order (workspace)
     __half* v_half;     // tensor-core forward: [B,Hkv,N,D] fp16 copy of V (workspace)
+    float* k_scale;     // split-operand forward, f16 tensors: [B,Hkv,N] factors that undo the scaling of the rows of k_pairs (workspace)
     int use_mma;        // backward: 1 = tensor-core main kernel (k_pairs / v_half are set), 0 = general kernel
     int B, Hq, Hkv, G, N, D;
     float sm_scale;
@@ -662,7 +663,7 @@ int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 int launch_rope_bwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 bool gqa_fwd_mma_supported(int N, int D, int dtype);
 // 16-bit tensors, D = 64 or 128, any N and strides; k_vec / v_vec: rows of k / v are aligned to 16 bytes; p.k_pairs and (without v_vec)
-// p.v_half: workspace of 2 B Hkv N D bytes each
+// p.v_half: workspace of 2 B Hkv N D bytes each; f16: p.k_scale, 4 B Hkv N bytes
 bool gqa_split_supported(int D, int dtype);
 int launch_gqa_fwd_split(const GqaParams& p, bool k_vec, bool v_vec, int dtype, cudaStream_t s);
 int launch_gqa_bwd_mma(const GqaParams& p, int dtype, cudaStream_t s);

@@ -3,14 +3,17 @@
 //
 // Same scheme as corope_fwd_mma.cu (one CTA = 8 query rows of one (batch, KV head), one warp per row, key tiles of 64 swept downward,
 // S^T = K' Q^T and O^T += V^T P^T with the keys as MMA rows and the group's heads as columns), but the operands stay exact: q, k, v
-// enter the MMAs in their own type; the rotation is formed in fp32 and K' enters as a hi + lo pair of that type (two MMAs), and so
-// does P.  The pair carries 16 bits for bf16 and 22 for f16 tensors, whose K' up to sqrt(2) * 65504 the saturated hi and lo still
-// cover.
+// enter the MMAs in their own type; the rotation is formed in fp32 and K' and P enter as the sum of several numbers of that type, hi
+// + rest.  bf16: three parts, which hold the 24 bits of an fp32 number.  f16: two parts for K' (22 bits; the rows of K are scaled by a
+// power of two so that none of it sinks into the subnormals), three for P, times 2^14 for the same reason.  The adder of the MMAs does
+// not round to nearest: products of the hi parts go through one MMA each, which fp32 additions join.
 //
-// 2-norm error of O against 64-bit arithmetic, N(0, 1) inputs, B1 Hq8 Hkv2 N500 D128: 1.603e-3 (bf16), 1.992e-4 (f16), the rounding
-// of the result and to the last digit what the CUDA-core kernel has; the fp16 operands of corope_fwd_mma.cu: 3.4e-4 (f16, N512).
-// B1 Hq32 Hkv8 N1500 D128 bf16 1442 -> 732 us, B2 Hq16 Hkv4 N2048 D64 bf16 1443 -> 688 us, B1 Hq16 Hkv2 N300 D64 f16 70 -> 25 us,
-// B4 Hq4 Hkv4 N100 D64 bf16 23 -> 19 us against the CUDA-core kernel, so it takes every size.
+// Error of O against 64-bit arithmetic, N(0, 1) inputs: the rounding of the result.  Results that are not the exact one rounded, next to
+// the CUDA-core kernel (Hq8 Hkv2, inputs times 0.3, where the phases matter least): bf16 N700 D128 0.030 % (0.037 %), f16 N333 D64 0.092 %
+// (0.133 %); at scale 1 f16 N512 D64 1.13 % (1.13 %), its LSE 4.9e-7 (4.8e-7).  Two bf16 parts, and f16 parts without the scaling, had
+// 0.22 % and 0.21 % at scale 0.3.
+// B1 Hq32 Hkv8 N1500 D128 bf16 1170 us (CUDA-core kernel 1347), f16 812 (1355), B2 Hq16 Hkv4 N2048 D64 bf16 970 (1298), B1 Hq16 Hkv2
+// N300 D64 f16 27.5 (68), B4 Hq4 Hkv4 N100 D64 bf16 22.9 (21.0) us, so it takes every size.
 // What bounds it: issue slots; the rotation costs two special-function operations and some 20 instructions per (query, key, pair)
 // triple, shared by the heads, against two per head and pair of the CUDA-core kernel on top of that.
 #include "corope_mma.cuh"
@@ -32,7 +35,7 @@ template <int D> struct Geo {
     static constexpr int kVRowBytes = 2 * D + 16;
     static constexpr int kKTileBytes = kKT * kKRow * 4, kVTileBytes = kKT * kVRowBytes;
     static constexpr int kAqBytes = kThreads * kChunks * 16;
-    static constexpr size_t kSmem = 2 * (kKTileBytes + kVTileBytes) + kRows * kPairs * 4 + 2 * kRows * kKT * 4 + 4 * kWStride * 4 + kAqBytes;
+    static constexpr size_t kSmem = 2 * (kKTileBytes + kVTileBytes) + kRows * kPairs * 4 + 2 * kRows * kKT * 4 + 4 * kWStride * 4 + kAqBytes + 2 * kKT * 4;
 };
 
 template <typename T> __device__ __forceinline__ void mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1);
@@ -42,23 +45,33 @@ template <> __device__ __forceinline__ void mma<__nv_bfloat16>(float (&d)[4], co
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-template <typename T> __device__ __forceinline__ uint32_t pack2_sat(float a, float b);
-template <> __device__ __forceinline__ uint32_t pack2_sat<__half>(float a, float b) { return pack_half2_sat(a, b); }
-template <> __device__ __forceinline__ uint32_t pack2_sat<__nv_bfloat16>(float a, float b) { return pack_bf162(a, b); }
-template <typename T>
-__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
-    hi = pack2_sat<T>(a, b);
-    const float2 f = unpack2<T>(hi);
-    lo = pack2_sat<T>(a - f.x, b - f.y);
+// (a, b) as the sum of PARTS pairs of T, each the rounded rest of those before
+template <typename T, int PARTS>
+__device__ __forceinline__ void split(float a, float b, uint32_t (&parts)[PARTS]) {
+#pragma unroll
+    for (int x = 0; x < PARTS; ++x) {
+        parts[x] = pack2<T>(a, b);
+        const float2 f = unpack2<T>(parts[x]);
+        a -= f.x;
+        b -= f.y;
+    }
 }
+// parts of a rotated K: bf16 needs three for the 24 bits of an fp32 number; two of f16 hold 22 where scaled rows keep them out of the
+// subnormals
+template <typename T> constexpr int kParts = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 2 : 3;
 // one (k1, k2) pair rotated by `angle` in fp32: (k1 cos + k2 sin, k2 cos - k1 sin), split
 template <typename T, bool DIRECT>
-__device__ __forceinline__ void rotate_split(uint32_t kpair, float angle, uint32_t& hi, uint32_t& lo) {
+__device__ __forceinline__ void rotate_split(uint32_t kpair, float angle, uint32_t (&parts)[kParts<T>]) {
     float sn, cs;
     gqa_mma::sincos_fast<DIRECT>(angle, &sn, &cs);
     const float2 k = unpack2<T>(kpair);
-    split2<T>(fmaf(k.x, cs, k.y * sn), fmaf(k.y, cs, -k.x * sn), hi, lo);
+    split<T, kParts<T>>(fmaf(k.x, cs, k.y * sn), fmaf(k.y, cs, -k.x * sn), parts);
 }
+// hi hi + the smaller products.  An infinity shows in hi hi with the sign it has in fp32; the other parts of such a product are
+// meaningless (NaN or either infinity).
+__device__ __forceinline__ float join(float main, float small) { return fabsf(main) < INFINITY ? main + small : main; }
+// P of f16 tensors enters its products times this
+template <typename T> constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 16384.f : 1.f;
 template <typename T>
 __device__ __forceinline__ uint32_t pair_bits(const T* row, int p, int half) {
     return (uint32_t)*reinterpret_cast<const uint16_t*>(row + p) | (uint32_t)*reinterpret_cast<const uint16_t*>(row + p + half) << 16;
@@ -76,17 +89,41 @@ __device__ __forceinline__ uint4 load8(const uint16_t* src, bool vec) {   // 8 e
     return make_uint4(w[0], w[1], w[2], w[3]);
 }
 // K -> (k1, k2) pairs of its own type in the permuted row order; V -> a contiguous copy where the main kernel's 16-byte copies
-// could not read it (vc, else null).  One thread per 8 pairs and 16 columns.
+// could not read it (vc, else null).  One thread per 8 pairs and 16 columns.  f16 rows are multiplied by the power of two that brings
+// their largest element into [2^13, 2^14) (K' stays below 2^15), its inverse goes to kscale: two f16 parts of K' then reach down to
+// 2^-38 of that element, whatever the magnitude of the row.  (An element that a row loses to the subnormals in being scaled down is
+// below 2^-39 of the largest.)
 template <typename T, int D>
-__global__ void __launch_bounds__(256) gqa_pack_k_kernel(const T* __restrict__ K, uint32_t* __restrict__ kp, const T* __restrict__ V, T* __restrict__ vc,
-                                                         size_t rows, RowAddr ak, RowAddr av, bool kvec) {
+__global__ void __launch_bounds__(256) gqa_pack_k_kernel(const T* __restrict__ K, uint32_t* __restrict__ kp, float* __restrict__ kscale, const T* __restrict__ V,
+                                                         T* __restrict__ vc, size_t rows, RowAddr ak, RowAddr av, bool kvec) {
     constexpr int kPairs = D / 2, kPerRow = kPairs / 8;
-    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x, r = idx / kPerRow;
-    if (r >= rows) return;
+    const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool live = idx / kPerRow < rows;
+    const size_t r = live ? idx / kPerRow : rows - 1;
     const int p0 = (int)(idx % kPerRow) * 8;
     const uint16_t* src = reinterpret_cast<const uint16_t*>(K + flat_row_offset(ak, r) + p0);
     const uint4 x1 = load8(src, kvec), x2 = load8(src + kPairs, kvec);
-    const uint32_t a[4] = {x1.x, x1.y, x1.z, x1.w}, b[4] = {x2.x, x2.y, x2.z, x2.w};
+    uint32_t a[4] = {x1.x, x1.y, x1.z, x1.w}, b[4] = {x2.x, x2.y, x2.z, x2.w};
+    if (Elem<T>::kDtype == COROPE_DTYPE_F16) {
+        float mx = 0.f;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
+            mx = fmaxf(fmaxf(mx, fmaxf(fabsf(fa.x), fabsf(fa.y))), fmaxf(fabsf(fb.x), fabsf(fb.y)));
+        }
+#pragma unroll
+        for (int off = kPerRow / 2; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+        const int e2 = mx > 0.f && mx < INFINITY ? 13 - ilogbf(mx) : 0;
+        const float up = exp2f((float)e2);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
+            a[e] = pack2<T>(fa.x * up, fa.y * up);
+            b[e] = pack2<T>(fb.x * up, fb.y * up);
+        }
+        if (live && p0 == 0) kscale[r] = exp2f((float)-e2);
+    }
+    if (!live) return;
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         kp[r * kPairs + perm_slot(p0 + 2 * e)] = __byte_perm(a[e], b[e], 0x5410);
@@ -104,6 +141,7 @@ template <typename T, int D, bool DIRECT>
 __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams p) {
     using M = Geo<D>;
     constexpr int kPairs = M::kPairs, CH = M::kChunks, DB = D / 16;
+    constexpr bool kScaled = Elem<T>::kDtype == COROPE_DTYPE_F16;
     extern __shared__ __align__(16) uint8_t smem_dyn[];
     uint8_t* ks_base = smem_dyn;                                              // 2 x K tile, (k1, k2) pairs, permuted rows
     uint8_t* vs_base = ks_base + 2 * M::kKTileBytes;                          // 2 x V tile, row-major
@@ -117,6 +155,8 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, r = lane >> 2, c = lane & 3;
     const int i = i0 + warp;                                                  // rows at or beyond N compute on zeros and store nothing
     uint4* aqs = reinterpret_cast<uint4*>(ws + 4 * kWStride) + warp * CH * 32;   // the query operand of every lane: chunk s of lane l at [warp][s][l]
+    float* kss = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(ws + 4 * kWStride) + M::kAqBytes);   // 2 x kscale of the tile's keys (f16)
+    auto key_scale = [&](int buf, int key) { return kScaled ? kss[buf * kKT + key] : 1.f; };
     const size_t q_head0 = (size_t)b * p.Hq + (size_t)g * G;
     const uint32_t* Kp = p.k_pairs + (size_t)bg * N * kPairs;
     const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, bg, 0);
@@ -130,6 +170,12 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
             const int pos = have ? j0 + row : 0;
             cp16(kd + row * (M::kKRow * 4) + ch * 16, Kp + (size_t)pos * kPairs + ch * 4, have);
             cp16(vd + row * M::kVRowBytes + ch * 16, V + (int64_t)pos * p.sv.n + ch * 8, have);
+        }
+        if (kScaled && tid < kKT) {
+            const bool have = j0 + tid < N;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(kss + buf * kKT + tid)),
+                         "l"(p.k_scale + (size_t)bg * N + (have ? j0 + tid : 0)), "r"(have ? 4 : 0)
+                         : "memory");
         }
         gqa_mma::cp_async_commit();
     };
@@ -185,8 +231,9 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
                 mma<T>(z, a1, kv.z, kv.w);
             }
             const int key = j0 + warp * 8 + 2 * c, qi = i0 + r;
-            zs[r * kKT + warp * 8 + 2 * c] = key <= qi ? 1.f / (1.f + __expf(-z[0] * p.sm_scale)) : 0.f;
-            zs[r * kKT + warp * 8 + 2 * c + 1] = key + 1 <= qi ? 1.f / (1.f + __expf(-z[1] * p.sm_scale)) : 0.f;
+            const float z0 = z[0] * key_scale(buf, warp * 8 + 2 * c), z1 = z[1] * key_scale(buf, warp * 8 + 2 * c + 1);
+            zs[r * kKT + warp * 8 + 2 * c] = key <= qi ? 1.f / (1.f + __expf(-z0 * p.sm_scale)) : 0.f;
+            zs[r * kKT + warp * 8 + 2 * c + 1] = key + 1 <= qi ? 1.f / (1.f + __expf(-z1 * p.sm_scale)) : 0.f;
         }
         __syncthreads();
         // 2. Delta of this warp's row: carry + sum of z over the keys of the tile above j
@@ -214,7 +261,7 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
             const float dA = dl[warp * kKT + kb * 16 + r], dB = dl[warp * kKT + kb * 16 + r + 8];
             const uint4* kpA = reinterpret_cast<const uint4*>(ks + (kb * 16 + r) * M::kKRow) + c;
             const uint4* kpB = reinterpret_cast<const uint4*>(ks + (kb * 16 + r + 8) * M::kKRow) + c;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f}, acl[4] = {0.f, 0.f, 0.f, 0.f};   // products of the hi and of the lo halves
+            float acc[4] = {0.f, 0.f, 0.f, 0.f}, acl[4] = {0.f, 0.f, 0.f, 0.f};   // products of the hi parts, and the smaller ones
 #pragma unroll
             for (int s = 0; s < CH; ++s) {
                 const uint4 kva = kpA[4 * s], kvb = kpB[4 * s], av = aqs[s * 32 + lane];
@@ -223,19 +270,27 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
                 const uint32_t ka[4] = {kva.x, kva.y, kva.z, kva.w}, kk[4] = {kvb.x, kvb.y, kvb.z, kvb.w}, q[4] = {av.x, av.y, av.z, av.w};
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
-                    uint32_t hi[4], lo[4];   // a0 / a2: key r, a1 / a3: key r + 8
+                    uint32_t kr[kParts<T>][4];   // a0 / a2: key r, a1 / a3: key r + 8
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        rotate_split<T, DIRECT>(ka[2 * t + e], dA * w[2 * t + e], hi[2 * e], lo[2 * e]);
-                        rotate_split<T, DIRECT>(kk[2 * t + e], dB * w[2 * t + e], hi[2 * e + 1], lo[2 * e + 1]);
+                        uint32_t x[kParts<T>], y[kParts<T>];
+                        rotate_split<T, DIRECT>(ka[2 * t + e], dA * w[2 * t + e], x);
+                        rotate_split<T, DIRECT>(kk[2 * t + e], dB * w[2 * t + e], y);
+#pragma unroll
+                        for (int part = 0; part < kParts<T>; ++part) kr[part][2 * e] = x[part], kr[part][2 * e + 1] = y[part];
                     }
-                    mma<T>(acc, hi, q[2 * t], q[2 * t + 1]);
-                    mma<T>(acl, lo, q[2 * t], q[2 * t + 1]);
+                    float hi[4] = {0.f, 0.f, 0.f, 0.f};
+                    mma<T>(hi, kr[0], q[2 * t], q[2 * t + 1]);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) acc[x] += hi[x];
+#pragma unroll
+                    for (int part = kParts<T> - 1; part > 0; --part) mma<T>(acl, kr[part], q[2 * t], q[2 * t + 1]);
                 }
             }
             const int keyA = j0 + kb * 16 + r;
-            if (keyA <= i) sc[kb][0] = (acc[0] + acl[0]) * sc2, sc[kb][1] = (acc[1] + acl[1]) * sc2;
-            if (keyA + 8 <= i) sc[kb][2] = (acc[2] + acl[2]) * sc2, sc[kb][3] = (acc[3] + acl[3]) * sc2;
+            const float sA = sc2 * key_scale(buf, kb * 16 + r), sB = sc2 * key_scale(buf, kb * 16 + r + 8);
+            if (keyA <= i) sc[kb][0] = join(acc[0], acl[0]) * sA, sc[kb][1] = join(acc[1], acl[1]) * sA;
+            if (keyA + 8 <= i) sc[kb][2] = join(acc[2], acl[2]) * sB, sc[kb][3] = join(acc[3], acl[3]) * sB;
         }
 
         // 4. online softmax of heads 2c, 2c + 1 (their 64 scores sit in the 8 lanes of class c), then O^T += V^T P^T
@@ -250,7 +305,7 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, off));
             mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, off));
         }
-        const float alpha0 = fast_exp2(m0 - mx0), alpha1 = fast_exp2(m1 - mx1);   // the first tile holds the diagonal: mx is finite
+        const float alpha0 = exp2f(m0 - mx0), alpha1 = exp2f(m1 - mx1);   // the first tile holds the diagonal: mx is finite
         m0 = mx0, m1 = mx1;
 #pragma unroll
         for (int db = 0; db < DB; ++db) {
@@ -261,23 +316,27 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
 #pragma unroll
         for (int kb = 0; kb < 4; ++kb) {
             if (j0 + kb * 16 > i) continue;   // nothing visible in this block (warp-uniform)
-            const float pA0 = fast_exp2(sc[kb][0] - mx0), pA1 = fast_exp2(sc[kb][1] - mx1);   // key r
-            const float pB0 = fast_exp2(sc[kb][2] - mx0), pB1 = fast_exp2(sc[kb][3] - mx1);   // key r + 8
+            const float pA0 = exp2f(sc[kb][0] - mx0), pA1 = exp2f(sc[kb][1] - mx1);   // key r
+            const float pB0 = exp2f(sc[kb][2] - mx0), pB1 = exp2f(sc[kb][3] - mx1);   // key r + 8
             ps0 += pA0 + pB0;
             ps1 += pA1 + pB1;
-            uint32_t ha, la, hb, lb;
-            split2<T>(pA0, pA1, ha, la);
-            split2<T>(pB0, pB1, hb, lb);
             // P^T as B operand: (keys 2c, 2c + 1 | head r) is the transpose of what the lane holds (key r | heads 2c, 2c + 1)
-            const uint32_t h0 = movmatrix_trans(ha), h1 = movmatrix_trans(hb), w0 = movmatrix_trans(la), w1 = movmatrix_trans(lb);
+            uint32_t pa[3], pb[3];
+            split<T, 3>(pA0 * kPScale<T>, pA1 * kPScale<T>, pa);
+            split<T, 3>(pB0 * kPScale<T>, pB1 * kPScale<T>, pb);
+#pragma unroll
+            for (int part = 0; part < 3; ++part) pa[part] = movmatrix_trans(pa[part]), pb[part] = movmatrix_trans(pb[part]);
             // V^T as A operand: four transposed 8x8 blocks (d 0-7 | 8-15) x (keys 0-7 | 8-15) of the block's V rows
             const uint8_t* vrow = vs + (kb * 16 + (lane & 7) + ((lane >> 4) & 1) * 8) * M::kVRowBytes + ((lane >> 3) & 1) * 16;
 #pragma unroll
-            for (int db = 0; db < DB; ++db) {
+            for (int db = 0; db < DB; ++db) {   // the block's own sum, then one fp32 addition: the adder of the MMAs does not round to nearest
                 uint32_t a[4];
                 gqa_mma::ldmatrix_x4_trans(a[0], a[1], a[2], a[3], vrow + db * 32);
-                mma<T>(o[db], a, h0, h1);
-                mma<T>(o[db], a, w0, w1);
+                float t[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                for (int part = 2; part >= 0; --part) mma<T>(t, a, pa[part], pb[part]);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) o[db][x] += t[x];
             }
         }
         l0 = l0 * alpha0 + ps0;
@@ -294,7 +353,7 @@ __global__ void __launch_bounds__(kThreads, 2) corope_fwd_split_kernel(GqaParams
     for (int x = 0; x < 2; ++x) {
         const int head = 2 * c + x;
         if (head >= G) continue;
-        const float inv = 1.f / (x ? l1 : l0);
+        const float inv = (1.f / kPScale<T>) / (x ? l1 : l0);
         T* O = reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.Hq, (int)q_head0 + head, i);
 #pragma unroll
         for (int db = 0; db < DB; ++db) {
@@ -310,7 +369,7 @@ template <typename T, int D>
 int launch_t(GqaParams p, bool k_vec, bool v_vec, cudaStream_t s) {
     const size_t rows = (size_t)p.B * p.Hkv * p.N;
     T* vc = v_vec ? nullptr : reinterpret_cast<T*>(p.v_half);
-    gqa_pack_k_kernel<T, D><<<(unsigned)((rows * (D / 16) + 255) / 256), 256, 0, s>>>((const T*)p.k, p.k_pairs, (const T*)p.v, vc, rows,
+    gqa_pack_k_kernel<T, D><<<(unsigned)((rows * (D / 16) + 255) / 256), 256, 0, s>>>((const T*)p.k, p.k_pairs, p.k_scale, (const T*)p.v, vc, rows,
                                                                                      row_addr(p.sk, p.Hkv, p.N), row_addr(p.sv, p.Hkv, p.N), k_vec);
     if (vc) {
         p.v = vc;
