@@ -111,12 +111,6 @@ __device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3
         b = fabsf(b - f.y) < INFINITY ? b - f.y : 0.f;
     }
 }
-// two rotation pairs (a.x, b.x), (a.y, b.y) by neighbouring table entries
-__device__ __forceinline__ void rotate(float2& a, float2& b, const float* c, const float* s) {
-    const float2 x = a, y = b;
-    a = make_float2(x.x * c[0] - y.x * s[0], x.y * c[1] - y.y * s[1]);
-    b = make_float2(y.x * c[0] + x.x * s[0], y.y * c[1] + x.y * s[1]);
-}
 // two neighbouring 8-column accumulator tiles as the A operand of one k-step, split: a[part]
 template <typename T>
 __device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[4], float scale, uint32_t (&a)[3][4]) {
@@ -204,13 +198,13 @@ __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
-        float2 ra = fa, rb = fb;
+        float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
         if (cosT != nullptr) {   // null tables: plain attention
             const float *c = cosT + (int64_t)n * ts + d + 2 * e, *s = sinT + (int64_t)n * ts + d + 2 * e;
-            rotate(ra, rb, c, s);
+            c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
         }
-        split3_any<__nv_bfloat16>(ra.x * scale, ra.y * scale, pa[e]);
-        split3_any<__nv_bfloat16>(rb.x * scale, rb.y * scale, pb[e]);
+        split3_any<__nv_bfloat16>((fa.x * c0 - fb.x * s0) * scale, (fa.y * c1 - fb.y * s1) * scale, pa[e]);
+        split3_any<__nv_bfloat16>((fb.x * c0 + fa.x * s0) * scale, (fb.y * c1 + fa.y * s1) * scale, pb[e]);
     }
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
@@ -238,8 +232,8 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sm = smem_u32(smem);
     // heads run fastest and the longest causal rows come first
-    const int N = p.N, heads = p.B * p.H, bh = blockIdx.x % heads, kvh = bh / (p.H / p.Hkv);
-    const int m0 = (gridDim.x / heads - 1 - blockIdx.x / heads) * F::kRows;
+    const int N = p.N, bh = blockIdx.x, kvh = bh / (p.H / p.Hkv);
+    const int m0 = (gridDim.y - 1 - blockIdx.y) * F::kRows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int row0 = m0 + warp * 16 + g;   // the lane's rows: row0 and row0 + 8
     const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0);
@@ -262,17 +256,21 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
             for (int x = 0; x < 4; ++x) {
                 const int pos = row0 + (x & 1) * 8, d = ks2 * 16 + (x >> 1) * 8 + c2;
                 float2 a = make_float2(0.f, 0.f), b = a;
+                float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
                 if (pos < N) {
                     const T* q = Q + (int64_t)pos * p.sq.n + d;
                     a = unpack2<T>(*reinterpret_cast<const uint32_t*>(q));
                     b = unpack2<T>(*reinterpret_cast<const uint32_t*>(q + D / 2));
-                    if (p.cos != nullptr) rotate(a, b, p.cos + (int64_t)pos * p.table_stride + d, p.sin + (int64_t)pos * p.table_stride + d);
+                    if (p.cos != nullptr) {
+                        const float *c = p.cos + (int64_t)pos * p.table_stride + d, *s = p.sin + (int64_t)pos * p.table_stride + d;
+                        c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
+                    }
                 }
                 uint32_t w[3];
-                split3_any<__nv_bfloat16>(a.x * scale, a.y * scale, w);
+                split3_any<__nv_bfloat16>((a.x * c0 - b.x * s0) * scale, (a.y * c1 - b.y * s1) * scale, w);
 #pragma unroll
                 for (int part = 0; part < 3; ++part) qa[ks2][part][x] = w[part];
-                split3_any<__nv_bfloat16>(b.x * scale, b.y * scale, w);
+                split3_any<__nv_bfloat16>((b.x * c0 + a.x * s0) * scale, (b.y * c1 + a.y * s1) * scale, w);
 #pragma unroll
                 for (int part = 0; part < 3; ++part) qa[ks2 + KS / 2][part][x] = w[part];
             }
@@ -395,9 +393,9 @@ __global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_spli
     const uint32_t sm = smem_u32(smem), stages = sm + 4 * W::kOwn;
     const int N = p.N, G = p.H / p.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
-    const int heads = p.B * (KV ? p.Hkv : p.H), own_head = blockIdx.x % heads, block = blockIdx.x / heads;   // KV: a K / V head, otherwise a query head
+    const int own_head = blockIdx.x;                         // KV: a K / V head, otherwise a query head
     const int kvh = KV ? own_head : own_head / G;
-    const int own0 = (KV ? block : gridDim.x / heads - 1 - block) * kRows;   // long causal sweeps first
+    const int own0 = (KV ? blockIdx.y : gridDim.y - 1 - blockIdx.y) * kRows;   // long causal sweeps first
     const int row0 = own0 + warp * 16 + g;                   // the lane's owned rows: row0 and row0 + 8
     const int first = KV && p.causal ? own0 / BS * BS : 0, end = !KV && p.causal ? min(N, own0 + kRows) : N;
     const int steps = (end - first + BS - 1) / BS, total = KV ? steps * G : steps;
@@ -576,7 +574,7 @@ int fwd(const RopeParams& p, void* ws, cudaStream_t s) {
     auto kern = rope_fwd_split_kernel<T, D>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, F::kSmem, smem_ok)) return e;
-    kern<<<rope_split_fwd_grid(p.B, p.H, p.N).blocks(), F::kThreads, F::kSmem, s>>>(p, k);
+    kern<<<dim3(p.B * p.H, (p.N + F::kRows - 1) / F::kRows), F::kThreads, F::kSmem, s>>>(p, k);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -587,24 +585,21 @@ int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
     const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D), q = take_rows(at, p.B, p.H, p.N, D);
     if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
     if (int e = split_rows<T, D>(p.q, p.sq, p.H, p, p.sm_scale * kLog2e, q, s)) return e;
+    const unsigned blocks = (p.N + W::kRows - 1) / W::kRows;
     auto kv = rope_bwd_split_kernel<T, D, true>;
     auto dq = rope_bwd_split_kernel<T, D, false>;
     static std::atomic<uint64_t> kv_ok, dq_ok;
     if (int e = allow_smem(kv, W::kSmem, kv_ok)) return e;
     if (int e = allow_smem(dq, W::kSmem, dq_ok)) return e;
-    kv<<<rope_split_bwd_grid(p.B, p.Hkv, p.N, D).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
+    kv<<<dim3(p.B * p.Hkv, blocks), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     if (cudaError_t e = cudaGetLastError()) return (int)e;
-    dq<<<rope_split_bwd_grid(p.B, p.H, p.N, D).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
+    dq<<<dim3(p.B * p.H, blocks), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     return (int)cudaGetLastError();
 }
 
 }  // namespace
-
-FlatGrid rope_split_fwd_grid(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, Fwd<64>::kRows)}; }
-static_assert(Fwd<64>::kRows == Fwd<128>::kRows, "one grid for both head dimensions");
-FlatGrid rope_split_bwd_grid(int B, int H, int N, int D) { return {(unsigned)(B * H), ceil_div(N, D == 64 ? Bwd<64>::kRows : Bwd<128>::kRows)}; }
 
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D) {
     return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 3 * sizeof(__nv_bfloat16);
