@@ -111,6 +111,12 @@ __device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3
         b = fabsf(b - f.y) < INFINITY ? b - f.y : 0.f;
     }
 }
+// two rotation pairs (a.x, b.x), (a.y, b.y) by neighbouring table entries
+__device__ __forceinline__ void rotate(float2& a, float2& b, const float* c, const float* s) {
+    const float2 x = a, y = b;
+    a = make_float2(x.x * c[0] - y.x * s[0], x.y * c[1] - y.y * s[1]);
+    b = make_float2(y.x * c[0] + x.x * s[0], y.y * c[1] + x.y * s[1]);
+}
 // two neighbouring 8-column accumulator tiles as the A operand of one k-step, split: a[part]
 template <typename T>
 __device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[4], float scale, uint32_t (&a)[3][4]) {
@@ -198,13 +204,13 @@ __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
         const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
-        float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
+        float2 ra = fa, rb = fb;
         if (cosT != nullptr) {   // null tables: plain attention
             const float *c = cosT + (int64_t)n * ts + d + 2 * e, *s = sinT + (int64_t)n * ts + d + 2 * e;
-            c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
+            rotate(ra, rb, c, s);
         }
-        split3_any<__nv_bfloat16>((fa.x * c0 - fb.x * s0) * scale, (fa.y * c1 - fb.y * s1) * scale, pa[e]);
-        split3_any<__nv_bfloat16>((fb.x * c0 + fa.x * s0) * scale, (fb.y * c1 + fa.y * s1) * scale, pb[e]);
+        split3_any<__nv_bfloat16>(ra.x * scale, ra.y * scale, pa[e]);
+        split3_any<__nv_bfloat16>(rb.x * scale, rb.y * scale, pb[e]);
     }
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
@@ -256,21 +262,17 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
             for (int x = 0; x < 4; ++x) {
                 const int pos = row0 + (x & 1) * 8, d = ks2 * 16 + (x >> 1) * 8 + c2;
                 float2 a = make_float2(0.f, 0.f), b = a;
-                float c0 = 1.f, c1 = 1.f, s0 = 0.f, s1 = 0.f;
                 if (pos < N) {
                     const T* q = Q + (int64_t)pos * p.sq.n + d;
                     a = unpack2<T>(*reinterpret_cast<const uint32_t*>(q));
                     b = unpack2<T>(*reinterpret_cast<const uint32_t*>(q + D / 2));
-                    if (p.cos != nullptr) {
-                        const float *c = p.cos + (int64_t)pos * p.table_stride + d, *s = p.sin + (int64_t)pos * p.table_stride + d;
-                        c0 = c[0], c1 = c[1], s0 = s[0], s1 = s[1];
-                    }
+                    if (p.cos != nullptr) rotate(a, b, p.cos + (int64_t)pos * p.table_stride + d, p.sin + (int64_t)pos * p.table_stride + d);
                 }
                 uint32_t w[3];
-                split3_any<__nv_bfloat16>((a.x * c0 - b.x * s0) * scale, (a.y * c1 - b.y * s1) * scale, w);
+                split3_any<__nv_bfloat16>(a.x * scale, a.y * scale, w);
 #pragma unroll
                 for (int part = 0; part < 3; ++part) qa[ks2][part][x] = w[part];
-                split3_any<__nv_bfloat16>((b.x * c0 + a.x * s0) * scale, (b.y * c1 + a.y * s1) * scale, w);
+                split3_any<__nv_bfloat16>(b.x * scale, b.y * scale, w);
 #pragma unroll
                 for (int part = 0; part < 3; ++part) qa[ks2 + KS / 2][part][x] = w[part];
             }

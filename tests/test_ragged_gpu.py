@@ -168,3 +168,22 @@ def test_ragged_lengths_are_as_accurate_as_fp32_kernels(N, D, causal, dtype, sca
         errors[policy] += [(a != b.to(dtype)).double().mean().item() for a, b in zip((saved[3],) + tuple(grads), (exact_o,) + exact)]
     for name, new, old in zip(("LSE", "O", "dQ", "dK", "dV"), errors[0], errors[1]):
         assert new <= 1.25 * old + (0.0 if name == "LSE" else 1e-4), (name, new, old)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_keys_masked_by_an_infinite_channel(D, dtype):
+    # a channel that is 1 in every query and -inf in some keys takes those keys out, as in fp32 arithmetic
+    N = 150
+    q, k, v = (draw((1, 2, N, D), 290 + i, dtype) for i in range(3))
+    q[..., 3] = 1.0
+    k[..., 3] = 0.0
+    hidden = torch.arange(N) % 3 == 1
+    plain = k.clone()
+    k[:, :, hidden, 3] = float("-inf")
+    o = pkg.flash_attention(q.cuda(), k.cuda(), v.cuda(), False, D ** -0.5)
+    ext.check_status()
+    seen = [t[:, :, ~hidden] for t in (plain, v)]
+    w = q.double() @ seen[0].double().transpose(-1, -2) * D ** -0.5
+    ref = w.softmax(-1) @ seen[1].double()
+    assert ((o.cpu().double() - ref).norm() / ref.norm()).item() < 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
