@@ -148,6 +148,9 @@ def lib():
             if hasattr(L, "corope_debug_synth_tables"):
                 L.corope_debug_synth_tables.restype = i32
                 L.corope_debug_synth_tables.argtypes = [vp, vp, vp, i32, i32, vp]
+            if hasattr(L, "corope_debug_grid"):
+                L.corope_debug_grid.restype = i32
+                L.corope_debug_grid.argtypes = [i32] * 6 + [ctypes.POINTER(ctypes.c_uint32)]
             if hasattr(L, "corope_debug_expire_wait"):
                 L.corope_debug_expire_wait.restype = i32
                 L.corope_debug_expire_wait.argtypes = [vp, ctypes.c_uint, vp]

@@ -79,6 +79,20 @@ __host__ __device__ inline int64_t flat_row_offset(const RowAddr& a, size_t row)
     return row_offset(a.st, a.H, (int)bh, (int)(r - bh * (unsigned)a.N));
 }
 
+// A grid of inner x outer blocks laid out along x alone, inner index fastest: x goes to 2^31 - 1, y and z only to 65 535, which heads
+// (up to 2 097 120) and row blocks (N / 16 of them) both exceed.
+struct FlatGrid {
+    unsigned inner, outer;
+    unsigned blocks() const { return inner * outer; }
+};
+__host__ __device__ inline unsigned ceil_div(unsigned a, unsigned b) { return (a + b - 1) / b; }
+// of the kernels that use it (also read by corope_debug_grid)
+FlatGrid rope_fp32_fwd_grid(int B, int H, int N);                 // heads x row blocks
+FlatGrid rope_fp32_bwd_grid(int B, int H, int Hkv, int N);        // K / V heads x (key block, its query heads' row blocks)
+FlatGrid rope_split_fwd_grid(int B, int H, int N);                // heads x row blocks
+FlatGrid rope_split_bwd_grid(int B, int H, int N, int D);         // heads (of K / V for dK and dV) x row blocks
+FlatGrid rope_prepass_grid(bool bwd, int B, int H, int N, int D); // position blocks x groups of heads
+
 // Launch parameters common to the fused-RoPE kernels.
 struct RopeParams {
     const void* q;

@@ -34,3 +34,22 @@ extern "C" int corope_debug_synth_tables(const float* inv_freq, float* cos_out, 
     if (!inv_freq || !cos_out || !sin_out || N <= 0 || half_d <= 0) return COROPE_ERR_NULL_POINTER;
     return corope::launch_synth_tables(inv_freq, 0.f, cos_out, sin_out, N, half_d, (cudaStream_t)stream);
 }
+
+extern "C" int corope_debug_grid(int kernel, int B, int Hq, int Hkv, int N, int D, uint32_t* inner_outer) {
+    if (!inner_outer) return COROPE_ERR_NULL_POINTER;
+    if (B <= 0 || Hq <= 0 || Hkv <= 0 || N <= 0) return COROPE_ERR_BAD_SHAPE;
+    corope::FlatGrid g;
+    switch (kernel) {
+        case 0: g = corope::rope_fp32_fwd_grid(B, Hq, N); break;
+        case 1: g = corope::rope_fp32_bwd_grid(B, Hq, Hkv, N); break;
+        case 2: g = corope::rope_split_fwd_grid(B, Hq, N); break;
+        case 3: g = corope::rope_split_bwd_grid(B, Hq, N, D); break;
+        case 4: g = corope::rope_split_bwd_grid(B, Hkv, N, D); break;
+        case 5: g = corope::rope_prepass_grid(false, B, Hkv, N, D); break;
+        case 6: g = corope::rope_prepass_grid(true, B, Hq, N, D); break;
+        default: return COROPE_ERR_BAD_SHAPE;
+    }
+    inner_outer[0] = g.inner;
+    inner_outer[1] = g.outer;
+    return COROPE_OK;
+}

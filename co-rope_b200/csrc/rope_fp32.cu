@@ -194,8 +194,8 @@ __global__ void __launch_bounds__(kThreads, 2) rope_fwd_fp32_kernel(RopeParams p
     float* row_s = s_s + BM * LDS_;  // [BM] rescale factor of the row, at the end its sum
 
     // heads run fastest and the longest causal rows come first: dealt to the SMs in this order the CTAs balance
-    const int N = p.N, bh = blockIdx.x;
-    const int m0 = (gridDim.y - 1 - blockIdx.y) * BM;
+    const int N = p.N, heads = p.B * p.H, bh = blockIdx.x % heads;
+    const int m0 = (gridDim.x / heads - 1 - blockIdx.x / heads) * BM;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int ty = (warp >> 2) * 8 + (lane >> 2), tx = (warp & 3) * 4 + (lane & 3);
     const int kvh = bh / (p.H / p.Hkv);                 // the heads of a group are adjacent
@@ -530,9 +530,9 @@ __device__ void dkdv_block(const RopeParams& p, const Flags& f, float* smem, int
 template <int D>
 __global__ void __launch_bounds__(kThreads, 2) rope_bwd_fp32_kernel(RopeParams p, Flags f) {
     extern __shared__ __align__(16) float smem[];
-    const int blocks = (p.N + kBR - 1) / kBR, G = p.H / p.Hkv;
-    // blockIdx.y = block * (G + 1) + kind: kind 0 is dK / dV of KV head x, kinds 1 .. G are dQ of its G query heads
-    const int block = blockIdx.y / (G + 1), kind = blockIdx.y % (G + 1), kvh = blockIdx.x;
+    const int blocks = (p.N + kBR - 1) / kBR, G = p.H / p.Hkv, heads = p.B * p.Hkv;
+    // outer index = block * (G + 1) + kind: kind 0 is dK / dV of the KV head, kinds 1 .. G are dQ of its G query heads
+    const int kvh = blockIdx.x % heads, outer = blockIdx.x / heads, block = outer / (G + 1), kind = outer % (G + 1);
     if (kind == 0)
         dkdv_block<D>(p, f, smem, kvh, block * kBR);
     else
@@ -565,6 +565,9 @@ Flags flags_of(const RopeParams& p, size_t elem) {
     return f;
 }
 
+FlatGrid fwd_grid(int B, int H, int N, int BM) { return {(unsigned)(B * H), ceil_div(N, BM)}; }
+bool fwd_64_rows(int B, int H, int N) { return (int64_t)((N + 63) / 64) * B * H >= 4 * sm_count(); }
+
 template <typename T, int D, int BM>
 int launch_fwd(const RopeParams& p, cudaStream_t s) {
     constexpr int BN = D == 128 ? 32 : 64;
@@ -572,7 +575,7 @@ int launch_fwd(const RopeParams& p, cudaStream_t s) {
     auto kern = rope_fwd_fp32_kernel<T, D, BM>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, smem, smem_ok)) return e;
-    kern<<<dim3(p.B * p.H, (p.N + BM - 1) / BM), kThreads, smem, s>>>(p, flags_of(p, sizeof(T)));
+    kern<<<fwd_grid(p.B, p.H, p.N, BM).blocks(), kThreads, smem, s>>>(p, flags_of(p, sizeof(T)));
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -580,7 +583,7 @@ int launch_fwd(const RopeParams& p, cudaStream_t s) {
 // balance and hide latency better.
 template <typename T, int D>
 int launch_fwd_rows(const RopeParams& p, cudaStream_t s) {
-    return (int64_t)((p.N + 63) / 64) * p.B * p.H >= 4 * sm_count() ? launch_fwd<T, D, 64>(p, s) : launch_fwd<T, D, 32>(p, s);
+    return fwd_64_rows(p.B, p.H, p.N) ? launch_fwd<T, D, 64>(p, s) : launch_fwd<T, D, 32>(p, s);
 }
 template <int D>
 int launch_bwd(const RopeParams& p, cudaStream_t s) {
@@ -592,8 +595,7 @@ int launch_bwd(const RopeParams& p, cudaStream_t s) {
     auto kern = rope_bwd_fp32_kernel<D>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, Bwd<D>::kSmem, smem_ok)) return e;
-    const dim3 grid(p.B * p.Hkv, (unsigned)((p.N + kBR - 1) / kBR) * (p.H / p.Hkv + 1));
-    kern<<<grid, kThreads, Bwd<D>::kSmem, s>>>(p, flags_of(p, 4));
+    kern<<<rope_fp32_bwd_grid(p.B, p.H, p.Hkv, p.N).blocks(), kThreads, Bwd<D>::kSmem, s>>>(p, flags_of(p, 4));
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -608,6 +610,9 @@ int fwd_d(const RopeParams& p, cudaStream_t s) {
 }
 
 }  // namespace
+
+FlatGrid rope_fp32_fwd_grid(int B, int H, int N) { return fwd_grid(B, H, N, fwd_64_rows(B, H, N) ? 64 : 32); }
+FlatGrid rope_fp32_bwd_grid(int B, int H, int Hkv, int N) { return {(unsigned)(B * Hkv), ceil_div(N, kBR) * (unsigned)(H / Hkv + 1)}; }
 
 int launch_rope_fwd_general(const RopeParams& p, int dtype, cudaStream_t s) {
     switch (dtype) {

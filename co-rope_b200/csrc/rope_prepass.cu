@@ -60,24 +60,25 @@ struct PrepassTable {
     uint32_t* packed;   // read (kPacked) or written by the blocks of the first heads; the work counter follows it
 };
 
-// Forward: D / 16 threads per row, 8 pairs each.  grid (position blocks, head groups).
+// Forward: D / 16 threads per row, 8 pairs each.  Position blocks run fastest, then groups of heads.
 template <typename T, int D, int MODE>
 __global__ void __launch_bounds__(kThreads) rope_fwd_prepass_kernel(const T* __restrict__ k, __half* __restrict__ k_rot, PrepassTable tab, int N,
                                                                     int BH, int heads_per_block, RowAddr ak) {
     constexpr int kPerRow = D / 16, kRows = kThreads / kPerRow, kUnroll = 4;
-    const int n = blockIdx.x * kRows + threadIdx.x / kPerRow;
+    const unsigned pbs = ceil_div(N, kRows), group = blockIdx.x / pbs;
+    const int n = (blockIdx.x % pbs) * kRows + threadIdx.x / kPerRow;
     const int c = (threadIdx.x % kPerRow) * 8;
-    if (MODE != kPacked && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) tab.packed[(size_t)N * (D / 2)] = 0u;   // work counter
+    if (MODE != kPacked && blockIdx.x == 0 && threadIdx.x == 0) tab.packed[(size_t)N * (D / 2)] = 0u;   // work counter
     if (n >= N) return;
     uint4 t0, t1;
     table_entries<MODE, D / 2>(t0, t1, tab.cos, tab.sin, tab.stride, tab.vec, tab.packed, n, c);
-    if (MODE != kPacked && blockIdx.y == 0) {
+    if (MODE != kPacked && group == 0) {
         uint4* out = reinterpret_cast<uint4*>(tab.packed + (size_t)n * (D / 2) + c);
         out[0] = t0;
         out[1] = t1;
     }
-    const int h1 = min(BH, (int)(blockIdx.y + 1) * heads_per_block);
-    for (int h = blockIdx.y * heads_per_block; h < h1; h += kUnroll) {
+    const int h1 = min(BH, (int)(group + 1) * heads_per_block);
+    for (int h = group * heads_per_block; h < h1; h += kUnroll) {
         uint4 x1[kUnroll], x2[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u)
@@ -106,22 +107,23 @@ __global__ void __launch_bounds__(kThreads) rope_bwd_prepass_kernel(const T* __r
                                                                     int N, int BH, int heads_per_block, float scale, RowAddr aq,
                                                                     RowAddr ao, RowAddr ado) {
     constexpr int kPerRow = D / 8, kRows = kThreads / kPerRow, kUnroll = 2;
-    const int n = blockIdx.x * kRows + threadIdx.x / kPerRow;
+    const unsigned pbs = ceil_div(N, kRows), group = blockIdx.x / pbs;
+    const int n = (blockIdx.x % pbs) * kRows + threadIdx.x / kPerRow;
     const int part = threadIdx.x % kPerRow;
     const bool live = n < N, rot = live && part < kPerRow / 2;
     const int c = part * 8;
-    if (MODE != kPacked && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) tab.packed[(size_t)N * (D / 2)] = 0u;   // work counter
+    if (MODE != kPacked && blockIdx.x == 0 && threadIdx.x == 0) tab.packed[(size_t)N * (D / 2)] = 0u;   // work counter
     uint4 t0 = make_uint4(0u, 0u, 0u, 0u), t1 = t0;
     if (rot) {
         table_entries<MODE, D / 2>(t0, t1, tab.cos, tab.sin, tab.stride, tab.vec, tab.packed, n, c);
-        if (MODE != kPacked && blockIdx.y == 0) {
+        if (MODE != kPacked && group == 0) {
             uint4* out = reinterpret_cast<uint4*>(tab.packed + (size_t)n * (D / 2) + c);
             out[0] = t0;
             out[1] = t1;
         }
     }
-    const int h1 = min(BH, (int)(blockIdx.y + 1) * heads_per_block);
-    for (int h = blockIdx.y * heads_per_block; h < h1; h += kUnroll) {
+    const int h1 = min(BH, (int)(group + 1) * heads_per_block);
+    for (int h = group * heads_per_block; h < h1; h += kUnroll) {
         uint4 a[kUnroll], b[kUnroll], x1[kUnroll], x2[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; ++u) {
@@ -219,26 +221,23 @@ PrepassTable prepass_table(const TableSource& src, uint32_t* packed) {
 
 // Heads per block: as many as still leave about eight blocks per SM, at most eight.
 int heads_per_block_for(int position_blocks, int BH) {
-    const int want = position_blocks * BH / (148 * 8);
-    return want < 1 ? 1 : want > 8 ? 8 : want;
+    const int64_t want = (int64_t)position_blocks * BH / (sm_count() * 8);
+    return want < 1 ? 1 : want > 8 ? 8 : (int)want;
 }
+int prepass_rows(bool bwd, int D) { return kThreads / (D / (bwd ? 8 : 16)); }   // positions per block
 
 template <typename T, int D, int MODE>
 int fwd_prepass_t(const RopeParams& p, const PrepassTable& tab, cudaStream_t s) {
-    constexpr int kRows = kThreads / (D / 16);
-    const int BH = p.B * p.Hkv, pb = (p.N + kRows - 1) / kRows, hpb = heads_per_block_for(pb, BH);
-    const dim3 grid(pb, (BH + hpb - 1) / hpb);
-    rope_fwd_prepass_kernel<T, D, MODE><<<grid, kThreads, 0, s>>>((const T*)p.k, (__half*)const_cast<void*>(p.k_rot), tab, p.N, BH, hpb,
+    const int BH = p.B * p.Hkv, hpb = heads_per_block_for(ceil_div(p.N, prepass_rows(false, D)), BH);
+    rope_fwd_prepass_kernel<T, D, MODE><<<rope_prepass_grid(false, p.B, p.Hkv, p.N, D).blocks(), kThreads, 0, s>>>((const T*)p.k, (__half*)const_cast<void*>(p.k_rot), tab, p.N, BH, hpb,
                                                                   row_addr(p.sk, p.Hkv, p.N));
     count_launch();
     return (int)cudaGetLastError();
 }
 template <typename T, int D, int MODE>
 int bwd_prepass_t(const RopeParams& p, const PrepassTable& tab, cudaStream_t s) {
-    constexpr int kRows = kThreads / (D / 8);
-    const int BH = p.B * p.H, pb = (p.N + kRows - 1) / kRows, hpb = heads_per_block_for(pb, BH);
-    const dim3 grid(pb, (BH + hpb - 1) / hpb);
-    rope_bwd_prepass_kernel<T, D, MODE><<<grid, kThreads, 0, s>>>((const T*)p.q, (const T*)p.o, (const T*)p.d_o, tab,
+    const int BH = p.B * p.H, hpb = heads_per_block_for(ceil_div(p.N, prepass_rows(true, D)), BH);
+    rope_bwd_prepass_kernel<T, D, MODE><<<rope_prepass_grid(true, p.B, p.H, p.N, D).blocks(), kThreads, 0, s>>>((const T*)p.q, (const T*)p.o, (const T*)p.d_o, tab,
                                                                   (__half*)const_cast<void*>(p.q_rot), p.delta, p.dq_acc, p.N, BH, hpb,
                                                                   p.sm_scale * kLog2e, row_addr(p.sq, p.H, p.N), row_addr(p.so, p.H, p.N),
                                                                   row_addr(p.sdo, p.H, p.N));
@@ -260,6 +259,11 @@ int prepass(bool bwd, const RopeParams& p, const TableSource& src, uint32_t* pac
 }
 
 }  // namespace
+
+FlatGrid rope_prepass_grid(bool bwd, int B, int H, int N, int D) {
+    const unsigned pbs = ceil_div(N, prepass_rows(bwd, D));
+    return {pbs, ceil_div(B * H, heads_per_block_for(pbs, B * H))};
+}
 
 int launch_rope_fwd_prepass(const RopeParams& p, const TableSource& src, uint32_t* packed, int dtype, cudaStream_t s) {
     return prepass(false, p, src, packed, dtype, s);

@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sm = smem_u32(smem);
     // heads run fastest and the longest causal rows come first
-    const int N = p.N, bh = blockIdx.x, kvh = bh / (p.H / p.Hkv);
-    const int m0 = (gridDim.y - 1 - blockIdx.y) * F::kRows;
+    const int N = p.N, heads = p.B * p.H, bh = blockIdx.x % heads, kvh = bh / (p.H / p.Hkv);
+    const int m0 = (gridDim.x / heads - 1 - blockIdx.x / heads) * F::kRows;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int row0 = m0 + warp * 16 + g;   // the lane's rows: row0 and row0 + 8
     const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0);
@@ -395,9 +395,9 @@ __global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_spli
     const uint32_t sm = smem_u32(smem), stages = sm + 4 * W::kOwn;
     const int N = p.N, G = p.H / p.Hkv;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
-    const int own_head = blockIdx.x;                         // KV: a K / V head, otherwise a query head
+    const int heads = p.B * (KV ? p.Hkv : p.H), own_head = blockIdx.x % heads, block = blockIdx.x / heads;   // KV: a K / V head, otherwise a query head
     const int kvh = KV ? own_head : own_head / G;
-    const int own0 = (KV ? blockIdx.y : gridDim.y - 1 - blockIdx.y) * kRows;   // long causal sweeps first
+    const int own0 = (KV ? block : gridDim.x / heads - 1 - block) * kRows;   // long causal sweeps first
     const int row0 = own0 + warp * 16 + g;                   // the lane's owned rows: row0 and row0 + 8
     const int first = KV && p.causal ? own0 / BS * BS : 0, end = !KV && p.causal ? min(N, own0 + kRows) : N;
     const int steps = (end - first + BS - 1) / BS, total = KV ? steps * G : steps;
@@ -576,7 +576,7 @@ int fwd(const RopeParams& p, void* ws, cudaStream_t s) {
     auto kern = rope_fwd_split_kernel<T, D>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, F::kSmem, smem_ok)) return e;
-    kern<<<dim3(p.B * p.H, (p.N + F::kRows - 1) / F::kRows), F::kThreads, F::kSmem, s>>>(p, k);
+    kern<<<rope_split_fwd_grid(p.B, p.H, p.N).blocks(), F::kThreads, F::kSmem, s>>>(p, k);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -587,21 +587,24 @@ int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
     const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D), q = take_rows(at, p.B, p.H, p.N, D);
     if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
     if (int e = split_rows<T, D>(p.q, p.sq, p.H, p, p.sm_scale * kLog2e, q, s)) return e;
-    const unsigned blocks = (p.N + W::kRows - 1) / W::kRows;
     auto kv = rope_bwd_split_kernel<T, D, true>;
     auto dq = rope_bwd_split_kernel<T, D, false>;
     static std::atomic<uint64_t> kv_ok, dq_ok;
     if (int e = allow_smem(kv, W::kSmem, kv_ok)) return e;
     if (int e = allow_smem(dq, W::kSmem, dq_ok)) return e;
-    kv<<<dim3(p.B * p.Hkv, blocks), W::kThreads, W::kSmem, s>>>(p, q, k);
+    kv<<<rope_split_bwd_grid(p.B, p.Hkv, p.N, D).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     if (cudaError_t e = cudaGetLastError()) return (int)e;
-    dq<<<dim3(p.B * p.H, blocks), W::kThreads, W::kSmem, s>>>(p, q, k);
+    dq<<<rope_split_bwd_grid(p.B, p.H, p.N, D).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     return (int)cudaGetLastError();
 }
 
 }  // namespace
+
+FlatGrid rope_split_fwd_grid(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, Fwd<64>::kRows)}; }
+static_assert(Fwd<64>::kRows == Fwd<128>::kRows, "one grid for both head dimensions");
+FlatGrid rope_split_bwd_grid(int B, int H, int N, int D) { return {(unsigned)(B * H), ceil_div(N, D == 64 ? Bwd<64>::kRows : Bwd<128>::kRows)}; }
 
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D) {
     return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 3 * sizeof(__nv_bfloat16);

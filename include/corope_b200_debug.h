@@ -45,6 +45,12 @@ int corope_debug_expire_wait(int* status_word, unsigned max_polls, void* stream)
  */
 int corope_debug_synth_tables(const float* inv_freq, float* cos_out, float* sin_out, int N, int half_d, void* stream);
 
+/*
+ * The grid of a launch, without a launch (inner_outer[2], host): inner * outer blocks along x.  kernel: 0 fp32 forward, 1 fp32 backward,
+ * 2 split-operand forward, 3 / 4 its backward for dQ / for dK and dV, 5 / 6 pre-pass of the tcgen05 forward / backward.
+ */
+int corope_debug_grid(int kernel, int B, int Hq, int Hkv, int N, int D, uint32_t* inner_outer);
+
 #ifdef __cplusplus
 }
 #endif

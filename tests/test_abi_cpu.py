@@ -114,3 +114,25 @@ def test_fused_entry_point_asserts_head_dim_like_the_reference():
     t = torch.zeros(8, 48)
     with pytest.raises(AssertionError):
         fused_attention(q, q, q, True, 1.0, t, t)
+
+
+@pytest.mark.parametrize("kernel", range(7))
+@pytest.mark.parametrize("B,Hq,Hkv,N,D", [(1, 64, 1, 32768, 64), (1, 128, 1, 65536, 128), (1, 8, 1, 1 << 20, 64), (1, 600000, 600000, 128, 64),
+                                          (2097120, 1, 1, 128, 128), (1, 1, 1, (1 << 31) - 1, 64), (1, 2097120, 1, 1000, 64), (1, 3, 1, 1, 32)])
+def test_every_admitted_size_has_a_grid_that_launches(kernel, B, Hq, Hkv, N, D):
+    # blocks lie along x, which goes to 2^31 - 1; y would end at 65 535.  Every row of every head has its block.
+    out = (ctypes.c_uint32 * 2)()
+    assert ext.lib().corope_debug_grid(kernel, B, Hq, Hkv, N, D, out) == 0
+    inner, outer = out
+    assert inner * outer <= 2 ** 31 - 1
+    G = Hq // Hkv
+    rows = (None, 32, 64, 64 if D == 64 else 128, 64 if D == 64 else 128)
+    if kernel == 0:
+        assert inner == B * Hq and outer in (-(-N // 32), -(-N // 64))
+    elif kernel == 1:
+        assert inner == B * Hkv and outer == -(-N // 32) * (G + 1)
+    elif kernel in (2, 3, 4):
+        assert inner == B * (Hkv if kernel == 4 else Hq) and outer == -(-N // rows[kernel])
+    else:
+        heads = B * (Hkv if kernel == 5 else Hq)
+        assert inner == -(-N // (256 // (D // (16 if kernel == 5 else 8)))) and -(-heads // 8) <= outer <= heads

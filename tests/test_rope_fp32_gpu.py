@@ -48,3 +48,15 @@ def test_grouped_heads_many_ctas_and_unaligned_rows(pad):
     refs = (oracle.attn_gqa_fwd(q, k, v, True, D ** -0.5),) + tuple(oracle.attn_gqa_bwd(q, k, v, do, True, D ** -0.5))
     for a, b in zip(outs, refs):
         assert maxdiff(a, b) < TOL_32
+
+
+def test_backward_of_a_very_large_group():
+    # 32 768 query heads on one K / V head: 65 538 row blocks of one key head.  dK and dV are sums over all of them, so the tolerance is
+    # relative to their largest value.
+    B, Hq, Hkv, N, D = 1, 32768, 1, 33, 32
+    q, do = (draw((B, Hq, N, D), 420 + i, torch.float32) for i in range(2))
+    k, v = (draw((B, Hkv, N, D), 422 + i, torch.float32) for i in range(2))
+    outs = _run(pkg.flash_attention, *(t.cuda() for t in (q, k, v, do)), True, D ** -0.5)
+    refs = (oracle.attn_gqa_fwd(q, k, v, True, D ** -0.5),) + tuple(oracle.attn_gqa_bwd(q, k, v, do, True, D ** -0.5))
+    for a, b in zip(outs, refs):
+        assert maxdiff(a, b) < TOL_32 * max(1.0, b.abs().max().item())
