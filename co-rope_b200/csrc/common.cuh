@@ -205,11 +205,15 @@ __device__ __forceinline__ bool mbar_wait_limited(uint64_t* bar, uint32_t parity
     if (status) atomicCAS(status, 0, COROPE_DEV_WAIT_EXPIRED | id);
     return false;
 }
-// A kernel that gave up leaves its code in the host mirror too, so that the host learns of it without a copy or a synchronisation.
-__device__ __forceinline__ void report_to_mirror(const int* status, int* mirror) {
-    if (status == nullptr || mirror == nullptr) return;
-    *reinterpret_cast<volatile int*>(mirror) = *reinterpret_cast<const volatile int*>(status);
+// A kernel that gave up, or that did not start because an earlier one had, leaves the code in the host mirror too: the host learns of
+// every launch that did not compute without a copy or a synchronisation.
+__device__ __forceinline__ void report_to_mirror(int code, int* mirror) {
+    if (code == 0 || mirror == nullptr) return;
+    *reinterpret_cast<volatile int*>(mirror) = code;
     __threadfence_system();
+}
+__device__ __forceinline__ void report_to_mirror(const int* status, int* mirror) {
+    if (status != nullptr) report_to_mirror(*reinterpret_cast<const volatile int*>(status), mirror);
 }
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, int id, volatile int* abort_flag) {
     return mbar_wait_limited(bar, parity, status, id, abort_flag, kWaitLimit);

@@ -156,12 +156,22 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // item's last tiles are still in the MMAs and its output is being written.
 
     if (reinterpret_cast<uintptr_t>(sm) - reinterpret_cast<uintptr_t>(smem_raw) > kSmemSlack) {   // base less aligned than assumed
-        if (threadIdx.x == 0 && p.status) atomicCAS(p.status, 0, COROPE_DEV_WAIT_EXPIRED | 0xfff);
+        if (threadIdx.x == 0 && p.status) {
+            atomicCAS(p.status, 0, COROPE_DEV_WAIT_EXPIRED | 0xfff);
+            report_to_mirror(COROPE_DEV_WAIT_EXPIRED | 0xfff, p.status_mirror);
+        }
         return;
     }
     // A non-zero status word means an earlier CTA (of this or a previous launch) gave up on a wait: do not pile up
-    // more timeouts behind it.  The word stays set until the host reads and clears it.
-    if (p.status != nullptr && *reinterpret_cast<volatile int*>(p.status) != 0) return;
+    // more timeouts behind it.  The word stays set until the host reads and clears it; the mirror may already be clear (the host resets it
+    // at once, the word in stream order), so this launch reports too.
+    if (p.status != nullptr) {
+        const int code = *reinterpret_cast<volatile int*>(p.status);
+        if (code != 0) {
+            if (threadIdx.x == 0) report_to_mirror(code, p.status_mirror);
+            return;
+        }
+    }
     if (threadIdx.x == 0) {
         *abort_flag = 0;
         for (int i = 0; i < 2; ++i) {

@@ -23,6 +23,33 @@ def test_a_failing_kernel_writes_the_host_mirror_itself():
     ext.check_status(dev)
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("backward", [False, True])
+def test_a_launch_that_does_not_compute_is_reported(D, backward):
+    # the word is set and the mirror clear: what a call on another stream meets after a failure has been raised and before the word has
+    # been cleared in stream order.  The kernels skip their work then, so the next call has to raise.
+    dev = torch.device("cuda", 0)
+    ext.check_status(dev)
+    q, k, v, do = (draw((1, 2, 256, D), 10 + i, torch.bfloat16).cuda() for i in range(4))
+    cos, sin = (t.cuda() for t in oracle.precompute_freqs_cis(D, 256, 10000.0))
+    rope = pkg.fused_rope_attn
+    saved = rope._forward(q, k, v, True, D ** -0.5, cos, sin)
+    word, mirror = ext.status_word(dev), ext._status(dev).mirror_view
+    assert ext.lib().corope_debug_expire_wait(word.data_ptr(), 100, torch.cuda.current_stream(dev).cuda_stream) == 0
+    torch.cuda.synchronize()
+    mirror[0] = 0
+    if backward:
+        rope._backward(*saved, do, True, D ** -0.5)
+    else:
+        rope._forward(q, k, v, True, D ** -0.5, cos, sin)
+    torch.cuda.synchronize()
+    assert int(word.item()) == 0x107e
+    with pytest.raises(RuntimeError, match="0x107e"):
+        rope._forward(q, k, v, True, D ** -0.5, cos, sin)
+    rope._forward(q, k, v, True, D ** -0.5, cos, sin)   # cleared
+    ext.check_status(dev)
+
+
 def test_broadcast_output_gradient_and_partial_requires_grad():
     # o.sum().backward() hands over a dO with zero strides; only v asks for a gradient
     B, H, N, D = 1, 2, 160, 64
