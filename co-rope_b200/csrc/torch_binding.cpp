@@ -395,42 +395,44 @@ PYBIND11_MODULE(_corope_torch, m) {
             PyErr_SetString(PyExc_ValueError, e.what());
         }
     });
+    // The GIL is released for every call: a launch blocks once the launch queue is full, and other Python threads go on meanwhile.
     // autograd entry points
+    using NoGil = py::call_guard<py::gil_scoped_release>;
     m.def("rope_attention", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double sm_scale, const Tensor& cos, const Tensor& sin) {
         return RopeFunction::apply(q, k, v, causal, sm_scale, cos, sin);
-    });
+    }, NoGil());
     m.def("theta_attention", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double sm_scale, double theta) {
         return MhaFunction::apply((int64_t)kTheta, q, k, v, causal, sm_scale, theta);
-    });
+    }, NoGil());
     m.def("flash_attention", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double sm_scale) {
         return MhaFunction::apply((int64_t)kFlash, q, k, v, causal, sm_scale, 0.0);
-    });
+    }, NoGil());
     m.def("gqa_attention", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double sm_scale, double theta) {
         return GqaFunction::apply(q, k, v, causal, sm_scale, theta);
-    });
+    }, NoGil());
     // the library calls alone, without autograd
     m.def("rope_forward", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double sm_scale, const Tensor& cos, const Tensor& sin) {
         Saved s = mha_forward(kRope, q, k, v, causal, sm_scale, cos, sin, 0.0);
-        return py::make_tuple(s.q, s.k, s.v, s.o, s.m, s.tab.cos, s.tab.sin, s.tab.stride);
-    });
+        return std::make_tuple(s.q, s.k, s.v, s.o, s.m, s.tab.cos, s.tab.sin, s.tab.stride);
+    }, NoGil());
     m.def("rope_backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse, const Tensor& cos, const Tensor& sin,
                               int64_t stride, const Tensor& d_o, bool causal, double sm_scale) {
         Grads g = mha_backward(kRope, Saved{q, k, v, o, lse, Tables{cos, sin, stride}}, d_o, causal, sm_scale, 0.0);
-        return py::make_tuple(g.dq, g.dk, g.dv);
-    });
+        return std::make_tuple(g.dq, g.dk, g.dv);
+    }, NoGil());
     m.def("gqa_forward", [](const Tensor& q, const Tensor& k, const Tensor& v, bool causal, double sm_scale, double theta) {
         GqaSaved s = gqa_forward(q, k, v, causal, sm_scale, theta);
-        return py::make_tuple(s.q, s.k, s.v, s.o, s.lse2, s.a_diag);
-    });
+        return std::make_tuple(s.q, s.k, s.v, s.o, s.lse2, s.a_diag);
+    }, NoGil());
     m.def("gqa_backward", [](const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, const Tensor& lse2, const Tensor& a_diag, const Tensor& d_o,
                              double sm_scale, double theta) {
         Grads g = gqa_backward(GqaSaved{q, k, v, o, lse2, a_diag}, d_o, sm_scale, theta);
-        return py::make_tuple(g.dq, g.dk, g.dv);
-    });
+        return std::make_tuple(g.dq, g.dk, g.dv);
+    }, NoGil());
     // (status word tensor, pinned mirror tensor) of a device, created on first use
     m.def("device_status", [](int index) {
         c10::cuda::CUDAGuard guard((c10::DeviceIndex)index);
         DeviceStatus& st = device_status(index);
-        return py::make_tuple(st.word, st.mirror);
-    });
+        return std::make_tuple(st.word, st.mirror);
+    }, NoGil());
 }

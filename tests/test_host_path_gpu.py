@@ -1,6 +1,9 @@
 """The C++ host path of the entry points: a device-side failure reaches the host without any call in between, and output
 gradients and masks in forms a caller may hand over."""
 
+import threading
+import time
+
 import pytest
 import torch
 
@@ -74,3 +77,39 @@ def test_wrong_tables_and_dtypes_raise_the_python_errors():
         fused_attention(q, q, q.float(), True, 1.0, t, t)
     with pytest.raises(AssertionError):
         pkg.flash_attention(q, q, q[..., :32], True, 1.0)
+
+
+@pytest.mark.parametrize("entry", ["rope", "theta", "flash", "corope"])
+def test_other_threads_run_while_launches_wait(entry):
+    # the GPU is busy for about half a second and the launch queue fills up behind that: the calls block in the launch, and a thread
+    # that wants to run every millisecond must not be held up for that time
+    q = torch.zeros(1, 1, 128, 64, device="cuda", dtype=torch.bfloat16)
+    t = torch.zeros(128, 64, device="cuda")
+    call = {"rope": lambda: fused_attention(q, q, q, True, 1.0, t, t), "theta": lambda: pkg.fused_rope_attention_theta(q, q, q, True, 1.0, 1e4),
+            "flash": lambda: pkg.flash_attention(q, q, q, True, 1.0), "corope": lambda: pkg.corope_gqa_attention(q, q, q, True, 1.0, 1e4)}[entry]
+    call()
+    torch.cuda.synchronize()
+    stop, longest = threading.Event(), [0.0]
+
+    def tick():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            longest[0], last = max(longest[0], now - last), now
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        time.sleep(0.01)
+        torch.cuda._sleep(10 ** 9)   # cycles: 0.5 s at the highest clock
+        began = time.perf_counter()
+        for _ in range(4000):
+            call()
+        took = time.perf_counter() - began
+    finally:
+        stop.set()
+        thread.join()
+        torch.cuda.synchronize()
+    assert took > 0.3          # the queue did fill up
+    assert longest[0] < 0.1, longest
