@@ -104,6 +104,8 @@ Tensor kernel_layout(const Tensor& t) {
     if (st[3] == 1 && st[0] > 0 && st[1] > 0 && st[2] >= t.size(3)) return t;
     return t.contiguous();
 }
+// Outputs and gradients: laid out like the input, or contiguous (the entry point that takes theta)
+Tensor new_like(const Tensor& t, bool contiguous) { return contiguous ? at::empty(t.sizes(), t.options()) : at::empty_like(t); }
 void set_strides(int64_t (&dst)[3], const Tensor& t) {
     const auto st = t.strides();
     dst[0] = st[0]; dst[1] = st[1]; dst[2] = st[2];
@@ -188,7 +190,7 @@ Saved mha_forward(Kind kind, const Tensor& q_in, const Tensor& k_in, const Tenso
     s.q = kernel_layout(q_in);
     s.k = kernel_layout(k_in);
     s.v = kernel_layout(v_in);
-    s.o = at::empty_like(s.q);
+    s.o = new_like(s.q, kind == kTheta);
     s.m = new_rows(s.q, B, Hq, N);
     const int op = kind == kRope ? COROPE_OP_ROPE_FWD : kind == kTheta ? COROPE_OP_ROPE_FWD_FREQS : COROPE_OP_FLASH_FWD;
     Workspace ws(op, B, Hq, Hkv, N, D, dt, s.q);
@@ -229,7 +231,7 @@ Grads mha_backward(Kind kind, const Saved& s, const Tensor& d_out, bool causal, 
     Call call(s.q);
     const Tensor d_o = kernel_layout(d_out);
     TORCH_CHECK(d_o.is_cuda() && d_o.scalar_type() == s.q.scalar_type() && d_o.sizes() == s.o.sizes(), "dO must match o");
-    Grads g{at::empty_like(s.q), at::empty_like(s.k), at::empty_like(s.v)};
+    Grads g{new_like(s.q, kind == kTheta), new_like(s.k, kind == kTheta), new_like(s.v, kind == kTheta)};
     const int op = kind == kRope ? COROPE_OP_ROPE_BWD : kind == kTheta ? COROPE_OP_ROPE_BWD_FREQS : COROPE_OP_FLASH_BWD;
     Workspace ws(op, B, Hq, Hkv, N, D, dt, s.q);
     corope_strides_t st;

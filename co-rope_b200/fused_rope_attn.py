@@ -4,7 +4,7 @@
 
 q, k, v: [B, H, N, D] CUDA tensors of one dtype (bf16, fp16 or fp32).  freqs_cos / freqs_sin: [N, D]
 ("cat" layout of precompute_freqs_cis) or [N, D/2]; only columns [0, D/2) are read, as in the
-reference (fused_rope_attn.py:88-93).  Positional-only, like torch.autograd.Function.apply.
+reference (fused_rope_attn.py:88-93).
 The CUDA kernels are reached through the C ABI in include/corope_b200.h; the checks (those of the reference's entry point,
 fused_rope_attn.py:657-661), allocations and autograd nodes are C++ (csrc/torch_binding.cpp).
 
@@ -52,5 +52,5 @@ def inv_freq_of(theta, D, device):
 
 
 def attention_theta(q, k, v, causal, sm_scale, theta):
-    """Positions 0 .. N-1, base theta."""
+    """Positions 0 .. N-1, base theta.  O and the gradients are contiguous whatever the inputs' strides are."""
     return _ext.native().theta_attention(q, k, v, causal, sm_scale, theta)

@@ -295,3 +295,22 @@ def test_strided_entry_point_rejects_bad_strides():
     rc = lib.corope_gqa_fwd_strided(t.data_ptr(), t.data_ptr(), t.data_ptr(), t.data_ptr(), g.data_ptr(), g.data_ptr(), 1, 1, 1, 128, 128, 1,
                                     0.1, 10000.0, ws.data_ptr(), nbytes, None, None, st)
     assert rc == -11
+
+
+@pytest.mark.parametrize("dtype,N,D", [(torch.bfloat16, 256, 128), (torch.float16, 200, 64), (torch.float32, 100, 64)])
+def test_theta_results_are_contiguous(dtype, N, D):
+    # inputs viewed from [B, N, H, D] buffers: O and the gradients are contiguous [B, H, N, D] tensors, with the values of contiguous inputs
+    B, H = 2, 3
+    q, k, v, do = (draw((B, H, N, D), 140 + i, dtype).cuda() for i in range(4))
+
+    def run(make):
+        leaves = [make(t).detach().requires_grad_(True) for t in (q, k, v)]
+        o = pkg.fused_rope_attention_theta(*leaves, True, D ** -0.5, 10000.0)
+        return (o,) + torch.autograd.grad(o, leaves, make(do))
+
+    ref, got = run(lambda t: t.clone()), run(_as_bnhd_view)
+    ext.check_status()
+    assert all(t.is_contiguous() for t in got)
+    got[0].view(B, H * N, D)
+    for i, (a, b) in enumerate(zip(got, ref)):
+        assert torch.equal(a, b) if i != 1 else maxdiff(a, b) < 1e-2   # dQ of whole tiles is summed in an order that varies
