@@ -19,7 +19,8 @@ import torch
 _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, "csrc")
 LIB_PATH = os.path.join(_HERE, "libcorope_b200.so")
-NATIVE_PATH = os.path.join(_HERE, "_corope_torch.so")
+# the module is bound to torch's C++ interface: one file per torch version, so that another version builds its own
+NATIVE_PATH = os.path.join(_HERE, "_corope_torch-%s.so" % torch.__version__)
 HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200.h")
 DEBUG_HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200_debug.h")
 
@@ -108,7 +109,8 @@ def native():
             mod = sys.modules.get("_corope_torch")   # one copy per process, whatever name this package was imported under
             if mod is None:
                 if not os.path.exists(NATIVE_PATH):
-                    raise RuntimeError("corope_b200: %s is missing; build it with `python -c \"import __graft_entry__ as g; g.build()\"`." % NATIVE_PATH)
+                    raise RuntimeError("corope_b200: %s is missing (torch %s); build it with `python -c \"import __graft_entry__ as g; g.build()\"`."
+                                       % (NATIVE_PATH, torch.__version__))
                 loader = importlib.machinery.ExtensionFileLoader("_corope_torch", NATIVE_PATH)
                 mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_corope_torch", loader))
                 loader.exec_module(mod)

@@ -136,3 +136,17 @@ def test_every_admitted_size_has_a_grid_that_launches(kernel, B, Hq, Hkv, N, D):
     else:
         heads = B * (Hkv if kernel == 5 else Hq)
         assert inner == -(-N // (256 // (D // (16 if kernel == 5 else 8)))) and -(-heads // 8) <= outer <= heads
+
+
+def test_the_extension_module_of_another_torch_version_is_not_loaded(monkeypatch):
+    import sys
+    import torch
+
+    ext.build()
+    assert torch.__version__ in os.path.basename(ext.NATIVE_PATH) and os.path.exists(ext.NATIVE_PATH)
+    # as another version would look for it, in a process that has not loaded the module yet
+    monkeypatch.setattr(ext, "_native", None)
+    monkeypatch.delitem(sys.modules, "_corope_torch", raising=False)
+    monkeypatch.setattr(ext, "NATIVE_PATH", ext.NATIVE_PATH.replace(torch.__version__, "0.0.0"))
+    with pytest.raises(RuntimeError, match="missing"):
+        ext.native()
