@@ -246,6 +246,13 @@ def metric_name(kind):
 # ------------------------------------------------------------------------------------------------------------------
 # timing helpers shared by the sweep and the Triton baseline
 # ------------------------------------------------------------------------------------------------------------------
+def kernel_family(lib, op, whole_tiles):
+    """Name of the kernels that the last call of an op ran on; `whole_tiles`: that of its kernels for whole tiles."""
+    if lib.corope_last_kernel_family(op) == 1:
+        return whole_tiles
+    return "mma.sync, split operands" if lib.corope_last_kernel_split(op) == 1 else "cuda-core fp32"
+
+
 def timed_like_do_bench(fn, reps, flush):
     """The reference's method (triton.testing.do_bench, fused-rope/bench_compare.py:28-58): per repetition the L2 is flushed,
     then one call sits between two events; nothing synchronises until all repetitions are queued, so the host's launch work
@@ -315,7 +322,7 @@ def run_sweep(args):
         pkg.check_status()
         F = flops_fwd(B, H, N, D)
         f, b = f_ms[len(f_ms) // 2], b_ms[len(b_ms) // 2]
-        fam = "tcgen05" if pkg._ext.lib().corope_last_kernel_family(0) == 1 else "cuda-core fp32"
+        fam = kernel_family(pkg._ext.lib(), 0, "tcgen05")
         row = "| %s (%d, %d, %d, %d) | %.3f ms (%.1f TFLOP/s) | %.3f ms (%.1f TFLOP/s) | %s |" % (name, B, H, N, D, f, F / f / 1e9, b, 2.5 * F / b / 1e9, fam)
         del q, k, v, do, qq, kk, vv
         if tri:
@@ -767,7 +774,8 @@ def main():
         sustained["frac_of_sustained_peak"] = sustained["value"] / world / peaks["tflops_sustained"] if kind == "rope" else None
         sustained["peak_sustained"] = peaks["tflops_sustained"]
     dom_is_bwd = bwd_ms >= fwd_ms
-    fam = lib.corope_last_kernel_family((1 if dom_is_bwd else 0) + (0 if kind == "rope" else 2))
+    op = (1 if dom_is_bwd else 0) + (0 if kind == "rope" else 2)
+    fam = lib.corope_last_kernel_family(op)
     # per-launch figures of this rank's dominant kernel: algorithmic FLOPs of one launch over its average duration
     dom_ms = bwd_ms if dom_is_bwd else fwd_ms
     F_launch = (2.5 if dom_is_bwd else 1.0) * F_rank
@@ -775,7 +783,7 @@ def main():
     if kind == "rope":
         roofline = {
             "bound": "tensor", "kernel": "fused_rope_bwd" if dom_is_bwd else "fused_rope_fwd",
-            "kernel_family": "tcgen05" if fam == 1 else "cuda-core fp32",
+            "kernel_family": kernel_family(lib, op, "tcgen05"),
             "achieved": ach, "peak": peaks["tflops"], "unit": "TFLOP/s", "frac": ach / peaks["tflops"],
             "peak_source": peaks["source"] + " cuBLAS bf16 burst", "frac_of_sustained": ach / peaks["tflops_sustained"],
             "frac_of_nominal_2250": ach / 2250.0,
@@ -795,7 +803,7 @@ def main():
         xu_peak = 16.0 * sms * 1965.0e6
         roofline = {
             "bound": "xu", "kernel": "corope_bwd" if dom_is_bwd else "corope_fwd",
-            "kernel_family": "mma.sync contractions + cuda-core rotation" if fam == 1 else "cuda-core fp32",
+            "kernel_family": kernel_family(lib, op, "mma.sync contractions + cuda-core rotation"),
             "achieved": 2.0 * triples / (dom_ms * 1e-3) / 1e12, "peak": xu_peak / 1e12, "unit": "T sin-or-cos/s",
             "frac": 2.0 * triples / (dom_ms * 1e-3) / xu_peak,
             "peak_source": "16 special-function results per clock per SM x %d SMs x 1965 MHz (nominal maximum clock)" % sms,

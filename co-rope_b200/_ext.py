@@ -147,6 +147,8 @@ def lib():
             L.corope_set_kernel_policy.argtypes = [i32]
             L.corope_last_kernel_family.restype = i32
             L.corope_last_kernel_family.argtypes = [i32]
+            L.corope_last_kernel_split.restype = i32
+            L.corope_last_kernel_split.argtypes = [i32]
             if hasattr(L, "corope_debug_synth_tables"):
                 L.corope_debug_synth_tables.restype = i32
                 L.corope_debug_synth_tables.argtypes = [vp, vp, vp, i32, i32, vp]

@@ -10,6 +10,12 @@ namespace {
 std::atomic<int> g_policy{0};
 std::atomic<unsigned long long> g_launches{0};
 std::atomic<int> g_last_family[4] = {{0}, {0}, {0}, {0}};
+std::atomic<int> g_last_split[4] = {{0}, {0}, {0}, {0}};
+// what the call in hand of an op takes: 1 tensor-core kernels at whole tiles, 0 the others, of those `split` with split operands
+void note_kernels(int op, int family, bool split) {
+    g_last_family[op] = family;
+    g_last_split[op] = split ? 1 : 0;
+}
 
 constexpr size_t kAlign = 256;
 
@@ -120,7 +126,7 @@ int sm_count() {
 }
 void count_launch(int n) { g_launches.fetch_add((unsigned long long)n); }
 void note_kernel_family(int op, int family) {
-    if (op >= 0 && op < 4) g_last_family[op] = family;
+    if (op >= 0 && op < 4) note_kernels(op, family, false);
 }
 int kernel_policy() { return g_policy.load(); }
 
@@ -258,6 +264,8 @@ int corope_set_kernel_policy(int policy) { return g_policy.exchange(policy); }
 
 int corope_last_kernel_family(int op) { return (op >= 0 && op < 4) ? g_last_family[op].load() : -1; }
 
+int corope_last_kernel_split(int op) { return (op >= 0 && op < 4) ? g_last_split[op].load() : -1; }
+
 }  // extern "C"
 
 namespace {
@@ -377,13 +385,14 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
         } else if (!src.packed) {
             if (int e = launch_pack_tables(src, tab, N, D / 2, s)) return e;
         }
-        g_last_family[kFamFwd] = 1;
+        note_kernels(kFamFwd, 1, false);
         return launch_rope_fwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
-    g_last_family[kFamFwd] = 0;
     // ragged N, rows that can be moved in 16-byte vectors: split operands at fp32 accuracy (rope_split.cu has both sides' figures)
-    if (w.split && policy == 0) return launch_rope_fwd_split(p, (char*)workspace + w.rot, dtype, s);
+    const bool split = w.split && policy == 0;
+    note_kernels(kFamFwd, 0, split);
+    if (split) return launch_rope_fwd_split(p, (char*)workspace + w.rot, dtype, s);
     return launch_rope_fwd_general(p, dtype, s);
 }
 
@@ -425,14 +434,15 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
             if (!src.packed)
                 if (int e = launch_pack_tables(src, tab, N, D / 2, s)) return e;
         }
-        g_last_family[kFamBwd] = 1;
+        note_kernels(kFamBwd, 1, false);
         return launch_rope_bwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
-    g_last_family[kFamBwd] = 0;
+    const bool split = w.split && policy == 0;
+    note_kernels(kFamBwd, 0, split);
     if (dtype == COROPE_DTYPE_F32) return launch_rope_bwd_fp32(p, s);
     if (int e = launch_rope_delta(p, dtype, s)) return e;
-    if (w.split && policy == 0) return launch_rope_bwd_split(p, (char*)workspace + w.rot, dtype, s);
+    if (split) return launch_rope_bwd_split(p, (char*)workspace + w.rot, dtype, s);
     return launch_rope_bwd_general(p, dtype, s);
 }
 
@@ -588,13 +598,14 @@ int corope_gqa_fwd_strided(const void* q, const void* k, const void* v, void* o,
     if (g_policy.load() == 0 && gqa_fwd_mma_supported(N, D, dtype) && vec_ok(q, p.sq) && vec_ok(k, p.sk) && vec_ok(v, p.sv) && vec_ok(o, p.so)) {
         p.k_pairs = reinterpret_cast<uint32_t*>((char*)workspace + w.k_pairs);
         p.v_half = reinterpret_cast<__half*>((char*)workspace + w.v_half);
-        g_last_family[COROPE_OP_GQA_FWD] = 1;
+        note_kernels(COROPE_OP_GQA_FWD, 1, false);
         return launch_gqa_fwd_mma(p, dtype, (cudaStream_t)stream);
     }
-    g_last_family[COROPE_OP_GQA_FWD] = 0;
     // D = 64, a ragged N, or rows that the mma kernels cannot read: fp32 accuracy on tensor cores where the workspace has room
     const GqaWorkspace any = gqa_workspace_layout(false, B, Hq, Hkv, N, D, dtype, true);
-    if (g_policy.load() == 0 && gqa_split_supported(D, dtype) && workspace_bytes >= any.total) {
+    const bool split = g_policy.load() == 0 && gqa_split_supported(D, dtype) && workspace_bytes >= any.total;
+    note_kernels(COROPE_OP_GQA_FWD, 0, split);
+    if (split) {
         p.k_pairs = reinterpret_cast<uint32_t*>((char*)workspace + any.k_pairs);
         p.v_half = reinterpret_cast<__half*>((char*)workspace + any.v_half);
         p.k_scale = reinterpret_cast<float*>((char*)workspace + any.k_scale);
@@ -635,7 +646,7 @@ int corope_gqa_bwd_strided(const void* q, const void* k, const void* v, const vo
         p.v_half = reinterpret_cast<__half*>((char*)workspace + w.v_half);
         p.use_mma = 1;
     }
-    g_last_family[COROPE_OP_GQA_BWD] = p.use_mma;
+    note_kernels(COROPE_OP_GQA_BWD, p.use_mma, false);
     return launch_gqa_bwd_general(p, dtype, (cudaStream_t)stream);
 }
 

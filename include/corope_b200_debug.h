@@ -27,6 +27,9 @@ int corope_set_kernel_policy(int policy);
  * (N a multiple of 128, Co-RoPE: of 64), 0 = the kernels with fp32 accuracy: on CUDA cores, or with split operands. */
 int corope_last_kernel_family(int op);
 
+/* Of a last call of family 0: 1 if it ran on the split-operand kernels, 0 if on CUDA cores. */
+int corope_last_kernel_split(int op);
+
 /* Number of GPU kernel launches this library has issued in this process so far. */
 uint64_t corope_launch_count(void);
 

@@ -122,5 +122,16 @@ def test_unaligned_f16_rows_at_a_whole_tile_length():
         buf[..., :D] = t.cuda()
     o = corope_attention(*(b[..., :D] for b in padded), True, D ** -0.5, 10000.0)
     ext.check_status()
+    assert ext.lib().corope_last_kernel_split(ext.OP_GQA_FWD) == 1
     ref = _exact_o(q.cuda(), k.cuda(), v.cuda(), D ** -0.5, 10000.0)
     assert ((o.double() - ref).norm() / ref.norm()).item() < 2.0 ** -12
+
+
+@pytest.mark.parametrize("N,D", [(130, 128), (128, 64), (130, 64)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_16_bit_forwards_outside_whole_tiles_take_the_split_operand_kernel(N, D, dtype):
+    q, k, v, _ = _case(1, 4, 2, N, D, dtype, 600)
+    run_corope(q, k, v, None, D ** -0.5, 10000.0)
+    assert (ext.lib().corope_last_kernel_family(ext.OP_GQA_FWD), ext.lib().corope_last_kernel_split(ext.OP_GQA_FWD)) == (0, 1)
+    run_corope(q.float(), k.float(), v.float(), None, D ** -0.5, 10000.0)
+    assert ext.lib().corope_last_kernel_split(ext.OP_GQA_FWD) == 0

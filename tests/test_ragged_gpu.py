@@ -187,3 +187,20 @@ def test_keys_masked_by_an_infinite_channel(D, dtype):
     w = q.double() @ seen[0].double().transpose(-1, -2) * D ** -0.5
     ref = w.softmax(-1) @ seen[1].double()
     assert ((o.cpu().double() - ref).norm() / ref.norm()).item() < 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_ragged_calls_take_the_split_operand_kernels(D, dtype):
+    # every check above would pass on the slower CUDA-core kernels too
+    B, H, N = 1, 2, 130
+    q, k, v, do = (draw((B, H, N, D), 300 + i, dtype) for i in range(4))
+    cos, sin = (t.cuda() for t in oracle.precompute_freqs_cis(D, N, 10000.0))
+    lib = ext.lib()
+    for fn, args in ((pkg.fused_rope_attention, (True, 1.0, cos, sin)), (pkg.fused_rope_attention_theta, (True, 1.0, 1e4)), (pkg.flash_attention, (True, 1.0))):
+        _run(fn, q, k, v, do, *args)
+        for op in (ext.OP_ROPE_FWD, ext.OP_ROPE_BWD):
+            assert (lib.corope_last_kernel_family(op), lib.corope_last_kernel_split(op)) == (0, 1)
+    _run(pkg.flash_attention, *(t.float() for t in (q, k, v, do)), True, 1.0)
+    for op in (ext.OP_ROPE_FWD, ext.OP_ROPE_BWD):
+        assert (lib.corope_last_kernel_family(op), lib.corope_last_kernel_split(op)) == (0, 0)
