@@ -177,7 +177,7 @@ __device__ __forceinline__ void row_tile(float (&acc)[MI][C::kN], const float* A
 }
 
 struct Flags {
-    bool q, k, v, o, d_o, dq, dk, dv, tab;   // rows can be moved in vectors of four elements
+    bool q, k, v, o, d_o, tab;   // rows can be moved in vectors of four elements
 };
 
 // ------------------------------------------------------------------------------------------------
@@ -560,13 +560,17 @@ bool vec_rows(const void* ptr, const Strides& st, size_t elem) {
 Flags flags_of(const RopeParams& p, size_t elem) {
     Flags f;
     f.q = vec_rows(p.q, p.sq, elem); f.k = vec_rows(p.k, p.sk, elem); f.v = vec_rows(p.v, p.sv, elem); f.o = vec_rows(p.out_o, p.so, elem);
-    f.d_o = vec_rows(p.d_o, p.sdo, elem); f.dq = vec_rows(p.dq, p.sdq, elem); f.dk = f.dv = false;
+    f.d_o = vec_rows(p.d_o, p.sdo, elem);
     f.tab = ((uintptr_t)p.cos % 16) == 0 && ((uintptr_t)p.sin % 16) == 0 && p.table_stride % 4 == 0;
     return f;
 }
 
 FlatGrid fwd_grid(int B, int H, int N, int BM) { return {(unsigned)(B * H), ceil_div(N, BM)}; }
-bool fwd_64_rows(int B, int H, int N) { return (int64_t)((N + 63) / 64) * B * H >= 4 * sm_count(); }
+// 64 rows per CTA load the shared memory least (8 FMAs per 16-byte load of the scores' 4 x 4 tiles against 5.3); below two such CTAs per
+// SM, 32-row CTAs balance and hide latency better.  Forward with 32 / 64 rows, in 64-row CTAs per SM: 0.4 (B1 H8 N512 D64) 35 / 50 us,
+// 1.7 (B1 H8 N2048 D64) 213 / 236, 1.7 (B4 H8 N512 D128) 113 / 130, 2.6 (B4 H16 N384 D128) 134 / 113, 3.5 (B8 H8 N512 D64) 116 / 87,
+// 3.5 (B2 H8 N2048 D128) 810 / 586, 6.9 (B4 H8 N2048 D64) 786 / 560.
+bool fwd_64_rows(int B, int H, int N) { return (int64_t)((N + 63) / 64) * B * H >= 2 * sm_count(); }
 
 template <typename T, int D, int BM>
 int launch_fwd(const RopeParams& p, cudaStream_t s) {
@@ -579,8 +583,6 @@ int launch_fwd(const RopeParams& p, cudaStream_t s) {
     count_launch();
     return (int)cudaGetLastError();
 }
-// 64 rows per CTA load the shared memory least (16 FMAs per 16-byte load against 11); below four such CTAs per SM, 32-row CTAs
-// balance and hide latency better.
 template <typename T, int D>
 int launch_fwd_rows(const RopeParams& p, cudaStream_t s) {
     return fwd_64_rows(p.B, p.H, p.N) ? launch_fwd<T, D, 64>(p, s) : launch_fwd<T, D, 32>(p, s);

@@ -1,6 +1,8 @@
 """The fp32 CUDA-core kernels at the edges of their 32- and 64-row tiles, for each head dimension, grouped heads and rows that
 cannot be moved in vectors; tolerance: the 1e-4 of the other fp32 tests."""
 
+import ctypes
+
 import pytest
 import torch
 
@@ -33,9 +35,12 @@ def test_rope_fp32_at_tile_edges(N, D, causal):
 
 
 @pytest.mark.parametrize("pad", [0, 1])
-def test_grouped_heads_many_ctas_and_unaligned_rows(pad):
-    # enough 64-row tiles to fill the chip (the 64-row forward CTA), 4 query heads per K / V head, rows of 64 + pad floats
-    B, Hq, Hkv, N, D = 2, 16, 4, 330, 64
+@pytest.mark.parametrize("D", [32, 64, 128])
+def test_grouped_heads_many_ctas_and_unaligned_rows(pad, D):
+    # enough 64-row tiles to fill the chip (the 64-row forward CTA), 4 query heads per K / V head, rows of D + pad floats
+    B, Hq, Hkv, N = 2, 32, 8, 330
+    grid = (ctypes.c_uint32 * 2)()
+    assert ext.lib().corope_debug_grid(0, B, Hq, Hkv, N, D, grid) == 0 and list(grid) == [B * Hq, 6]   # 64-row blocks
 
     def make(heads, seed):
         t = draw((B, heads, N, D), seed, torch.float32)
