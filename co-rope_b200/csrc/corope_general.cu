@@ -334,7 +334,9 @@ __global__ void gqa_finalize_kernel(const float* __restrict__ dk_acc, const floa
 }
 
 // Shared memory of the backward (floats).  The (cos, sin) of every (row, key, pair) of a tile are kept from the score phase for the
-// two gradient phases where they fit and are worth it: sincosf costs some 40 instructions, the hardware approximations two.
+// two gradient phases where they fit and are worth it: sincosf costs some 40 instructions, the hardware approximations two.  Kept /
+// formed again: fp32 B1 Hq8 Hkv2 N512 D64 152 / 200 us, D128 288 / 349, B1 Hq4 Hkv4 N600 D128 335 / 490; 16 bits B2 Hq16 Hkv4 N2048 D64
+// 2.89 / 3.02 ms, B1 Hq32 Hkv8 N1500 D128 3.78 / 3.29 ms (the table leaves room for one CTA per SM there, where two fit without).
 template <typename T, int D, int G, bool ACCURATE> struct BwdSmem {
     static constexpr int kPitch = D + 2;                          // floats per (row, key) of the (cos, sin) table: lane = key writes 8 bytes without conflicts
     static constexpr size_t kTile2 = 2 * kTile * (D + kPad);      // one tile of K and of V

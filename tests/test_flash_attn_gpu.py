@@ -49,7 +49,7 @@ def _inputs(B, Hq, Hkv, N, D, dtype, seed):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("cfg,causal", [((1, 4, 2, 200, 64), True), ((2, 6, 2, 96, 32), False), ((1, 8, 1, 130, 128), True)])
 def test_flash_attention_general_kernels_16bit(dtype, cfg, causal):
-    # ragged N and D = 32: the CUDA-core kernels, groups of 2, 3 and 8 query heads per K / V head
+    # ragged N (split operands) and D = 32 (CUDA cores): groups of 2, 3 and 8 query heads per K / V head
     B, Hq, Hkv, N, D = cfg
     q, k, v, do = _inputs(B, Hq, Hkv, N, D, dtype, 60)
     outs = run_flash(q, k, v, do, causal, D ** -0.5)
@@ -64,7 +64,7 @@ def test_flash_attention_general_kernels_16bit(dtype, cfg, causal):
 @pytest.mark.parametrize("cfg,causal", [((1, 2, 2, 256, 128), True), ((2, 8, 2, 512, 128), True), ((1, 6, 2, 384, 128), False),
                                         ((1, 8, 1, 1024, 128), True), ((2, 4, 2, 256, 64), True), ((1, 6, 3, 384, 64), False)])
 def test_flash_attention_tensor_core_groups(dtype, cfg, causal):
-    # the tcgen05 kernels with the rotation off: group sizes 1, 2, 3, 4 and 8; D = 64 runs zero-padded on them
+    # the tcgen05 kernels with the rotation off: group sizes 1, 2, 3, 4 and 8, both head dimensions
     B, Hq, Hkv, N, D = cfg
     q, k, v, do = _inputs(B, Hq, Hkv, N, D, dtype, 70)
     outs = run_flash(q, k, v, do, causal, D ** -0.5)

@@ -508,7 +508,7 @@ def test_bounded_wait_expiry_is_reported_and_cleared():
     B, H, N, D = 1, 1, 256, 128
     q, k, v, _ = (t.cuda() for t in rope_inputs(B, H, N, D, torch.bfloat16, seed=21))
     cos, sin = (t.cuda() for t in oracle.precompute_freqs_cis(D, N, 10000.0))
-    ext.post_call(dev)          # what every entry point does after its launch: refresh the host mirror of the word
+    ext.post_call(dev)          # refreshes the host mirror of the word (a failing kernel writes it too)
     torch.cuda.synchronize()
     # ... and the next call through the drop-in entry point raises before launching anything, and clears the word
     with pytest.raises(RuntimeError, match="0x107e"):

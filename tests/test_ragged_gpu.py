@@ -68,11 +68,8 @@ def test_rows_of_the_next_head_are_not_seen(causal):
         t[:, 1] *= 100
     v[0, 1, 0, 0] = do[0, 1, 0, 0] = float("inf")
     outs = _run(pkg.flash_attention, q, k, v, do, causal, D ** -0.5)
-    for i, (a, b) in enumerate(zip(base, outs)):
-        if i == 1:   # dQ is summed with floating-point reductions in an order that varies
-            assert (a[:, 0] - b[:, 0]).abs().max().item() < 1e-2
-        else:
-            assert torch.equal(a[:, 0], b[:, 0])
+    for a, b in zip(base, outs):   # every sum has one owner and one order
+        assert torch.equal(a[:, 0], b[:, 0])
 
 
 def test_theta_with_a_ragged_length():
