@@ -1,23 +1,23 @@
 // Fused-RoPE / plain attention for 16-bit tensors at lengths that are not whole 128-row tiles, D = 64 or 128: tensor-core products
 // (mma.sync m16n8k16) of fp32 operands.  Every fp32 operand x enters the MMAs as hi + mid + lo, hi = x rounded to 16 bits, mid = (x - hi)
 // rounded, lo = the rest.  Three bf16 numbers hold the 24 bits of an fp32 number exactly, so nothing is lost in the operands:
-//     S  = Q~ K~^T        Q~, K~ rotated in fp32, both split into bf16      6 MMAs (without mid lo, lo mid, lo lo: below 2^-24)
+//     S  = Q~ K~^T        Q~, K~ rotated in fp32, both split into bf16      6 MMAs (without mid lo, lo mid, lo lo: about 2^-24)
 //     dP = dO V^T         inputs as they are                                1 MMA
 //     O += P V, dV += P^T dO     P split into the inputs' own type          3 MMAs
 //     dQ += dS K~, dK += dS^T Q~  dS split into bf16                        6 MMAs
 // bf16 for everything that is not bounded, so that no magnitude of the inputs leaves the range.  P <= 1 of f16 tensors enters its
 // products times 2^14: the three numbers then reach down to 2^-38 of the row's largest probability.  The adder of the MMAs does not round to
-// nearest; the large products therefore go through short chains (their own accumulators for a row's scores, one 16-row step for the
-// sums over keys or queries), which fp32 additions join.
+// nearest; the large products therefore go through one 16-wide step each (with the smaller ones in front for the sums over keys or
+// queries), which fp32 additions join.
 //
 // Error against 64-bit arithmetic next to the CUDA-core kernels with fp32 operands (N(0, 1) inputs, B1 H4 N1777 D128 causal f16): LSE
 // 3.75e-7 (3.87e-7), results that are not the exact one rounded: O 0.11 % (0.33 %), dV 0.21 % (0.36 %); with q and k times 4 (scores
 // with a standard deviation of 16) LSE 4.5e-6 (1.2e-5), O 0.29 % (0.71 %).  Two parts per operand (16 bits; half the MMAs, half the time)
 // had 2 to 10 times the error of the fp32 kernels.
 //
-// B1 H32 N1777 D128 bf16 causal forward 405 us (64 TFLOP/s; the CUDA-core kernel 909 us), backward 1262 us (5081 us); B4 H16 N1000 D64
-// bf16 full forward 244 us (572 us), backward 763 us (2890 us).  Below some 100 rows the CUDA-core forward is as fast or faster (B1 H1
-// N50 D128 12.6 against 16.8 us with the host's part), its backward never.
+// B1 H32 N1777 D128 bf16 causal forward 396 us (65 TFLOP/s; the CUDA-core kernel 909 us), backward 1315 us (5081 us); B4 H16 N1000 D64
+// bf16 full forward 243 us (572 us), backward 777 us (2890 us).  Below some 100 rows the CUDA-core forward is as fast or faster (B1 H1
+// N50 D128 12.6 against 16.5 us with the host's part), its backward never.
 // What bounds it: mma.sync, measured at 553 TFLOP/s with all operands in registers (B200, 8 warps per SM); with 8 warps per SM
 // (D = 128: 255 registers; D = 64: 12 warps) the latency between a tile's ldmatrix, MMAs and softmax is not fully hidden, and the
 // shared-memory port is close behind, a warp's 16 rows reading every streamed tile, all three parts of it, once per product.
@@ -26,6 +26,8 @@
 //
 // Math: fused-rope/rope_attn_pytorch.py:108-155 (forward), :187-222 (backward); exp2-domain softmax and log2-domain LSE as
 // fused-rope/fused_rope_attn.py:103-114, 316.
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace corope {
@@ -74,17 +76,18 @@ __device__ __forceinline__ void add4(float (*d)[4], const float (&t)[4][4]) {
 #pragma unroll
         for (int x = 0; x < 4; ++x) d[n][x] += t[n][x];
 }
-// product of two split operands for four neighbouring accumulator tiles, b[part][two ldmatrix_x4 results]: hi hi into `d`, the five
-// smaller ones into `e`, smallest first
-__device__ __forceinline__ void mma4_split(float (*d)[4], float (*e)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2][4]) {
+// the products of two split operands (PA and PB parts) for four neighbouring accumulator tiles, b[part][two ldmatrix_x4 results]: hi hi
+// into `d` by way of an fp32 addition, the others into `e`, smallest first
+template <int PA, int PB>
+__device__ __forceinline__ void mma4_split(float (*d)[4], float (*e)[4], const uint32_t (&a)[PA][4], const uint32_t (&b)[PB][2][4]) {
     using B = __nv_bfloat16;
     float t[4][4] = {};
-    mma4<B>(e, a[1], b[1][0], b[1][1]);
-    mma4<B>(e, a[0], b[2][0], b[2][1]);
-    mma4<B>(e, a[2], b[0][0], b[0][1]);
+    if constexpr (PA > 1 && PB > 1) mma4<B>(e, a[1], b[1][0], b[1][1]);
+    if constexpr (PB > 2) mma4<B>(e, a[0], b[2][0], b[2][1]);
+    if constexpr (PA > 2) mma4<B>(e, a[2], b[0][0], b[0][1]);
     mma4<B>(t, a[0], b[0][0], b[0][1]);
-    mma4<B>(e, a[0], b[1][0], b[1][1]);
-    mma4<B>(e, a[1], b[0][0], b[0][1]);
+    if constexpr (PB > 1) mma4<B>(e, a[0], b[1][0], b[1][1]);
+    if constexpr (PA > 1) mma4<B>(e, a[1], b[0][0], b[0][1]);
     add4(d, t);
 }
 // hi hi + the smaller products.  An infinity shows in hi hi with the sign it has in fp32; the other parts of such a product are
@@ -143,13 +146,14 @@ __device__ __forceinline__ void add_products(float (*d)[4], const uint32_t (&a)[
     add4(d, t);
 }
 // the same with both operands split
-__device__ __forceinline__ void add_products_split(float (*d)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2][4]) {
-    float t[4][4] = {};
+template <int PB>
+__device__ __forceinline__ void add_products_split(float (*d)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[PB][2][4]) {
     using B = __nv_bfloat16;
-    mma4<B>(t, a[1], b[1][0], b[1][1]);
-    mma4<B>(t, a[0], b[2][0], b[2][1]);
+    float t[4][4] = {};
+    if constexpr (PB > 1) mma4<B>(t, a[1], b[1][0], b[1][1]);
+    if constexpr (PB > 2) mma4<B>(t, a[0], b[2][0], b[2][1]);
     mma4<B>(t, a[2], b[0][0], b[0][1]);
-    mma4<B>(t, a[0], b[1][0], b[1][1]);
+    if constexpr (PB > 1) mma4<B>(t, a[0], b[1][0], b[1][1]);
     mma4<B>(t, a[1], b[0][0], b[0][1]);
     mma4<B>(t, a[0], b[0][0], b[0][1]);
     add4(d, t);
@@ -184,6 +188,16 @@ template <int D, int ROWS, int THREADS>
 __device__ __forceinline__ void load_split(uint32_t dst, uint32_t step, const SplitRows& x, int head, int r0, int N) {
 #pragma unroll
     for (int part = 0; part < 3; ++part) load_rows<D, ROWS, THREADS>(dst + part * step, x.rows + part * x.plane + (size_t)head * N * D, D, r0, N);
+}
+
+// Rotated K: three parts.  K of plain attention on bf16 tensors is its own hi part and is read where the caller has it (KP = 1): 3 MMAs per
+// score product and 3 for dQ instead of 6, no pass over K.  (f16 K would need two bf16 parts: 5 instead of 6.)
+template <typename T, int D, int KP, int ROWS, int THREADS>
+__device__ __forceinline__ void load_k(uint32_t dst, uint32_t step, const RopeParams& p, const SplitRows& ks, int head, int r0) {
+    if constexpr (KP == 1)
+        load_rows<D, ROWS, THREADS>(dst, reinterpret_cast<const T*>(p.k) + row_offset(p.sk, p.Hkv, head, 0), p.sk.n, r0, p.N);
+    else
+        load_split<D, ROWS, THREADS>(dst, step, ks, head, r0, p.N);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -223,17 +237,17 @@ __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__
 // ------------------------------------------------------------------------------------------------
 // forward: 64 query rows per CTA (4 warps of 16), double-buffered key tiles of 64 (D = 64) or 32 keys
 // ------------------------------------------------------------------------------------------------
-template <int D> struct Fwd {
+template <int D, int KP> struct Fwd {
     static constexpr int kThreads = 128, kRows = 64, kCtas = D == 64 ? 3 : 2;
     static constexpr int kBN = D == 64 ? 64 : 32;
     static constexpr uint32_t kTile = kBN * Pitch<D>::kBytes;
-    static constexpr uint32_t kStage = 4 * kTile;   // K~ hi, mid, lo, V
+    static constexpr uint32_t kStage = (KP + 1) * kTile;   // parts of K~, V
     static constexpr size_t kSmem = 2 * kStage;
 };
 
-template <typename T, int D>
-__global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_split_kernel(RopeParams p, SplitRows ks) {
-    using F = Fwd<D>;
+template <typename T, int D, int KP>
+__global__ void __launch_bounds__(Fwd<D, KP>::kThreads, Fwd<D, KP>::kCtas) rope_fwd_split_kernel(RopeParams p, SplitRows ks) {
+    using F = Fwd<D, KP>;
     constexpr int BN = F::kBN, KS = D / 16, NT = BN / 8, DT = D / 8;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t sm = smem_u32(smem);
@@ -245,8 +259,8 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
     const T* V = reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0);
     auto load = [&](int j0, int buf) {
         const uint32_t st = sm + buf * F::kStage;
-        load_split<D, BN, F::kThreads>(st, F::kTile, ks, kvh, j0, N);
-        load_rows<D, BN, F::kThreads>(st + 3 * F::kTile, V, p.sv.n, j0, N);
+        load_k<T, D, KP, BN, F::kThreads>(st, F::kTile, p, ks, kvh, j0);
+        load_rows<D, BN, F::kThreads>(st + KP * F::kTile, V, p.sv.n, j0, N);
         cp_commit();
     };
     load(0, 0);
@@ -256,26 +270,29 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
     {
         const T* Q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, 0);
         const float scale = p.sm_scale * kLog2e;
+        // rows beyond the head repeat its last one (their results are not stored): no branch stands between the loads
+        auto load_q = [&](auto rot) {
 #pragma unroll
-        for (int ks2 = 0; ks2 < KS / 2; ++ks2)
+            for (int k = 0; k < KS / 2; ++k)
 #pragma unroll
-            for (int x = 0; x < 4; ++x) {
-                const int pos = row0 + (x & 1) * 8, d = ks2 * 16 + (x >> 1) * 8 + c2;
-                float2 a = make_float2(0.f, 0.f), b = a;
-                if (pos < N) {
+                for (int x = 0; x < 4; ++x) {
+                    const int pos = min(row0 + (x & 1) * 8, N - 1), d = k * 16 + (x >> 1) * 8 + c2;
                     const T* q = Q + (int64_t)pos * p.sq.n + d;
-                    a = unpack2<T>(*reinterpret_cast<const uint32_t*>(q));
-                    b = unpack2<T>(*reinterpret_cast<const uint32_t*>(q + D / 2));
-                    if (p.cos != nullptr) rotate(a, b, p.cos + (int64_t)pos * p.table_stride + d, p.sin + (int64_t)pos * p.table_stride + d);
+                    float2 a = unpack2<T>(*reinterpret_cast<const uint32_t*>(q)), b = unpack2<T>(*reinterpret_cast<const uint32_t*>(q + D / 2));
+                    if constexpr (decltype(rot)::value) rotate(a, b, p.cos + (int64_t)pos * p.table_stride + d, p.sin + (int64_t)pos * p.table_stride + d);
+                    uint32_t w[3];
+                    split3_any<__nv_bfloat16>(a.x * scale, a.y * scale, w);
+#pragma unroll
+                    for (int part = 0; part < 3; ++part) qa[k][part][x] = w[part];
+                    split3_any<__nv_bfloat16>(b.x * scale, b.y * scale, w);
+#pragma unroll
+                    for (int part = 0; part < 3; ++part) qa[k + KS / 2][part][x] = w[part];
                 }
-                uint32_t w[3];
-                split3_any<__nv_bfloat16>(a.x * scale, a.y * scale, w);
-#pragma unroll
-                for (int part = 0; part < 3; ++part) qa[ks2][part][x] = w[part];
-                split3_any<__nv_bfloat16>(b.x * scale, b.y * scale, w);
-#pragma unroll
-                for (int part = 0; part < 3; ++part) qa[ks2 + KS / 2][part][x] = w[part];
-            }
+        };
+        if (p.cos != nullptr)
+            load_q(std::true_type{});
+        else
+            load_q(std::false_type{});   // plain attention
     }
     float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f}, o[DT][4];
 #pragma unroll
@@ -288,7 +305,7 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
         __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
         if (j0 + BN < n_end) load(j0 + BN, buf ^ 1);
         if (p.causal && j0 > m0 + warp * 16 + 15) continue;   // no key of the tile is seen by the warp's rows
-        const uint32_t st = sm + buf * F::kStage, kk = st + lane_b<D>(lane), vv = st + 3 * F::kTile + lane_bt<D>(lane);
+        const uint32_t st = sm + buf * F::kStage, kk = st + lane_b<D>(lane), vv = st + KP * F::kTile + lane_bt<D>(lane);
         float s[NT][4];
 #pragma unroll
         for (int np = 0; np < NT / 4; ++np) {   // 32 keys
@@ -299,9 +316,9 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
                 for (int x = 0; x < 4; ++x) main[n][x] = small[n][x] = 0.f;
 #pragma unroll
             for (int k = 0; k < KS; ++k) {
-                uint32_t b[3][2][4];
+                uint32_t b[KP][2][4];
 #pragma unroll
-                for (int part = 0; part < 3; ++part)
+                for (int part = 0; part < KP; ++part)
 #pragma unroll
                     for (int y = 0; y < 2; ++y) ldm_x4(b[part][y], kk + part * F::kTile + (2 * np + y) * 16 * Pitch<D>::kBytes + k * 32);
                 mma4_split(main, small, qa[k], b);
@@ -373,53 +390,60 @@ __global__ void __launch_bounds__(Fwd<D>::kThreads, Fwd<D>::kCtas) rope_fwd_spli
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward: two kernels of one form.  KV = false: dQ of the owned query rows, sweeping the keys.  KV = true: dK, dV of the owned keys,
-// sweeping the query rows of the group's heads (everything transposed).  The owned rows are the A operands, the streamed rows (32 per
-// step) the B operands of both score products, and the streamed rotated rows again those of the gradient product.  The scores are
-// formed twice (29 MMAs against 22), but every sum has one owner and one order: the same bits every time, and no fp32 accumulator
-// of dQ.
+// backward: two kernels of one form.  KV = false: dQ of 64 query rows, sweeping the keys.  KV = true: dK, dV of 64 keys, sweeping
+// the query rows of the group's heads (everything transposed).  The owned rows are the A operands, the streamed rows the B operands of
+// both score products, and the streamed rotated rows again those of the gradient product.  The scores are formed twice (29 MMAs against
+// 22), but every sum has one owner and one order: the same bits every time, and no fp32 accumulator of dQ.
+// A warp owns 16 rows and takes 32 streamed rows per step.  D = 64: 4 warps, three CTAs per SM.  D = 128: the parts of the owned rows fill
+// half of the shared memory, so 8 warps share them, two per 16 rows, each with its half of the streamed rows; their sums meet at the
+// end: B1 H32 N1777 1315 us, B1 H2 N1023 244 us, forward + backward of B1 Hq8 Hkv2 N2400 without rotation 1349 us.  (8 warps on 128 owned
+// rows, half the CTAs: 1262, 417 and 2776 us.)
 // ------------------------------------------------------------------------------------------------
-template <int D> struct Bwd {
-    static constexpr int kThreads = D == 64 ? 128 : 256, kCtas = D == 64 ? 3 : 1;
-    static constexpr int kRows = kThreads / 2, kBS = 32;   // rows a CTA owns, 16 per warp; rows streamed per step
-    static constexpr uint32_t kOwn = kRows * Pitch<D>::kBytes, kTile = kBS * Pitch<D>::kBytes, kStage = 4 * kTile;
-    static constexpr size_t kSmem = 4 * kOwn + 2 * kStage;
+template <int D, int KP, bool KV> struct Bwd {
+    static constexpr int kGroups = D == 64 ? 1 : 2, kThreads = 128 * kGroups, kCtas = D == 64 ? 3 : 1;
+    static constexpr int kRows = 64, kStep = 32, kBS = kStep * kGroups;   // owned rows; streamed rows per step of a warp and of the CTA
+    static constexpr int kOwnParts = KV ? KP : 3, kStrParts = KV ? 3 : KP;   // parts of the rotated rows; the plain rows follow them
+    static constexpr uint32_t kOwn = kRows * Pitch<D>::kBytes, kTile = kBS * Pitch<D>::kBytes, kStage = (kStrParts + 1) * kTile;
+    static constexpr size_t kSmem = (kOwnParts + 1) * kOwn + 2 * kStage;
+    static_assert(kGroups == 1 || kSmem >= (KV ? 2 : 1) * kRows * (D + 4) * sizeof(float), "room for the sums of the second group");
 };
 
-template <typename T, int D, bool KV>
-__global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
-    using W = Bwd<D>;
-    constexpr int BS = W::kBS, KS = D / 16, NT = BS / 8, DT = D / 8, kThreads = W::kThreads, kRows = W::kRows;
+template <typename T, int D, int KP, bool KV>
+__global__ void __launch_bounds__(Bwd<D, KP, KV>::kThreads, Bwd<D, KP, KV>::kCtas) rope_bwd_split_kernel(RopeParams p, SplitRows qs, SplitRows ks) {
+    using W = Bwd<D, KP, KV>;
+    constexpr int BS = W::kBS, SR = W::kStep, KS = D / 16, NT = SR / 8, DT = D / 8, kThreads = W::kThreads, kRows = W::kRows, OP = W::kOwnParts, SP = W::kStrParts;
     static_assert(NT == 4, "the score products of a step are four accumulator tiles");
     extern __shared__ __align__(16) uint8_t smem[];
-    const uint32_t sm = smem_u32(smem), stages = sm + 4 * W::kOwn;
+    const uint32_t sm = smem_u32(smem), stages = sm + (OP + 1) * W::kOwn;
     const int N = p.N, G = p.H / p.Hkv;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
+    const int warp = (threadIdx.x >> 5) & 3, group = threadIdx.x >> 7, lane = threadIdx.x & 31, g = lane >> 2, c2 = (lane & 3) * 2;
     const int heads = p.B * (KV ? p.Hkv : p.H), own_head = blockIdx.x % heads, block = blockIdx.x / heads;   // KV: a K / V head, otherwise a query head
     const int kvh = KV ? own_head : own_head / G;
     const int own0 = (KV ? block : gridDim.x / heads - 1 - block) * kRows;   // long causal sweeps first
     const int row0 = own0 + warp * 16 + g;                   // the lane's owned rows: row0 and row0 + 8
-    const int first = KV && p.causal ? own0 / BS * BS : 0, end = !KV && p.causal ? min(N, own0 + kRows) : N;
+    const int first = KV && p.causal ? own0 : 0, end = !KV && p.causal ? min(N, own0 + kRows) : N;
     const int steps = (end - first + BS - 1) / BS, total = KV ? steps * G : steps;
 
     auto load = [&](int step, int buf) {
         const uint32_t st = stages + buf * W::kStage;
         const int r0 = first + (KV ? step % steps : step) * BS;
-        if (KV) {
+        if constexpr (KV) {
             const int qh = kvh * G + step / steps;
             load_split<D, BS, kThreads>(st, W::kTile, qs, qh, r0, N);
-            load_rows<D, BS, kThreads>(st + 3 * W::kTile, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, qh, 0), p.sdo.n, r0, N);
+            load_rows<D, BS, kThreads>(st + SP * W::kTile, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, qh, 0), p.sdo.n, r0, N);
         } else {
-            load_split<D, BS, kThreads>(st, W::kTile, ks, kvh, r0, N);
-            load_rows<D, BS, kThreads>(st + 3 * W::kTile, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0), p.sv.n, r0, N);
+            load_k<T, D, KP, BS, kThreads>(st, W::kTile, p, ks, kvh, r0);
+            load_rows<D, BS, kThreads>(st + SP * W::kTile, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, kvh, 0), p.sv.n, r0, N);
         }
         cp_commit();
     };
-    load_split<D, kRows, kThreads>(sm, W::kOwn, KV ? ks : qs, own_head, own0, N);
-    if (KV)
-        load_rows<D, kRows, kThreads>(sm + 3 * W::kOwn, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, own_head, 0), p.sv.n, own0, N);
-    else
-        load_rows<D, kRows, kThreads>(sm + 3 * W::kOwn, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, own_head, 0), p.sdo.n, own0, N);
+    if constexpr (KV) {
+        load_k<T, D, KP, kRows, kThreads>(sm, W::kOwn, p, ks, own_head, own0);
+        load_rows<D, kRows, kThreads>(sm + OP * W::kOwn, reinterpret_cast<const T*>(p.v) + row_offset(p.sv, p.Hkv, own_head, 0), p.sv.n, own0, N);
+    } else {
+        load_split<D, kRows, kThreads>(sm, W::kOwn, qs, own_head, own0, N);
+        load_rows<D, kRows, kThreads>(sm + OP * W::kOwn, reinterpret_cast<const T*>(p.d_o) + row_offset(p.sdo, p.H, own_head, 0), p.sdo.n, own0, N);
+    }
     load(0, 0);
     float lse_r[2], dl_r[2];
     if (!KV) {
@@ -435,16 +459,16 @@ __global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_spli
     for (int n = 0; n < DT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
 #pragma unroll
     for (int n = 0; n < (KV ? DT : 1); ++n) dv[n][0] = dv[n][1] = dv[n][2] = dv[n][3] = 0.f;
-    const uint32_t a_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane);   // of the hi rows; mid, lo and plain rows follow
+    const uint32_t a_addr = sm + warp * 16 * Pitch<D>::kBytes + lane_a<D>(lane);   // of the hi rows; the other parts and the plain rows follow
 
     for (int step = 0, buf = 0; step < total; ++step, buf ^= 1) {
         cp_wait_all();
         __syncthreads();   // the tile has landed for every thread, and every warp is done with the other buffer
         if (step + 1 < total) load(step + 1, buf ^ 1);
-        const uint32_t st = stages + buf * W::kStage;
-        const int r0 = first + (KV ? step % steps : step) * BS;
-        // no pair of the step's and the warp's rows is visible
-        if (p.causal && (KV ? r0 + BS - 1 < own0 + warp * 16 : r0 > own0 + warp * 16 + 15)) continue;
+        const uint32_t st = stages + buf * W::kStage + group * SR * Pitch<D>::kBytes;
+        const int r0 = first + (KV ? step % steps : step) * BS + group * SR;
+        // no pair of the warp's owned and streamed rows is visible
+        if (r0 >= N || (p.causal && (KV ? r0 + SR - 1 < own0 + warp * 16 : r0 > own0 + warp * 16 + 15))) continue;
         float s[NT][4], dp[NT][4], small[NT][4];
 #pragma unroll
         for (int n = 0; n < NT; ++n)
@@ -453,26 +477,26 @@ __global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_spli
         const uint32_t b_addr = st + lane_b<D>(lane);
 #pragma unroll
         for (int k = 0; k < KS; ++k) {
-            uint32_t a[3][4], ax[4], b[3][2][4], bx[2][4];   // split and plain rows
+            uint32_t a[OP][4], ax[4], b[SP][2][4], bx[2][4];   // split and plain rows
 #pragma unroll
-            for (int y = 0; y < 2; ++y) ldm_x4(bx[y], b_addr + 3 * W::kTile + y * 16 * Pitch<D>::kBytes + k * 32);
-            ldm_x4(ax, a_addr + 3 * W::kOwn + k * 32);
+            for (int y = 0; y < 2; ++y) ldm_x4(bx[y], b_addr + SP * W::kTile + y * 16 * Pitch<D>::kBytes + k * 32);
+            ldm_x4(ax, a_addr + OP * W::kOwn + k * 32);
             {
                 float t[4][4] = {};
                 mma4<T>(t, ax, bx[0], bx[1]);
                 add4(dp, t);
             }
 #pragma unroll
-            for (int x = 0; x < 3; ++x) {
-                ldm_x4(a[x], a_addr + x * W::kOwn + k * 32);
+            for (int x = 0; x < OP; ++x) ldm_x4(a[x], a_addr + x * W::kOwn + k * 32);
+#pragma unroll
+            for (int x = 0; x < SP; ++x)
 #pragma unroll
                 for (int y = 0; y < 2; ++y) ldm_x4(b[x][y], b_addr + x * W::kTile + y * 16 * Pitch<D>::kBytes + k * 32);
-            }
             mma4_split(s, small, a, b);
         }
         // P and dS = P (dP - delta), in place of S and dP
         const size_t head = KV ? (size_t)(kvh * G + step / steps) * N : 0;
-        const bool edge = KV ? (p.causal && r0 < own0 + warp * 16 + 15) : (r0 + BS > N || (p.causal && r0 + BS - 1 > own0 + warp * 16));
+        const bool edge = KV ? (p.causal && r0 < own0 + warp * 16 + 15) : (r0 + SR > N || (p.causal && r0 + SR - 1 > own0 + warp * 16));
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
             float lse_c[2], dl_c[2];
@@ -498,27 +522,56 @@ __global__ void __launch_bounds__(Bwd<D>::kThreads, Bwd<D>::kCtas) rope_bwd_spli
         }
         const uint32_t t_addr = st + lane_bt<D>(lane);
 #pragma unroll
-        for (int t = 0; t < BS / 16; ++t) {
+        for (int t = 0; t < SR / 16; ++t) {
             uint32_t da[3][4], pa[3][4];
             split_a<__nv_bfloat16>(dp[2 * t], dp[2 * t + 1], 1.f, da);
             if (KV) split_a<T>(s[2 * t], s[2 * t + 1], kPScale<T>, pa);
 #pragma unroll
             for (int d = 0; d < DT / 2; d += 2) {
                 const uint32_t off = t * 16 * Pitch<D>::kBytes + d * 32;
-                uint32_t b[3][2][4];
+                uint32_t b[SP][2][4];
 #pragma unroll
-                for (int x = 0; x < 3; ++x)
+                for (int x = 0; x < SP; ++x)
 #pragma unroll
                     for (int y = 0; y < 2; ++y) ldm_x4_trans(b[x][y], t_addr + x * W::kTile + off + 32 * y);
                 add_products_split(acc + 2 * d, da, b);
                 if (KV) {
                     uint32_t bx0[4], bx1[4];
-                    ldm_x4_trans(bx0, t_addr + 3 * W::kTile + off);
-                    ldm_x4_trans(bx1, t_addr + 3 * W::kTile + off + 32);
+                    ldm_x4_trans(bx0, t_addr + SP * W::kTile + off);
+                    ldm_x4_trans(bx1, t_addr + SP * W::kTile + off + 32);
                     add_products<T>(dv + (KV ? 2 * d : 0), pa, bx0, bx1);
                 }
             }
         }
+    }
+    if constexpr (W::kGroups == 2) {   // the second group's sums to the first, in the layout of the accumulators: rows of D + 4 floats
+        __syncthreads();               // every warp is done with the tiles
+        float* sums = reinterpret_cast<float*>(smem) + (warp * 16 + g) * (D + 4) + c2;
+        constexpr int kSecond = kRows * (D + 4);
+        if (group == 1) {
+#pragma unroll
+            for (int n = 0; n < DT; ++n)
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    *reinterpret_cast<float2*>(sums + r * 8 * (D + 4) + n * 8) = make_float2(acc[n][2 * r], acc[n][2 * r + 1]);
+                    if (KV) *reinterpret_cast<float2*>(sums + kSecond + r * 8 * (D + 4) + n * 8) = make_float2(dv[KV ? n : 0][2 * r], dv[KV ? n : 0][2 * r + 1]);
+                }
+        }
+        __syncthreads();
+        if (group == 1) return;
+#pragma unroll
+        for (int n = 0; n < DT; ++n)
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                const float2 x = *reinterpret_cast<const float2*>(sums + r * 8 * (D + 4) + n * 8);
+                acc[n][2 * r] += x.x;
+                acc[n][2 * r + 1] += x.y;
+                if (KV) {
+                    const float2 y = *reinterpret_cast<const float2*>(sums + kSecond + r * 8 * (D + 4) + n * 8);
+                    dv[KV ? n : 0][2 * r] += y.x;
+                    dv[KV ? n : 0][2 * r + 1] += y.y;
+                }
+            }
     }
 
     // gradients of the rotated rows turned back (both columns of a pair belong to the same lane); Q~ carries sm_scale * log2e, so
@@ -567,58 +620,62 @@ SplitRows take_rows(__nv_bfloat16*& ws, int B, int H, int N, int D) {
     return r;
 }
 
-template <typename T, int D>
+template <typename T, int D, int KP>
 int fwd(const RopeParams& p, void* ws, cudaStream_t s) {
-    using F = Fwd<D>;
+    using F = Fwd<D, KP>;
     __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
     const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D);
-    if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
-    auto kern = rope_fwd_split_kernel<T, D>;
+    if (KP > 1)
+        if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
+    auto kern = rope_fwd_split_kernel<T, D, KP>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, F::kSmem, smem_ok)) return e;
     kern<<<rope_split_fwd_grid(p.B, p.H, p.N).blocks(), F::kThreads, F::kSmem, s>>>(p, k);
     count_launch();
     return (int)cudaGetLastError();
 }
-template <typename T, int D>
-int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
-    using W = Bwd<D>;
-    __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
-    const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D), q = take_rows(at, p.B, p.H, p.N, D);
-    if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
-    if (int e = split_rows<T, D>(p.q, p.sq, p.H, p, p.sm_scale * kLog2e, q, s)) return e;
-    auto kv = rope_bwd_split_kernel<T, D, true>;
-    auto dq = rope_bwd_split_kernel<T, D, false>;
-    static std::atomic<uint64_t> kv_ok, dq_ok;
-    if (int e = allow_smem(kv, W::kSmem, kv_ok)) return e;
-    if (int e = allow_smem(dq, W::kSmem, dq_ok)) return e;
-    kv<<<rope_split_bwd_grid(p.B, p.Hkv, p.N, D).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
-    count_launch();
-    if (cudaError_t e = cudaGetLastError()) return (int)e;
-    dq<<<rope_split_bwd_grid(p.B, p.H, p.N, D).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
+template <typename T, int D, int KP, bool KV>
+int bwd_sweep(const RopeParams& p, const SplitRows& q, const SplitRows& k, cudaStream_t s) {
+    using W = Bwd<D, KP, KV>;
+    auto kern = rope_bwd_split_kernel<T, D, KP, KV>;
+    static std::atomic<uint64_t> smem_ok;
+    if (int e = allow_smem(kern, W::kSmem, smem_ok)) return e;
+    kern<<<rope_split_bwd_grid(p.B, KV ? p.Hkv : p.H, p.N).blocks(), W::kThreads, W::kSmem, s>>>(p, q, k);
     count_launch();
     return (int)cudaGetLastError();
+}
+template <typename T, int D, int KP>
+int bwd(const RopeParams& p, void* ws, cudaStream_t s) {
+    __nv_bfloat16* at = reinterpret_cast<__nv_bfloat16*>(ws);
+    const SplitRows k = take_rows(at, p.B, p.Hkv, p.N, D), q = take_rows(at, p.B, p.H, p.N, D);
+    if (KP > 1)
+        if (int e = split_rows<T, D>(p.k, p.sk, p.Hkv, p, 1.f, k, s)) return e;
+    if (int e = split_rows<T, D>(p.q, p.sq, p.H, p, p.sm_scale * kLog2e, q, s)) return e;
+    if (int e = bwd_sweep<T, D, KP, true>(p, q, k, s)) return e;
+    return bwd_sweep<T, D, KP, false>(p, q, k, s);
+}
+template <typename T, int KP>
+int run(bool backward, const RopeParams& p, void* ws, cudaStream_t s) {
+    if (backward) return p.D == 64 ? bwd<T, 64, KP>(p, ws, s) : bwd<T, 128, KP>(p, ws, s);
+    return p.D == 64 ? fwd<T, 64, KP>(p, ws, s) : fwd<T, 128, KP>(p, ws, s);
+}
+int run(bool backward, const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
+    if (dtype == COROPE_DTYPE_F16) return run<__half, 3>(backward, p, ws, s);
+    return p.cos == nullptr ? run<__nv_bfloat16, 1>(backward, p, ws, s) : run<__nv_bfloat16, 3>(backward, p, ws, s);
 }
 
 }  // namespace
 
-FlatGrid rope_split_fwd_grid(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, Fwd<64>::kRows)}; }
-static_assert(Fwd<64>::kRows == Fwd<128>::kRows, "one grid for both head dimensions");
-FlatGrid rope_split_bwd_grid(int B, int H, int N, int D) { return {(unsigned)(B * H), ceil_div(N, D == 64 ? Bwd<64>::kRows : Bwd<128>::kRows)}; }
+constexpr int kSplitRows = 64;   // rows per CTA, forward and backward
+static_assert(Fwd<64, 3>::kRows == kSplitRows && Fwd<128, 3>::kRows == kSplitRows && Bwd<64, 3, true>::kRows == kSplitRows && Bwd<128, 3, true>::kRows == kSplitRows, "grids");
+FlatGrid rope_split_fwd_grid(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, kSplitRows)}; }
+FlatGrid rope_split_bwd_grid(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, kSplitRows)}; }
 
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D) {
     return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 3 * sizeof(__nv_bfloat16);
 }
 
-int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
-    if (dtype == COROPE_DTYPE_BF16) return p.D == 64 ? fwd<__nv_bfloat16, 64>(p, ws, s) : fwd<__nv_bfloat16, 128>(p, ws, s);
-    return p.D == 64 ? fwd<__half, 64>(p, ws, s) : fwd<__half, 128>(p, ws, s);
-}
-
-// delta computed before
-int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
-    if (dtype == COROPE_DTYPE_BF16) return p.D == 64 ? bwd<__nv_bfloat16, 64>(p, ws, s) : bwd<__nv_bfloat16, 128>(p, ws, s);
-    return p.D == 64 ? bwd<__half, 64>(p, ws, s) : bwd<__half, 128>(p, ws, s);
-}
+int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) { return run(false, p, ws, dtype, s); }
+int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) { return run(true, p, ws, dtype, s); }   // delta computed before
 
 }  // namespace corope

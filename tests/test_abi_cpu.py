@@ -127,13 +127,12 @@ def test_every_admitted_size_has_a_grid_that_launches(kernel, B, Hq, Hkv, N, D):
     inner, outer = out
     assert inner * outer <= 2 ** 31 - 1
     G = Hq // Hkv
-    rows = (None, 32, 64, 64 if D == 64 else 128, 64 if D == 64 else 128)
     if kernel == 0:
         assert inner == B * Hq and outer in (-(-N // 32), -(-N // 64))
     elif kernel == 1:
         assert inner == B * Hkv and outer == -(-N // 32) * (G + 1)
     elif kernel in (2, 3, 4):
-        assert inner == B * (Hkv if kernel == 4 else Hq) and outer == -(-N // rows[kernel])
+        assert inner == B * (Hkv if kernel == 4 else Hq) and outer == -(-N // 64)
     else:
         heads = B * (Hkv if kernel == 5 else Hq)
         assert inner == -(-N // (256 // (D // (16 if kernel == 5 else 8)))) and -(-heads // 8) <= outer <= heads

@@ -201,3 +201,34 @@ def test_ragged_calls_take_the_split_operand_kernels(D, dtype):
     _run(pkg.flash_attention, *(t.float() for t in (q, k, v, do)), True, 1.0)
     for op in (ext.OP_ROPE_FWD, ext.OP_ROPE_BWD):
         assert (lib.corope_last_kernel_family(op), lib.corope_last_kernel_split(op)) == (0, 0)
+
+
+@pytest.mark.parametrize("N", [1, 31, 33, 65, 97, 130])
+@pytest.mark.parametrize("D,causal,dtype", [(128, True, torch.bfloat16), (128, False, torch.bfloat16), (64, True, torch.bfloat16), (128, True, torch.float16)])
+def test_plain_attention_at_step_edges(N, D, causal, dtype):
+    # 32 streamed rows per warp and step, 64 owned rows; D = 128: two warps share 16 rows and each sees every other 32 streamed ones.  bf16
+    # keys are read from the caller's tensor, here a transposed one, f16 keys from their split copies
+    B, Hq, Hkv = 2, 6, 2
+    q, do = (draw((B, Hq, N, D), 310 + i, dtype) for i in range(2))
+    k, v = (draw((B, N, Hkv, D), 312 + i, dtype).transpose(1, 2) for i in range(2))
+    outs = _run(pkg.flash_attention, q, k, v, do, causal, D ** -0.5)
+    refs = (oracle.attn_gqa_fwd(q, k, v, causal, D ** -0.5),) + tuple(oracle.attn_gqa_bwd(q, k, v, do, causal, D ** -0.5))
+    _check(outs, refs, dtype)
+
+
+@pytest.mark.parametrize("N,D,causal", [(1000, 128, True), (1001, 64, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_plain_attention_is_as_accurate_as_fp32_kernels(N, D, causal, dtype):
+    q, k, v, do = (draw((1, 4, N, D), 320 + i, dtype) * (2.0 if i < 2 else 1.0) for i in range(4))
+    one, zero = torch.ones(N, D), torch.zeros(N, D)
+    exact = _exact(q, k, v, do, causal, D ** -0.5, one, zero)
+    wrong = {}
+    for policy in (0, 1):
+        prev = ext.lib().corope_set_kernel_policy(policy)
+        try:
+            outs = _run(pkg.flash_attention, q, k, v, do, causal, D ** -0.5)
+        finally:
+            ext.lib().corope_set_kernel_policy(prev)
+        wrong[policy] = [(a.to(dtype) != b.cpu().to(dtype)).double().mean().item() for a, b in zip((outs[0], outs[3]), (exact[0], exact[3]))]
+    for new, old in zip(*(wrong[x] for x in (0, 1))):   # O, dV
+        assert new <= 1.25 * old + 1e-4, wrong
