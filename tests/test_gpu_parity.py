@@ -155,7 +155,7 @@ def test_fused_rope_tensor_core_non_causal(dtype, shape):
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape,causal", [((2, 3, 256, 64), True), ((1, 2, 1024, 64), True), ((2, 2, 384, 64), False)])
 def test_fused_rope_head_dim_64_on_tensor_cores(dtype, shape, causal):
-    # D = 64 with N % 128 == 0 runs zero-padded to D = 128 on the tensor-core kernels
+    # D = 64 with N % 128 == 0 on the tensor-core kernels
     B, H, N, D = shape
     q, k, v, do = rope_inputs(B, H, N, D, dtype, seed=8)
     cos, sin = oracle.precompute_freqs_cis(D, N, 10000.0)
