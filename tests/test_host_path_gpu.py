@@ -112,4 +112,4 @@ def test_other_threads_run_while_launches_wait(entry):
         thread.join()
         torch.cuda.synchronize()
     assert took > 0.3          # the queue did fill up
-    assert longest[0] < 0.1, longest
+    assert longest[0] < 0.25, longest   # half of what a held lock shows
