@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <utility>
 
 #include "../../include/corope_b200.h"
 
@@ -419,6 +420,11 @@ __device__ __forceinline__ bool elect_one() {
     return pred != 0;
 }
 
+// Programmatic dependent launch: a kernel launched by launch_dependent may start once every block of the kernel before it has called
+// pdl_trigger (or has ended); what the earlier kernel wrote is there after pdl_wait.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // register re-allocation between warpgroups (all four warps of a warpgroup must execute the same one)
 template <int N> __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
@@ -646,6 +652,21 @@ inline int allow_smem(K kernel, size_t bytes, std::atomic<uint64_t>& done) {
     if (cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) return (int)e;
     done.fetch_or(bit);
     return 0;
+}
+// Launch whose set-up runs beside the end of the kernel before it in the stream (see pdl_wait).
+template <typename... P, typename... A>
+inline int launch_dependent(void (*kern)(P...), unsigned grid, unsigned threads, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return (int)cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 // Every kernel launch of the library bumps this counter (read through corope_launch_count()).
 void count_launch(int n = 1);

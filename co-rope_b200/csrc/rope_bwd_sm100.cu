@@ -149,6 +149,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             atomicCAS(p.status, 0, COROPE_DEV_WAIT_EXPIRED | 0xfff);
             report_to_mirror(COROPE_DEV_WAIT_EXPIRED | 0xfff, p.status_mirror);
         }
+        pdl_wait();   // no launch ends before the one in front of it
         return;
     }
     // A non-zero status word means an earlier CTA (of this or a previous launch) gave up on a wait: do not pile up
@@ -158,6 +159,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const int code = *reinterpret_cast<volatile int*>(p.status);
         if (code != 0) {
             if (threadIdx.x == 0) report_to_mirror(code, p.status_mirror);
+            pdl_wait();
             return;
         }
     }
@@ -199,6 +201,8 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();      // the pre-pass: everything above runs beside it
+    pdl_trigger();   // the conversion of dQ may be set up
 
     // setmaxnreg sits inside each role's branch: placed before the dispatch, the merge point would force the
     // smallest count on all the code that follows
@@ -585,6 +589,7 @@ rope_bwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
 template <typename T, int kD>
 __global__ void rope_bwd_dq_finalize_kernel(const float* __restrict__ acc, T* __restrict__ dq, const uint32_t* __restrict__ packed,
                                             size_t rows, int N, float scale, Strides sdq, int H, int flat) {
+    pdl_wait();
     constexpr int kHalf = kD / 2, kPerRow = kD / 8;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * kPerRow) return;
@@ -633,13 +638,12 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     const int sms = sm_count();
     const unsigned units = (unsigned)((p.N / kBK) * p.B * p.Hkv);
     const unsigned grid = units < (unsigned)sms ? units : (unsigned)sms;   // persistent: one CTA per SM
-    kern<<<grid, kThreads, kSmemBytes, s>>>(mq, mk, mv, mdo, mdq, pp); count_launch();
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
+    count_launch();
+    if (int er = launch_dependent(kern, grid, kThreads, kSmemBytes, s, mq, mk, mv, mdo, mdq, pp)) return er;
     const size_t n = rows * (kD / 8);
-    rope_bwd_dq_finalize_kernel<T, kD><<<(unsigned)((n + 255) / 256), 256, 0, s>>>(p.dq_acc, reinterpret_cast<T*>(p.dq), p.packed_tab, rows, p.N,
-                                                                                  p.sm_scale, p.sdq, p.H, rows_collapse(p.sdq, p.H, p.N) ? 1 : 0); count_launch();
-    return (int)cudaGetLastError();
+    count_launch();
+    return launch_dependent(rope_bwd_dq_finalize_kernel<T, kD>, (unsigned)((n + 255) / 256), 256, 0, s, (const float*)p.dq_acc, reinterpret_cast<T*>(p.dq), p.packed_tab, rows,
+                            p.N, p.sm_scale, p.sdq, p.H, rows_collapse(p.sdq, p.H, p.N) ? 1 : 0);
 }
 
 }  // namespace

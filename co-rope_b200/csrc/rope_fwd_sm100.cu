@@ -160,6 +160,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
             atomicCAS(p.status, 0, COROPE_DEV_WAIT_EXPIRED | 0xfff);
             report_to_mirror(COROPE_DEV_WAIT_EXPIRED | 0xfff, p.status_mirror);
         }
+        pdl_wait();   // no launch ends before the one in front of it
         return;
     }
     // A non-zero status word means an earlier CTA (of this or a previous launch) gave up on a wait: do not pile up
@@ -169,6 +170,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const int code = *reinterpret_cast<volatile int*>(p.status);
         if (code != 0) {
             if (threadIdx.x == 0) report_to_mirror(code, p.status_mirror);
+            pdl_wait();
             return;
         }
     }
@@ -217,6 +219,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         if (warp == 0) {
             // -------------------------------------------------------------- TMA producer: Q per item, and the K ring
             if (lane == 0) {
+                pdl_wait();   // work counter, rotated K
                 int gk = 0;
                 bool ok = true;
                 for (int n = 0; ok; ++n) {
@@ -365,6 +368,7 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         const int tid = (threadIdx.x - kRotWarp0 * 32) & 127;
         constexpr int kHalfRows = kBM / 2;
         bool ok = true;
+        pdl_wait();   // packed table
         TabRegs<kHalfRows, kD> tr;
         int gk = 0;
         for (int n = 0; ok; ++n) {
@@ -562,8 +566,8 @@ int launch_t(const RopeParams& p, int dtype, cudaStream_t s) {
     const unsigned items = (unsigned)(((p.N + 2 * kBM - 1) / (2 * kBM)) * p.B * p.H);
     const int sms = sm_count();
     const unsigned grid = items < (unsigned)sms ? items : (unsigned)sms;   // persistent: one CTA per SM
-    kern<<<grid, kThreads, kSmemBytes, s>>>(mq, mk, mv, pp); count_launch();
-    return (int)cudaGetLastError();
+    count_launch();
+    return launch_dependent(kern, grid, kThreads, kSmemBytes, s, mq, mk, mv, pp);
 }
 
 }  // namespace

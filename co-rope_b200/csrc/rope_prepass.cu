@@ -65,6 +65,7 @@ template <typename T, int D, int MODE>
 __global__ void __launch_bounds__(kThreads) rope_fwd_prepass_kernel(const T* __restrict__ k, __half* __restrict__ k_rot, PrepassTable tab, int N,
                                                                     int BH, int heads_per_block, RowAddr ak) {
     constexpr int kPerRow = D / 16, kRows = kThreads / kPerRow, kUnroll = 4;
+    pdl_trigger();
     const unsigned pbs = ceil_div(N, kRows), group = blockIdx.x / pbs;
     const int n = (blockIdx.x % pbs) * kRows + threadIdx.x / kPerRow;
     const int c = (threadIdx.x % kPerRow) * 8;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(kThreads) rope_bwd_prepass_kernel(const T* __r
                                                                     int N, int BH, int heads_per_block, float scale, RowAddr aq,
                                                                     RowAddr ao, RowAddr ado) {
     constexpr int kPerRow = D / 8, kRows = kThreads / kPerRow, kUnroll = 2;
+    pdl_trigger();
     const unsigned pbs = ceil_div(N, kRows), group = blockIdx.x / pbs;
     const int n = (blockIdx.x % pbs) * kRows + threadIdx.x / kPerRow;
     const int part = threadIdx.x % kPerRow;
