@@ -392,6 +392,7 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
     // ragged N, rows that can be moved in 16-byte vectors: split operands at fp32 accuracy (rope_split.cu has both sides' figures)
     const bool split = w.split && policy == 0;
     note_kernels(kFamFwd, 0, split);
+    p.sched_counter = reinterpret_cast<int*>((char*)workspace + w.packed_tab) + (size_t)N * (D / 2);   // the table itself is not used
     if (split) return launch_rope_fwd_split(p, (char*)workspace + w.rot, dtype, s);
     return launch_rope_fwd_general(p, dtype, s);
 }

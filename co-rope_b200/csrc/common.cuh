@@ -400,6 +400,22 @@ __device__ __forceinline__ void umma_ts2(uint32_t d_tmem, uint32_t a_tmem, uint3
         "r"(r[31])                                                                                                                  \
         : "memory")
 
+#define COROPE_TMEM_LD16(taddr, r)                                                                                                  \
+    asm volatile(                                                                                                                   \
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"                     \
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),   \
+          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])                                              \
+        : "r"(taddr))
+
+#define COROPE_TMEM_ST8(taddr, r)                                                                                              \
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),   \
+                 "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])                                              \
+                 : "memory")
+#define COROPE_TMEM_ST4(taddr, r)                                                                                              \
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),    \
+                 "r"(r[3])                                                                                                     \
+                 : "memory")
+
 #define COROPE_TMEM_ST16(taddr, r)                                                                                              \
     asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr), \
                  "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),       \
@@ -410,6 +426,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
+__device__ __forceinline__ void named_bar_arrive(int id, int nthreads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
 
 // Elects one lane of a fully converged warp.  The MMA issuer runs its whole loop warp-uniformly (all 32 lanes wait
 // on the barriers and compute the descriptors) and only the issue itself is predicated on the elected lane: the
@@ -432,6 +449,13 @@ template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("s
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+// the same, NaN if one of them is
+__device__ __forceinline__ float fmax3_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
 
@@ -705,7 +729,8 @@ bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types
 // 16-bit tensors at any N, D = 64 or 128, 16-byte aligned rows: split operands, `ws` of rope_split_workspace_bytes; backward with
 // delta computed before
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D);
-int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
+int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);   // p.sched_counter: a word of workspace
+int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s);   // the tcgen05 form of the forward
 int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
 int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s);
 int launch_rope_bwd_tc(const RopeParams& p, int dtype, cudaStream_t s);

@@ -15,9 +15,8 @@
 // with a standard deviation of 16) LSE 4.5e-6 (1.2e-5), O 0.29 % (0.71 %).  Two parts per operand (16 bits; half the MMAs, half the time)
 // had 2 to 10 times the error of the fp32 kernels.
 //
-// B1 H32 N1777 D128 bf16 causal forward 396 us (65 TFLOP/s; the CUDA-core kernel 909 us), backward 1315 us (5081 us); B4 H16 N1000 D64
-// bf16 full forward 243 us (572 us), backward 777 us (2890 us).  Below some 100 rows the CUDA-core forward is as fast or faster (B1 H1
-// N50 D128 12.6 against 16.5 us with the host's part), its backward never.
+// The forward below is what short sequences take; the others run on tcgen05 MMAs (rope_split_fwd_sm100.cu).  Backward: B1 H32 N1777 D128
+// bf16 causal 1315 us (the CUDA-core kernel 5081 us), B4 H16 N1000 D64 bf16 full 777 us (2890 us).
 // What bounds it: mma.sync, measured at 553 TFLOP/s with all operands in registers (B200, 8 warps per SM); with 8 warps per SM
 // (D = 128: 255 registers; D = 64: 12 warps) the latency between a tile's ldmatrix, MMAs and softmax is not fully hidden, and the
 // shared-memory port is close behind, a warp's 16 rows reading every streamed tile, all three parts of it, once per product.
@@ -28,7 +27,7 @@
 // fused-rope/fused_rope_attn.py:103-114, 316.
 #include <type_traits>
 
-#include "common.cuh"
+#include "rope_split.cuh"
 
 namespace corope {
 namespace {
@@ -93,33 +92,6 @@ __device__ __forceinline__ void mma4_split(float (*d)[4], float (*e)[4], const u
 // hi hi + the smaller products.  An infinity shows in hi hi with the sign it has in fp32; the other parts of such a product are
 // meaningless (0 or either infinity).
 __device__ __forceinline__ float join(float main, float small) { return fabsf(main) < INFINITY ? main + small : main; }
-// parts[] = hi, mid, lo of (a, b); a non-finite number is its own hi
-template <typename T>
-__device__ __forceinline__ void split3(float a, float b, uint32_t (&parts)[3]) {
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        parts[x] = pack2<T>(a, b);
-        const float2 f = unpack2<T>(parts[x]);
-        a -= f.x;
-        b -= f.y;
-    }
-}
-template <typename T>
-__device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3]) {
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        parts[x] = pack2<T>(a, b);
-        const float2 f = unpack2<T>(parts[x]);
-        a = fabsf(a - f.x) < INFINITY ? a - f.x : 0.f;
-        b = fabsf(b - f.y) < INFINITY ? b - f.y : 0.f;
-    }
-}
-// two rotation pairs (a.x, b.x), (a.y, b.y) by neighbouring table entries
-__device__ __forceinline__ void rotate(float2& a, float2& b, const float* c, const float* s) {
-    const float2 x = a, y = b;
-    a = make_float2(x.x * c[0] - y.x * s[0], x.y * c[1] - y.y * s[1]);
-    b = make_float2(y.x * c[0] + x.x * s[0], y.y * c[1] + x.y * s[1]);
-}
 // two neighbouring 8-column accumulator tiles as the A operand of one k-step, split: a[part]
 template <typename T>
 __device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[4], float scale, uint32_t (&a)[3][4]) {
@@ -133,9 +105,6 @@ __device__ __forceinline__ void split_a(const float (&c0)[4], const float (&c1)[
 #pragma unroll
         for (int e = 0; e < 4; ++e) a[x][e] = w[e][x];
 }
-// P of f16 tensors enters its products times this
-template <typename T> constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 16384.f : 1.f;
-
 // d += P b for four neighbouring tiles of columns, one 16-row step: its own sum, then one fp32 addition
 template <typename T>
 __device__ __forceinline__ void add_products(float (*d)[4], const uint32_t (&a)[3][4], const uint32_t (&b0)[4], const uint32_t (&b1)[4]) {
@@ -179,10 +148,6 @@ __device__ __forceinline__ void load_rows(uint32_t dst, const E* X, int64_t xs, 
     }
 }
 
-struct SplitRows {   // three bf16 copies [B, H, N, D], `plane` elements apart: hi, mid, lo
-    __nv_bfloat16* rows;
-    size_t plane;
-};
 // the three parts of ROWS rows of head `head` into three tiles `step` bytes apart
 template <int D, int ROWS, int THREADS>
 __device__ __forceinline__ void load_split(uint32_t dst, uint32_t step, const SplitRows& x, int head, int r0, int N) {
@@ -201,31 +166,43 @@ __device__ __forceinline__ void load_k(uint32_t dst, uint32_t step, const RopePa
 }
 
 // ------------------------------------------------------------------------------------------------
-// pre-pass: rows of X rotated in fp32, times `scale`, split.  One thread per 8 pairs.
+// pre-pass: rows of X rotated in fp32, times `scale`, split.  One thread per 8 pairs; the threads of a row are neighbouring lanes.
 // ------------------------------------------------------------------------------------------------
 template <typename T, int D>
 __global__ void __launch_bounds__(256) split_rotate_kernel(const T* __restrict__ X, RowAddr ax, const float* __restrict__ cosT, const float* __restrict__ sinT,
-                                                           int64_t ts, float scale, SplitRows out, size_t rows) {
+                                                           int64_t ts, float scale, SplitRows out, size_t rows, int* counter) {
     constexpr int kPerRow = D / 16;
     const size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const size_t row = idx / kPerRow;
-    if (row >= rows) return;
+    pdl_trigger();
+    if (idx == 0 && counter != nullptr) *counter = 0;
+    const bool live = idx / kPerRow < rows;
+    const size_t row = live ? idx / kPerRow : rows - 1;   // threads beyond the last row take part in the shuffles with it
     const int d = (int)(idx % kPerRow) * 8, n = (int)(row % (size_t)ax.N);
     const T* src = X + flat_row_offset(ax, row) + d;
     const uint4 xa = *reinterpret_cast<const uint4*>(src), xb = *reinterpret_cast<const uint4*>(src + D / 2);
     const uint32_t a[4] = {xa.x, xa.y, xa.z, xa.w}, b[4] = {xb.x, xb.y, xb.z, xb.w};
+    float2 ra[4], rb[4];
+    float largest = 0.f;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        ra[e] = unpack2<T>(a[e]), rb[e] = unpack2<T>(b[e]);
+        if (cosT != nullptr) {   // null tables: plain attention
+            const float *c = cosT + (int64_t)n * ts + d + 2 * e, *s = sinT + (int64_t)n * ts + d + 2 * e;
+            rotate(ra[e], rb[e], c, s);
+        }
+        ra[e].x *= scale, ra[e].y *= scale, rb[e].x *= scale, rb[e].y *= scale;
+        largest = fmax3_nan(largest, fmax3_nan(0.f, fabsf(ra[e].x), fabsf(ra[e].y)), fmax3_nan(0.f, fabsf(rb[e].x), fabsf(rb[e].y)));
+    }
+#pragma unroll
+    for (int off = 1; off < kPerRow; off <<= 1) largest = fmax3_nan(0.f, largest, __shfl_xor_sync(0xffffffffu, largest, off));
+    const RowUnit unit = row_unit(largest);
     uint32_t pa[4][3], pb[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        const float2 fa = unpack2<T>(a[e]), fb = unpack2<T>(b[e]);
-        float2 ra = fa, rb = fb;
-        if (cosT != nullptr) {   // null tables: plain attention
-            const float *c = cosT + (int64_t)n * ts + d + 2 * e, *s = sinT + (int64_t)n * ts + d + 2 * e;
-            rotate(ra, rb, c, s);
-        }
-        split3_any<__nv_bfloat16>(ra.x * scale, ra.y * scale, pa[e]);
-        split3_any<__nv_bfloat16>(rb.x * scale, rb.y * scale, pb[e]);
+        split_row_pair(ra[e].x, ra[e].y, unit, pa[e]);
+        split_row_pair(rb[e].x, rb[e].y, unit, pb[e]);
     }
+    if (!live) return;
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
         __nv_bfloat16* o = out.rows + part * out.plane + row * D + d;
@@ -606,10 +583,10 @@ __global__ void __launch_bounds__(Bwd<D, KP, KV>::kThreads, Bwd<D, KP, KV>::kCta
 
 // ------------------------------------------------------------------------------------------------ launchers
 template <typename T, int D>
-int split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, SplitRows out, cudaStream_t s) {
+int split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, SplitRows out, cudaStream_t s, int* counter = nullptr) {
     const size_t rows = (size_t)p.B * H * p.N;
     split_rotate_kernel<T, D><<<(unsigned)((rows * (D / 16) + 255) / 256), 256, 0, s>>>((const T*)x, row_addr(st, H, p.N), p.cos, p.sin, p.table_stride, scale,
-                                                                                       out, rows);
+                                                                                       out, rows, counter);
     count_launch();
     return (int)cudaGetLastError();
 }
@@ -675,7 +652,23 @@ size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D
     return ((size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0)) * N * D * 3 * sizeof(__nv_bfloat16);
 }
 
-int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) { return run(false, p, ws, dtype, s); }
+int launch_split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, const SplitRows& out, int* counter, int dtype, cudaStream_t s) {
+    if (dtype == COROPE_DTYPE_BF16)
+        return p.D == 64 ? split_rows<__nv_bfloat16, 64>(x, st, H, p, scale, out, s, counter) : split_rows<__nv_bfloat16, 128>(x, st, H, p, scale, out, s, counter);
+    return p.D == 64 ? split_rows<__half, 64>(x, st, H, p, scale, out, s, counter) : split_rows<__half, 128>(x, st, H, p, scale, out, s, counter);
+}
+
+// The forward on mma.sync where its short start counts more than its rate: one block of rows, and for bf16 keys without rotation, which it
+// reads as they are, a few.  GPU time of it and of the tcgen05 kernel (pre-pass included): B1 H1 N50 D64 8.6 / 9.6 us, N50 D128 11.9 / 12.5,
+// N129 D64 13.8 / 11.5, N129 D128 19.0 / 15.3; without rotation B1 H1 N129 D64 9.3 / 11.1, N200 D128 17.4 / 16.0, B4 H16 N300 D64 19.1 / 21.6,
+// N500 D64 32.2 / 26.8, B2 H32 N200 D128 21.7 / 18.5.
+bool short_forward(const RopeParams& p, int dtype) {
+    if (p.cos == nullptr && dtype == COROPE_DTYPE_BF16) return p.N < (p.D == 64 ? 320 : 160);
+    return p.N <= 64;
+}
+int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
+    return short_forward(p, dtype) ? run(false, p, ws, dtype, s) : launch_rope_fwd_split_tc(p, ws, dtype, s);
+}
 int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) { return run(true, p, ws, dtype, s); }   // delta computed before
 
 }  // namespace corope

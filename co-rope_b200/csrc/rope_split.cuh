@@ -1,0 +1,108 @@
+// Operands of the split-operand kernels: fp32 numbers as sums of three 16-bit ones.
+#pragma once
+
+#include "common.cuh"
+
+namespace corope {
+
+struct SplitRows {   // three bf16 copies [B, H, N, D], `plane` elements apart: hi, mid, lo
+    __nv_bfloat16* rows;
+    size_t plane;
+};
+
+#ifdef __CUDACC__
+// parts[] = hi, mid, lo of (a, b), each rounded to T; a non-finite number is its own hi
+template <typename T>
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&parts)[3]) {
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        parts[x] = pack2<T>(a, b);
+        const float2 f = unpack2<T>(parts[x]);
+        a -= f.x;
+        b -= f.y;
+    }
+}
+// the same for two positive numbers, bf16 parts cut off instead of rounded (the three then hold the 24 bits exactly): byte permutes and
+// masks instead of conversions
+template <typename T>
+__device__ __forceinline__ void split3_pos(float a, float b, uint32_t (&parts)[3]) {
+    if constexpr (Elem<T>::kDtype == COROPE_DTYPE_BF16) {
+#pragma unroll
+        for (int x = 0; x < 3; ++x) {
+            const uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
+            parts[x] = __byte_perm(ua, ub, 0x7632);
+            if (x < 2) f2_unpack(f2_sub(f2_pack(a, b), f2_pack_bits(ua & 0xffff0000u, ub & 0xffff0000u)), a, b);
+        }
+    } else {
+        split3<T>(a, b, parts);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3]) {
+#pragma unroll
+    for (int x = 0; x < 3; ++x) {
+        parts[x] = pack2<T>(a, b);
+        const float2 f = unpack2<T>(parts[x]);
+        a = fabsf(a - f.x) < INFINITY ? a - f.x : 0.f;
+        b = fabsf(b - f.y) < INFINITY ? b - f.y : 0.f;
+    }
+}
+
+// Rows whose products are formed exactly: hi is the number rounded to a multiple of u = 2^-7 of the power of two below the row's largest
+// magnitude, at most 2^8 of them, mid and lo are the rest as bf16 numbers (2^-25 of the row's largest magnitude and below is lost).  A
+// product of two hi parts is an integer of at most 2^16 times one power of two per row and column, a sum of 128 of them stays below 2^24:
+// the adder of the MMAs, which truncates, has nothing to truncate however many of them it chains.  Rows with a non-finite (or nearly
+// so) number are split element by element.
+struct RowUnit {
+    float u, inv;   // inv = 0: element by element
+};
+__device__ __forceinline__ RowUnit row_unit(float largest) {
+    RowUnit r{0.f, 0.f};
+    if (largest < 8.5e37f) {   // 2^126
+        const int e = max((int)((__float_as_uint(largest) >> 23) & 255), 16);   // biased exponent of the largest number
+        r.u = __uint_as_float((uint32_t)(e - 7) << 23);
+        r.inv = __uint_as_float((uint32_t)(254 - (e - 7)) << 23);
+    }
+    return r;
+}
+__device__ __forceinline__ void split_row_pair(float a, float b, const RowUnit& r, uint32_t (&parts)[3]) {
+    if (r.inv == 0.f) {
+        split3_any<__nv_bfloat16>(a, b, parts);
+        return;
+    }
+    const float ha = rintf(a * r.inv) * r.u, hb = rintf(b * r.inv) * r.u;
+    parts[0] = pack_bf162(ha, hb);
+    a -= ha;
+    b -= hb;
+    parts[1] = pack_bf162(a, b);
+    const float2 f = unpack_bf162(parts[1]);
+    parts[2] = pack_bf162(a - f.x, b - f.y);
+}
+// two rotation pairs (a.x, b.x), (a.y, b.y) by neighbouring table entries
+__device__ __forceinline__ void rotate(float2& a, float2& b, const float* c, const float* s) {
+    const float2 x = a, y = b;
+    a = make_float2(x.x * c[0] - y.x * s[0], x.y * c[1] - y.y * s[1]);
+    b = make_float2(y.x * c[0] + x.x * s[0], y.y * c[1] + x.y * s[1]);
+}
+// rows of both tables are aligned to 16 bytes
+__device__ __forceinline__ bool tables_aligned(const RopeParams& p) {
+    return (((uintptr_t)p.cos | (uintptr_t)p.sin) & 15) == 0 && (p.table_stride & 3) == 0;
+}
+__device__ __forceinline__ void load_table8(const float* __restrict__ src, bool vec, float (&x)[8]) {
+    if (vec) {
+        const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
+        x[0] = a.x, x[1] = a.y, x[2] = a.z, x[3] = a.w, x[4] = b.x, x[5] = b.y, x[6] = b.z, x[7] = b.w;
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = src[i];
+    }
+}
+// P of f16 tensors enters its products times this
+template <typename T> constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 16384.f : 1.f;
+#endif
+
+// Pre-pass: rows of x (H heads, strides st), rotated in fp32 by the tables of p (none: as they are), times `scale`, split; `counter`, if
+// not null, is zeroed.
+int launch_split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, const SplitRows& out, int* counter, int dtype, cudaStream_t s);
+
+}  // namespace corope
