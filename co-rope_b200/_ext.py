@@ -24,7 +24,7 @@ NATIVE_PATH = os.path.join(_HERE, "_corope_torch-%s.so" % torch.__version__)
 HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200.h")
 DEBUG_HEADER_PATH = os.path.join(os.path.dirname(_HERE), "include", "corope_b200_debug.h")
 
-SOURCES = ["abi.cu", "rope_general.cu", "rope_fp32.cu", "rope_split.cu", "rope_split_fwd_sm100.cu", "rope_prepass.cu", "rope_fwd_sm100.cu", "rope_bwd_sm100.cu", "corope_general.cu", "corope_fwd_mma.cu", "corope_fwd_split.cu", "corope_bwd_mma.cu", "noalloc.cu",
+SOURCES = ["abi.cu", "rope_general.cu", "rope_fp32.cu", "rope_split.cu", "rope_split_fwd_sm100.cu", "rope_split_bwd_sm100.cu", "rope_split_prepass.cu", "rope_prepass.cu", "rope_fwd_sm100.cu", "rope_bwd_sm100.cu", "corope_general.cu", "corope_fwd_mma.cu", "corope_fwd_split.cu", "corope_bwd_mma.cu", "noalloc.cu",
            "debug.cu"]
 
 DTYPE_CODES = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}

@@ -44,9 +44,9 @@ RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int
         w.synth_sin = off;
         off += align_up((size_t)N * (D / 2) * sizeof(float), kAlign);
     }
-    w.rot = off;   // tcgen05 kernels: fp16 copy of the rotated K (forward) / rotated and scaled Q (backward); the other ones: bf16 hi and lo
+    w.rot = off;   // tcgen05 kernels: fp16 copy of the rotated K (forward) / rotated and scaled Q (backward); the split-operand kernels: parts of K and Q
     if (w.tc) off += align_up((bwd ? q_elems : kv_elems) * 2, kAlign);
-    if (w.split) off += align_up(rope_split_workspace_bytes(bwd, B, Hq, Hkv, N, D), kAlign);
+    if (w.split) off += align_up(rope_split_workspace_bytes(bwd, B, Hq, Hkv, N, D, dtype), kAlign);
     if (bwd) {
         w.delta = off;
         off += align_up((size_t)B * Hq * N * sizeof(float), kAlign);
@@ -441,9 +441,10 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
     const bool split = w.split && policy == 0;
     note_kernels(kFamBwd, 0, split);
+    p.sched_counter = reinterpret_cast<int*>((char*)workspace + w.packed_tab) + (size_t)N * (D / 2);   // the table itself is not used
+    if (split) return launch_rope_bwd_split(p, (char*)workspace + w.rot, dtype, s);
     if (dtype == COROPE_DTYPE_F32) return launch_rope_bwd_fp32(p, s);
     if (int e = launch_rope_delta(p, dtype, s)) return e;
-    if (split) return launch_rope_bwd_split(p, (char*)workspace + w.rot, dtype, s);
     return launch_rope_bwd_general(p, dtype, s);
 }
 

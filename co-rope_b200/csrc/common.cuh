@@ -91,7 +91,7 @@ __host__ __device__ inline unsigned ceil_div(unsigned a, unsigned b) { return (a
 FlatGrid rope_fp32_fwd_grid(int B, int H, int N);                 // heads x row blocks
 FlatGrid rope_fp32_bwd_grid(int B, int H, int Hkv, int N);        // K / V heads x (key block, its query heads' row blocks)
 FlatGrid rope_split_fwd_grid(int B, int H, int N);                // heads x row blocks
-FlatGrid rope_split_bwd_grid(int B, int H, int N);                // heads (of K / V for dK and dV) x row blocks
+FlatGrid rope_split_bwd_grid(int B, int H, int N);                // heads (of K / V for dK and dV) x 64-row blocks; persistent, one block per SM
 FlatGrid rope_prepass_grid(bool bwd, int B, int H, int N, int D); // position blocks x groups of heads
 
 // Launch parameters common to the fused-RoPE kernels.
@@ -333,6 +333,15 @@ __device__ __forceinline__ void umma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64
         : "memory");
 }
 
+// 128 rows x 32 bytes (one k-step of a 16-bit operand) from a shared-memory tile, described as an A operand, to 8 TMEM columns
+__device__ __forceinline__ void tmem_copy_128x256b(uint32_t d_tmem, uint32_t s_lo, uint32_t s_hi) {
+    asm volatile(
+        "{\n\t.reg .b64 ds;\n\tmov.b64 ds, {%1, %2};\n\t"
+        "tcgen05.cp.cta_group::1.128x256b [%0], ds;\n\t}" ::"r"(d_tmem),
+        "r"(s_lo), "r"(s_hi)
+        : "memory");
+}
+
 // Instruction descriptor for kind::f16: fp32 accumulator, A/B formats 0 = f16, 1 = bf16,
 // a_mn / b_mn = 1 when the operand's M/N extent (not K) is the contiguous one in memory.
 __host__ __device__ constexpr uint32_t make_idesc(int a_fmt, int b_fmt, int a_mn, int b_mn, int M, int N) {
@@ -406,6 +415,11 @@ __device__ __forceinline__ void umma_ts2(uint32_t d_tmem, uint32_t a_tmem, uint3
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),   \
           "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])                                              \
         : "r"(taddr))
+
+#define COROPE_TMEM_LD8(taddr, r)                                                                                              \
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"                                      \
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])               \
+                 : "r"(taddr))
 
 #define COROPE_TMEM_ST8(taddr, r)                                                                                              \
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]),   \
@@ -726,10 +740,10 @@ int launch_rope_fwd_prepass(const RopeParams& p, const TableSource& src, uint32_
 // p.dq_acc
 int launch_rope_bwd_prepass(const RopeParams& p, const TableSource& src, uint32_t* packed, int dtype, cudaStream_t s);
 bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types, D = 64 or 128
-// 16-bit tensors at any N, D = 64 or 128, 16-byte aligned rows: split operands, `ws` of rope_split_workspace_bytes; backward with
-// delta computed before
-size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D);
-int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);   // p.sched_counter: a word of workspace
+// 16-byte aligned rows at any N, 16-bit tensors of D = 64 or 128: split operands, `ws` of rope_split_workspace_bytes, two words of workspace
+// at p.sched_counter; the backward computes delta
+size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype);
+int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
 int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s);   // the tcgen05 form of the forward
 int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
 int launch_rope_fwd_tc(const RopeParams& p, int dtype, cudaStream_t s);

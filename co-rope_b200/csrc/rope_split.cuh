@@ -11,6 +11,40 @@ struct SplitRows {   // three bf16 copies [B, H, N, D], `plane` elements apart: 
 };
 
 #ifdef __CUDACC__
+// How V and dO enter the MMAs: 16-bit tensors as they are, fp32 tensors as three bf16 parts; P in parts of the same type.
+template <typename T> struct Plain {
+    using Mma = T;
+    static constexpr int kParts = 1, kDtype = Elem<T>::kDtype;
+};
+template <> struct Plain<float> {
+    using Mma = __nv_bfloat16;
+    static constexpr int kParts = 3, kDtype = COROPE_DTYPE_BF16;
+};
+// the products of two split operands, smallest first: parts of the one and of the other
+constexpr int kProducts = 6;
+__host__ __device__ constexpr int product_a(int i) { return i == 0 ? 1 : i == 2 ? 2 : i == 4 ? 1 : 0; }
+__host__ __device__ constexpr int product_b(int i) { return i == 0 ? 1 : i == 1 ? 2 : i == 3 ? 1 : 0; }
+// eight neighbouring numbers of a row, aligned to 16 bytes
+template <typename T>
+__device__ __forceinline__ void load8(const T* __restrict__ x, float2 (&to)[4]) {
+    if constexpr (sizeof(T) == 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x), b = *reinterpret_cast<const float4*>(x + 4);
+        to[0] = make_float2(a.x, a.y), to[1] = make_float2(a.z, a.w), to[2] = make_float2(b.x, b.y), to[3] = make_float2(b.z, b.w);
+    } else {
+        const uint4 a = *reinterpret_cast<const uint4*>(x);
+        to[0] = unpack2<T>(a.x), to[1] = unpack2<T>(a.y), to[2] = unpack2<T>(a.z), to[3] = unpack2<T>(a.w);
+    }
+}
+template <typename T>
+__device__ __forceinline__ void store8(T* to, const float2 (&x)[4]) {
+    if constexpr (sizeof(T) == 4) {
+        *reinterpret_cast<float4*>(to) = make_float4(x[0].x, x[0].y, x[1].x, x[1].y);
+        *reinterpret_cast<float4*>(to + 4) = make_float4(x[2].x, x[2].y, x[3].x, x[3].y);
+    } else {
+        *reinterpret_cast<uint4*>(to) = make_uint4(pack2<T>(x[0].x, x[0].y), pack2<T>(x[1].x, x[1].y), pack2<T>(x[2].x, x[2].y), pack2<T>(x[3].x, x[3].y));
+    }
+}
+
 // parts[] = hi, mid, lo of (a, b), each rounded to T; a non-finite number is its own hi
 template <typename T>
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&parts)[3]) {
@@ -22,10 +56,10 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t (&parts)[3]) {
         b -= f.y;
     }
 }
-// the same for two positive numbers, bf16 parts cut off instead of rounded (the three then hold the 24 bits exactly): byte permutes and
+// the same for two finite numbers, bf16 parts cut off instead of rounded (the three then hold the 24 bits exactly): byte permutes and
 // masks instead of conversions
 template <typename T>
-__device__ __forceinline__ void split3_pos(float a, float b, uint32_t (&parts)[3]) {
+__device__ __forceinline__ void split3_cut(float a, float b, uint32_t (&parts)[3]) {
     if constexpr (Elem<T>::kDtype == COROPE_DTYPE_BF16) {
 #pragma unroll
         for (int x = 0; x < 3; ++x) {
@@ -97,12 +131,41 @@ __device__ __forceinline__ void load_table8(const float* __restrict__ src, bool 
         for (int i = 0; i < 8; ++i) x[i] = src[i];
     }
 }
+// One score by its definition, for operands with infinities or NaNs, whose parts do not multiply as the numbers do.
+template <typename T>
+__device__ __forceinline__ float plain_score(const RopeParams& p, int bh, int row, int key) {
+    const T* q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, row);
+    const T* k = reinterpret_cast<const T*>(p.k) + row_offset(p.sk, p.Hkv, bh / (p.H / p.Hkv), key);
+    const int half = p.D / 2;
+    const float scale = p.sm_scale * kLog2e;
+    float s = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < half; ++d) {
+        float q1 = Elem<T>::to_f32(q[d]), q2 = Elem<T>::to_f32(q[d + half]), k1 = Elem<T>::to_f32(k[d]), k2 = Elem<T>::to_f32(k[d + half]);
+        if (p.cos != nullptr) {
+            const float cq = p.cos[(int64_t)row * p.table_stride + d], sq = p.sin[(int64_t)row * p.table_stride + d];
+            const float ck = p.cos[(int64_t)key * p.table_stride + d], sk = p.sin[(int64_t)key * p.table_stride + d];
+            const float a = q1 * cq - q2 * sq, b = k1 * ck - k2 * sk;
+            q2 = q2 * cq + q1 * sq, q1 = a;
+            k2 = k2 * ck + k1 * sk, k1 = b;
+        }
+        s = fmaf(q1 * scale, k1, s);
+        s = fmaf(q2 * scale, k2, s);
+    }
+    return s;
+}
+
 // P of f16 tensors enters its products times this
 template <typename T> constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 16384.f : 1.f;
 #endif
 
-// Pre-pass: rows of x (H heads, strides st), rotated in fp32 by the tables of p (none: as they are), times `scale`, split; `counter`, if
-// not null, is zeroed.
-int launch_split_rows(const void* x, const Strides& st, int H, const RopeParams& p, float scale, const SplitRows& out, int* counter, int dtype, cudaStream_t s);
+// The split copies of a call in its workspace.  V and dO (rows null: not copied) of fp32 tensors only.
+struct SplitCopies {
+    SplitRows k, q, v, d_o;
+};
+SplitCopies split_copies(const RopeParams& p, void* ws, bool bwd, int dtype);
+// Pre-pass: the copies whose `rows` are set, K and Q rotated by the tables of p (none: as they are), Q times sm_scale * log2e; with_delta:
+// p.delta from p.o and p.d_o; the two words at p.sched_counter are zeroed.
+int launch_split_rows(const RopeParams& p, const SplitCopies& to, bool with_delta, int dtype, cudaStream_t s);
 
 }  // namespace corope

@@ -57,30 +57,6 @@ __device__ __forceinline__ WorkItem work_item(int w, int n_qt, int BH, int head_
     return {n_qt - 1 - within / heads_here, chunk * head_chunk + within % heads_here};
 }
 
-// One score by its definition, for operands with infinities or NaNs, whose parts do not multiply as the numbers do.
-template <typename T>
-__device__ __forceinline__ float plain_score(const RopeParams& p, int bh, int row, int key) {
-    const T* q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, row);
-    const T* k = reinterpret_cast<const T*>(p.k) + row_offset(p.sk, p.Hkv, bh / (p.H / p.Hkv), key);
-    const int half = p.D / 2;
-    const float scale = p.sm_scale * kLog2e;
-    float s = 0.f;
-#pragma unroll 1
-    for (int d = 0; d < half; ++d) {
-        float q1 = Elem<T>::to_f32(q[d]), q2 = Elem<T>::to_f32(q[d + half]), k1 = Elem<T>::to_f32(k[d]), k2 = Elem<T>::to_f32(k[d + half]);
-        if (p.cos != nullptr) {
-            const float cq = p.cos[(int64_t)row * p.table_stride + d], sq = p.sin[(int64_t)row * p.table_stride + d];
-            const float ck = p.cos[(int64_t)key * p.table_stride + d], sk = p.sin[(int64_t)key * p.table_stride + d];
-            const float a = q1 * cq - q2 * sq, b = k1 * ck - k2 * sk;
-            q2 = q2 * cq + q1 * sq, q1 = a;
-            k2 = k2 * ck + k1 * sk, k1 = b;
-        }
-        s = fmaf(q1 * scale, k1, s);
-        s = fmaf(q2 * scale, k2, s);
-    }
-    return s;
-}
-
 template <typename T, int D, int KP>
 __global__ void __launch_bounds__(kThreads, 1)
 rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const __grid_constant__ RopeParams p) {
@@ -416,7 +392,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                     x0 = fast_exp2(x0), x1 = fast_exp2(x1);
                     sum = f2_add(sum, f2_pack(x0, x1));
                     uint32_t y[3];
-                    split3_pos<T>(x0 * kPScale<T>, x1 * kPScale<T>, y);
+                    split3_cut<T>(x0 * kPScale<T>, x1 * kPScale<T>, y);
                     parts[0][i] = y[0], parts[1][i] = y[1], parts[2][i] = y[2];
                 }
 #pragma unroll
@@ -497,9 +473,8 @@ int launch_d(const RopeParams& p, const SplitRows& ks, int dtype, cudaStream_t s
 }  // namespace
 
 int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
-    const size_t plane = (size_t)p.B * p.Hkv * p.N * p.D;
-    const SplitRows ks{reinterpret_cast<__nv_bfloat16*>(ws), plane};
-    if (int e = launch_split_rows(p.k, p.sk, p.Hkv, p, 1.f, ks, p.sched_counter, dtype, s)) return e;
+    const SplitRows ks = split_copies(p, ws, false, dtype).k;
+    if (int e = launch_split_rows(p, SplitCopies{ks, {}, {}, {}}, false, dtype, s)) return e;
     if (dtype == COROPE_DTYPE_F16) return launch_d<__half, 3>(p, ks, dtype, s);
     // bf16 keys without rotation have 8 bits: hi and mid hold all of them
     return p.cos == nullptr ? launch_d<__nv_bfloat16, 2>(p, ks, dtype, s) : launch_d<__nv_bfloat16, 3>(p, ks, dtype, s);

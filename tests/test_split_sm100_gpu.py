@@ -1,0 +1,72 @@
+"""The tcgen05 split-operand kernels of ragged lengths where their persistent loops and rings wrap: more items than SMs, sweeps that end
+in the middle of a 64-row block, grouped heads whose sweep runs over several query heads, owned blocks that are nearly empty."""
+
+import pytest
+import torch
+
+from helpers import draw, ext, pkg
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(q, k, v, do, causal, s):
+    q, k, v, do = (t.cuda().double() for t in (q, k, v, do))
+    G = q.shape[1] // k.shape[1]
+    ke, ve = (t.repeat_interleave(G, 1) for t in (k, v))
+    w = q @ ke.transpose(-1, -2) * s
+    if causal:
+        w = w.masked_fill(torch.ones(w.shape[-2:], dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    p = w.softmax(-1)
+    o = p @ ve
+    ds = p * (do @ ve.transpose(-1, -2) - (o * do).sum(-1, keepdim=True)) * s
+    fold = lambda t: t.unflatten(1, (k.shape[1], G)).sum(2)
+    return o, ds @ ke, fold(ds.transpose(-1, -2) @ q), fold(p.transpose(-1, -2) @ do)
+
+
+def _run(q, k, v, do, causal, s):
+    q, k, v = (t.cuda().requires_grad_(True) for t in (q, k, v))
+    o = pkg.flash_attention(q, k, v, causal, s)
+    grads = torch.autograd.grad(o, (q, k, v), do.cuda())
+    ext.check_status()
+    return (o.detach(),) + grads
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,N", [(2, 40, 40, 257), (1, 160, 160, 65), (1, 12, 3, 385), (3, 8, 1, 191), (1, 2, 2, 1153), (1, 4, 2, 639)])
+@pytest.mark.parametrize("D,causal,dtype", [(128, True, torch.bfloat16), (64, False, torch.bfloat16), (64, True, torch.float16), (128, False, torch.float16)])
+def test_wraps_of_items_rings_and_sweeps(B, Hq, Hkv, N, D, causal, dtype):
+    # one rounding of the result is at most 2^-9 (bf16) or 2^-12 of a value, in the 2-norm about 0.8 of that; dQ and dK also see delta of the
+    # rounded O, whose error stands next to a dP - delta of about the same size
+    q, do = (draw((B, Hq, N, D), 400 + i, dtype) for i in range(2))
+    k, v = (draw((B, Hkv, N, D), 402 + i, dtype) for i in range(2))
+    ulp = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    for name, got, ref in zip(("O", "dQ", "dK", "dV"), _run(q, k, v, do, causal, D ** -0.5), _exact(q, k, v, do, causal, D ** -0.5)):
+        err = ((got.double() - ref).norm() / ref.norm()).item()
+        assert err < ulp * (1.0 if name in ("O", "dV") else 1.5), (name, err / ulp)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_results_are_reproducible(D):
+    q, do = (draw((1, 12, 700, D), 410 + i, torch.bfloat16) for i in range(2))
+    k, v = (draw((1, 4, 700, D), 412 + i, torch.bfloat16) for i in range(2))
+    first = _run(q, k, v, do, True, D ** -0.5)
+    for _ in range(3):
+        assert all(torch.equal(a, b) for a, b in zip(first, _run(q, k, v, do, True, D ** -0.5)))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("N", [40, 150])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_gradients_of_keys_masked_by_an_infinite_channel(D, N, dtype):
+    # as test_keys_masked_by_an_infinite_channel: hidden keys have no share in O, dK and dV (dQ takes 0 times their -inf)
+    q, k, v, do = (draw((1, 2, N, D), 420 + i, dtype) for i in range(4))
+    q[..., 3] = 1.0
+    k[..., 3] = 0.0
+    hidden = torch.arange(N) % 3 == 1
+    exact = _exact(q, k[:, :, ~hidden], v[:, :, ~hidden], do, False, D ** -0.5)
+    k[:, :, hidden, 3] = float("-inf")
+    o, _, dk, dv = _run(q, k, v, do, False, D ** -0.5)
+    ulp = 2.0 ** (-9 if dtype == torch.bfloat16 else -12)
+    assert ((o.double() - exact[0]).norm() / exact[0].norm()).item() < ulp
+    for got, ref, room in ((dk, exact[2], 1.5), (dv, exact[3], 1.0)):
+        assert not got[:, :, hidden].any()
+        assert ((got[:, :, ~hidden].double() - ref).norm() / ref.norm()).item() < ulp * room
