@@ -33,7 +33,7 @@ struct RopeWorkspace {
 RopeWorkspace rope_workspace_layout(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype, bool synth, bool any_n) {
     RopeWorkspace w{};
     w.tc = rope_tc_supported(D, dtype) && N % 128 == 0;
-    w.split = rope_tc_supported(D, dtype) && N % 128 != 0 && any_n;
+    w.split = any_n && (rope_tc_supported(D, dtype) ? N % 128 != 0 : rope_split_fp32(N, D, dtype));
     const size_t q_elems = (size_t)B * Hq * N * D, kv_elems = (size_t)B * Hkv * N * D;
     size_t off = 0;
     w.packed_tab = off;
@@ -389,7 +389,8 @@ int rope_fwd_impl(const void* q, const void* k, const void* v, Rotation rot, voi
         return launch_rope_fwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
-    // ragged N, rows that can be moved in 16-byte vectors: split operands at fp32 accuracy (rope_split.cu has both sides' figures)
+    // rows that can be moved in 16-byte vectors, ragged N or fp32 of D = 64: split operands at fp32 accuracy (rope_split*.cu have both
+    // sides' figures)
     const bool split = w.split && policy == 0;
     note_kernels(kFamFwd, 0, split);
     p.sched_counter = reinterpret_cast<int*>((char*)workspace + w.packed_tab) + (size_t)N * (D / 2);   // the table itself is not used

@@ -742,6 +742,10 @@ int launch_rope_bwd_prepass(const RopeParams& p, const TableSource& src, uint32_
 bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types, D = 64 or 128
 // 16-byte aligned rows at any N, 16-bit tensors of D = 64 or 128: split operands, `ws` of rope_split_workspace_bytes, two words of workspace
 // at p.sched_counter; the backward computes delta
+// fp32 tensors on split operands: D = 64, from this length on.  Forward + backward on them / on the CUDA cores: B1 H1 N200 84 / 80 us (as much
+// host as GPU time), B2 H4 N300 86 / 94, B4 H8 N512 causal 88 / 261, B1 H8 N1000 100 / 495, B1 H4 N2048 causal 152 / 519.  (D = 128: the
+// three parts of K, V and the streamed rows of the backward do not fit a shared memory.)
+inline bool rope_split_fp32(int N, int D, int dtype) { return dtype == COROPE_DTYPE_F32 && D == 64 && N >= 256; }
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype);
 int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
 int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s);   // the tcgen05 form of the forward

@@ -6,7 +6,7 @@
 //     KV = false   owns 128 queries, sweeps 64-row blocks of the keys: dQ
 // Owned rows are the A operands and the TMEM lanes, streamed rows the B operands:
 //     S  = own~ str~^T                 5 products of a smaller part into one accumulator, hi hi (exact) into another
-//     dP = V dO^T  (dO V^T)            inputs as they are
+//     dP = V dO^T  (dO V^T)            inputs as they are (fp32 tensors, D = 64: split too, 6 products, as of P dO)
 //     dV += P dO                       P in three parts of the inputs' type (f16: times 2^14)
 //     dK += dS Q~, (dQ += dS K~)       dS in three bf16 parts: 6 products
 // dV and dK / dQ of a block are their own sums in TMEM, which fp32 registers collect.
@@ -650,6 +650,7 @@ FlatGrid rope_split_bwd_grid(int B, int H, int N) { return {(unsigned)(B * H), c
 int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
     const SplitCopies x = split_copies(p, ws, true, dtype);
     if (int e = launch_split_rows(p, x, true, dtype, s)) return e;
+    if (dtype == COROPE_DTYPE_F32) return launch_both<float, 64, 3>(p, x, s);
     if (dtype == COROPE_DTYPE_F16) return launch_d<__half, 3>(p, x, s);
     // bf16 keys without rotation have 8 bits: hi and mid hold all of them
     return p.cos == nullptr ? launch_d<__nv_bfloat16, 2>(p, x, s) : launch_d<__nv_bfloat16, 3>(p, x, s);

@@ -4,7 +4,8 @@
 //                    products of a smaller part in a second one; one fp32 addition joins them (without mid lo, lo mid, lo lo: about 2^-25)
 //     O += P V       P split into three numbers of the inputs' type, V as it is; the product of each 64-key block is its own sum in
 //                    TMEM (small parts first), which fp32 registers collect
-// P <= 1 of f16 tensors enters its products times 2^14.
+// P <= 1 of f16 tensors enters its products times 2^14.  fp32 tensors of D = 64 run here at every length from rope_split_fp32 on: V is split too,
+// P V are 6 products.
 //
 // A work item is 128 query rows of one head; persistent CTAs (one per SM) take items from a counter, heaviest first.  640 threads:
 //   warp 0      TMA producer: fetches items; ring of stages, each the parts of 64 rows of K~ and the rows of V (zeros beyond the head)
@@ -35,9 +36,10 @@ static_assert(128 * (kRegsCtl + 4 * kRegsCompute) <= kThreads * kLaunchRegs, "re
 constexpr int kItemSlots = 2, kItemReaders = 1 + kComputeWarps;
 constexpr uint32_t kHi = sdesc_hi(1024);
 
-template <int D, int KP> struct Fwd {
-    static constexpr int kTile = kBN * D * 2, kStage = (KP + 1) * kTile;   // 64 rows; parts of K~, then V
-    static constexpr int kStages = D == 64 ? 5 : KP == 3 ? 3 : 4;
+// KP, VP: parts of K~ and V
+template <int D, int KP, int VP> struct Fwd {
+    static constexpr int kTile = kBN * D * 2, kStage = (KP + VP) * kTile;   // 64 rows; parts of K~, then V
+    static constexpr int kStages = VP == 3 ? 4 : D == 64 ? 5 : KP == 3 ? 3 : 4;
     static constexpr int kQTile = kBM * D * 2;   // one part of Q~ on its way to TMEM; D = 128: lo stays here
     enum Bar { FULL = 0, EMPTY = FULL + kStages, S_FULL = EMPTY + kStages, P_FULL = S_FULL + 2, O_FULL = P_FULL + 2, Q_READY, ITEM_FULL, ITEM_EMPTY = ITEM_FULL + kItemSlots, NUM_BARS = ITEM_EMPTY + kItemSlots };
     static constexpr size_t kXch = 4 * kBM * sizeof(float), kSlack = 512;
@@ -60,7 +62,8 @@ __device__ __forceinline__ WorkItem work_item(int w, int n_qt, int BH, int head_
 template <typename T, int D, int KP>
 __global__ void __launch_bounds__(kThreads, 1)
 rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __grid_constant__ CUtensorMap mapV, const __grid_constant__ RopeParams p) {
-    using F = Fwd<D, KP>;
+    constexpr int VP = Plain<T>::kParts;
+    using F = Fwd<D, KP, VP>;
     constexpr int ST = F::kStages;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -159,7 +162,12 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                         for (int c = 0; c < D / 64; ++c) {
 #pragma unroll
                             for (int part = 0; part < KP; ++part) tma_load_4d(dst + part * F::kTile + c * (kBN * 128), &mapK, c * 64, j * kBN, kvh, part, bar);
-                            tma_load_4d(dst + KP * F::kTile + c * (kBN * 128), &mapV, c * 64, j * kBN, vh, vb, bar);
+                            if constexpr (VP > 1) {   // the copies of fp32 V are laid out as those of K
+#pragma unroll
+                                for (int part = 0; part < VP; ++part) tma_load_4d(dst + (KP + part) * F::kTile + c * (kBN * 128), &mapV, c * 64, j * kBN, kvh, part, bar);
+                            } else {
+                                tma_load_4d(dst + KP * F::kTile + c * (kBN * 128), &mapV, c * 64, j * kBN, vh, vb, bar);
+                            }
                         }
                     }
                 }
@@ -168,7 +176,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
         } else if (warp == 1) {
             // -------------------------------------------------------------- MMA issuer
             const bool leader = elect_one();
-            constexpr int kVFmt = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 0 : 1;
+            constexpr int kVFmt = Plain<T>::kDtype == COROPE_DTYPE_F16 ? 0 : 1;
             const uint32_t idesc_qk = make_idesc(1, 1, 0, 0, kBM, kBN), idesc_pv = make_idesc(kVFmt, kVFmt, 0, 1, kBM, D);
             const uint32_t stage_lo = sdesc_lo(smem_u32(sm), 0), qlo_lo = sdesc_lo(smem_u32(sQ), 0), v_lo = sdesc_lo(smem_u32(sm) + KP * F::kTile, kBN * 128);
             // one product of a part of Q~ and a part of K~
@@ -217,10 +225,12 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                         if (j + 1 < nb) qk_tail();
                         const uint32_t b0 = v_lo + st * (F::kStage >> 4), a0 = tmem + F::kS + buf * 128;
 #pragma unroll
-                        for (int part = 2; part >= 0; --part)
+                        for (int i = 0; i < (VP > 1 ? kProducts : 3); ++i)   // small parts first
 #pragma unroll
                             for (int kk = 0; kk < kBN / 16; ++kk)
-                                if (leader) umma_ts2(tmem + F::kO, a0 + part * 32 + kk * 8, b0 + kk * (2048 >> 4), kHi, idesc_pv, (part == 2 && kk == 0) ? 0u : 1u);
+                                if (leader)
+                                    umma_ts2(tmem + F::kO, a0 + (VP > 1 ? product_a(i) : 2 - i) * 32 + kk * 8, b0 + (((VP > 1 ? product_b(i) : 0) * F::kTile + kk * 2048) >> 4), kHi,
+                                             idesc_pv, (i == 0 && kk == 0) ? 0u : 1u);
                         if (leader) umma_commit(&bars[F::O_FULL]);
                         if (leader) umma_commit(&bars[F::EMPTY + st]);
                         ++gp;
@@ -275,9 +285,9 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 for (int st = 0; st < STEPS; ++st) {
                     const int r = quad * 32 + wg * 8 + st * RPS + lane / LPR, n = min(wi.t * kBM + r, N - 1);   // rows beyond the head repeat its last one
                     const T* src = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, wi.bh, n) + u * 8;
-                    const uint4 xa = *reinterpret_cast<const uint4*>(src), xb = *reinterpret_cast<const uint4*>(src + D / 2);
-                    float2 a[4] = {unpack2<T>(xa.x), unpack2<T>(xa.y), unpack2<T>(xa.z), unpack2<T>(xa.w)};
-                    float2 b[4] = {unpack2<T>(xb.x), unpack2<T>(xb.y), unpack2<T>(xb.z), unpack2<T>(xb.w)};
+                    float2 a[4], b[4];
+                    load8(src, a);
+                    load8(src + D / 2, b);
                     if (p.cos != nullptr) {
                         float c[8], sn[8];
                         load_table8(p.cos + (int64_t)n * p.table_stride + u * 8, table_vec, c);
@@ -392,7 +402,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                     x0 = fast_exp2(x0), x1 = fast_exp2(x1);
                     sum = f2_add(sum, f2_pack(x0, x1));
                     uint32_t y[3];
-                    split3_cut<T>(x0 * kPScale<T>, x1 * kPScale<T>, y);
+                    split3_cut<typename Plain<T>::Mma>(x0 * kPScale<T>, x1 * kPScale<T>, y);
                     parts[0][i] = y[0], parts[1][i] = y[1], parts[2][i] = y[2];
                 }
 #pragma unroll
@@ -420,17 +430,16 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
             named_bar_sync(quad_bar, 128);
             if (pos < N) {
                 const float inv = total > 0.f ? (1.f / kPScale<T>) / total : 0.f;
-                uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.H, wi.bh, pos) + wg * OC);
+                T* dst = reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.H, wi.bh, pos) + wg * OC;
 #pragma unroll
                 for (int v = 0; v < OC / 8; ++v) {
-                    uint32_t o[4];
+                    float2 o[4];
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
-                        float x, y;
-                        f2_unpack(acc[4 * v + e], x, y);
-                        o[e] = pack2<T>(x * inv, y * inv);
+                        f2_unpack(acc[4 * v + e], o[e].x, o[e].y);
+                        o[e].x *= inv, o[e].y *= inv;
                     }
-                    dst[v] = make_uint4(o[0], o[1], o[2], o[3]);
+                    store8(dst + 8 * v, o);
                 }
                 if (wg == 0) p.lse2[(size_t)wi.bh * N + pos] = m + log2f(total);
             }
@@ -449,13 +458,16 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
 }
 
 template <typename T, int D, int KP>
-int launch_t(const RopeParams& p, const SplitRows& ks, int dtype, cudaStream_t s) {
-    using F = Fwd<D, KP>;
+int launch_t(const RopeParams& p, const SplitCopies& x, cudaStream_t s) {
+    constexpr int VP = Plain<T>::kParts;
+    using F = Fwd<D, KP, VP>;
     CUtensorMap mk, mv;
     Strides sk = contiguous_strides(p.B * p.Hkv, p.N, D);
-    sk.b = (int64_t)ks.plane;   // the parts take the place of the batch dimension
-    if (int e = encode_tensor_map_4d_sw128(&mk, ks.rows, KP, p.B * p.Hkv, p.N, D, sk, kBN, 64, COROPE_DTYPE_BF16)) return e;
-    if (int e = encode_tensor_map_4d_sw128(&mv, p.v, p.B, p.Hkv, p.N, D, p.sv, kBN, 64, dtype)) return e;
+    sk.b = (int64_t)x.k.plane;   // the parts take the place of the batch dimension
+    if (int e = encode_tensor_map_4d_sw128(&mk, x.k.rows, KP, p.B * p.Hkv, p.N, D, sk, kBN, 64, COROPE_DTYPE_BF16)) return e;
+    if (int e = VP > 1 ? encode_tensor_map_4d_sw128(&mv, x.v.rows, VP, p.B * p.Hkv, p.N, D, sk, kBN, 64, COROPE_DTYPE_BF16)
+                       : encode_tensor_map_4d_sw128(&mv, p.v, p.B, p.Hkv, p.N, D, p.sv, kBN, 64, Elem<T>::kDtype))
+        return e;
     RopeParams pp = p;
     pp.head_chunk = p.N >= 4096 ? 8 : 8 * (4096 / (p.N < 128 ? 128 : p.N));
     auto kern = rope_fwd_split_sm100_kernel<T, D, KP>;
@@ -466,18 +478,19 @@ int launch_t(const RopeParams& p, const SplitRows& ks, int dtype, cudaStream_t s
     return launch_dependent(kern, items < sms ? items : sms, kThreads, F::kSmem, s, mk, mv, pp);
 }
 template <typename T, int KP>
-int launch_d(const RopeParams& p, const SplitRows& ks, int dtype, cudaStream_t s) {
-    return p.D == 64 ? launch_t<T, 64, KP>(p, ks, dtype, s) : launch_t<T, 128, KP>(p, ks, dtype, s);
+int launch_d(const RopeParams& p, const SplitCopies& x, cudaStream_t s) {
+    return p.D == 64 ? launch_t<T, 64, KP>(p, x, s) : launch_t<T, 128, KP>(p, x, s);
 }
 
 }  // namespace
 
 int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
-    const SplitRows ks = split_copies(p, ws, false, dtype).k;
-    if (int e = launch_split_rows(p, SplitCopies{ks, {}, {}, {}}, false, dtype, s)) return e;
-    if (dtype == COROPE_DTYPE_F16) return launch_d<__half, 3>(p, ks, dtype, s);
+    const SplitCopies x = split_copies(p, ws, false, dtype);
+    if (int e = launch_split_rows(p, x, false, dtype, s)) return e;
+    if (dtype == COROPE_DTYPE_F32) return launch_t<float, 64, 3>(p, x, s);
+    if (dtype == COROPE_DTYPE_F16) return launch_d<__half, 3>(p, x, s);
     // bf16 keys without rotation have 8 bits: hi and mid hold all of them
-    return p.cos == nullptr ? launch_d<__nv_bfloat16, 2>(p, ks, dtype, s) : launch_d<__nv_bfloat16, 3>(p, ks, dtype, s);
+    return p.cos == nullptr ? launch_d<__nv_bfloat16, 2>(p, x, s) : launch_d<__nv_bfloat16, 3>(p, x, s);
 }
 
 }  // namespace corope

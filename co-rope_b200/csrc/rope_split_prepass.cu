@@ -116,7 +116,7 @@ int launch_d(const RopeParams& p, const SplitCopies& to, bool with_delta, cudaSt
 }  // namespace
 
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype) {
-    size_t heads = (size_t)B * Hkv + (size_t)B * Hq;
+    size_t heads = (size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0);
     if (dtype == COROPE_DTYPE_F32) heads += (size_t)B * Hkv + (bwd ? (size_t)B * Hq : 0);   // V, dO
     return heads * N * D * 3 * sizeof(__nv_bfloat16);
 }
@@ -129,7 +129,7 @@ SplitCopies split_copies(const RopeParams& p, void* ws, bool bwd, int dtype) {
     };
     SplitCopies c{};
     c.k = take(p.Hkv);
-    c.q = take(p.H);
+    if (bwd) c.q = take(p.H);   // the forward takes Q itself
     if (dtype == COROPE_DTYPE_F32) {
         c.v = take(p.Hkv);
         if (bwd) c.d_o = take(p.H);

@@ -70,3 +70,32 @@ def test_gradients_of_keys_masked_by_an_infinite_channel(D, N, dtype):
     for got, ref, room in ((dk, exact[2], 1.5), (dv, exact[3], 1.0)):
         assert not got[:, :, hidden].any()
         assert ((got[:, :, ~hidden].double() - ref).norm() / ref.norm()).item() < ulp * room
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,N", [(1, 2, 2, 256), (2, 3, 3, 257), (1, 8, 2, 321), (1, 160, 160, 260), (1, 2, 2, 1024), (1, 3, 1, 703)])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_fp32_tensors(B, Hq, Hkv, N, causal, transposed):
+    # sums of some hundred fp32 terms: 2^-24 of a term and a root of their number; the CUDA-core kernels show 2e-7 to 1.1e-6 here
+    def make(H, seed):
+        return draw((B, N, H, 64), seed, torch.float32).transpose(1, 2) if transposed else draw((B, H, N, 64), seed, torch.float32)
+
+    q, k, v, do = make(Hq, 440), make(Hkv, 441), make(Hkv, 442), make(Hq, 443)
+    lib = ext.lib()
+    outs = _run(q, k, v, do, causal, 0.125)
+    for op in (ext.OP_ROPE_FWD, ext.OP_ROPE_BWD):
+        assert (lib.corope_last_kernel_family(op), lib.corope_last_kernel_split(op)) == (0, 1)
+    for name, got, ref in zip(("O", "dQ", "dK", "dV"), outs, _exact(q, k, v, do, causal, 0.125)):
+        assert got.dtype == torch.float32 and ((got.double() - ref).norm() / ref.norm()).item() < 1e-6, name
+
+
+def test_fp32_rows_that_are_not_aligned_stay_on_the_cuda_cores():
+    wide = [draw((1, 2, 300, 66), 450 + i, torch.float32) for i in range(4)]
+    do = wide[3][..., 1:65]   # rows 4 bytes off
+    q, k, v = (w.cuda()[..., 1:65].detach().requires_grad_(True) for w in wide[:3])
+    o = pkg.flash_attention(q, k, v, True, 0.125)
+    grads = torch.autograd.grad(o, (q, k, v), do.cuda())
+    ext.check_status()
+    assert ext.lib().corope_last_kernel_split(ext.OP_ROPE_FWD) == 0
+    for got, ref in zip((o.detach(),) + grads, _exact(q.detach(), k.detach(), v.detach(), do, True, 0.125)):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 4e-6
