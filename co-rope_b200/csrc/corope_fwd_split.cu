@@ -12,11 +12,13 @@
 // the CUDA-core kernel (Hq8 Hkv2, inputs times 0.3, where the phases matter least): bf16 N700 D128 0.030 % (0.037 %), f16 N333 D64 0.092 %
 // (0.133 %); at scale 1 f16 N512 D64 1.13 % (1.13 %), its LSE 4.9e-7 (4.8e-7).  Two bf16 parts, and f16 parts without the scaling, had
 // 0.22 % and 0.21 % at scale 0.3.
-// B1 Hq32 Hkv8 N1500 D128 bf16 1170 us (CUDA-core kernel 1347), f16 812 (1355), B2 Hq16 Hkv4 N2048 D64 bf16 970 (1298), B1 Hq16 Hkv2
-// N300 D64 f16 27.5 (68), B4 Hq4 Hkv4 N100 D64 bf16 22.9 (21.0) us, so it takes every size.
+// B1 Hq32 Hkv8 N1500 D128 bf16 928 us (CUDA-core kernel 1347; 1160 with conversions in place of permutes and masks), f16 800 (1355), B2 Hq16
+// Hkv4 N2048 D64 bf16 899 (1298; 969), B1 Hq16 Hkv2 N300 D64 f16 27.5 (68), B4 Hq4 Hkv4 N100 D64 bf16 21.5 (21.0; 23.3) us, so it takes
+// every size.
 // What bounds it: issue slots; the rotation costs two special-function operations and some 20 instructions per (query, key, pair)
 // triple, shared by the heads, against two per head and pair of the CUDA-core kernel on top of that.
 #include "corope_mma.cuh"
+#include "rope_split.cuh"
 
 namespace corope {
 namespace {
@@ -45,9 +47,14 @@ template <> __device__ __forceinline__ void mma<__nv_bfloat16>(float (&d)[4], co
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-// (a, b) as the sum of PARTS pairs of T, each the rounded rest of those before
+// (a, b) as the sum of PARTS pairs of T, each the rounded rest of those before; three bf16 parts, which hold all 24 bits either way, are cut off
+// by byte permutes and masks instead of conversions
 template <typename T, int PARTS>
 __device__ __forceinline__ void split(float a, float b, uint32_t (&parts)[PARTS]) {
+    if constexpr (Elem<T>::kDtype == COROPE_DTYPE_BF16 && PARTS == 3) {
+        split3_cut<T>(a, b, parts);
+        return;
+    }
 #pragma unroll
     for (int x = 0; x < PARTS; ++x) {
         parts[x] = pack2<T>(a, b);
@@ -71,8 +78,6 @@ __device__ __forceinline__ void rotate_split(uint32_t kpair, float angle, uint32
 // hi hi + the smaller products.  An infinity shows in hi hi with the sign it has in fp32; the other parts of such a product are
 // meaningless (NaN or either infinity).
 __device__ __forceinline__ float join(float main, float small) { return fabsf(main) < INFINITY ? main + small : main; }
-// P of f16 tensors enters its products times this
-template <typename T> constexpr float kPScale = Elem<T>::kDtype == COROPE_DTYPE_F16 ? 16384.f : 1.f;
 template <typename T>
 __device__ __forceinline__ uint32_t pair_bits(const T* row, int p, int half) {
     return (uint32_t)*reinterpret_cast<const uint16_t*>(row + p) | (uint32_t)*reinterpret_cast<const uint16_t*>(row + p + half) << 16;
@@ -82,7 +87,7 @@ __device__ __forceinline__ void cp16(void* dst, const void* src, bool have) {   
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ uint4 load8(const uint16_t* src, bool vec) {   // 8 elements; one by one where rows are not aligned to 16 bytes
+__device__ __forceinline__ uint4 load8_any(const uint16_t* src, bool vec) {   // 8 elements; one by one where rows are not aligned to 16 bytes
     if (vec) return *reinterpret_cast<const uint4*>(src);
     uint32_t w[4];
 #pragma unroll
@@ -103,7 +108,7 @@ __global__ void __launch_bounds__(256) gqa_pack_k_kernel(const T* __restrict__ K
     const size_t r = live ? idx / kPerRow : rows - 1;
     const int p0 = (int)(idx % kPerRow) * 8;
     const uint16_t* src = reinterpret_cast<const uint16_t*>(K + flat_row_offset(ak, r) + p0);
-    const uint4 x1 = load8(src, kvec), x2 = load8(src + kPairs, kvec);
+    const uint4 x1 = load8_any(src, kvec), x2 = load8_any(src + kPairs, kvec);
     uint32_t a[4] = {x1.x, x1.y, x1.z, x1.w}, b[4] = {x2.x, x2.y, x2.z, x2.w};
     if (Elem<T>::kDtype == COROPE_DTYPE_F16) {
         float mx = 0.f;
@@ -133,8 +138,8 @@ __global__ void __launch_bounds__(256) gqa_pack_k_kernel(const T* __restrict__ K
     if (vc != nullptr) {
         const uint16_t* v = reinterpret_cast<const uint16_t*>(V + flat_row_offset(av, r) + 2 * p0);
         uint4* out = reinterpret_cast<uint4*>(vc + r * D + 2 * p0);
-        out[0] = load8(v, false);
-        out[1] = load8(v + 8, false);
+        out[0] = load8_any(v, false);
+        out[1] = load8_any(v + 8, false);
     }
 }
 
