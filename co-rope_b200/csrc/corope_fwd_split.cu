@@ -12,7 +12,8 @@
 // the CUDA-core kernel (Hq8 Hkv2, inputs times 0.3, where the phases matter least): bf16 N700 D128 0.030 % (0.037 %), f16 N333 D64 0.092 %
 // (0.133 %); at scale 1 f16 N512 D64 1.13 % (1.13 %), its LSE 4.9e-7 (4.8e-7).  Two bf16 parts, and f16 parts without the scaling, had
 // 0.22 % and 0.21 % at scale 0.3.
-// B1 Hq32 Hkv8 N1500 D128 bf16 928 us (CUDA-core kernel 1347; 1160 with conversions in place of permutes and masks), f16 800 (1355), B2 Hq16
+// B1 Hq32 Hkv8 N1500 D128 bf16 928 us (CUDA-core kernel 1347; 1160 with conversions in place of permutes and masks), f16 763 (1355; 810 with conversions
+// back to fp32 in place of mixed-precision additions), B2 Hq16
 // Hkv4 N2048 D64 bf16 899 (1298; 969), B1 Hq16 Hkv2 N300 D64 f16 27.5 (68), B4 Hq4 Hkv4 N100 D64 bf16 21.5 (21.0; 23.3) us, so it takes
 // every size.
 // What bounds it: issue slots; the rotation costs two special-function operations and some 20 instructions per (query, key, pair)
@@ -58,9 +59,7 @@ __device__ __forceinline__ void split(float a, float b, uint32_t (&parts)[PARTS]
 #pragma unroll
     for (int x = 0; x < PARTS; ++x) {
         parts[x] = pack2<T>(a, b);
-        const float2 f = unpack2<T>(parts[x]);
-        a -= f.x;
-        b -= f.y;
+        if (x + 1 < PARTS) subtract_pair<T>(parts[x], a, b);
     }
 }
 // parts of a rotated K: bf16 needs three for the 24 bits of an fp32 number; two of f16 hold 22 where scaled rows keep them out of the

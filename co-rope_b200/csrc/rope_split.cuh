@@ -45,15 +45,21 @@ __device__ __forceinline__ void store8(T* to, const float2 (&x)[4]) {
     }
 }
 
+// (a, b) minus a pair of T: fp32 additions that take the 16-bit number as it is, so nothing is converted back
+template <typename T>
+__device__ __forceinline__ void subtract_pair(uint32_t pair, float& a, float& b) {
+    if constexpr (Elem<T>::kDtype == COROPE_DTYPE_F16)
+        asm("{\n\t.reg .f16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.f16 %0, lo, %0;\n\tadd.rn.f32.f16 %1, hi, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(pair ^ 0x80008000u));
+    else
+        asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.bf16 %0, lo, %0;\n\tadd.rn.f32.bf16 %1, hi, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(pair ^ 0x80008000u));
+}
 // parts[] = hi, mid, lo of (a, b), each rounded to T; a non-finite number is its own hi
 template <typename T>
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&parts)[3]) {
 #pragma unroll
     for (int x = 0; x < 3; ++x) {
         parts[x] = pack2<T>(a, b);
-        const float2 f = unpack2<T>(parts[x]);
-        a -= f.x;
-        b -= f.y;
+        if (x < 2) subtract_pair<T>(parts[x], a, b);
     }
 }
 // the same for two finite numbers, bf16 parts cut off instead of rounded (the three then hold the 24 bits exactly): byte permutes and
