@@ -5,7 +5,7 @@
 //     KV = true    owns 128 keys of a K / V head, sweeps 64-row blocks of the queries of its group's heads: dK, dV
 //     KV = false   owns 128 queries, sweeps 64-row blocks of the keys: dQ
 // Owned rows are the A operands and the TMEM lanes, streamed rows the B operands:
-//     S  = own~ str~^T                 5 products of a smaller part into one accumulator, hi hi (exact) into another
+//     S  = own~ str~^T                 5 products of a smaller part into one accumulator, hi hi into another (join_products)
 //     dP = V dO^T  (dO V^T)            inputs as they are (fp32 tensors, D = 64: split too, 6 products, as of P dO)
 //     dV += P dO                       P in three parts of the inputs' type (f16: times 2^14)
 //     dK += dS Q~, (dQ += dS K~)       dS in three bf16 parts: 6 products
@@ -22,8 +22,9 @@
 // 5700.  D = 64: score products overlap the softmax of the block before.  Forward + backward of B1 H32 N1777 D128 bf16 causal 1720 ->
 // 567 us (two mma.sync kernels that form the scores at three parts before), B4 H16 N1000 D64 bf16 full 1032 -> 380 us, B1 H2 N5999
 // D128 1826 -> 604 us, B1 H8 N4001 D64 f16 1230 -> 326 us; GPU time of the backward of B1 H1 N65 D64 28.5 -> 14.8 us.  Share of results
-// off the exact rounding before and now (f16, N(0, 1) inputs, B1 H4 N1777 D128 causal): dQ 0.19 / 0.20, dK 0.22 / 0.21, dV 0.22 / 0.20 %; bf16
-// dQ 0.045 / 0.042, dK 0.042 / 0.040, dV 0.041 / 0.038 %.
+// off the exact rounding before and now (f16, N(0, 1) inputs, B1 H4 N1777 D128 causal): dQ 0.19 / 0.20, dK 0.22 / 0.22, dV 0.22 / 0.22 %; bf16
+// dQ 0.057 / 0.044, dK 0.041 / 0.041, dV 0.040 / 0.040 %.  fp32 (B1 H4 N512 D64 causal), CUDA cores / here: dQ 3.6e-7 / 2.5e-7, dK 5.7e-7 /
+// 2.7e-7, dV 5.5e-7 / 2.3e-7.
 //
 // Math: fused-rope/rope_attn_pytorch.py:187-222.
 #include "rope_split.cuh"
@@ -52,7 +53,7 @@ template <int D, int KP, int XP, bool KV> struct Bwd {
     // dP is summed in two (D = 64), three (dQ) or four (dK, dV) pieces of the head dimension that meet in registers, because the adder of the
     // MMAs truncates: with one sum the share of dQ off the exact rounding grew from 0.19 to 0.21 % (D = 128, f16).  The further pieces have
     // their own columns (D = 64), or those of dK / dQ and dV between the collection of the block before and the products of this one.
-    // Parts of V and dO (XP = 3): hi hi, exact, is one piece, the smaller products are the other.
+    // Parts of V and dO (XP = 3): hi hi is one piece, the smaller products are the other.
     static constexpr bool kOwnPieces = D == 64;
     static constexpr int kPieces = D == 64 ? 2 : KV ? 4 : 3;
     static_assert(XP == 1 || D == 64, "pieces of dP");
@@ -450,7 +451,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                     COROPE_TMEM_LD16(tS + 64 + wg * 16, small);
                     tmem_wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) f2_unpack(f2_add(f2_pack_bits(main[2 * i], main[2 * i + 1]), f2_pack_bits(small[2 * i], small[2 * i + 1])), s[2 * i], s[2 * i + 1]);
+                    for (int i = 0; i < 8; ++i) f2_unpack(join_products<D>(f2_pack_bits(main[2 * i], main[2 * i + 1]), f2_pack_bits(small[2 * i], small[2 * i + 1])), s[2 * i], s[2 * i + 1]);
                 }
                 float nan0 = 0.f, nan1 = 0.f;
 #pragma unroll
@@ -512,7 +513,11 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                             COROPE_TMEM_LD16(lanes + W::piece_col(c) + wg * 16 + h * kCols, r);
                         tmem_wait_ld();
 #pragma unroll
-                        for (int i = 0; i < kCols; ++i) dp[h * kCols + i] = c == 0 ? __uint_as_float(r[i]) : dp[h * kCols + i] + __uint_as_float(r[i]);
+                        for (int i = 0; i < kCols; i += 2) {
+                            float &d0 = dp[h * kCols + i], &d1 = dp[h * kCols + i + 1];
+                            const uint64_t x = f2_pack_bits(r[i], r[i + 1]);
+                            f2_unpack(c == 0 ? x : XP > 1 ? join_products<D>(f2_pack(d0, d1), x) : f2_add(f2_pack(d0, d1), x), d0, d1);
+                        }
                     }
                 }
                 if (KV) {

@@ -1,7 +1,7 @@
 // Fused-RoPE / plain attention forward for 16-bit tensors at lengths that are not whole 128-row tiles, D = 64 or 128, at the accuracy of
 // fp32 operands: tcgen05 MMAs on operands split into 16-bit parts (rope_split.cuh).
-//     S  = Q~ K~^T   both rotated in fp32 and split into three bf16 parts: hi hi in one accumulator (exact, see row_unit), the five
-//                    products of a smaller part in a second one; one fp32 addition joins them (without mid lo, lo mid, lo lo: about 2^-25)
+//     S  = Q~ K~^T   both rotated in fp32 and split into three bf16 parts: hi hi in one accumulator, the five products of a smaller
+//                    part in a second one; join_products adds them (without mid lo, lo mid, lo lo: about 2^-25)
 //     O += P V       P split into three numbers of the inputs' type, V as it is; the product of each 64-key block is its own sum in
 //                    TMEM (small parts first), which fp32 registers collect
 // P <= 1 of f16 tensors enters its products times 2^14.  fp32 tensors of D = 64 run here at every length from rope_split_fp32 on: V is split too,
@@ -20,7 +20,8 @@
 // What bounds it: 48 + 12 MMAs per block of 64 keys (D = 128; 2520 cycles), measured at 2800 cycles per block and 14 700 per item (rotation
 // and split of Q 8700).  B1 H32 N1777 D128 bf16 causal 397 -> 135 us (mma.sync kernel before), B4 H16 N1000 D64 bf16 full 243 -> 108 us,
 // B1 H2 N5999 D128 538 -> 160 us.  Error against 64-bit arithmetic next to that kernel (N(0, 1) inputs, B1 H4 N1777 D128 causal f16): LSE
-// 3.7e-7 (3.8e-7), results that are not the exact one rounded 0.093 % (0.117 %); q and k times 4: LSE 3.1e-6 (4.4e-6), 0.21 % (0.32 %).
+// 3.6e-7 (3.8e-7), results that are not the exact one rounded 0.119 % (0.123 %); q and k times 4: LSE 4.7e-6 (4.5e-6; CUDA cores 6.9e-6),
+// 0.31 % (0.30 %; 0.47 %).  fp32 (B1 H4 N512 D64 causal): O 1.3e-7 (CUDA cores 2.3e-7), also where channels differ in scale by 1000.
 //
 // Replaces _attn_fwd of the reference (fused-rope/fused_rope_attn.py:219-320) for these lengths; math: rope_attn_pytorch.py:108-155.
 #include "rope_split.cuh"
@@ -296,20 +297,11 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                         for (int e = 0; e < 4; ++e) rotate(a[e], b[e], c + 2 * e, sn + 2 * e);
                     }
                     const float scale = p.sm_scale * kLog2e;
-                    float largest = 0.f;
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) {
-                        a[e].x *= scale, a[e].y *= scale, b[e].x *= scale, b[e].y *= scale;
-                        largest = fmax3_nan(largest, fmax3_nan(0.f, fabsf(a[e].x), fabsf(a[e].y)), fmax3_nan(0.f, fabsf(b[e].x), fabsf(b[e].y)));
-                    }
-#pragma unroll
-                    for (int off = 1; off < LPR; off <<= 1) largest = fmax3_nan(0.f, largest, __shfl_xor_sync(0xffffffffu, largest, off));
-                    const RowUnit unit = row_unit(largest);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         uint32_t x[3], y[3];
-                        split_row_pair(a[e].x, a[e].y, unit, x);
-                        split_row_pair(b[e].x, b[e].y, unit, y);
+                        split3_any<__nv_bfloat16>(a[e].x * scale, a[e].y * scale, x);
+                        split3_any<__nv_bfloat16>(b[e].x * scale, b[e].y * scale, y);
 #pragma unroll
                         for (int part = 0; part < 3; ++part) pa[st][part][e] = x[part], pb[st][part][e] = y[part];
                     }
@@ -358,7 +350,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 const int key0 = j * kBN + wg * 16;
                 float s[16];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) f2_unpack(f2_add(f2_pack_bits(main[2 * i], main[2 * i + 1]), f2_pack_bits(small[2 * i], small[2 * i + 1])), s[2 * i], s[2 * i + 1]);
+                for (int i = 0; i < 8; ++i) f2_unpack(join_products<D>(f2_pack_bits(main[2 * i], main[2 * i + 1]), f2_pack_bits(small[2 * i], small[2 * i + 1])), s[2 * i], s[2 * i + 1]);
                 float mx = -INFINITY;
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) mx = fmax3_nan(mx, s[i], s[i + 1]);

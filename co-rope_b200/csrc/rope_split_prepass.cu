@@ -62,22 +62,13 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
 #pragma unroll
         for (int e = 0; e < 4; ++e) rotate(ra[e], rb[e], c + 2 * e, sn + 2 * e);
     }
-    float largest = 0.f;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        ra[e].x *= in.scale, ra[e].y *= in.scale, rb[e].x *= in.scale, rb[e].y *= in.scale;
-        largest = fmax3_nan(largest, fmax3_nan(0.f, fabsf(ra[e].x), fabsf(ra[e].y)), fmax3_nan(0.f, fabsf(rb[e].x), fabsf(rb[e].y)));
-    }
-#pragma unroll
-    for (int off = 1; off < kPerRow; off <<= 1) largest = fmax3_nan(0.f, largest, __shfl_xor_sync(0xffffffffu, largest, off));
-    const RowUnit unit = row_unit(largest);
+    if (!live) return;
     uint32_t pa[4][3], pb[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        split_row_pair(ra[e].x, ra[e].y, unit, pa[e]);
-        split_row_pair(rb[e].x, rb[e].y, unit, pb[e]);
+        split3_any<__nv_bfloat16>(ra[e].x * in.scale, ra[e].y * in.scale, pa[e]);
+        split3_any<__nv_bfloat16>(rb[e].x * in.scale, rb[e].y * in.scale, pb[e]);
     }
-    if (!live) return;
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
         __nv_bfloat16* to = in.out.rows + part * in.out.plane + row * D + d;
