@@ -185,10 +185,10 @@ __global__ void __launch_bounds__(Fwd<D, KP>::kThreads, Fwd<D, KP>::kCtas) rope_
                     float2 a = unpack2<T>(*reinterpret_cast<const uint32_t*>(q)), b = unpack2<T>(*reinterpret_cast<const uint32_t*>(q + D / 2));
                     if constexpr (decltype(rot)::value) rotate(a, b, p.cos + (int64_t)pos * p.table_stride + d, p.sin + (int64_t)pos * p.table_stride + d);
                     uint32_t w[3];
-                    split3_any<__nv_bfloat16>(a.x * scale, a.y * scale, w);
+                    split3_any(a.x * scale, a.y * scale, w);
 #pragma unroll
                     for (int part = 0; part < 3; ++part) qa[k][part][x] = w[part];
-                    split3_any<__nv_bfloat16>(b.x * scale, b.y * scale, w);
+                    split3_any(b.x * scale, b.y * scale, w);
 #pragma unroll
                     for (int part = 0; part < 3; ++part) qa[k + KS / 2][part][x] = w[part];
                 }

@@ -77,17 +77,17 @@ __device__ __forceinline__ void split3_cut(float a, float b, uint32_t (&parts)[3
         split3<T>(a, b, parts);
     }
 }
-// the same for operands of any value: what is not finite keeps to hi.  Three rounded bf16 parts hold the 24 bits of every number of its own,
-// whatever the size of its neighbours.
-template <typename T>
+// bf16 parts of operands of any value: three rounded ones hold the 24 bits of every number of its own, whatever the size of its neighbours.
+// What is not finite keeps to hi; a finite number beyond the largest bf16 number, which would round to an infinity, has that one as its hi.
 __device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3]) {
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-        parts[x] = pack2<T>(a, b);
-        const float2 f = unpack2<T>(parts[x]);
-        a = fabsf(a - f.x) < INFINITY ? a - f.x : 0.f;
-        b = fabsf(b - f.y) < INFINITY ? b - f.y : 0.f;
-    }
+    constexpr float kTop = 0x1.fep127f;
+    const bool fa = fabsf(a) < INFINITY, fb = fabsf(b) < INFINITY;
+    parts[0] = pack_bf162(fa ? fminf(fmaxf(a, -kTop), kTop) : a, fb ? fminf(fmaxf(b, -kTop), kTop) : b);
+    float2 f = unpack_bf162(parts[0]);
+    a = fa ? a - f.x : 0.f, b = fb ? b - f.y : 0.f;
+    parts[1] = pack_bf162(a, b);
+    f = unpack_bf162(parts[1]);
+    parts[2] = pack_bf162(a - f.x, b - f.y);
 }
 
 // The leading products of two split operands (hi hi) are one chain of MMAs per 16 columns, whose adder drops bits towards zero: 2^-26 of the

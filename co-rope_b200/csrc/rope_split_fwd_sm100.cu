@@ -300,8 +300,8 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
                         uint32_t x[3], y[3];
-                        split3_any<__nv_bfloat16>(a[e].x * scale, a[e].y * scale, x);
-                        split3_any<__nv_bfloat16>(b[e].x * scale, b[e].y * scale, y);
+                        split3_any(a[e].x * scale, a[e].y * scale, x);
+                        split3_any(b[e].x * scale, b[e].y * scale, y);
 #pragma unroll
                         for (int part = 0; part < 3; ++part) pa[st][part][e] = x[part], pb[st][part][e] = y[part];
                     }

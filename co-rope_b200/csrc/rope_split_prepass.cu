@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
     uint32_t pa[4][3], pb[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        split3_any<__nv_bfloat16>(ra[e].x * in.scale, ra[e].y * in.scale, pa[e]);
-        split3_any<__nv_bfloat16>(rb[e].x * in.scale, rb[e].y * in.scale, pb[e]);
+        split3_any(ra[e].x * in.scale, ra[e].y * in.scale, pa[e]);
+        split3_any(rb[e].x * in.scale, rb[e].y * in.scale, pb[e]);
     }
 #pragma unroll
     for (int part = 0; part < 3; ++part) {

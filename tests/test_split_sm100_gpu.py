@@ -171,3 +171,20 @@ def test_lse_with_channels_of_different_scale(N, D, dtype):
     new, old = run(), _by_policy(1, run)
     ext.check_status()
     assert new <= 1.25 * old, (new, old)
+
+
+@pytest.mark.parametrize("causal", [True, False])
+def test_fp32_values_at_the_end_of_the_range(causal):
+    # keys hidden by a channel of the lowest finite number, which is no bf16 number, and the largest one in V (where no query sees it alone)
+    N, s = 300, 0.125
+    q, k, v, do = (draw((1, 2, N, 64), 470 + i, torch.float32) for i in range(4))
+    q[..., 3] = 1.0
+    k[..., 3] = 0.0
+    k[:, :, torch.arange(N) % 3 == 1, 3] = torch.finfo(torch.float32).min
+    exact = _exact(q, k, v, do, causal, s)
+    for name, got, ref in zip(("O", "dQ", "dK", "dV"), _run(q, k, v, do, causal, s), exact):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < 1e-6, name
+    v[:, :, 42, 7] = torch.finfo(torch.float32).max
+    o, ref = pkg.flash_attention(q.cuda(), k.cuda(), v.cuda(), causal, s).double(), _exact(q, k, v, do, causal, s)[0]
+    ext.check_status()
+    assert ((o - ref).norm(dim=2) / ref.norm(dim=2)).max().item() < 2e-6   # of every channel
