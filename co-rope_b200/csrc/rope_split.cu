@@ -5,7 +5,8 @@
 // bf16 for everything that is not bounded, so that no magnitude of the inputs leaves the range.  P <= 1 of f16 tensors enters its
 // products times 2^14: the three numbers then reach down to 2^-38 of the row's largest probability.  The adder of the MMAs does not round to
 // nearest; the large products therefore go through one 16-wide step each (with the smaller ones in front for the sums over keys), which
-// fp32 additions join.
+// fp32 additions join.  Infinities in Q or K keep the scores they have in fp32; beyond that non-finite operands of 16-bit tensors give NaN
+// here and in the other split-operand kernels, also where fp32 sums would have been infinite (0 times an infinity where a part of P is 0).
 //
 // Longer sequences and the backward run on tcgen05 MMAs (rope_split_fwd_sm100.cu, rope_split_bwd_sm100.cu); the line is at short_forward.
 // What bounds this one: mma.sync, measured at 553 TFLOP/s with all operands in registers (B200, 8 warps per SM); with 8 warps per SM

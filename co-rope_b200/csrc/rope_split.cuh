@@ -78,16 +78,19 @@ __device__ __forceinline__ void split3_cut(float a, float b, uint32_t (&parts)[3
     }
 }
 // bf16 parts of operands of any value: three rounded ones hold the 24 bits of every number of its own, whatever the size of its neighbours.
-// What is not finite keeps to hi; a finite number beyond the largest bf16 number, which would round to an infinity, has that one as its hi.
-__device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3]) {
+// A finite number beyond the largest bf16 number, which would round to an infinity, has that one as its hi.  What is not finite is hi alone, or
+// (`in_lo`, for V and dO) lo alone: of the six products lo only meets the leading part of the other operand, so an infinity never meets a
+// part that is 0 where the number is not.
+__device__ __forceinline__ void split3_any(float a, float b, uint32_t (&parts)[3], bool in_lo = false) {
     constexpr float kTop = 0x1.fep127f;
     const bool fa = fabsf(a) < INFINITY, fb = fabsf(b) < INFINITY;
-    parts[0] = pack_bf162(fa ? fminf(fmaxf(a, -kTop), kTop) : a, fb ? fminf(fmaxf(b, -kTop), kTop) : b);
+    const float x = a, y = b;
+    parts[0] = pack_bf162(fa ? fminf(fmaxf(a, -kTop), kTop) : in_lo ? 0.f : x, fb ? fminf(fmaxf(b, -kTop), kTop) : in_lo ? 0.f : y);
     float2 f = unpack_bf162(parts[0]);
     a = fa ? a - f.x : 0.f, b = fb ? b - f.y : 0.f;
     parts[1] = pack_bf162(a, b);
     f = unpack_bf162(parts[1]);
-    parts[2] = pack_bf162(a - f.x, b - f.y);
+    parts[2] = pack_bf162(fa || !in_lo ? a - f.x : x, fb || !in_lo ? b - f.y : y);
 }
 
 // The leading products of two split operands (hi hi) are one chain of MMAs per 16 columns, whose adder drops bits towards zero: 2^-26 of the

@@ -12,7 +12,7 @@ template <typename T> struct Rows {   // rows to split
     SplitRows out;
     size_t rows;
     float scale;
-    int rotate, with_delta;
+    int rotate, with_delta, in_lo;   // in_lo: see split3_any
     unsigned end;   // the block behind its last one
 };
 template <typename T> struct Jobs {
@@ -66,8 +66,8 @@ __global__ void __launch_bounds__(256) split_rows_kernel(const __grid_constant__
     uint32_t pa[4][3], pb[4][3];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-        split3_any(ra[e].x * in.scale, ra[e].y * in.scale, pa[e]);
-        split3_any(rb[e].x * in.scale, rb[e].y * in.scale, pb[e]);
+        split3_any(ra[e].x * in.scale, ra[e].y * in.scale, pa[e], in.in_lo);
+        split3_any(rb[e].x * in.scale, rb[e].y * in.scale, pb[e], in.in_lo);
     }
 #pragma unroll
     for (int part = 0; part < 3; ++part) {
@@ -82,16 +82,16 @@ int launch_t(const RopeParams& p, const SplitCopies& to, bool with_delta, cudaSt
     Jobs<T> jobs{};
     unsigned blocks = 0;
     int n = 0;
-    auto add = [&](const void* x, const Strides& st, int H, const SplitRows& out, float scale, bool rotated, bool delta) {
+    auto add = [&](const void* x, const Strides& st, int H, const SplitRows& out, float scale, bool rotated, bool delta, bool in_lo) {
         if (out.rows == nullptr) return;
         Rows<T>& r = jobs.job[n++];
-        r = {(const T*)x, row_addr(st, H, p.N), out, (size_t)p.B * H * p.N, scale, rotated && p.cos != nullptr, delta, 0};
+        r = {(const T*)x, row_addr(st, H, p.N), out, (size_t)p.B * H * p.N, scale, rotated && p.cos != nullptr, delta, in_lo, 0};
         r.end = blocks += (unsigned)((r.rows * (D / 16) + 255) / 256);
     };
-    add(p.k, p.sk, p.Hkv, to.k, 1.f, true, false);
-    add(p.q, p.sq, p.H, to.q, p.sm_scale * kLog2e, true, with_delta);
-    add(p.v, p.sv, p.Hkv, to.v, 1.f, false, false);
-    add(p.d_o, p.sdo, p.H, to.d_o, 1.f, false, false);
+    add(p.k, p.sk, p.Hkv, to.k, 1.f, true, false, false);
+    add(p.q, p.sq, p.H, to.q, p.sm_scale * kLog2e, true, with_delta, false);
+    add(p.v, p.sv, p.Hkv, to.v, 1.f, false, false, true);
+    add(p.d_o, p.sdo, p.H, to.d_o, 1.f, false, false, true);
     for (; n < 4; ++n) jobs.job[n].end = blocks;
     const bool vec = (((uintptr_t)p.cos | (uintptr_t)p.sin) & 15) == 0 && (p.table_stride & 3) == 0;
     split_rows_kernel<T, D><<<blocks, 256, 0, s>>>(jobs, p.cos, p.sin, p.table_stride, vec, (const T*)p.o, row_addr(p.so, p.H, p.N), (const T*)p.d_o,

@@ -188,3 +188,20 @@ def test_fp32_values_at_the_end_of_the_range(causal):
     o, ref = pkg.flash_attention(q.cuda(), k.cuda(), v.cuda(), causal, s).double(), _exact(q, k, v, do, causal, s)[0]
     ext.check_status()
     assert ((o - ref).norm(dim=2) / ref.norm(dim=2)).max().item() < 2e-6   # of every channel
+
+
+def _same_kinds(outs, refs):
+    for name, a, b in zip(("O", "dQ", "dK", "dV"), outs, refs):
+        assert torch.equal(a.isnan(), b.isnan()), (name, int(a.isnan().sum()), int(b.isnan().sum()))
+        assert torch.equal(a.isinf(), b.isinf()) and torch.equal(a[a.isinf()] > 0, b[b.isinf()] > 0), name
+
+
+@pytest.mark.parametrize("value", [math.inf, -math.inf, math.nan])
+@pytest.mark.parametrize("which", ["v", "do"])
+def test_fp32_infinities_in_v_and_do(which, value):
+    # infinite or NaN exactly where the CUDA-core kernels are: 0 times an infinity must not come from a part of P that is 0
+    t = {n: draw((1, 2, 300, 64), 480 + i, torch.float32) for i, n in enumerate(("q", "k", "v", "do"))}
+    t[which][:, 0, 200, 5] = value
+    t[which][:, 1, 17, 40] = value
+    run = lambda: _run(t["q"], t["k"], t["v"], t["do"], False, 0.125)
+    _same_kinds(run(), _by_policy(1, run))
