@@ -388,6 +388,23 @@ __device__ __forceinline__ void umma_ts2(uint32_t d_tmem, uint32_t a_tmem, uint3
         : "memory");
 }
 
+// The same, but only lanes [FROM, TO) of the accumulator are written (the instruction takes one bit per lane that is not).
+template <int FROM, int TO>
+__device__ __forceinline__ void umma_ts2_lanes(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t b_hi, uint32_t idesc, uint32_t accumulate) {
+    auto off = [](int word) {
+        uint32_t bits = 0;
+        for (int x = 0; x < 32; ++x) bits |= (32 * word + x < FROM || 32 * word + x >= TO ? 1u : 0u) << x;
+        return bits;
+    };
+    constexpr uint32_t m0 = off(0), m1 = off(1), m2 = off(2), m3 = off(3);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "mov.b64 db, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, {%6, %7, %8, %9}, p;\n\t}" ::"r"(d_tmem),
+        "r"(a_tmem), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(accumulate), "r"(m0), "r"(m1), "r"(m2), "r"(m3)
+        : "memory");
+}
+
 // TMEM <-> registers: 32 lanes x 32-bit, N consecutive columns per thread.
 #define COROPE_TMEM_LD32(taddr, r)                                                                                                  \
     asm volatile(                                                                                                                   \

@@ -24,6 +24,30 @@ template <> struct Plain<float> {
 constexpr int kProducts = 6;
 __host__ __device__ constexpr int product_a(int i) { return i == 0 ? 1 : i == 2 ? 2 : i == 4 ? 1 : 0; }
 __host__ __device__ constexpr int product_b(int i) { return i == 0 ? 1 : i == 1 ? 2 : i == 3 ? 1 : 0; }
+// One product of a 64-row block of streamed rows as the K dimension, A from TMEM: a(kk), b(kk) for the k-step of 16 rows `kk`.  REL >= 0: a
+// block on the diagonal, REL rows (0 or 64) behind the first owned one.  Owned rows that a k-step's 16 rows are all hidden from are then left
+// out, because their 0 (P or dS) would make an infinity or a NaN of a row that they have no part in their own.  KEYS: the owned rows are
+// keys, seen by the streamed rows behind them, else queries.  The step with the most owned rows comes first and is the one that may start the sum.
+struct WholeBlock { static constexpr int kRel = -1; };
+// A copy that the compiler does not know the value of: the forms of a product that follow on a branch share no addresses then, which it would
+// otherwise form in front of the branch for all of them and spill (2 - 4 % of the backward).
+__device__ __forceinline__ uint32_t apart(uint32_t x) {
+    asm volatile("" : "+r"(x));
+    return x;
+}
+struct FirstOnDiagonal { static constexpr int kRel = 0; };
+struct SecondOnDiagonal { static constexpr int kRel = 64; };
+template <bool KEYS, typename Where, int X = 0, typename A, typename B>
+__device__ __forceinline__ void block_product(Where where, bool leader, uint32_t d, A a, B b, uint32_t b_hi, uint32_t idesc, bool start) {
+    constexpr int kk = KEYS && Where::kRel >= 0 ? 3 - X : X, rel = Where::kRel + 16 * kk;
+    const uint32_t accumulate = start && X == 0 ? 0u : 1u;
+    if constexpr (Where::kRel < 0) {
+        if (leader) umma_ts2(d, a(kk), b(kk), b_hi, idesc, accumulate);
+    } else {
+        if (leader) umma_ts2_lanes<KEYS ? 0 : rel, KEYS ? rel + 16 : 128>(d, a(kk), b(kk), b_hi, idesc, accumulate);
+    }
+    if constexpr (X < 3) block_product<KEYS, Where, X + 1>(where, leader, d, a, b, b_hi, idesc, start);
+}
 // eight neighbouring numbers of a row, aligned to 16 bytes
 template <typename T>
 __device__ __forceinline__ void load8(const T* __restrict__ x, float2 (&to)[4]) {

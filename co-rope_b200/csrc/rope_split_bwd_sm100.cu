@@ -9,7 +9,8 @@
 //     dP = V dO^T  (dO V^T)            inputs as they are (fp32 tensors, D = 64: split too, 6 products, as of P dO)
 //     dV += P dO                       P in three parts of the inputs' type (f16: times 2^14)
 //     dK += dS Q~, (dQ += dS K~)       dS in three bf16 parts: 6 products
-// dV and dK / dQ of a block are their own sums in TMEM, which fp32 registers collect.
+// dV and dK / dQ of a block are their own sums in TMEM, which fp32 registers collect.  On the diagonal the MMAs leave out the owned rows that a
+// k-step of 16 streamed rows is hidden from (block_product), so that a row with infinities or NaNs only reaches its own group of 16.
 //
 // Persistent CTAs (one per SM) take items (owned blocks, most work first) from a counter.  640 threads:
 //   warp 0      TMA producer: items; the owned rows; ring of stages, each the parts of 64 streamed rotated rows and their plain rows
@@ -301,7 +302,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
             for (int n = 0; ok; ++n) {
                 const int w = fetch_item(n);
                 if (w < 0) break;
-                const int nb = steps_of(item_of(w).t) * (KV ? G : 1), set = n % W::kOwnSets;
+                const int t = item_of(w).t, steps = steps_of(t), nb = steps * (KV ? G : 1), set = n % W::kOwnSets;
                 const uint32_t set_lo = own_lo + set * (W::kOwnSet >> 4);
                 if (W::kTmemTiles > 0 && g > 0 && !(ok = mbar_wait_warp(&bars[W::ACC_FULL], (g - 1) & 1, p.status, W::ACC_FULL, abort_flag))) break;   // the owned operands in TMEM are free
                 for (int i = 0; i < W::kTmemTiles; i += W::kPerStage, ++gs) {
@@ -321,7 +322,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 int grad_stage = gs % ST;
                 issue_s(set_lo);
                 if (ok) issue_dp(set_lo);
-                for (int j = 0; j < nb && ok; ++j, ++g) {
+                for (int j = 0, step = 0; j < nb && ok; ++j, ++g, step = step + 1 == steps ? 0 : step + 1) {
                     const bool more = j + 1 < nb;
                     if (W::kBufs == 2 && more) {
                         issue_s(set_lo);
@@ -329,30 +330,39 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                     }
                     const uint32_t t_lo = stage_lo + grad_stage * (W::kStage >> 4) + kLbo;
                     const int buf = g % W::kBufs;
+                    const int on_diagonal = !causal ? -1 : KV ? (step < 2 ? step : -1) : j - 2 * t;   // < 0: not
+                    auto by_place = [&](auto products) {
+                        if (on_diagonal < 0)
+                            products(WholeBlock{}, tmem, t_lo, buf);
+                        else if (on_diagonal == 0)
+                            products(FirstOnDiagonal{}, apart(tmem), apart(t_lo), apart(buf));
+                        else
+                            products(SecondOnDiagonal{}, apart(tmem), apart(t_lo), apart(buf));
+                    };
+                    auto product = [&](auto where, uint32_t d, uint32_t tm, auto a_col, uint32_t rows, int sp, uint32_t idesc, bool start) {
+                        block_product<KV>(where, leader, d, [&](int kk) { return tm + a_col(kk); }, [&](int kk) { return rows + ((sp * W::kTile + kk * 2048) >> 4); }, kHi, idesc, start);
+                    };
                     if (KV) {
                         if (!(ok = mbar_wait_warp(&bars[W::P_READY], g & 1, p.status, W::P_READY, abort_flag))) break;
                         tc_fence_after();
+                        by_place([&](auto where, uint32_t tm, uint32_t rows, int b) {
 #pragma unroll
-                        for (int i = 0; i < (XP > 1 ? kProducts : 3); ++i) {   // small parts first
-                            const int pp = XP > 1 ? product_a(i) : 2 - i, xp = XP > 1 ? product_b(i) : 0;
-#pragma unroll
-                            for (int kk = 0; kk < kBN / 16; ++kk)
-                                if (leader) umma_ts2(tmem + W::kDV, tmem + W::p_col(buf, pp, kk), t_lo + (((SP + xp) * W::kTile + kk * 2048) >> 4), kHi, idesc_dv, (i == 0 && kk == 0) ? 0u : 1u);
-                        }
+                            for (int i = 0; i < (XP > 1 ? kProducts : 3); ++i)   // small parts first
+                                product(where, tm + W::kDV, tm, [&](int kk) { return W::p_col(b, XP > 1 ? product_a(i) : 2 - i, kk); }, rows, SP + (XP > 1 ? product_b(i) : 0), idesc_dv,
+                                        i == 0);
+                        });
                     }
                     if (!(ok = mbar_wait_warp(&bars[W::DS_READY], g & 1, p.status, W::DS_READY, abort_flag))) break;
                     tc_fence_after();
-                    auto gradient = [&](int dp, int sp, bool first) {
-#pragma unroll
-                        for (int kk = 0; kk < kBN / 16; ++kk)
-                            if (leader) umma_ts2(tmem + W::kAcc, tmem + W::ds_col(buf, dp, kk), t_lo + ((sp * W::kTile + kk * 2048) >> 4), kHi, idesc_acc, (first && kk == 0) ? 0u : 1u);
-                    };
-                    gradient(1, 1, true);
-                    if (SP > 2) gradient(0, 2, false);
-                    gradient(2, 0, false);
-                    gradient(0, 1, false);
-                    gradient(1, 0, false);
-                    gradient(0, 0, false);
+                    by_place([&](auto where, uint32_t tm, uint32_t rows, int b) {
+                        auto gradient = [&](int dp, int sp, bool start) { product(where, tm + W::kAcc, tm, [&](int kk) { return W::ds_col(b, dp, kk); }, rows, sp, idesc_acc, start); };
+                        gradient(1, 1, true);
+                        if (SP > 2) gradient(0, 2, false);
+                        gradient(2, 0, false);
+                        gradient(0, 1, false);
+                        gradient(1, 0, false);
+                        gradient(0, 0, false);
+                    });
                     if (leader) umma_commit(&bars[W::ACC_FULL]);
                     if (leader) umma_commit(&bars[W::EMPTY + grad_stage]);
                     grad_stage = grad_stage + 1 == ST ? 0 : grad_stage + 1;
@@ -393,13 +403,17 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
 #pragma unroll
             for (int i = 0; i < E / 2; ++i) to[i] = f2_add(to[i], f2_pack_bits(r[2 * i], r[2 * i + 1]));
         };
-        auto collect = [&](int block) {
+        // Nothing is added where none of the warp's owned rows has a part in the block (`seen`): their products have not been formed.  Keys: in the
+        // first block of a sweep; queries: in the last one.
+        auto collect = [&](int block, bool seen) {
             if (!(ok = mbar_wait_warp(&bars[W::ACC_FULL], block & 1, p.status, W::ACC_FULL, abort_flag))) return;
             tc_fence_after();
+            if (seen) {
 #pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                add_columns(W::kAcc + half * (D / 2) + wg * E, acc[half]);
-                if constexpr (KV) add_columns(W::kDV + half * (D / 2) + wg * E, dv[half]);
+                for (int half = 0; half < 2; ++half) {
+                    add_columns(W::kAcc + half * (D / 2) + wg * E, acc[half]);
+                    if constexpr (KV) add_columns(W::kDV + half * (D / 2) + wg * E, dv[half]);
+                }
             }
             tc_fence_before();
             if (!W::kOwnPieces) mbar_arrive_warp(&bars[W::ACC_READ], lane);
@@ -420,6 +434,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 const size_t at = (size_t)(wi.head * G + j / steps) * N + q;
                 return lane < 16 ? (q < N ? p.lse2[at] : INFINITY) : (q < N ? p.delta[at] : 0.f);
             };
+            bool seen = true;   // the block before
             float stat = KV ? stream_stat(0) : 0.f;
 #pragma unroll
             for (int half = 0; half < 2; ++half)
@@ -432,7 +447,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 const int buf = g % W::kBufs;
                 const uint32_t tS = lanes + buf * W::kBuf;
                 if (W::kBufs == 1 && j > 0) {
-                    collect(g - 1);
+                    collect(g - 1, seen);
                     if (!ok) break;
                 }
                 if (KV) {
@@ -522,7 +537,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 }
                 if (KV) {
                     if (W::kBufs == 2 && j > 0) {   // dV and dK of the block before leave TMEM to this one
-                        collect(g - 1);
+                        collect(g - 1, seen);
                         if (!ok) break;
                     }
                     tc_fence_before();
@@ -546,14 +561,16 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 }
                 tmem_wait_st();
                 if (!KV && W::kBufs == 2 && j > 0) {   // dQ of the block before leaves TMEM to this one
-                    collect(g - 1);
+                    collect(g - 1, true);
                     if (!ok) break;
                 }
                 tc_fence_before();
                 mbar_arrive_warp(&bars[W::DS_READY], lane);
+                if (KV) seen = !(causal && quad >= 2 && j % steps == 0);
             }
             if (!ok) break;
-            collect(g - 1);
+            if (!KV) seen = !causal || (nb - 1) * kBN <= own0 + quad * 32 + 31;
+            collect(g - 1, seen);
             if (!ok) break;
             // gradients of the rotated rows turned back; Q~ carries sm_scale * log2e, so dK only takes the log2e off again
             if (pos < N) {

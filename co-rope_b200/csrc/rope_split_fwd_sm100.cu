@@ -3,7 +3,8 @@
 //     S  = Q~ K~^T   both rotated in fp32 and split into three bf16 parts: hi hi in one accumulator, the five products of a smaller
 //                    part in a second one; join_products adds them (without mid lo, lo mid, lo lo: about 2^-25)
 //     O += P V       P split into three numbers of the inputs' type, V as it is; the product of each 64-key block is its own sum in
-//                    TMEM (small parts first), which fp32 registers collect
+//                    TMEM (small parts first), which fp32 registers collect; on the diagonal the MMAs leave out the rows that a k-step of 16 keys is
+//                    hidden from (block_product), so that a key with infinities or NaNs only reaches the rows of its own group of 16
 // P <= 1 of f16 tensors enters its products times 2^14.  fp32 tensors of D = 64 run here at every length from rope_split_fp32 on: V is split too,
 // P V are 6 products.
 //
@@ -215,7 +216,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
             for (int n = 0; ok; ++n) {
                 const int w = fetch_item(n);
                 if (w < 0) break;
-                const int nb = blocks_of(work_item(w, n_qt, BH, p.head_chunk).t);
+                const int t = work_item(w, n_qt, BH, p.head_chunk).t, nb = blocks_of(t);
                 if (!(ok = mbar_wait_warp(&bars[F::Q_READY], n & 1, p.status, F::Q_READY, abort_flag))) break;
                 tc_fence_after();
                 for (int j = -2; j < nb && ok; ++j) {   // P V of block j; Q K^T of block j + 2, and at j = -2 alone all of block 0's
@@ -225,13 +226,18 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                         tc_fence_after();
                         if (j + 1 < nb) qk_tail();
                         const uint32_t b0 = v_lo + st * (F::kStage >> 4), a0 = tmem + F::kS + buf * 128;
+                        auto pv = [&](auto where, uint32_t p0, uint32_t v0) {
 #pragma unroll
-                        for (int i = 0; i < (VP > 1 ? kProducts : 3); ++i)   // small parts first
-#pragma unroll
-                            for (int kk = 0; kk < kBN / 16; ++kk)
-                                if (leader)
-                                    umma_ts2(tmem + F::kO, a0 + (VP > 1 ? product_a(i) : 2 - i) * 32 + kk * 8, b0 + (((VP > 1 ? product_b(i) : 0) * F::kTile + kk * 2048) >> 4), kHi,
-                                             idesc_pv, (i == 0 && kk == 0) ? 0u : 1u);
+                            for (int i = 0; i < (VP > 1 ? kProducts : 3); ++i)   // small parts first
+                                block_product<false>(where, leader, tmem + F::kO, [&](int kk) { return p0 + (VP > 1 ? product_a(i) : 2 - i) * 32 + kk * 8; },
+                                                     [&](int kk) { return v0 + (((VP > 1 ? product_b(i) : 0) * F::kTile + kk * 2048) >> 4); }, kHi, idesc_pv, i == 0);
+                        };
+                        if (!causal || j < 2 * t)
+                            pv(WholeBlock{}, a0, b0);
+                        else if (j == 2 * t)
+                            pv(FirstOnDiagonal{}, apart(a0), apart(b0));
+                        else
+                            pv(SecondOnDiagonal{}, apart(a0), apart(b0));
                         if (leader) umma_commit(&bars[F::O_FULL]);
                         if (leader) umma_commit(&bars[F::EMPTY + st]);
                         ++gp;
@@ -253,8 +259,9 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
         int g = 0;                                                     // blocks so far
         bool ok = true;
         uint64_t acc[OC / 2];
-        // O += product of the block before, alpha = what the reference max moved by at that block
-        auto collect = [&](int block, float alpha, bool last) {
+        // O += product of the block before, alpha = what the reference max moved by at that block; nothing where the warp's rows all lie in front
+        // of the block (`seen`; an item's last block alone can be such a one): their product has not been formed
+        auto collect = [&](int block, float alpha, bool seen, bool last) {
             if (!(ok = mbar_wait_warp(&bars[F::O_FULL], block & 1, p.status, F::O_FULL, abort_flag))) return;
             tc_fence_after();
             uint32_t r[OC];
@@ -265,6 +272,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
             tmem_wait_ld();
             tc_fence_before();
             if (!last) mbar_arrive_warp(&bars[F::P_FULL + ((block + 1) & 1)], lane);   // P of the next block, and O is free
+            if (!seen) return;
             const uint64_t a2 = f2_pack(alpha, alpha);
 #pragma unroll
             for (int i = 0; i < OC / 2; ++i) acc[i] = f2_fma(acc[i], a2, f2_pack_bits(r[2 * i], r[2 * i + 1]));
@@ -404,7 +412,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 l = l * alpha + (s0 + s1);   // this group's keys only
                 tmem_wait_st();
                 if (j > 0) {
-                    collect(g - 1, alpha_before, false);
+                    collect(g - 1, alpha_before, true, false);
                     if (!ok) break;
                 } else {
                     tc_fence_before();
@@ -414,7 +422,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 named_bar_sync(quad_bar, 128);   // all four have read the exchanged maxima
             }
             if (!ok) break;
-            collect(g - 1, alpha_before, true);
+            collect(g - 1, alpha_before, !causal || (nb - 1) * kBN <= wi.t * kBM + quad * 32 + 31, true);
             if (!ok) break;
             xch[wg * kBM + row] = l;
             named_bar_sync(quad_bar, 128);

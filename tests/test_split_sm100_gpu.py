@@ -205,3 +205,20 @@ def test_fp32_infinities_in_v_and_do(which, value):
     t[which][:, 1, 17, 40] = value
     run = lambda: _run(t["q"], t["k"], t["v"], t["do"], False, 0.125)
     _same_kinds(run(), _by_policy(1, run))
+
+
+@pytest.mark.parametrize("at", [140, 200, 255, 390])   # in the first and the second 64 columns of a 128-row block, at its end, in the last block
+@pytest.mark.parametrize("D,dtype", [(64, torch.float32), (64, torch.bfloat16), (128, torch.bfloat16), (64, torch.float16), (128, torch.float16)])
+def test_causal_rows_do_not_see_what_is_not_finite_in_hidden_rows(D, dtype, at):
+    # rows in front of a key (behind a query) by its group of 16 rows or more must not change by a bit
+    t = [draw((1, h, 400, D), 490 + i, dtype) for i, h in enumerate((4, 2, 2, 4))]
+    base = _run(*t, True, D ** -0.5)
+    for value in (math.inf, math.nan):
+        for which in range(4):
+            x = [y.clone() for y in t]
+            x[which][:, :, at, 5] = value
+            outs = _run(*x, True, D ** -0.5)
+            front, behind = slice(0, at // 16 * 16), slice(at // 16 * 16 + 16, None)
+            names = ((0, "O", front), (1, "dQ", front)) if which in (1, 2) else ((2, "dK", behind), (3, "dV", behind))
+            for i, name, rows in names:
+                assert torch.equal(outs[i][:, :, rows], base[i][:, :, rows]), ("QKV"[which:which + 1] or "dO", value, name)
