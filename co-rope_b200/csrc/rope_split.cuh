@@ -146,28 +146,17 @@ __device__ __forceinline__ void load_table8(const float* __restrict__ src, bool 
         for (int i = 0; i < 8; ++i) x[i] = src[i];
     }
 }
-// One score by its definition, for operands with infinities or NaNs, whose parts do not multiply as the numbers do.
-template <typename T>
-__device__ __forceinline__ float plain_score(const RopeParams& p, int bh, int row, int key) {
-    const T* q = reinterpret_cast<const T*>(p.q) + row_offset(p.sq, p.H, bh, row);
-    const T* k = reinterpret_cast<const T*>(p.k) + row_offset(p.sk, p.Hkv, bh / (p.H / p.Hkv), key);
-    const int half = p.D / 2;
-    const float scale = p.sm_scale * kLog2e;
-    float s = 0.f;
-#pragma unroll 1
-    for (int d = 0; d < half; ++d) {
-        float q1 = Elem<T>::to_f32(q[d]), q2 = Elem<T>::to_f32(q[d + half]), k1 = Elem<T>::to_f32(k[d]), k2 = Elem<T>::to_f32(k[d + half]);
-        if (p.cos != nullptr) {
-            const float cq = p.cos[(int64_t)row * p.table_stride + d], sq = p.sin[(int64_t)row * p.table_stride + d];
-            const float ck = p.cos[(int64_t)key * p.table_stride + d], sk = p.sin[(int64_t)key * p.table_stride + d];
-            const float a = q1 * cq - q2 * sq, b = k1 * ck - k2 * sk;
-            q2 = q2 * cq + q1 * sq, q1 = a;
-            k2 = k2 * ck + k1 * sk, k1 = b;
-        }
-        s = fmaf(q1 * scale, k1, s);
-        s = fmaf(q2 * scale, k2, s);
+// Scores that joined to NaN: an infinity of an operand is its leading part alone, so the leading products have it with the sign it has in fp32
+// (the smaller ones may be 0 times it).  `col`: their TMEM column, still as the MMAs left it; the whole warp comes here.
+__device__ __forceinline__ void infinite_scores(uint32_t col, float (&s)[16]) {
+#pragma unroll
+    for (int half = 0; half < 16; half += 8) {
+        uint32_t leading[8];
+        COROPE_TMEM_LD8(col + half, leading);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[half + i] = fabsf(__uint_as_float(leading[i])) == INFINITY ? __uint_as_float(leading[i]) : s[half + i];
     }
-    return s;
 }
 
 // P of f16 tensors enters its products times this

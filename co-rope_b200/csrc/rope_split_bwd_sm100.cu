@@ -35,7 +35,7 @@ namespace {
 
 constexpr int kBM = 128, kBN = 64;
 constexpr int kThreads = 640, kComputeWarp0 = 4, kComputeWarps = 16;
-constexpr int kLaunchRegs = 96, kRegsCtl = 48, kRegsCompute = 104;
+constexpr int kLaunchRegs = 96, kRegsCtl = 64, kRegsCompute = 104;
 static_assert(128 * (kRegsCtl + 4 * kRegsCompute) <= kThreads * kLaunchRegs, "register budget");
 constexpr int kItemSlots = 2, kItemReaders = 1 + kComputeWarps;
 constexpr uint32_t kHi = sdesc_hi(1024);
@@ -471,18 +471,7 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 float nan0 = 0.f, nan1 = 0.f;
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) nan0 = fmax3_nan(nan0, s[i], s[i + 1]), nan1 = fmax3_nan(nan1, s[i + 2], s[i + 3]);
-                if (__any_sync(0xffffffffu, nan0 != nan0 || nan1 != nan1)) {   // infinities or NaNs among the operands
-                    const int own = min(pos, N - 1), qh = KV ? wi.head * G + j / steps : wi.head;
-#pragma unroll 1
-                    for (int i = 0; i < 16; ++i) {
-                        float x = 0.f;
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) x = c == i ? s[c] : x;
-                        if (x != x) x = plain_score<T>(p, qh, KV ? min(str0 + i, N - 1) : own, KV ? own : min(str0 + i, N - 1));
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) s[c] = c == i ? x : s[c];
-                    }
-                }
+                if (__any_sync(0xffffffffu, nan0 != nan0 || nan1 != nan1)) infinite_scores(tS + wg * 16, s);   // infinities or NaNs among the operands
 #pragma unroll
                 for (int i = 0; i < 16; i += 4) {
                     const float4 l = KV ? *reinterpret_cast<const float4*>(slot + i) : make_float4(lse, lse, lse, lse);

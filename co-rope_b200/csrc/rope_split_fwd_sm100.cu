@@ -33,7 +33,7 @@ namespace {
 constexpr int kBM = 128, kBN = 64;
 constexpr int kThreads = 640, kComputeWarp0 = 4, kComputeWarps = 16;
 // launch registers 65536 / 640 rounded down to a multiple of 8; what the control warps give up the others may take
-constexpr int kLaunchRegs = 96, kRegsCtl = 40, kRegsCompute = 104;
+constexpr int kLaunchRegs = 96, kRegsCtl = 64, kRegsCompute = 104;
 static_assert(128 * (kRegsCtl + 4 * kRegsCompute) <= kThreads * kLaunchRegs, "register budget");
 constexpr int kItemSlots = 2, kItemReaders = 1 + kComputeWarps;
 constexpr uint32_t kHi = sdesc_hi(1024);
@@ -281,7 +281,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
             const int w = fetch_item(n);
             if (w < 0) break;
             const WorkItem wi = work_item(w, n_qt, BH, p.head_chunk);
-            const int nb = blocks_of(wi.t), pos = wi.t * kBM + row, pos_in = min(pos, N - 1);   // rows beyond the head repeat its last one
+            const int nb = blocks_of(wi.t), pos = wi.t * kBM + row;
             {   // Q~: 8 rotation pairs of a row per lane (whole rows are read at a time), the parts by way of shared memory to the threads
                 // that own the rows in TMEM.  Every MMA of the item before has completed (its last O_FULL).
                 constexpr int LPR = D / 16, RPS = 32 / LPR, STEPS = 8 / RPS;   // lanes per row, rows per step, steps of a warp's 8 rows
@@ -363,16 +363,8 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
 #pragma unroll
                 for (int i = 0; i < 16; i += 2) mx = fmax3_nan(mx, s[i], s[i + 1]);
                 if (__any_sync(0xffffffffu, mx != mx)) {   // infinities or NaNs among the operands
+                    infinite_scores(tS + wg * 16, s);
                     mx = -INFINITY;
-#pragma unroll 1
-                    for (int i = 0; i < 16; ++i) {
-                        float x = 0.f;
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) x = c == i ? s[c] : x;
-                        if (x != x) x = plain_score<T>(p, wi.bh, pos_in, min(key0 + i, N - 1));
-#pragma unroll
-                        for (int c = 0; c < 16; ++c) s[c] = c == i ? x : s[c];
-                    }
 #pragma unroll
                     for (int i = 0; i < 16; i += 2) mx = fmax3(mx, s[i], s[i + 1]);
                 }

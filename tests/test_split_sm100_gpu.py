@@ -222,3 +222,28 @@ def test_causal_rows_do_not_see_what_is_not_finite_in_hidden_rows(D, dtype, at):
             names = ((0, "O", front), (1, "dQ", front)) if which in (1, 2) else ((2, "dK", behind), (3, "dV", behind))
             for i, name, rows in names:
                 assert torch.equal(outs[i][:, :, rows], base[i][:, :, rows]), ("QKV"[which:which + 1] or "dO", value, name)
+
+
+@pytest.mark.parametrize("D,dtype", [(64, torch.float32), (64, torch.float16), (128, torch.bfloat16)])
+def test_keys_masked_by_an_infinite_channel_cost_nothing(D, dtype):
+    # 0 times an infinity among the smaller products is no reason to form scores one by one (4 to 58 times the time); room for noise
+    q, k, v, do = (draw((1, 8, 1000, D), 500 + i, dtype).cuda() for i in range(4))
+    q[..., 3] = 1.0
+    k[..., 3] = 0.0
+    hidden = k.clone()
+    hidden[:, :, torch.arange(1000) % 3 == 1, 3] = float("-inf")
+    times = {}
+    for name, key in (("plain", k), ("hidden", hidden)) * 2:
+        x = [t.clone().requires_grad_(True) for t in (q, key, v)]
+        spans = []
+        for _ in range(8):
+            begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            begin.record()
+            for _ in range(4):
+                torch.autograd.grad(pkg.flash_attention(*x, False, D ** -0.5), x, do)
+            end.record()
+            end.synchronize()
+            spans.append(begin.elapsed_time(end))
+        times[name] = min(spans)
+    ext.check_status()
+    assert times["hidden"] < 2.0 * times["plain"], times
