@@ -29,12 +29,6 @@ __host__ __device__ constexpr int product_b(int i) { return i == 0 ? 1 : i == 1 
 // out, because their 0 (P or dS) would make an infinity or a NaN of a row that they have no part in their own.  KEYS: the owned rows are
 // keys, seen by the streamed rows behind them, else queries.  The step with the most owned rows comes first and is the one that may start the sum.
 struct WholeBlock { static constexpr int kRel = -1; };
-// A copy that the compiler does not know the value of: the forms of a product that follow on a branch share no addresses then, which it would
-// otherwise form in front of the branch for all of them and spill (2 - 4 % of the backward).
-__device__ __forceinline__ uint32_t apart(uint32_t x) {
-    asm volatile("" : "+r"(x));
-    return x;
-}
 struct FirstOnDiagonal { static constexpr int kRel = 0; };
 struct SecondOnDiagonal { static constexpr int kRel = 64; };
 template <bool KEYS, typename Where, int X = 0, typename A, typename B>

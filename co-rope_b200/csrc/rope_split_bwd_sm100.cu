@@ -322,52 +322,49 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
                 int grad_stage = gs % ST;
                 issue_s(set_lo);
                 if (ok) issue_dp(set_lo);
-                for (int j = 0, step = 0; j < nb && ok; ++j, ++g, step = step + 1 == steps ? 0 : step + 1) {
-                    const bool more = j + 1 < nb;
+                int left = nb;
+                auto block = [&](auto where) {
+                    const bool more = --left > 0;
                     if (W::kBufs == 2 && more) {
                         issue_s(set_lo);
-                        if (!ok) break;
+                        if (!ok) return;
                     }
                     const uint32_t t_lo = stage_lo + grad_stage * (W::kStage >> 4) + kLbo;
                     const int buf = g % W::kBufs;
-                    const int on_diagonal = !causal ? -1 : KV ? (step < 2 ? step : -1) : j - 2 * t;   // < 0: not
-                    auto by_place = [&](auto products) {
-                        if (on_diagonal < 0)
-                            products(WholeBlock{}, tmem, t_lo, buf);
-                        else if (on_diagonal == 0)
-                            products(FirstOnDiagonal{}, apart(tmem), apart(t_lo), apart(buf));
-                        else
-                            products(SecondOnDiagonal{}, apart(tmem), apart(t_lo), apart(buf));
-                    };
-                    auto product = [&](auto where, uint32_t d, uint32_t tm, auto a_col, uint32_t rows, int sp, uint32_t idesc, bool start) {
-                        block_product<KV>(where, leader, d, [&](int kk) { return tm + a_col(kk); }, [&](int kk) { return rows + ((sp * W::kTile + kk * 2048) >> 4); }, kHi, idesc, start);
+                    auto product = [&](uint32_t d, auto a_col, int sp, uint32_t idesc, bool start) {
+                        block_product<KV>(where, leader, d, [&](int kk) { return tmem + a_col(kk); }, [&](int kk) { return t_lo + ((sp * W::kTile + kk * 2048) >> 4); }, kHi, idesc, start);
                     };
                     if (KV) {
-                        if (!(ok = mbar_wait_warp(&bars[W::P_READY], g & 1, p.status, W::P_READY, abort_flag))) break;
+                        if (!(ok = mbar_wait_warp(&bars[W::P_READY], g & 1, p.status, W::P_READY, abort_flag))) return;
                         tc_fence_after();
-                        by_place([&](auto where, uint32_t tm, uint32_t rows, int b) {
 #pragma unroll
-                            for (int i = 0; i < (XP > 1 ? kProducts : 3); ++i)   // small parts first
-                                product(where, tm + W::kDV, tm, [&](int kk) { return W::p_col(b, XP > 1 ? product_a(i) : 2 - i, kk); }, rows, SP + (XP > 1 ? product_b(i) : 0), idesc_dv,
-                                        i == 0);
-                        });
+                        for (int i = 0; i < (XP > 1 ? kProducts : 3); ++i)   // small parts first
+                            product(tmem + W::kDV, [&](int kk) { return W::p_col(buf, XP > 1 ? product_a(i) : 2 - i, kk); }, SP + (XP > 1 ? product_b(i) : 0), idesc_dv, i == 0);
                     }
-                    if (!(ok = mbar_wait_warp(&bars[W::DS_READY], g & 1, p.status, W::DS_READY, abort_flag))) break;
+                    if (!(ok = mbar_wait_warp(&bars[W::DS_READY], g & 1, p.status, W::DS_READY, abort_flag))) return;
                     tc_fence_after();
-                    by_place([&](auto where, uint32_t tm, uint32_t rows, int b) {
-                        auto gradient = [&](int dp, int sp, bool start) { product(where, tm + W::kAcc, tm, [&](int kk) { return W::ds_col(b, dp, kk); }, rows, sp, idesc_acc, start); };
-                        gradient(1, 1, true);
-                        if (SP > 2) gradient(0, 2, false);
-                        gradient(2, 0, false);
-                        gradient(0, 1, false);
-                        gradient(1, 0, false);
-                        gradient(0, 0, false);
-                    });
+                    auto gradient = [&](int dp, int sp, bool start) { product(tmem + W::kAcc, [&](int kk) { return W::ds_col(buf, dp, kk); }, sp, idesc_acc, start); };
+                    gradient(1, 1, true);
+                    if (SP > 2) gradient(0, 2, false);
+                    gradient(2, 0, false);
+                    gradient(0, 1, false);
+                    gradient(1, 0, false);
+                    gradient(0, 0, false);
                     if (leader) umma_commit(&bars[W::ACC_FULL]);
                     if (leader) umma_commit(&bars[W::EMPTY + grad_stage]);
                     grad_stage = grad_stage + 1 == ST ? 0 : grad_stage + 1;
+                    ++g;
                     if (W::kBufs == 1 && more) issue_s(set_lo);
                     if (ok && more) issue_dp(set_lo);
+                };
+                // the blocks on the diagonal, a sweep's first two (keys) or last two (queries), stand outside the loop: see the forward
+                for (int sweep = 0; sweep < (KV ? G : 1) && ok; ++sweep) {
+                    const int whole = !causal ? steps : KV ? max(steps - 2, 0) : 2 * t, diagonal = steps - whole;
+                    if (KV && diagonal > 0) block(FirstOnDiagonal{});
+                    if (KV && diagonal > 1 && ok) block(SecondOnDiagonal{});
+                    for (int x = 0; x < whole && ok; ++x) block(WholeBlock{});
+                    if (!KV && diagonal > 0 && ok) block(FirstOnDiagonal{});
+                    if (!KV && diagonal > 1 && ok) block(SecondOnDiagonal{});
                 }
                 if (W::kSmemTiles > 0 && leader) umma_commit(&bars[W::OWN_EMPTY + set]);
             }
