@@ -44,7 +44,7 @@ template <int D, int KP, int VP> struct Fwd {
     static constexpr int kStages = VP == 3 ? 4 : D == 64 ? 5 : KP == 3 ? 3 : 4;
     static constexpr int kQTile = kBM * D * 2;   // one part of Q~ on its way to TMEM; D = 128: lo stays here
     enum Bar { FULL = 0, EMPTY = FULL + kStages, S_FULL = EMPTY + kStages, P_FULL = S_FULL + 2, O_FULL = P_FULL + 2, Q_READY, ITEM_FULL, ITEM_EMPTY = ITEM_FULL + kItemSlots, NUM_BARS = ITEM_EMPTY + kItemSlots };
-    static constexpr size_t kXch = 4 * kBM * sizeof(float), kSlack = 512;
+    static constexpr size_t kXch = 4 * kBM * sizeof(float) + 4 * sizeof(int), kSlack = 512;
     static constexpr size_t kSmem = (size_t)kStages * kStage + kQTile + kXch + NUM_BARS * 8 + 32 + kSlack;
     static_assert(kSmem <= 232448, "shared memory budget");
     // TMEM columns
@@ -71,6 +71,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t* sQ = sm + ST * F::kStage;
     float* xch = reinterpret_cast<float*>(sQ + F::kQTile);   // [group][row]
+    volatile int* left = reinterpret_cast<volatile int*>(xch + 4 * kBM);   // per four warps with the same rows: they leave together
     uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(xch) + F::kXch);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + F::NUM_BARS);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
@@ -100,6 +101,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
     }
     if (threadIdx.x == 0) {
         *abort_flag = 0;
+        for (int i = 0; i < 4; ++i) left[i] = 0;
         for (int i = 0; i < ST; ++i) {
             mbar_init(&bars[F::FULL + i], 1);
             mbar_init(&bars[F::EMPTY + i], 1);
@@ -127,10 +129,10 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    // the n-th item of this CTA, or -1 when there is none left (or a wait gave up); one arrival per warp
+    // the n-th item of this CTA, -1 when there is none left, -2 where the wait gave up; one arrival per warp
     auto fetch_item = [&](int n) {
         const int slot = n % kItemSlots;
-        if (!mbar_wait_warp(&bars[F::ITEM_FULL + slot], (n / kItemSlots) & 1, p.status, F::ITEM_FULL, abort_flag)) return -1;
+        if (!mbar_wait_warp(&bars[F::ITEM_FULL + slot], (n / kItemSlots) & 1, p.status, F::ITEM_FULL, abort_flag)) return -2;
         const int w = item_ring[slot];
         mbar_arrive_warp(&bars[F::ITEM_EMPTY + slot], lane);
         return w;
@@ -275,9 +277,14 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
 #pragma unroll
             for (int i = 0; i < OC / 2; ++i) acc[i] = f2_fma(acc[i], a2, f2_pack_bits(r[2 * i], r[2 * i + 1]));
         };
-        for (int n = 0; ok; ++n) {
-            const int w = fetch_item(n);
-            if (w < 0) break;
+        // A warp whose wait gave up must not leave the three that meet it at quad_bar alone: it goes on to the next of two places where they
+        // look for it, the start of an item (`left`) and the exchange of a block's maxima (NaN, which no maximum is), and all four leave behind it.
+        // tests/test_give_up_cpu.py goes through every order of this.
+        for (int n = 0;; ++n) {
+            const int w = ok ? fetch_item(n) : -2;
+            if (w == -2) left[quad] = 1;
+            named_bar_sync(quad_bar, 128);
+            if (w < 0 || left[quad] != 0) break;
             const WorkItem wi = work_item(w, n_qt, BH, p.head_chunk);
             const int nb = blocks_of(wi.t), pos = wi.t * kBM + row;
             {   // Q~: 8 rotation pairs of a row per lane (whole rows are read at a time), the parts by way of shared memory to the threads
@@ -342,11 +349,18 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 mbar_arrive_warp(&bars[F::Q_READY], lane);
             }
             float m = -INFINITY, l = 0.f, alpha_before = 0.f;
+            bool all_here = false;
 #pragma unroll
             for (int i = 0; i < OC / 2; ++i) acc[i] = 0;
             for (int j = 0; j < nb; ++j, ++g) {
                 const int buf = g & 1;
-                if (!(ok = mbar_wait_warp(&bars[F::S_FULL + buf], (g >> 1) & 1, p.status, F::S_FULL, abort_flag))) break;
+                if (ok) ok = mbar_wait_warp(&bars[F::S_FULL + buf], (g >> 1) & 1, p.status, F::S_FULL, abort_flag);
+                if (!ok) {
+                    xch[wg * kBM + row] = __int_as_float(0x7fffffff);
+                    named_bar_sync(quad_bar, 128);
+                    named_bar_sync(quad_bar, 128);
+                    break;
+                }
                 tc_fence_after();
                 const uint32_t tS = lanes + F::kS + buf * 128;
                 uint32_t main[16], small[16];
@@ -376,9 +390,8 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 }
                 xch[wg * kBM + row] = mx;
                 named_bar_sync(quad_bar, 128);   // also: all four have read their S, so P may be written anywhere over it
-                float m_new = fmaxf(m, mx);
-#pragma unroll
-                for (int x = 1; x < 4; ++x) m_new = fmaxf(m_new, xch[(wg ^ x) * kBM + row]);
+                const float others = fmax3_nan(xch[(wg ^ 1) * kBM + row], xch[(wg ^ 2) * kBM + row], xch[(wg ^ 3) * kBM + row]);
+                const float m_new = fmax3(m, mx, others);
                 const float ref = m_new == -INFINITY ? 0.f : m_new;   // a row that has seen no key yet
                 const float alpha = fast_exp2(m - ref);
                 m = m_new;
@@ -403,22 +416,22 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
                 tmem_wait_st();
                 if (j > 0) {
                     collect(g - 1, alpha_before, true, false);
-                    if (!ok) break;
                 } else {
                     tc_fence_before();
                     mbar_arrive_warp(&bars[F::P_FULL + buf], lane);
                 }
                 alpha_before = alpha;
                 named_bar_sync(quad_bar, 128);   // all four have read the exchanged maxima
+                if (others != others) break;     // one of them gave up; in all lanes alike
+                all_here = j + 1 == nb;
             }
-            if (!ok) break;
-            collect(g - 1, alpha_before, !causal || (nb - 1) * kBN <= wi.t * kBM + quad * 32 + 31, true);
-            if (!ok) break;
+            if (!all_here) break;
+            if (ok) collect(g - 1, alpha_before, !causal || (nb - 1) * kBN <= wi.t * kBM + quad * 32 + 31, true);
             xch[wg * kBM + row] = l;
             named_bar_sync(quad_bar, 128);
             const float total = (xch[row] + xch[kBM + row]) + (xch[2 * kBM + row] + xch[3 * kBM + row]);
             named_bar_sync(quad_bar, 128);
-            if (pos < N) {
+            if (ok && pos < N) {
                 const float inv = total > 0.f ? (1.f / kPScale<T>) / total : 0.f;
                 T* dst = reinterpret_cast<T*>(p.out_o) + row_offset(p.so, p.H, wi.bh, pos) + wg * OC;
 #pragma unroll
@@ -435,9 +448,6 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
             }
         }
         tc_fence_before();
-        // warps that gave up do not meet the others at the barriers any more: arrive for all that can come before those give up too
-        if (*abort_flag)
-            for (int i = 0; i < 8; ++i) named_bar_arrive(quad_bar, 128);
     }
     __syncthreads();
     if (threadIdx.x == 0 && *abort_flag) report_to_mirror(p.status, p.status_mirror);
