@@ -32,9 +32,11 @@ namespace {
 
 constexpr int kBM = 128, kBN = 64;
 constexpr int kThreads = 640, kComputeWarp0 = 4, kComputeWarps = 16;
-// launch registers 65536 / 640 rounded down to a multiple of 8; what the control warps give up the others may take
-constexpr int kLaunchRegs = 96, kRegsCtl = 64, kRegsCompute = 104;
-static_assert(128 * (kRegsCtl + 4 * kRegsCompute) <= kThreads * kLaunchRegs, "register budget");
+// launch registers 65536 / 640 rounded down to a multiple of 8; what the control warps give up the others may take.  The issue loop is scheduled by what
+// it may keep: 40 / 48 / 64 registers, B4 H16 N1000 D64 102.8 / 108.0 / 103.8 us, B1 H32 N1777 D128 113.4 / 111.6 / 113.1 us.
+constexpr int kLaunchRegs = 96, kRegsCompute = 104;
+template <int D> constexpr int kRegsCtl = D == 64 ? 40 : 48;
+static_assert(128 * (kRegsCtl<128> + 4 * kRegsCompute) <= kThreads * kLaunchRegs && kRegsCtl<64> <= kRegsCtl<128>, "register budget");
 constexpr int kItemSlots = 2, kItemReaders = 1 + kComputeWarps;
 constexpr uint32_t kHi = sdesc_hi(1024);
 
@@ -139,7 +141,7 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
     };
 
     if (warp < kComputeWarp0) {
-        reg_dealloc<kRegsCtl>();
+        reg_dealloc<kRegsCtl<D>>();
         if (warp == 0) {
             // -------------------------------------------------------------- TMA producer
             if (lane == 0) {
