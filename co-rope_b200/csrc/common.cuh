@@ -91,7 +91,7 @@ __host__ __device__ inline unsigned ceil_div(unsigned a, unsigned b) { return (a
 FlatGrid rope_fp32_fwd_grid(int B, int H, int N);                 // heads x row blocks
 FlatGrid rope_fp32_bwd_grid(int B, int H, int Hkv, int N);        // K / V heads x (key block, its query heads' row blocks)
 FlatGrid rope_split_fwd_grid(int B, int H, int N);                // heads x row blocks
-FlatGrid rope_split_bwd_grid(int B, int H, int N);                // heads (of K / V for dK and dV) x 64-row blocks; persistent, one block per SM
+FlatGrid rope_split_items(int B, int H, int N);                   // heads (of K / V for dK and dV) x 128-row blocks, the items of persistent kernels
 FlatGrid rope_prepass_grid(bool bwd, int B, int H, int N, int D); // position blocks x groups of heads
 
 // Launch parameters common to the fused-RoPE kernels.

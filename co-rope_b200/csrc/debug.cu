@@ -43,8 +43,8 @@ extern "C" int corope_debug_grid(int kernel, int B, int Hq, int Hkv, int N, int 
         case 0: g = corope::rope_fp32_fwd_grid(B, Hq, N); break;
         case 1: g = corope::rope_fp32_bwd_grid(B, Hq, Hkv, N); break;
         case 2: g = corope::rope_split_fwd_grid(B, Hq, N); break;
-        case 3: g = corope::rope_split_bwd_grid(B, Hq, N); break;
-        case 4: g = corope::rope_split_bwd_grid(B, Hkv, N); break;
+        case 3: g = corope::rope_split_items(B, Hq, N); break;
+        case 4: g = corope::rope_split_items(B, Hkv, N); break;
         case 5: g = corope::rope_prepass_grid(false, B, Hkv, N, D); break;
         case 6: g = corope::rope_prepass_grid(true, B, Hq, N, D); break;
         default: return COROPE_ERR_BAD_SHAPE;

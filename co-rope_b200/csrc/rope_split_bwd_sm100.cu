@@ -637,7 +637,7 @@ int launch_t(const RopeParams& p, const SplitCopies& x, int* counter, cudaStream
     auto kern = rope_bwd_split_sm100_kernel<T, D, KP, KV>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, W::kSmem, smem_ok)) return e;
-    const unsigned items = ceil_div(p.N, kBM) * (unsigned)(p.B * (KV ? p.Hkv : p.H)), sms = (unsigned)sm_count();
+    const unsigned items = rope_split_items(p.B, KV ? p.Hkv : p.H, p.N).blocks(), sms = (unsigned)sm_count();
     count_launch();
     return launch_dependent(kern, items < sms ? items : sms, kThreads, W::kSmem, s, KV ? mk : mq, KV ? mv : mdo, KV ? mq : mk, KV ? mdo : mv, pp);
 }
@@ -652,8 +652,6 @@ int launch_d(const RopeParams& p, const SplitCopies& x, cudaStream_t s) {
 }
 
 }  // namespace
-
-FlatGrid rope_split_bwd_grid(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, kBN)}; }
 
 int launch_rope_bwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
     const SplitCopies x = split_copies(p, ws, true, dtype);

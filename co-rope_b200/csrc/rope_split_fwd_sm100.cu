@@ -475,7 +475,7 @@ int launch_t(const RopeParams& p, const SplitCopies& x, cudaStream_t s) {
     auto kern = rope_fwd_split_sm100_kernel<T, D, KP>;
     static std::atomic<uint64_t> smem_ok;
     if (int e = allow_smem(kern, F::kSmem, smem_ok)) return e;
-    const unsigned items = ceil_div(p.N, kBM) * (unsigned)(p.B * p.H), sms = (unsigned)sm_count();
+    const unsigned items = rope_split_items(p.B, p.H, p.N).blocks(), sms = (unsigned)sm_count();
     count_launch();
     return launch_dependent(kern, items < sms ? items : sms, kThreads, F::kSmem, s, mk, mv, pp);
 }
@@ -485,6 +485,8 @@ int launch_d(const RopeParams& p, const SplitCopies& x, cudaStream_t s) {
 }
 
 }  // namespace
+
+FlatGrid rope_split_items(int B, int H, int N) { return {(unsigned)(B * H), ceil_div(N, kBM)}; }
 
 int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
     const SplitCopies x = split_copies(p, ws, false, dtype);

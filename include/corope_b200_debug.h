@@ -50,8 +50,9 @@ int corope_debug_synth_tables(const float* inv_freq, float* cos_out, float* sin_
 
 /*
  * The grid of a launch, without a launch (inner_outer[2], host): inner * outer blocks along x.  kernel: 0 fp32 forward, 1 fp32 backward,
- * 2 split-operand forward of short sequences, 5 / 6 pre-pass of the tcgen05 forward / backward.  3 / 4 the split-operand backward for dQ / for dK
- * and dV: heads x 64-row blocks, the work of kernels that never launch more than one block per SM.
+ * 2 split-operand forward of short sequences, 5 / 6 pre-pass of the tcgen05 forward / backward.  3 / 4 the work items (query heads / K and V heads
+ * x 128-row blocks) of the persistent split-operand kernels, forward and dQ / dK and dV, which launch a block per item, but not more than one
+ * per SM.
  */
 int corope_debug_grid(int kernel, int B, int Hq, int Hkv, int N, int D, uint32_t* inner_outer);
 

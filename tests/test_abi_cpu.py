@@ -131,8 +131,8 @@ def test_every_admitted_size_has_a_grid_that_launches(kernel, B, Hq, Hkv, N, D):
         assert inner == B * Hq and outer in (-(-N // 32), -(-N // 64))
     elif kernel == 1:
         assert inner == B * Hkv and outer == -(-N // 32) * (G + 1)
-    elif kernel in (2, 3, 4):
-        assert inner == B * (Hkv if kernel == 4 else Hq) and outer == -(-N // 64)
+    elif kernel in (2, 3, 4):   # 3, 4: what the launchers of the persistent kernels take the minimum of, with the SMs of the GPU
+        assert inner == B * (Hkv if kernel == 4 else Hq) and outer == -(-N // (64 if kernel == 2 else 128))
     else:
         heads = B * (Hkv if kernel == 5 else Hq)
         assert inner == -(-N // (256 // (D // (16 if kernel == 5 else 8)))) and -(-heads // 8) <= outer <= heads

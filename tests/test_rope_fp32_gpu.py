@@ -49,7 +49,13 @@ def test_grouped_heads_many_ctas_and_unaligned_rows(pad, D):
         return t, buf[..., :D]
 
     (q, qv), (do, dov), (k, kv), (v, vv) = make(Hq, 410), make(Hq, 411), make(Hkv, 412), make(Hkv, 413)
-    outs = _run(pkg.flash_attention, qv.detach(), kv.detach(), vv.detach(), dov, True, D ** -0.5)
+    prev = ext.lib().corope_set_kernel_policy(1)   # aligned rows of D = 64 run on split operands otherwise
+    try:
+        outs = _run(pkg.flash_attention, qv.detach(), kv.detach(), vv.detach(), dov, True, D ** -0.5)
+    finally:
+        ext.lib().corope_set_kernel_policy(prev)
+    for op in (ext.OP_ROPE_FWD, ext.OP_ROPE_BWD):
+        assert (ext.lib().corope_last_kernel_family(op), ext.lib().corope_last_kernel_split(op)) == (0, 0)
     refs = (oracle.attn_gqa_fwd(q, k, v, True, D ** -0.5),) + tuple(oracle.attn_gqa_bwd(q, k, v, do, True, D ** -0.5))
     for a, b in zip(outs, refs):
         assert maxdiff(a, b) < TOL_32

@@ -247,3 +247,24 @@ def test_keys_masked_by_an_infinite_channel_cost_nothing(D, dtype):
         times[name] = min(spans)
     ext.check_status()
     assert times["hidden"] < 2.0 * times["plain"], times
+
+
+@pytest.mark.parametrize("N,D,dtype", [(300, 64, torch.float32), (333, 64, torch.float16), (333, 128, torch.bfloat16)])
+def test_tables_that_are_not_aligned(N, D, dtype):
+    # rows of the tables 4 bytes off a multiple of 16, an odd number of floats apart: the same bits as from aligned tables
+    q, k, v, do = (draw((1, 2, N, D), 510 + i, dtype).cuda() for i in range(4))
+    cos, sin = (t[:, :D // 2].cuda() for t in oracle.precompute_freqs_cis(D, N, 10000.0))
+
+    def run(tables):
+        x = [t.clone().requires_grad_(True) for t in (q, k, v)]
+        o = pkg.fused_rope_attention(*x, True, D ** -0.5, *tables)
+        return (o.detach(),) + torch.autograd.grad(o, x, do)
+
+    off = []
+    for t in (cos, sin):
+        wide = torch.full((N, D // 2 + 3), float("nan"), device="cuda")
+        wide[:, 1:D // 2 + 1] = t
+        off.append(wide[:, 1:D // 2 + 1])
+    for a, b in zip(run((cos.contiguous(), sin.contiguous())), run(off)):
+        assert torch.equal(a, b)
+    ext.check_status()
