@@ -125,7 +125,15 @@ struct Workspace {
     size_t bytes;
     Workspace(int op, int64_t B, int64_t Hq, int64_t Hkv, int64_t N, int64_t D, int dtype, const Tensor& like) {
         bytes = corope_workspace_bytes_any_n(op, (int)B, (int)Hq, (int)Hkv, (int)N, (int)D, dtype);
-        buf = at::empty({(int64_t)std::max<size_t>(bytes, 256)}, like.options().dtype(at::kByte));
+        auto allocate = [&] { buf = at::empty({(int64_t)std::max<size_t>(bytes, 256)}, like.options().dtype(at::kByte)); };
+        try {
+            allocate();
+        } catch (const c10::OutOfMemoryError&) {   // the split copies are for speed: without them a call runs on the CUDA cores
+            const size_t least = corope_workspace_bytes(op, (int)B, (int)Hq, (int)Hkv, (int)N, (int)D, dtype);
+            if (least >= bytes) throw;
+            bytes = least;
+            allocate();
+        }
     }
     void* ptr() const { return buf.data_ptr(); }
 };

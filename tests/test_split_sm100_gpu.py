@@ -268,3 +268,24 @@ def test_tables_that_are_not_aligned(N, D, dtype):
     for a, b in zip(run((cos.contiguous(), sin.contiguous())), run(off)):
         assert torch.equal(a, b)
     ext.check_status()
+
+
+def test_without_memory_for_split_copies():
+    # a call whose split copies do not fit runs on the CUDA cores, which need none
+    H, N, D = 64, 2048, 64
+    q, k, v, do = (draw((1, H, N, D), 520 + i, torch.float32).cuda().requires_grad_(i < 3) for i in range(4))
+    run = lambda: pkg.flash_attention(q, k, v, True, 0.125)
+    with_copies = run()
+    assert ext.lib().corope_last_kernel_split(ext.OP_ROPE_FWD) == 1
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    room = q.numel() * 4 + (8 << 20)   # o and the LSE, but not 12 bytes per element of k and v
+    try:
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + room) / total)
+        o = run()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert ext.lib().corope_last_kernel_split(ext.OP_ROPE_FWD) == 0
+    ext.check_status()
+    assert ((o - with_copies).norm() / o.norm()).item() < 2e-6
