@@ -440,7 +440,7 @@ int rope_bwd_impl(const void* q, const void* k, const void* v, const void* o, co
         return launch_rope_bwd_tc(p, dtype, s);
     }
     if (int e = fp32_tables(p, rot, workspace, w, s)) return e;
-    const bool split = w.split && policy == 0;
+    const bool split = w.split && policy == 0 && (dtype == COROPE_DTYPE_F32 || (no_shared_heads(p.sv, B, Hkv) && no_shared_heads(p.sdo, B, Hq)));
     note_kernels(kFamBwd, 0, split);
     p.sched_counter = reinterpret_cast<int*>((char*)workspace + w.packed_tab) + (size_t)N * (D / 2);   // the table itself is not used
     if (split) return launch_rope_bwd_split(p, (char*)workspace + w.rot, dtype, s);

@@ -762,6 +762,8 @@ bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types
 // host as GPU time), B2 H4 N300 86 / 94, B4 H8 N512 causal 88 / 261, B1 H8 N1000 100 / 495, B1 H4 N2048 causal 152 / 519.  (D = 128: the
 // three parts of K, V and the streamed rows of the backward do not fit a shared memory.)
 inline bool rope_split_fp32(int N, int D, int dtype) { return dtype == COROPE_DTYPE_F32 && D == 64 && N >= 256; }
+// Tensors that TMA steps over head by head: a stride of 0 (one head or batch entry shared by all) is none that a tensor map is documented to take.
+inline bool no_shared_heads(const Strides& st, int B, int H) { return (B == 1 || st.b > 0) && (H == 1 || st.h > 0); }
 size_t rope_split_workspace_bytes(bool bwd, int B, int Hq, int Hkv, int N, int D, int dtype);
 int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s);
 int launch_rope_fwd_split_tc(const RopeParams& p, void* ws, int dtype, cudaStream_t s);   // the tcgen05 form of the forward

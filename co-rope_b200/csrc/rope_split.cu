@@ -328,7 +328,8 @@ bool short_forward(const RopeParams& p, int dtype) {
     return p.N <= 64;
 }
 int launch_rope_fwd_split(const RopeParams& p, void* ws, int dtype, cudaStream_t s) {
-    if (dtype == COROPE_DTYPE_F32 || !short_forward(p, dtype)) return launch_rope_fwd_split_tc(p, ws, dtype, s);
+    // 16-bit V is read by TMA there, by plain copies here
+    if (dtype == COROPE_DTYPE_F32 || (!short_forward(p, dtype) && no_shared_heads(p.sv, p.B, p.Hkv))) return launch_rope_fwd_split_tc(p, ws, dtype, s);
     if (dtype == COROPE_DTYPE_F16) return fwd<__half, 3>(p, ws, s);
     return p.cos == nullptr ? fwd<__nv_bfloat16, 1>(p, ws, s) : fwd<__nv_bfloat16, 3>(p, ws, s);
 }

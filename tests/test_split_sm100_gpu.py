@@ -289,3 +289,27 @@ def test_without_memory_for_split_copies():
     assert ext.lib().corope_last_kernel_split(ext.OP_ROPE_FWD) == 0
     ext.check_status()
     assert ((o - with_copies).norm() / o.norm()).item() < 2e-6
+
+
+@pytest.mark.parametrize("N,D,dtype", [(400, 64, torch.bfloat16), (333, 128, torch.float16), (300, 64, torch.float32)])
+def test_heads_that_share_one_v_through_the_c_abi(N, D, dtype):
+    # head strides of 0 in V and dO, which the C entry points take (the Python ones copy such tensors first)
+    B, H, L = 1, 3, ext.lib()
+    q, k = (draw((B, H, N, D), 530 + i, dtype).cuda() for i in range(2))
+    v, do = (draw((B, 1, N, D), 532 + i, dtype).cuda().expand(B, H, N, D) for i in range(2))
+    s, code = D ** -0.5, ext.DTYPE_CODES[dtype]
+    o, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+    m = torch.empty((B, H, N), device="cuda")
+    st = ext.strides_of(q=q, k=k, v=v, o=o, d_o=do, dq=dq, dk=dk, dv=dv)
+    assert list(st.v)[1] == 0 and list(st.d_o)[1] == 0
+    status, stream = ext.status_word(q.device).data_ptr(), torch.cuda.current_stream().cuda_stream
+    ws, n = ext.workspace(ext.OP_FLASH_FWD, B, H, H, N, D, dtype, q.device)
+    assert L.corope_flash_attn_fwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), m.data_ptr(), B, H, H, N, D, code, 1, s, ws.data_ptr(), n, status,
+                                           stream, st) == 0
+    ws, n = ext.workspace(ext.OP_FLASH_BWD, B, H, H, N, D, dtype, q.device)
+    assert L.corope_flash_attn_bwd_strided(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), do.data_ptr(), m.data_ptr(), dq.data_ptr(), dk.data_ptr(),
+                                           dv.data_ptr(), B, H, H, N, D, code, 1, s, ws.data_ptr(), n, status, stream, st) == 0
+    ext.check_status()
+    tol = 1e-6 if dtype == torch.float32 else 2.0 ** (-9 if dtype == torch.bfloat16 else -12) * 1.5   # as in the tests above
+    for name, got, ref in zip(("O", "dQ", "dK", "dV"), (o, dq, dk, dv), _exact(q, k, v, do, True, s)):
+        assert ((got.double() - ref).norm() / ref.norm()).item() < tol, name
