@@ -31,9 +31,8 @@ __device__ __forceinline__ void ldm_x4(uint32_t (&r)[4], uint32_t addr) {
 __device__ __forceinline__ void ldm_x4_trans(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-// byte offsets of a lane's ldmatrix row inside a tile.  A operand (16 rows x 16 k): registers a0..a3.  B operand from a tile with
-// k contiguous: (b0, b1) of columns 0-7, then of columns 8-15.  B operand from a tile with the columns contiguous (.trans): the same.
-template <int D> __device__ __forceinline__ uint32_t lane_a(int lane) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * Pitch<D>::kBytes + (lane >> 4) * 16; }
+// byte offsets of a lane's ldmatrix row inside a tile.  B operand from a tile with k contiguous: (b0, b1) of columns 0-7, then of columns
+// 8-15.  B operand from a tile with the columns contiguous (.trans): the same.
 template <int D> __device__ __forceinline__ uint32_t lane_b(int lane) { return ((lane & 7) + (lane >> 4) * 8) * Pitch<D>::kBytes + ((lane >> 3) & 1) * 16; }
 template <int D> __device__ __forceinline__ uint32_t lane_bt(int lane) { return ((lane & 7) + ((lane >> 3) & 1) * 8) * Pitch<D>::kBytes + (lane >> 4) * 16; }
 
@@ -63,18 +62,18 @@ __device__ __forceinline__ void add4(float (*d)[4], const float (&t)[4][4]) {
 #pragma unroll
         for (int x = 0; x < 4; ++x) d[n][x] += t[n][x];
 }
-// the products of two split operands (PA and PB parts) for four neighbouring accumulator tiles, b[part][two ldmatrix_x4 results]: hi hi
+// the products of two split operands (three and PB parts) for four neighbouring accumulator tiles, b[part][two ldmatrix_x4 results]: hi hi
 // into `d` by way of an fp32 addition, the others into `e`, smallest first
-template <int PA, int PB>
-__device__ __forceinline__ void mma4_split(float (*d)[4], float (*e)[4], const uint32_t (&a)[PA][4], const uint32_t (&b)[PB][2][4]) {
+template <int PB>
+__device__ __forceinline__ void mma4_split(float (*d)[4], float (*e)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[PB][2][4]) {
     using B = __nv_bfloat16;
     float t[4][4] = {};
-    if constexpr (PA > 1 && PB > 1) mma4<B>(e, a[1], b[1][0], b[1][1]);
+    if constexpr (PB > 1) mma4<B>(e, a[1], b[1][0], b[1][1]);
     if constexpr (PB > 2) mma4<B>(e, a[0], b[2][0], b[2][1]);
-    if constexpr (PA > 2) mma4<B>(e, a[2], b[0][0], b[0][1]);
+    mma4<B>(e, a[2], b[0][0], b[0][1]);
     mma4<B>(t, a[0], b[0][0], b[0][1]);
     if constexpr (PB > 1) mma4<B>(e, a[0], b[1][0], b[1][1]);
-    if constexpr (PA > 1) mma4<B>(e, a[1], b[0][0], b[0][1]);
+    mma4<B>(e, a[1], b[0][0], b[0][1]);
     add4(d, t);
 }
 // hi hi + the smaller products.  An infinity shows in hi hi with the sign it has in fp32; the other parts of such a product are

@@ -128,7 +128,7 @@ __device__ __forceinline__ void rotate(float2& a, float2& b, const float* c, con
     b = make_float2(y.x * c[0] + x.x * s[0], y.y * c[1] + x.y * s[1]);
 }
 // rows of both tables are aligned to 16 bytes
-__device__ __forceinline__ bool tables_aligned(const RopeParams& p) {
+__host__ __device__ __forceinline__ bool tables_aligned(const RopeParams& p) {
     return (((uintptr_t)p.cos | (uintptr_t)p.sin) & 15) == 0 && (p.table_stride & 3) == 0;
 }
 __device__ __forceinline__ void load_table8(const float* __restrict__ src, bool vec, float (&x)[8]) {

@@ -93,8 +93,7 @@ int launch_t(const RopeParams& p, const SplitCopies& to, bool with_delta, cudaSt
     add(p.v, p.sv, p.Hkv, to.v, 1.f, false, false, true);
     add(p.d_o, p.sdo, p.H, to.d_o, 1.f, false, false, true);
     for (; n < 4; ++n) jobs.job[n].end = blocks;
-    const bool vec = (((uintptr_t)p.cos | (uintptr_t)p.sin) & 15) == 0 && (p.table_stride & 3) == 0;
-    split_rows_kernel<T, D><<<blocks, 256, 0, s>>>(jobs, p.cos, p.sin, p.table_stride, vec, (const T*)p.o, row_addr(p.so, p.H, p.N), (const T*)p.d_o,
+    split_rows_kernel<T, D><<<blocks, 256, 0, s>>>(jobs, p.cos, p.sin, p.table_stride, tables_aligned(p), (const T*)p.o, row_addr(p.so, p.H, p.N), (const T*)p.d_o,
                                                    row_addr(p.sdo, p.H, p.N), p.delta, p.sched_counter);
     count_launch();
     return (int)cudaGetLastError();
