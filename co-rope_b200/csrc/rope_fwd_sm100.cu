@@ -167,9 +167,9 @@ rope_fwd_sm100_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     // more timeouts behind it.  The word stays set until the host reads and clears it; the mirror may already be clear (the host resets it
     // at once, the word in stream order), so this launch reports too.
     if (p.status != nullptr) {
-        const int code = *reinterpret_cast<volatile int*>(p.status);
-        if (code != 0) {
-            if (threadIdx.x == 0) report_to_mirror(code, p.status_mirror);
+        // one answer for the whole block: a launch beside this one may set the word while its threads read it
+        if (__syncthreads_or(*reinterpret_cast<volatile int*>(p.status))) {
+            if (threadIdx.x == 0) report_to_mirror(p.status, p.status_mirror);
             pdl_wait();
             return;
         }

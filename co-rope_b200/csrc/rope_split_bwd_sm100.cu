@@ -116,9 +116,9 @@ rope_bwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapOwn, const __
         return;
     }
     if (p.status != nullptr) {   // an earlier launch gave up on a wait: see rope_fwd_sm100_kernel
-        const int code = *reinterpret_cast<volatile int*>(p.status);
-        if (code != 0) {
-            if (threadIdx.x == 0) report_to_mirror(code, p.status_mirror);
+        // one answer for the whole block: a launch beside this one may set the word while its threads read it
+        if (__syncthreads_or(*reinterpret_cast<volatile int*>(p.status))) {
+            if (threadIdx.x == 0) report_to_mirror(p.status, p.status_mirror);
             pdl_wait();
             return;
         }
