@@ -759,8 +759,9 @@ bool rope_tc_supported(int D, int dtype);   // the tcgen05 kernels: 16-bit types
 // 16-byte aligned rows at any N, 16-bit tensors of D = 64 or 128: split operands, `ws` of rope_split_workspace_bytes, two words of workspace
 // at p.sched_counter; the backward computes delta
 // fp32 tensors on split operands: D = 64, from this length on.  Forward + backward on them / on the CUDA cores: B1 H1 N200 84 / 80 us (as much
-// host as GPU time), B2 H4 N300 86 / 94, B4 H8 N512 causal 88 / 261, B1 H8 N1000 100 / 495, B1 H4 N2048 causal 152 / 519.  (D = 128: the
-// three parts of K, V and the streamed rows of the backward do not fit a shared memory.)
+// host as GPU time), B2 H4 N300 86 / 94, B4 H8 N512 causal 86 / 261, B1 H8 N1000 100 / 495, B1 H4 N2048 causal 152 / 519.  (D = 128: the
+// three parts of K, V and the streamed rows of the backward do not fit a shared memory; those of the forward would, with two stages, which is not
+// built.)
 inline bool rope_split_fp32(int N, int D, int dtype) { return dtype == COROPE_DTYPE_F32 && D == 64 && N >= 256; }
 // Tensors that TMA steps over head by head: a stride of 0 (one head or batch entry shared by all) is none that a tensor map is documented to take.
 inline bool no_shared_heads(const Strides& st, int B, int H) { return (B == 1 || st.b > 0) && (H == 1 || st.h > 0); }

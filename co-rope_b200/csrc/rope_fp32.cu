@@ -1,6 +1,6 @@
-// Fused-RoPE / plain attention in fp32 arithmetic on the CUDA cores: the accuracy path (fp32 inputs must match the fp32 reference
-// to 1e-4, which rules out 16-bit tensor-core operands) and the forward of every shape the tensor-core kernels do not take
-// (D = 32, strides that are no multiples of 16 bytes).  Any N, causal or full, D in {32, 64, 128}.
+// Fused-RoPE / plain attention in fp32 arithmetic on the CUDA cores: fp32 inputs (which must match the fp32 reference to 1e-4) where they do not
+// run on split operands (rope_split_fp32: aligned rows of D = 64 from 256 rows on do), and the forward of every 16-bit shape the
+// tensor-core kernels do not take (D = 32, strides that are no multiples of 16 bytes).  Any N, causal or full, D in {32, 64, 128}.
 //
 // Every product is a register-blocked tile product out of shared memory.  What bounds it is the rate at which shared memory fills
 // registers, 128 bytes per clock and SM whatever is broadcast: a thread tile of m x n needs (m + n) / (m n) floats per FMA, so the

@@ -19,11 +19,11 @@
 //               columns of S that it alone reads, reads dP, writes dS likewise; D / 4 columns of dK / dQ and of dV in registers
 //
 // What bounds it: D = 128, dK and dV: 96 MMAs per block of 64 queries (4750 cycles at a shared-memory port shared with the tiles' arrival) and
-// the chain of waits, exponentials and splits between them, which nothing overlaps in the 512 columns: 8400 cycles per block.  dQ:
-// 5700.  D = 64: score products overlap the softmax of the block before.  Forward + backward of B1 H32 N1777 D128 bf16 causal 1720 ->
-// 567 us (two mma.sync kernels that form the scores at three parts before), B4 H16 N1000 D64 bf16 full 1032 -> 380 us, B1 H2 N5999
-// D128 1826 -> 604 us, B1 H8 N4001 D64 f16 1230 -> 326 us; GPU time of the backward of B1 H1 N65 D64 28.5 -> 14.8 us.  Share of results
-// off the exact rounding before and now (f16, N(0, 1) inputs, B1 H4 N1777 D128 causal): dQ 0.19 / 0.20, dK 0.22 / 0.22, dV 0.22 / 0.22 %; bf16
+// the chain of waits, exponentials and splits between them, which nothing overlaps in the 512 columns: 4.15 us (8160 cycles of 1965
+// MHz) per block, 17 us per launch besides.  D = 64: score products overlap the softmax of the block before, 2.06 us per block.  GPU time of forward and
+// backward of B1 H32 N1777 D128 bf16 causal 1720 -> 541 us (two mma.sync kernels that form the scores at three parts before), B4 H16 N1000 D64
+// bf16 full 1032 -> 353 us, B1 H2 N5999 D128 1826 -> 570 us, B1 H8 N4001 D64 f16 1230 -> 312 us; of the backward of B1 H1 N65 D64 28.5 -> 14.8 us.
+// Share of results off the exact rounding before and now (f16, N(0, 1) inputs, B1 H4 N1777 D128 causal): dQ 0.19 / 0.20, dK 0.22 / 0.22, dV 0.22 / 0.22 %; bf16
 // dQ 0.057 / 0.044, dK 0.041 / 0.041, dV 0.040 / 0.040 %.  fp32 (B1 H4 N512 D64 causal), CUDA cores / here: dQ 3.6e-7 / 2.5e-7, dK 5.7e-7 /
 // 2.7e-7, dV 5.5e-7 / 2.3e-7.
 //

@@ -18,9 +18,9 @@
 // MMA; D = 128: lo has no room and sits in shared memory) | two S buffers of 64 + 64 columns, so that Q K^T of the next block runs beside
 // the softmax of this one | O of a block.
 //
-// What bounds it: 48 + 12 MMAs per block of 64 keys (D = 128; 2520 cycles), measured at 2800 cycles per block and 14 700 per item (rotation
-// and split of Q 8700).  B1 H32 N1777 D128 bf16 causal 397 -> 135 us (mma.sync kernel before), B4 H16 N1000 D64 bf16 full 243 -> 108 us,
-// B1 H2 N5999 D128 538 -> 160 us.  Error against 64-bit arithmetic next to that kernel (N(0, 1) inputs, B1 H4 N1777 D128 causal f16): LSE
+// What bounds it: 48 + 12 MMAs per block of 64 keys (D = 128; 2520 cycles), measured at 1.52 us (2990 cycles of 1965 MHz) per block, D = 64 at
+// 1.17 us; a launch with one item per SM takes 8 us besides (launch, rotation and split of Q, output).  GPU time: B1 H32 N1777 D128 bf16 causal
+// 397 -> 112 us (mma.sync kernel before), B4 H16 N1000 D64 bf16 full 243 -> 104 us, B1 H2 N5999 D128 538 -> 153 us.  Error against 64-bit arithmetic next to that kernel (N(0, 1) inputs, B1 H4 N1777 D128 causal f16): LSE
 // 3.6e-7 (3.8e-7), results that are not the exact one rounded 0.119 % (0.123 %); q and k times 4: LSE 4.7e-6 (4.5e-6; CUDA cores 6.9e-6),
 // 0.31 % (0.30 %; 0.47 %).  fp32 (B1 H4 N512 D64 causal): O 1.3e-7 (CUDA cores 2.3e-7), also where channels differ in scale by 1000.
 //
@@ -199,8 +199,8 @@ rope_fwd_split_sm100_kernel(const __grid_constant__ CUtensorMap mapK, const __gr
             };
             int gq = 0, gp = 0;   // blocks so far: Q K^T, P V
             bool ok = true;
-            // Q K^T in two pieces: a wait costs 280 cycles even where its phase is complete, about what the MMAs still queued in front of it
-            // take, so the wait for P stands between the pieces and the one for the K~ stage behind P V
+            // Q K^T in two pieces, so that MMAs are still queued while the warp waits: the wait for P (85 cycles even where its phase is
+            // complete, and the fences around it) stands between the pieces, the one for the K~ stage behind P V
             auto qk_head = [&]() {
                 const int st = gq % ST;
                 if (!(ok = mbar_wait_warp(&bars[F::FULL + st], (gq / ST) & 1, p.status, F::FULL, abort_flag))) return;

@@ -91,8 +91,8 @@ const char* corope_status_string(int status);
 size_t corope_workspace_bytes(int op, int B, int Hq, int Hkv, int N, int D, int dtype);
 
 /* The size with which an op runs on tensor cores at every N, not only at whole tiles: 16-bit D = 64 or 128 inputs of a ragged N, and
- * fp32 D = 64 inputs of 256 rows or more, then go to kernels that split every fp32 operand into several 16-bit ones and keep fp32
- * accuracy (6 bytes per element of k, in the backward also of q; for fp32 also of v and, backward, of d_o); so does the Co-RoPE forward
+ * fp32 D = 64 inputs of 256 rows or more, then go to kernels that split every fp32 operand into three 16-bit numbers, which hold its
+ * 24 bits, and keep fp32 accuracy (6 bytes per element of k, in the backward also of q; for fp32 also of v and, backward, of d_o); so does the Co-RoPE forward
  * at D = 64, a ragged N or rows that are not aligned to 16 bytes.  A call that is handed at least this much uses them; with
  * corope_workspace_bytes() bytes it runs on the CUDA-core kernels.  Never more than corope_workspace_bytes() for the fused-RoPE and plain
  * ops on 16-bit inputs where N is a whole number of tiles. */
